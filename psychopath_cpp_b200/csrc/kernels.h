@@ -17,6 +17,11 @@ struct RaySoA {
 	const uint16_t* type;
 };
 
+// What a caller of psy_trace asks for beyond hit, id and t: nothing, u and v
+// alone, fields without derivatives, or any of u, v and the derivatives
+// beside other fields.
+enum : int { WANT_NONE = 0, WANT_UV, WANT_POINT, WANT_ALL };
+
 struct HitSoA {
 	uint8_t* hit;
 	uint64_t* id;
@@ -27,12 +32,12 @@ struct HitSoA {
 	float* space;
 	uint8_t* closure;
 	float* closure_color;
-	int want_geometry;  // any geometry field requested
+	int want_geometry;  // WANT_*: which of the fields beyond hit, id and t are requested
 };
 
 struct HaltonDev {
 	const uint16_t* perm;
-	const uint4* dims;     // base, pow_base, groups, perm_offset
+	const uint4* dims;     // floor(2^32 / pow_base), pow_base, groups, perm_offset
 	const double* cmul;
 };
 
@@ -155,6 +160,9 @@ cudaError_t launch_batch_wave(const DevScene* scenes, const RenderParams* render
 
 cudaError_t launch_light_sample(const DevScene& sc, const LightQuerySoADev& q, const LightSampleSoADev& o, uint32_t n,
                                 float ident_inv, unsigned* status, cudaStream_t st);
+
+// Fills pairs[0 .. n - 1] from the light nodes (DevLightPair).
+cudaError_t launch_light_pairs(const DevLightNode* nodes, int n, DevLightPair* pairs, cudaStream_t st);
 
 cudaError_t launch_trace(const DevScene& sc, const RaySoA& rays, const HitSoA& hits, uint32_t n, unsigned* status,
                          cudaStream_t stream);

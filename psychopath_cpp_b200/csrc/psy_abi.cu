@@ -517,7 +517,7 @@ int psy_ctx_create(int device, psy_ctx** out) {
 	{
 		const HaltonTables ht = build_halton_tables();
 		std::vector<uint4> dims;
-		for (const HaltonDim& d : ht.dims) dims.push_back(make_uint4(d.base, d.pow_base, d.groups, d.perm_offset));
+		for (const HaltonDim& d : ht.dims) dims.push_back(make_uint4(d.pow_base ? (uint32_t)((1ull << 32) / d.pow_base) : 0u, d.pow_base, d.groups, d.perm_offset));
 		void *p0, *p1, *p2;
 		if (cudaMalloc(&p0, ht.perm.size() * sizeof(uint16_t)) != cudaSuccess) return PSY_ERR_OOM;
 		ctx->const_allocs.push_back(p0);
@@ -662,6 +662,18 @@ int psy_scene_upload_ex(psy_ctx* ctx, const psy_scene_desc* desc, uint32_t flags
 		UP(light_nodes, b->light_nodes);
 		UP(light_extra, b->light_extra);
 	}
+	{
+		// the light tree's children side by side, as the walk reads them
+		const size_t n = b->light_nodes.size() + (ctx->gpu_light_nodes > 0 ? (size_t)ctx->gpu_light_nodes : 0);
+		void* lp = nullptr;
+		if ((rc = ctx_cuda(ctx, cudaMalloc(&lp, (n ? n : 1) * sizeof(DevLightPair)), "cudaMalloc(light_pairs)"))) return rc;
+		ctx->scene_allocs.push_back(lp);
+		ctx->device_bytes += n * sizeof(DevLightPair);
+		d.light_pairs = static_cast<const DevLightPair*>(lp);
+		if ((rc = ctx_cuda(ctx, launch_light_pairs(d.light_nodes, (int)n, static_cast<DevLightPair*>(lp), nullptr),
+		                   "light pairs")))
+			return rc;
+	}
 	UP(assemblies, b->assemblies);
 	UP(instances, b->instances);
 	UP(objects, b->objects);
@@ -798,10 +810,9 @@ static int make_hit_soa(const psy_hit_soa* h, HitSoA* o) {
 	o->space = h->space;
 	o->closure = h->closure;
 	o->closure_color = h->closure_color;
-	o->want_geometry = (h->uv || h->p || h->n || h->dpdu || h->dpdv || h->dndu || h->dndv || h->backfacing ||
-	                    h->light_pdf || h->offset || h->space || h->closure || h->closure_color)
-	                       ? 1
-	                       : 0;
+	const bool point = h->p || h->n || h->backfacing || h->light_pdf || h->offset || h->space || h->closure || h->closure_color;
+	const bool derivs = h->dpdu || h->dpdv || h->dndu || h->dndv;
+	o->want_geometry = derivs || (point && h->uv) ? WANT_ALL : point ? WANT_POINT : h->uv ? WANT_UV : WANT_NONE;
 	return PSY_OK;
 }
 

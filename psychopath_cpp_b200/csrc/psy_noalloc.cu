@@ -161,7 +161,7 @@ extern "C" int psy_trace_host_noalloc(psy_ctx* ctx, const psy_ray_soa* rays, uin
 	hs.closure_color = static_cast<float*>(dev[15]);
 	hs.want_geometry = 0;
 	for (int k = 3; k < 16; ++k)
-		if (dev[k]) hs.want_geometry = 1;
+		if (dev[k]) hs.want_geometry = psy::WANT_ALL;
 
 	const psy::RaySoA rs{dr[0], dr[1], dr[2], dr[3], dr[4], dr[5], d_time, rays->type ? d_type : nullptr};
 	if ((rc = ctx_cuda(ctx, psy::launch_trace(ctx->dev, rs, hs, n, d_status, st), "psy_trace_host_noalloc: launch")))

@@ -108,6 +108,21 @@ struct alignas(16) DevLightNode {
 	int c1, c2;          // children (global) or, for leaves, c1 = local instance index
 };
 
+// The two children of an inner light node as the tree walk reads them, at the
+// node's own index: box centre, half diagonal squared (-1: the bounds move,
+// read the node), energy over that, and where the child leads (an inner
+// node's index, or -(local instance + 1) of a leaf).  Filled on the device
+// after the upload (light_pairs_kernel).
+struct alignas(64) DevLightPair {
+	float c1[3], r2_1;
+	float c2[3], r2_2;
+	float e1, e2;
+	float pad0[2];
+	int ref1, ref2;
+	int pad1[2];
+};
+static_assert(sizeof(DevLightPair) == 64, "DevLightPair must be 64 bytes");
+
 struct alignas(16) DevShader {
 	int kind;
 	float col[3];
@@ -130,6 +145,7 @@ struct DevScene {
 	const float* xforms;
 	const float* fpool;
 	const DevLightNode* light_nodes;
+	const DevLightPair* light_pairs;  // one per light node (inner nodes' are set)
 	const float* light_extra;
 	const DevShader* shaders;
 	int assembly_count;

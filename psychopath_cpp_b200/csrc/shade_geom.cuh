@@ -50,10 +50,11 @@ __device__ __forceinline__ void normal_derivs(const V3& n, const V3& dpdu, const
 __device__ __forceinline__ V3 bl_eval_p(float u, V3 p0, V3 p1) { return (p0 * (1.0f - u)) + (p1 * u); }
 __device__ __forceinline__ V3 bl_eval_pd(V3 p0, V3 p1) { return (p0 * -1.0f) + (p1 * 1.0f); }
 
-__device__ __forceinline__ void bilinear_geo(const Patch<4>& p, float u, float v, Geo* g) {
+__device__ __forceinline__ void bilinear_geo(const Patch<4>& p, float u, float v, Geo* g, bool derivs) {
 	g->dpdu = bl_eval_pd(bl_eval_p(v, p.p[0], p.p[2]), bl_eval_p(v, p.p[1], p.p[3]));
 	g->dpdv = bl_eval_pd(bl_eval_p(u, p.p[0], p.p[1]), bl_eval_p(u, p.p[2], p.p[3]));
 	g->n = normalized(cross(g->dpdv, g->dpdu));
+	if (!derivs) return;
 	const V3 zero(0.0f);
 	const V3 d2pduv = bl_eval_pd(bl_eval_pd(p.p[0], p.p[1]), bl_eval_pd(p.p[2], p.p[3]));
 	normal_derivs(g->n, g->dpdu, g->dpdv, zero, d2pduv, zero, &g->dndu, &g->dndv);
@@ -84,17 +85,20 @@ __device__ __forceinline__ V3 bc_eval_pdd(float u, V3 p0, V3 p1, V3 p2, V3 p3) {
 	return (p0 * dd0) + (p1 * dd1) + (p2 * dd2) + (p3 * dd3);
 }
 
-__device__ __forceinline__ void bicubic_geo(const Patch<16>& p, float u, float v, Geo* g) {
-	V3 pu[4], pv[4], pdv[4];
+__device__ __forceinline__ void bicubic_geo(const Patch<16>& p, float u, float v, Geo* g, bool derivs) {
+	V3 pu[4], pv[4];
 #pragma unroll
 	for (int i = 0; i < 4; ++i) {
 		pu[i] = bc_eval_p(v, p.p[i], p.p[i + 4], p.p[i + 8], p.p[i + 12]);
 		pv[i] = bc_eval_p(u, p.p[i * 4], p.p[i * 4 + 1], p.p[i * 4 + 2], p.p[i * 4 + 3]);
-		pdv[i] = bc_eval_pd(u, p.p[i * 4], p.p[i * 4 + 1], p.p[i * 4 + 2], p.p[i * 4 + 3]);
 	}
 	g->dpdu = bc_eval_pd(u, pu[0], pu[1], pu[2], pu[3]);
 	g->dpdv = bc_eval_pd(v, pv[0], pv[1], pv[2], pv[3]);
 	g->n = normalized(cross(g->dpdv, g->dpdu));
+	if (!derivs) return;
+	V3 pdv[4];
+#pragma unroll
+	for (int i = 0; i < 4; ++i) pdv[i] = bc_eval_pd(u, p.p[i * 4], p.p[i * 4 + 1], p.p[i * 4 + 2], p.p[i * 4 + 3]);
 	const V3 d2pduu = bc_eval_pdd(u, pu[0], pu[1], pu[2], pu[3]);
 	const V3 d2pduv = bc_eval_pd(v, pdv[0], pdv[1], pdv[2], pdv[3]);
 	const V3 d2pdvv = bc_eval_pdd(v, pv[0], pv[1], pv[2], pv[3]);
@@ -186,8 +190,11 @@ __device__ __forceinline__ void closure_of_shader(const DevScene& sc, int shader
 }
 
 // Fills the Intersection data of a closest hit. `lo`, `ld` are the ray
-// origin and direction in the hit object's space.
-static __device__ void hit_geometry(const DevScene& sc, const HitRec& rec, float time, V3 lo, V3 ld, HitInfo* h) {
+// origin and direction in the hit object's space.  The derivatives (and a
+// sphere's u, v, which come with them) cost more than the rest of a hit's
+// geometry and are left out unless `derivs` asks for them or the closure is
+// the one that reads them (GTR).
+static __device__ __forceinline__ void hit_geometry(const DevScene& sc, const HitRec& rec, float time, V3 lo, V3 ld, bool derivs, HitInfo* h) {
 	const DevObject ob = sc.objects[rec.obj];
 	const float t = rec.t;
 	h->light_pdf = 9999.0f;
@@ -199,6 +206,9 @@ static __device__ void hit_geometry(const DevScene& sc, const HitRec& rec, float
 		g.p = lo + (ld * t);
 		g.n = normalized(g.p - cent);
 		h->backfacing = dot(g.n, normalized(ld)) > 0.0f;
+		h->offset = g.n * 0.000001f;
+		closure_of_shader(sc, rec.shader, h);
+		if (!derivs && h->closure != CLOSURE_GTR) return;
 		const V3 unit_p = g.n;
 		const V3 p = unit_p * radi;
 		const float lat_cos = unit_p.z;
@@ -221,8 +231,6 @@ static __device__ void hit_geometry(const DevScene& sc, const HitRec& rec, float
 		const V3 d2pduv = ((V3(-long_sin, long_cos, 0.0f) * pif) * p.z) * pi2;
 		const V3 d2pdvv = V3(p.x, p.y, p.z) * (float)(-PSY_PI_D * PSY_PI_D);
 		normal_derivs(g.n, g.dpdu, g.dpdv, d2pduu, d2pduv, d2pdvv, &g.dndu, &g.dndv);
-		h->offset = g.n * 0.000001f;
-		closure_of_shader(sc, rec.shader, h);
 	} else if (ob.kind == OBJ_SPHERE_LIGHT) {
 		V3 cent;
 		float radi;
@@ -267,18 +275,19 @@ static __device__ void hit_geometry(const DevScene& sc, const HitRec& rec, float
 		g.u = rec.u;
 		g.v = rec.v;
 		const float* verts = sc.fpool + ob.data;
+		closure_of_shader(sc, rec.shader, h);
+		derivs = derivs || h->closure == CLOSURE_GTR;
 		if (ob.kind == OBJ_BILINEAR) {
 			Patch<4> q;
 			patch_at<4>(verts, ob.n0, time, &q);
-			bilinear_geo(q, rec.u, rec.v, &g);
+			bilinear_geo(q, rec.u, rec.v, &g, derivs);
 		} else {
 			Patch<16> q;
 			patch_at<16>(verts, ob.n0, time, &q);
-			bicubic_geo(q, rec.u, rec.v, &g);
+			bicubic_geo(q, rec.u, rec.v, &g, derivs);
 		}
 		h->backfacing = dot(g.n, normalized(ld)) > 0.0f;
 		h->offset = g.n * (rec.max_dim * 1.74f);
-		closure_of_shader(sc, rec.shader, h);
 	}
 }
 

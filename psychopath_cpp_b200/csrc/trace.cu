@@ -49,7 +49,11 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
 	if (hits.hit) hits.hit[i] = hit ? 1 : 0;
 	if (hits.id) hits.id[i] = hit ? rec.id : 0ull;
 	if (hits.t) hits.t[i] = (hit && !wr.occl) ? rec.t : INFINITY;
-	if (hit && !wr.occl && hits.want_geometry) {
+	if (hit && !wr.occl && hits.want_geometry == WANT_UV && (rec.kind == OBJ_BILINEAR || rec.kind == OBJ_BICUBIC)) {
+		// a patch's u, v are the bisection's own: no geometry to evaluate
+		hits.uv[2 * (size_t)i] = rec.u;
+		hits.uv[2 * (size_t)i + 1] = rec.v;
+	} else if (hit && !wr.occl && hits.want_geometry) {
 		M44 space;
 		const bool xf = hit_space<F>(sc, rec, wr.time, &space, &err);
 		V3 lo = wr.o, ld = wr.d;
@@ -60,7 +64,7 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
 			space = m44_identity();
 		}
 		HitInfo h;
-		hit_geometry(sc, rec, wr.time, lo, ld, &h);
+		hit_geometry(sc, rec, wr.time, lo, ld, hits.want_geometry != WANT_POINT, &h);
 		if (hits.uv) {
 			hits.uv[2 * (size_t)i] = h.geo.u;
 			hits.uv[2 * (size_t)i + 1] = h.geo.v;
