@@ -161,6 +161,12 @@ cudaError_t launch_batch_wave(const DevScene* scenes, const RenderParams* render
 cudaError_t launch_light_sample(const DevScene& sc, const LightQuerySoADev& q, const LightSampleSoADev& o, uint32_t n,
                                 float ident_inv, unsigned* status, cudaStream_t st);
 
+// Puts the nodes [0, n) and the roots into the traversal's form (REF_NODE_*,
+// LEAF_* classes, absent children); flags is scratch for n ints.
+cudaError_t launch_finish_nodes(DevNode* nodes, float* extra, int n, const DevLeaf* leaves, const DevAssembly* assemblies,
+                                int assembly_count, DevPlace* places, int place_count, int* flags, int* asmb_root,
+                                cudaStream_t st);
+
 // Fills pairs[0 .. n - 1] from the light nodes (DevLightPair).
 cudaError_t launch_light_pairs(const DevLightNode* nodes, int n, DevLightPair* pairs, cudaStream_t st);
 

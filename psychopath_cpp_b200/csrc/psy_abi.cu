@@ -680,6 +680,29 @@ int psy_scene_upload_ex(psy_ctx* ctx, const psy_scene_desc* desc, uint32_t flags
 	UP(xforms, b->xforms);
 	UP(fpool, b->fpool);
 	UP(shaders, b->shaders);
+	{
+		SceneTables tb;
+		const size_t node_count = b->nodes.size() + (ctx->gpu_bvh_nodes > 0 ? (size_t)ctx->gpu_bvh_nodes : 0);
+		if (b->instances.size() > (size_t)REF_MAX_INSTANCES || node_count > (size_t)REF_MAX_NODES) {
+			ctx->free_scene();
+			return ctx_fail(ctx, PSY_ERR_ARG, "scene: more than %d instances or %d tree nodes", REF_MAX_INSTANCES,
+			                REF_MAX_NODES);
+		}
+		build_tables(*b, PSY_MAX_PLACES, &tb);
+		UP(leaves, tb.leaves);
+		UP(places, tb.places);
+		UP(place_frames, tb.frames);
+		std::vector<int> work(node_count + b->assemblies.size());  // node flags, then the assemblies' roots
+		UP(asmb_root, work);
+		int* flags = const_cast<int*>(d.asmb_root);
+		d.asmb_root = flags + node_count;
+		if ((rc = ctx_cuda(ctx, launch_finish_nodes(const_cast<DevNode*>(d.nodes), const_cast<float*>(d.node_extra),
+		                                            (int)node_count, d.leaves, d.assemblies, (int)b->assemblies.size(),
+		                                            const_cast<DevPlace*>(d.places), (int)tb.places.size(), flags,
+		                                            flags + node_count, nullptr),
+		                   "scene tables")))
+			return rc;
+	}
 	UP(cam_xforms, b->cam_xforms);
 	UP(cam_tfovs, b->cam_tfovs);
 	UP(cam_apertures, b->cam_apertures);
@@ -701,6 +724,8 @@ int psy_scene_upload_ex(psy_ctx* ctx, const psy_scene_desc* desc, uint32_t flags
 		ctx->free_scene();
 		return ctx_fail(ctx, PSY_ERR_ARG, "assembly nesting %d deeper than %d", b->max_depth, PSY_MAX_LEVELS_HOST);
 	}
+	// the last steps ran on the default stream; renders may use any
+	if ((rc = ctx_cuda(ctx, cudaStreamSynchronize(nullptr), "scene tables"))) return rc;
 	ctx->host = std::move(b);
 	ctx->has_scene = true;
 	return PSY_OK;

@@ -3,6 +3,8 @@
  *
  * One flat set of arrays per uploaded scene, resident in HBM:
  *   assemblies[]   per-assembly roots and table bases
+ *   leaves[]       per instance: what the traversal reads of it
+ *   places[]       the unrolled assembly instances (DevPlace)
  *   instances[]    global instance table (all assemblies, contiguous per assembly)
  *   objects[]      global object table; geometry in the float pool
  *   nodes[]        BVH4 inner nodes, 128-byte records: the 4 child boxes of
@@ -55,12 +57,34 @@ inline unsigned feature_variant(unsigned f) {
 	return FEAT_ALL;
 }
 
-// A child reference in a BVH4 node or an assembly root:
+// A child reference in a BVH4 node or an assembly root, as the builders
+// leave it:
 //   >= 0          inner node index (global)
-//   < 0, != EMPTY leaf: local instance index = -(ref + 1)
+//   < 0, != EMPTY leaf: global instance index = -(ref + 1)
 static constexpr int REF_EMPTY = (int)0x80000000;
-PSY_HD int leaf_ref(int local_instance) { return -(local_instance + 1); }
+PSY_HD int leaf_ref(int instance) { return -(instance + 1); }
 PSY_HD int leaf_instance(int ref) { return -(ref + 1); }
+
+// The form the traversal reads (finish_nodes, scene_device.cu): an inner
+// node's index with what its test needs to know before the node is read, or
+// a leaf's class and global instance index.
+static constexpr int REF_NODE_MOVING = 1 << 30;  // more than one time sample
+static constexpr int REF_NODE_ODD = 1 << 29;     // a box is not finite
+static constexpr int REF_NODE_MASK = (1 << 29) - 1;
+static constexpr int REF_LEAF_MASK = (1 << 28) - 1;
+static constexpr int REF_MAX_NODES = 1 << 29, REF_MAX_INSTANCES = 1 << 28;
+enum : int {
+	LEAF_ENTER = 1,   // assembly instance
+	LEAF_SPHERE = 2,  // sphere or sphere light at rest in its assembly's space
+	LEAF_SIMPLE = 3,  // other spheres, sphere lights and rectangle lights
+	LEAF_PATCH = 4    // bilinear and bicubic patches
+};
+PSY_HD int leaf_class(int ref) { return (int)(((unsigned)ref >> 28) & 7u); }
+PSY_HD int class_ref(int cls, int instance) { return (int)(0x80000000u | ((unsigned)cls << 28) | (unsigned)instance); }
+
+// The planes of an absent child's box: inverted, so that no ray hits it, and
+// finite, so that interpolating them stays so.
+static constexpr float ABSENT_PLANE = 3.0e38f;
 
 struct alignas(16) DevNode {
 	float b[24];      // time sample 0 child bounds, BBox4 SoA
@@ -80,6 +104,39 @@ struct alignas(16) DevInstance {
 	int shader;       // -1 = none
 	int pad[3];
 };
+
+// What the traversal reads of an instance, by its global index.
+struct alignas(16) DevLeaf {
+	float sphere[4];  // LEAF_SPHERE: centre, radius
+	int data;         // patches: float pool offset; assemblies: rank among its assembly's assembly instances
+	int xforms;       // the instance's own motion samples
+	int asmb;         // assemblies: assembly index
+	int kind;         // patches: PM_* | LEAF_PATCH_ODD; bits 4..6: LEAF_* class
+};
+static constexpr int LEAF_PATCH_ODD = 8;  // a coordinate so large that sums of two may overflow
+
+// An assembly instance as the walk from the root meets it: one entry per
+// path of assembly instances (entry 0 is the root assembly), children of an
+// entry in a row.  Holds what the path gives the level: the merged motion
+// frame (place_frames, 16 floats per sample), the inherited shader and the
+// element id so far.
+struct alignas(16) DevPlace {
+	int root;         // root reference of its assembly
+	int child_base;   // entry of its first assembly instance
+	int frame;        // first matrix of the merged frame
+	int frame_count;  // its motion samples: 0 = no transform, -1 = more than supported
+	int parent;
+	int inst_base;    // of its assembly
+	int shader;
+	int id_bits;      // of its assembly
+	uint64_t id;
+	int asmb, pad;
+};
+static_assert(sizeof(DevPlace) == 48, "DevPlace must be 48 bytes");
+// Scenes that unroll to more entries than this are traversed with a level
+// stack per ray instead (12 MB of entries, and the frames of as many
+// transformed ones; a scene's upload spends about 0.1 us per entry).
+#define PSY_MAX_PLACES (1 << 18)
 
 struct alignas(16) DevObject {
 	int kind;
@@ -139,6 +196,10 @@ struct alignas(16) DevShader {
 struct DevScene {
 	const DevAssembly* assemblies;
 	const DevInstance* instances;
+	const DevLeaf* leaves;
+	const DevPlace* places;        // null: more than PSY_MAX_PLACES
+	const float* place_frames;
+	const int* asmb_root;          // per assembly: root reference (traversal form)
 	const DevObject* objects;
 	const DevNode* nodes;
 	const float* node_extra;

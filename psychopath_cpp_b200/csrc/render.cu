@@ -52,38 +52,6 @@ cudaError_t launch_batch_wave(const DevScene* scenes, const RenderParams* render
 }
 
 // ---------------------------------------------------------------------
-// The light trees' children side by side (DevLightPair), with the parts of
-// node_prob that depend on the node alone, in its float operations.
-// ---------------------------------------------------------------------
-__global__ void light_pairs_kernel(const DevLightNode* __restrict__ nodes, int n, DevLightPair* __restrict__ pairs) {
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n || nodes[i].is_leaf) return;
-	DevLightPair p = {};
-	auto child = [&](int c, float* centre, float* r2, float* e, int* ref) {
-		const DevLightNode nd = nodes[c];
-		Box b;
-		b.lo = V3(nd.lo[0], nd.lo[1], nd.lo[2]);
-		b.hi = V3(nd.hi[0], nd.hi[1], nd.hi[2]);
-		const V3 m = box_center(b);
-		centre[0] = m.x; centre[1] = m.y; centre[2] = m.z;
-		const float r = box_diagonal(b) * 0.5f;
-		*r2 = r * r;
-		*e = nd.energy * (1.0f / *r2);
-		if (nd.ts > 1) *r2 = -1.0f;
-		*ref = nd.is_leaf ? -(nd.c1 + 1) : c;
-	};
-	child(nodes[i].c1, p.c1, &p.r2_1, &p.e1, &p.ref1);
-	child(nodes[i].c2, p.c2, &p.r2_2, &p.e2, &p.ref2);
-	pairs[i] = p;
-}
-
-cudaError_t launch_light_pairs(const DevLightNode* nodes, int n, DevLightPair* pairs, cudaStream_t st) {
-	if (n == 0) return cudaSuccess;
-	light_pairs_kernel<<<(n + 255) / 256, 256, 0, st>>>(nodes, n, pairs);
-	return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------
 // Batched LightTree::sample queries (psy_light_sample)
 // ---------------------------------------------------------------------
 __global__ void light_sample_kernel(DevScene sc, LightQuerySoADev q, LightSampleSoADev o, uint32_t n, float ident_inv,

@@ -74,30 +74,19 @@ __device__ __forceinline__ int load_ray(const float4* rb, int cap, int i, WorldR
 	return __float_as_int(e.w);
 }
 
-// Hit planes: 0: t, u, v, max_dim (float4)   1: obj, kind | depth << 8,
-// shader, path[0]   2: path[1..4]   3: path[5..7] (int4).  The path planes
-// beyond the hit's depth are neither written nor read.
-__device__ __forceinline__ void store_rec(const WaveBufs& wb, int i, const HitRec& h) {
-	wb.hit_f[i] = make_float4(h.t, h.u, h.v, h.max_dim);
-	const int cap = wb.cap;
-	if (h.obj < 0) {
-		wb.hit_i[i] = make_int4(-1, 0, -1, 0);
-		return;
-	}
-	wb.hit_i[i] = make_int4(h.obj, h.kind | (h.depth << 8), h.shader, h.path[0]);
-	if (h.depth > 1) wb.hit_i[cap + i] = make_int4(h.path[1], h.path[2], h.path[3], h.path[4]);
-	if (h.depth > 5) wb.hit_i[2 * cap + i] = make_int4(h.path[5], h.path[6], h.path[7], 0);
-}
+// Hit planes: 0: t, u, v, max_dim (float4)   1: instance, placement, depth,
+// path[0]   2: path[1..4]   3: path[5..7] (int4).  The path is written and
+// read in scenes without placements only, as far as the hit's depth.
 __device__ __forceinline__ void load_rec(const WaveBufs& wb, int i, HitRec* h) {
+	const int4 a = wb.hit_i[i];
+	h->inst = a.x;
+	if (a.x < 0) return;
 	const float4 f = wb.hit_f[i];
 	h->t = f.x; h->u = f.y; h->v = f.z; h->max_dim = f.w;
-	const int4 a = wb.hit_i[i];
-	h->obj = a.x;
-	h->kind = a.y & 0xff;
-	h->depth = a.y >> 8;
-	h->shader = a.z;
+	h->place = a.y;
+	if (a.y >= 0) return;
+	h->depth = a.z;
 	h->path[0] = a.w;
-	h->id = 0;
 	const int cap = wb.cap;
 	if (h->depth > 1) {
 		const int4 b = wb.hit_i[cap + i];
@@ -108,6 +97,46 @@ __device__ __forceinline__ void load_rec(const WaveBufs& wb, int i, HitRec* h) {
 		h->path[5] = c.x; h->path[6] = c.y; h->path[7] = c.z;
 	}
 }
+
+// A ray of the wave's queue (Trav's IO).  Hits go straight to the ray's
+// place in the hit planes: a lane carries nothing of them.
+struct WaveIO {
+	const float4* rb;
+	const WaveBufs* wb;
+	int i;  // queue position, -1 = no ray
+	__device__ __forceinline__ V3 origin() const {
+		const float4 a = rb[i];
+		return V3(a.x, a.y, a.z);
+	}
+	__device__ __forceinline__ V3 direction() const {
+		const float4 b = rb[wb->cap + i];
+		return V3(b.x, b.y, b.z);
+	}
+	__device__ __forceinline__ void differentials(V3* odx, V3* ody, V3* ddx, V3* ddy) const {
+		WorldRayD r;
+		load_ray(rb, wb->cap, i, &r);
+		*odx = r.odx;
+		*ody = r.ody;
+		*ddx = r.ddx;
+		*ddy = r.ddy;
+	}
+	template <class T>
+	__device__ __forceinline__ void hit(const T& tr, int inst, float t, float u, float v, float md) const {
+		if (tr.flags & RAY_OCCL) return;
+		wb->hit_f[i] = make_float4(t, u, v, md);
+		if (!T::NESTED || tr.place >= 0) {
+			wb->hit_i[i] = make_int4(inst, tr.place, 0, 0);
+			return;
+		}
+		int p[PSY_MAX_LEVELS] = {};
+		for (int k = 1; k <= tr.L; ++k) p[k - 1] = tr.lv_inst[k];
+		p[tr.L] = inst;
+		const int cap = wb->cap;
+		wb->hit_i[i] = make_int4(inst, -1, tr.L + 1, p[0]);
+		if (tr.L > 0) wb->hit_i[cap + i] = make_int4(p[1], p[2], p[3], p[4]);
+		if (tr.L > 4) wb->hit_i[2 * cap + i] = make_int4(p[5], p[6], p[7], 0);
+	}
+};
 
 // World-space shading data of the stored intersection (the PTState::inter
 // and prev_ray the reference keeps per path).
@@ -478,29 +507,18 @@ __global__ void __launch_bounds__(256) camera_gen_kernel(W w, HaltonDev hd, Wave
 //
 // Persistent warps with per-lane ray replacement: a lane whose ray is
 // finished takes the next ray of the queue between traversal steps instead
-// of idling until the slowest ray of its warp is done.  128 registers a
-// thread (16 resident warps an SM) hide more latency than the
-// register-unbounded variant's 8 warps (measured: +13% on the many-light
-// scene, no change on flat scenes).
+// of idling until the slowest ray of its warp is done.
 //
-// Scenes with instance levels (the large traversal kernels): one block of
-// 512 threads per SM, whose warps run the same kind of work while they
-// can.  The kernel is bound by instruction fetch (the lanes of 16 warps
-// spread over more code than an SM's instruction cache holds), so a warp
-// that has lanes for the kind the block is running runs that kind, and
-// only a warp without any takes its own most common kind, which the block
-// then follows.  The preference is a shared word read and written without
-// synchronisation (a stale value only costs time).  A warp also refills
-// its lanes from 4 idle lanes instead of 8.  Measured on the many-light
-// render: 11% off the traversal time against blocks of 128 threads that
-// each vote alone.  Flat scenes (a small kernel) keep the render's block
-// size and the per-warp vote, which are 3-4% faster there.
+// Registers: 128 a thread where a lane's step can be a bicubic split (96
+// floats live), 80 in flat scenes, where more warps hide the walk's latency
+// (1280x720x4 many-light frame: 169 ms with 2 x 256 or 1 x 512 threads an
+// SM, 192 with 6 x 128, 223 with 2 x 512; 512x384x16 with 50,000
+// primitives: 18.2 ms with 3 or 4 x 256, 18.9 with 2).
 template <unsigned F>
 struct TraceCfg {
 	static constexpr bool NESTED = (F & FEAT_NESTED) != 0;
-	static constexpr int BLOCK = NESTED ? 512 : 256;      // launch bound (flat: the render's block size)
-	static constexpr int MIN_BLOCKS = NESTED ? 1 : 2;
-	static constexpr bool FOLLOW = NESTED;                // warps follow the block's kind of work
+	static constexpr int BLOCK = 256;                     // launch bound
+	static constexpr int MIN_BLOCKS = NESTED ? 2 : 3;     // 128 and 80 registers a thread
 	static constexpr int REFILL_MIN = NESTED ? 4 : 8;     // idle lanes that trigger a refill while rays remain
 	static int launch_block(int render_block) { return NESTED ? BLOCK : render_block; }
 };
@@ -509,24 +527,23 @@ struct TraceCfg {
 // classes (entering an assembly instance, testing a simple object, starting
 // a patch bisection) and bisection iterations (PSY_PATCH_UNITS at a time).
 // Each loop iteration of a warp runs the kind that most of its lanes have
-// next (leaf visits counted PSY_LEAF_WEIGHT times, bisections
-// PSY_PATCH_WEIGHT times), so that the lanes doing the same work run
-// together instead of one lane's long bisection or transformed-instance
-// entry holding up the others.  (Measured on the many-light render: 4 node
-// visits a step 1.4% faster than 8 and 16; 16 bisection iterations and a
-// refill threshold of 16 slower than 8.)
+// next, so that the lanes doing the same work run together instead of one
+// lane's long bisection or transformed-instance entry holding up the others.
+// (2, 4 or 8 node visits: within 1%; 16 bisection iterations: 2% better than
+// 8 on the many-light frame.  Warps that follow one kind of work per block,
+// which paid while a step's code and state did not fit the caches, cost 5%.)
 #ifndef PSY_WALK_NODES
 #define PSY_WALK_NODES 4
 #endif
 #ifndef PSY_PATCH_UNITS
-#define PSY_PATCH_UNITS 8
+#define PSY_PATCH_UNITS 16
 #endif
-#ifndef PSY_PATCH_WEIGHT
-#define PSY_PATCH_WEIGHT 1
-#endif
-#ifndef PSY_LEAF_WEIGHT
-#define PSY_LEAF_WEIGHT 1
-#endif
+// Kinds of work of a lane: idle, inner nodes, a leaf visit of one of three
+// classes, a bisection in progress.  Leaf visits are told apart so that the
+// lanes of a warp step run one branch together: assembly entries (ray
+// transform), simple objects (spheres, sphere and rectangle lights), patches
+// (root box, ray widths, bisection set-up).
+enum : int { KIND_IDLE = 0, KIND_NODES, KIND_ENTER, KIND_SIMPLE, KIND_BEGIN, KIND_PATCH, KIND_COUNT };
 
 template <class W, unsigned F, bool OCCL>
 __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS) trace_wave_kernel(W w, WaveBufs wb, const float4* __restrict__ rb,
@@ -538,103 +555,102 @@ __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS) t
 	unsigned err = 0;
 	// per-lane work counters (TC_*), and the warp's own (lane 0 keeps them)
 	unsigned rays = 0, c_nodes = 0, c_leaves = 0, c_iters = 0, c_warp = 0, c_lanes = 0;
-	TraceState<F> st;
-	int my = -1;    // queue position of this lane's ray, -1 = idle
-	int leaf = 0;   // walk_nodes stopped at a leaf (st.leaf): its LEAF_* class, else 0
+	Trav<F, WaveIO> tr;
+	tr.io.rb = rb;
+	tr.io.wb = &wb;
+	tr.io.i = -1;
+	tr.pmode = PM_NONE;
+	tr.cur = REF_NONE;
 	int rid = 0;
 	bool more = true;  // the queue may still hold rays (warp-uniform)
-	__shared__ int s_kind;  // the kind of work the block's warps run
-	if (threadIdx.x == 0) s_kind = KIND_NODES;
-	__syncthreads();
 	while (true) {
-		const unsigned idle = __ballot_sync(0xffffffffu, my < 0);
+		const unsigned idle = __ballot_sync(0xffffffffu, tr.io.i < 0);
 		if (more && (__popc(idle) >= TraceCfg<F>::REFILL_MIN || idle == 0xffffffffu)) {
 			int base = 0;
 			if (lane == 0) base = atomicAdd(work, __popc(idle));
 			base = __shfl_sync(0xffffffffu, base, 0);
 			if (base + __popc(idle) >= n) more = false;
-			if (my < 0) {
+			if (tr.io.i < 0) {
 				const int k = base + __popc(idle & lt_mask);
 				if (k < n) {
-					WorldRayD wr;
-					const int tag = load_ray(rb, wb.cap, k, &wr);
-					wr.occl = OCCL;
+					const int tag = __float_as_int(rb[4 * (size_t)wb.cap + k].w);
 					if (tag & 1) {
 						// no ray: a shadow step without a light sample, or a
 						// path of a shorter render in a batch that has ended
 						if (OCCL) wb.occl[k] = 1;
 					} else {
 						rid = tag >> 1;
-						trace_init<F>(w.scene(rid), st, wr);
-						my = k;
-						leaf = 0;
+						tr.io.i = k;
+						const float4 a = rb[k], b = rb[wb.cap + k];
+						tr.init(w.scene(rid), V3(a.x, a.y, a.z), V3(b.x, b.y, b.z), a.w, OCCL);
 						++rays;
+						if (tr.cur == REF_EMPTY) {
+							// an empty scene
+							if (OCCL) wb.occl[k] = 0;
+							else wb.hit_i[k] = make_int4(-1, 0, 0, 0);
+							tr.io.i = -1;
+						}
 					}
 				}
 			}
 		}
-		// KIND_IDLE, KIND_NODES (node visits), a leaf visit of one of the
-		// LEAF_* classes, or KIND_PATCH (bisection)
-		const int kind = my < 0 ? KIND_IDLE : st.pmode != PM_NONE ? KIND_PATCH : leaf ? leaf : KIND_NODES;
-		unsigned m[KIND_PATCH + 1];
+		// KIND_IDLE, KIND_NODES (inner nodes), a leaf visit of one of three
+		// kinds, or KIND_PATCH (bisection)
+		int kind = KIND_IDLE;
+		if (tr.io.i >= 0) {
+			const int cls = leaf_class(tr.cur);
+			kind = tr.pmode != PM_NONE ? KIND_PATCH : tr.cur >= 0 ? KIND_NODES
+			     : cls == LEAF_ENTER ? KIND_ENTER : cls == LEAF_PATCH ? KIND_BEGIN : KIND_SIMPLE;
+		}
+		unsigned m[KIND_COUNT];
 #pragma unroll
-		for (int k = KIND_NODES; k <= KIND_PATCH; ++k) m[k] = __ballot_sync(0xffffffffu, kind == k);
-		if ((m[KIND_NODES] | m[LEAF_ENTER] | m[LEAF_SIMPLE] | m[LEAF_PATCH] | m[KIND_PATCH]) == 0u) {
+		for (int k = KIND_NODES; k < KIND_COUNT; ++k) m[k] = __ballot_sync(0xffffffffu, kind == k);
+		if ((m[KIND_NODES] | m[KIND_ENTER] | m[KIND_SIMPLE] | m[KIND_BEGIN] | m[KIND_PATCH]) == 0u) {
 			if (!more) break;
 			continue;
 		}
-		// the block's kind if this warp has lanes for it, else the kind most
-		// of its lanes have next (later kinds win ties), which the block takes
-		int run = *(volatile int*)&s_kind;
-		bool has = false;
-		if (TraceCfg<F>::FOLLOW) {
+		// the kind most of the lanes have next (later kinds win ties)
+		int run = KIND_NODES;
+		int best = __popc(m[KIND_NODES]);
 #pragma unroll
-			for (int k = KIND_NODES; k <= KIND_PATCH; ++k)
-				if (run == k) has = m[k] != 0u;
-		}
-		if (!has) {
-			run = KIND_NODES;
-			int best = __popc(m[KIND_NODES]);
-#pragma unroll
-			for (int k = LEAF_ENTER; k <= KIND_PATCH; ++k) {
-				const int c = __popc(m[k]) * (k == KIND_PATCH ? PSY_PATCH_WEIGHT : PSY_LEAF_WEIGHT);
-				if (c >= best && c > 0) {
-					best = c;
-					run = k;
-				}
+		for (int k = KIND_ENTER; k < KIND_COUNT; ++k) {
+			const int c = __popc(m[k]);
+			if (c >= best && c > 0) {
+				best = c;
+				run = k;
 			}
-			if (TraceCfg<F>::FOLLOW && lane == 0) *(volatile int*)&s_kind = run;
 		}
 		++c_warp;
-		unsigned runmask = m[KIND_NODES];
-#pragma unroll
-		for (int k = LEAF_ENTER; k <= KIND_PATCH; ++k)
-			if (run == k) runmask = m[k];
-		c_lanes += __popc(runmask);
-		bool live = true;
+		c_lanes += best;
 		if (kind == run) {
 			const DevScene& sc = w.scene(rid);
-			if (run == KIND_PATCH) {
-				int left = PSY_PATCH_UNITS;
-				live = patch_step<F>(sc, st, left);
-				c_iters += PSY_PATCH_UNITS - left;
-			} else if (run == KIND_NODES) {
-				int left = PSY_WALK_NODES;
-				const int r = walk_nodes<F>(sc, st, left);
-				c_nodes += PSY_WALK_NODES - left;
-				live = r != WALK_DONE;
-				leaf = r == WALK_LEAF ? leaf_class<F>(sc, st) : 0;
+			bool live = true;
+			if (run == KIND_NODES) {
+#pragma unroll 1
+				for (int k = 0; k < PSY_WALK_NODES; ++k) {
+					++c_nodes;
+					live = tr.node_step(sc) && tr.pop(sc);
+					if (!live || tr.cur < 0) break;
+				}
 			} else {
-				leaf = 0;
-				++c_leaves;
-				live = leaf_visit<F>(sc, st);
+				if (run == KIND_PATCH) {
+					int left = PSY_PATCH_UNITS;
+					live = tr.patch_step(sc, left);
+					c_iters += PSY_PATCH_UNITS - left;
+				} else {
+					++c_leaves;
+					if (TraceCfg<F>::NESTED && run == KIND_ENTER) live = tr.enter(sc);
+					else if ((F & (FEAT_BILINEAR | FEAT_BICUBIC)) && run == KIND_BEGIN) live = tr.template patch_leaf<false>(sc);
+					else live = leaf_class(tr.cur) == LEAF_SPHERE ? tr.sphere_leaf(sc) : tr.simple_leaf(sc);
+				}
+				if (live && tr.pmode == PM_NONE) live = tr.pop(sc);
 			}
-		}
-		if (!live) {
-			err |= st.err;
-			if (OCCL) wb.occl[my] = st.rec.obj >= 0 ? 1 : 0;
-			else store_rec(wb, my, st.rec);
-			my = -1;
+			if (!live) {
+				err |= tr.err;
+				if (OCCL) wb.occl[tr.io.i] = (tr.flags & RAY_HIT) ? 1 : 0;
+				else if (!(tr.flags & RAY_HIT)) wb.hit_i[tr.io.i] = make_int4(-1, 0, 0, 0);
+				tr.io.i = -1;
+			}
 		}
 	}
 	unsigned long long c[4] = {rays, c_nodes, c_leaves, c_iters};
@@ -708,7 +724,8 @@ __global__ void __maxnreg__(PSY_SHADE_MAXNREG) shade_hit_kernel(W w, HaltonDev h
 			load_rec(wb, i, &rec);
 			bool done = false;
 			StoredHit sh;
-			if (rec.obj >= 0) {
+			if (rec.inst >= 0) {
+				hit_surface(sc, &rec);
 				int closure;
 				float ecol[3], lpdf;
 				make_stored<F>(sc, rec, wr, rp.ident_inv, &sh, &closure, ecol, &lpdf, &err);

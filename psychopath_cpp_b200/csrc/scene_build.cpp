@@ -652,7 +652,7 @@ struct Builder {
 			i += std::max<uint32_t>(recs[i].ts, 1);
 		}
 		auto ref_of = [&](size_t ri) -> int {
-			if (recs[ri].leaf_data) return leaf_ref((int)recs[ri].data);
+			if (recs[ri].leaf_data) return leaf_ref(da.inst_base + (int)recs[ri].data);
 			return dev_of[ri];
 		};
 		for (size_t i = 0; i < recs.size();) {
@@ -1018,6 +1018,102 @@ int build_scene(const psy_scene_desc* desc, BuiltScene* out, std::string* err, b
 	b.err = err;
 	b.gpu_root_bvh = gpu_root_bvh;
 	return b.run() ? PSY_OK : PSY_ERR_ARG;
+}
+
+// merge() of transform sequences (math/transform.hpp:241-272) with the
+// operations of the device's frame_merge: parent `a` (na matrices) with
+// instance transforms `b`; the result is appended to `out`.  Returns its
+// count, -1 if it needs more than 4 samples.
+static int merge_frames(const std::vector<M44>& a, const float* b, int nb, std::vector<M44>* out) {
+	const int na = (int)a.size();
+	if (na > 4 || nb > 4) return -1;
+	const int n = std::max(na, nb);
+	const float inv_s = n > 1 ? 1.0f / (float)(n - 1) : 0.0f;
+	auto own = [&](int i) {
+		M44 m;
+		std::memcpy(&m, b + 16 * i, sizeof(m));
+		return m;
+	};
+	auto at = [](const SeqPos& sp, auto get) { return sp.single ? get(sp.i0) : m44_lerp(sp.nalpha, get(sp.i0), get(sp.i0 + 1)); };
+	for (int i = 0; i < n; ++i) {
+		if (na == nb) out->push_back(m44_mul(a[i], own(i)));
+		else if (na > nb) out->push_back(nb == 0 ? a[i] : m44_mul(a[i], at(seq_pos((float)i * inv_s, nb), own)));
+		else out->push_back(na == 0 ? own(i) : m44_mul(own(i), at(seq_pos((float)i * inv_s, na), [&](int k) { return a[k]; })));
+	}
+	return n;
+}
+
+void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
+	out->leaves.resize(b.instances.size());
+	std::vector<int> rank(b.instances.size(), 0);
+	for (const DevAssembly& as : b.assemblies) {
+		int r = 0;
+		for (int i = 0; i < as.inst_count; ++i) {
+			const int gi = as.inst_base + i;
+			const DevInstance& inst = b.instances[gi];
+			DevLeaf& lf = out->leaves[gi];
+			lf = DevLeaf{};
+			lf.xforms = inst.xform_count;
+			int cls = LEAF_SIMPLE, pm = 0;
+			if (inst.kind == INST_ASSEMBLY) {
+				cls = LEAF_ENTER;
+				lf.data = rank[gi] = r++;
+				lf.asmb = inst.data;
+			} else {
+				const DevObject& ob = b.objects[inst.data];
+				const float* p = b.fpool.data() + ob.data;
+				if (ob.kind == OBJ_BILINEAR || ob.kind == OBJ_BICUBIC) {
+					cls = LEAF_PATCH;
+					lf.data = ob.data;
+					pm = (ob.kind == OBJ_BILINEAR ? 1 : 3) + (ob.n0 != 1 ? 1 : 0);
+					const int n = ob.n0 * (ob.kind == OBJ_BILINEAR ? 12 : 48);
+					for (int k = 0; k < n; ++k)
+						if (!(std::fabs(p[k]) < 1e37f)) pm |= LEAF_PATCH_ODD;
+				} else if (inst.xform_count == 0 && ((ob.kind == OBJ_SPHERE && ob.n0 == 1) ||
+				                                     (ob.kind == OBJ_SPHERE_LIGHT && ob.n0 == 1 && ob.n1 == 1))) {
+					cls = LEAF_SPHERE;
+					for (int k = 0; k < 4; ++k) lf.sphere[k] = p[k];
+				}
+			}
+			lf.kind = pm | (cls << 4);
+		}
+	}
+	// breadth first: an entry's children follow one another
+	std::vector<DevPlace>& pl = out->places;
+	std::vector<float>& fr = out->frames;
+	const DevAssembly& root = b.assemblies[0];
+	pl.push_back(DevPlace{REF_EMPTY, 0, 0, 0, -1, root.inst_base, -1, root.id_bits, 0, 0, 0});
+	for (size_t k = 0; k < pl.size(); ++k) {
+		pl[k].child_base = (int)pl.size();
+		const DevPlace at = pl[k];
+		const DevAssembly& as = b.assemblies[at.asmb];
+		std::vector<M44> parent(at.frame_count > 0 ? at.frame_count : 0);
+		for (size_t m = 0; m < parent.size(); ++m) std::memcpy(&parent[m], fr.data() + (size_t)(at.frame + m) * 16, sizeof(M44));
+		for (int i = 0; i < as.inst_count; ++i) {
+			const DevInstance& inst = b.instances[as.inst_base + i];
+			if (inst.kind != INST_ASSEMBLY) continue;
+			if ((int)pl.size() >= limit) {
+				pl.clear();
+				fr.clear();
+				return;
+			}
+			const DevAssembly& sub = b.assemblies[inst.data];
+			DevPlace q = at;
+			q.parent = (int)k;
+			q.asmb = inst.data;
+			q.inst_base = sub.inst_base;
+			q.id_bits = sub.id_bits;
+			q.id = id_push(at.id, (uint64_t)i, at.id_bits);
+			if (inst.shader >= 0) q.shader = inst.shader;
+			if (inst.xform_count > 0 && at.frame_count >= 0) {
+				std::vector<M44> merged;
+				q.frame = (int)(fr.size() / 16);
+				q.frame_count = merge_frames(parent, b.xforms.data() + (size_t)inst.xform * 16, inst.xform_count, &merged);
+				if (q.frame_count > 0) fr.insert(fr.end(), &merged[0].m[0][0], &merged[0].m[0][0] + merged.size() * 16);
+			}
+			pl.push_back(q);
+		}
+	}
 }
 
 }  // namespace psy

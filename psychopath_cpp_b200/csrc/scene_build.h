@@ -61,6 +61,16 @@ struct BuiltScene {
 	std::vector<int> gpu_light_first;
 };
 
+// The traversal's tables of a built scene: a leaf record per instance, and
+// the unrolled assembly instances with their merged frames (places is empty
+// when there are more than `limit`).
+struct SceneTables {
+	std::vector<DevLeaf> leaves;
+	std::vector<DevPlace> places;
+	std::vector<float> frames;  // 16 floats per matrix
+};
+void build_tables(const BuiltScene& b, int limit, SceneTables* out);
+
 // Validates the description and builds every assembly (children first).
 // gpu_root_bvh: leave the root assembly's traversal tree and light tree to
 // the device builds (see gpu_root_pending and gpu_light_pending).  Returns PSY_OK or

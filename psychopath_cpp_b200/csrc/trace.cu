@@ -18,14 +18,44 @@ __device__ __forceinline__ void st3(float* p, uint32_t i, V3 v) {
 	p[3 * (size_t)i + 2] = v.z;
 }
 
-// Register cap of the kernel: flat scenes (spheres, lights, bilinear
-// patches in one level) run at 64 registers, where more resident warps hide
-// the walk's memory latency (the 4M-ray heightfield stream: 1.92 -> 2.15 G
-// rays/s against the compiler's 127; 96 and 48 are slower); the larger
-// variants keep the compiler's choice.
+// A ray of the stream and the hit it ends with (Trav's IO).
+struct StreamIO {
+	const RaySoA* rays;
+	HitRec* rec;
+	uint32_t i;
+	__device__ __forceinline__ V3 origin() const { return ld3(rays->o, i); }
+	__device__ __forceinline__ V3 direction() const { return ld3(rays->d, i); }
+	__device__ __forceinline__ void differentials(V3* odx, V3* ody, V3* ddx, V3* ddy) const {
+		*odx = ld3(rays->odx, i);
+		*ody = ld3(rays->ody, i);
+		*ddx = ld3(rays->ddx, i);
+		*ddy = ld3(rays->ddy, i);
+	}
+	template <class T>
+	__device__ __forceinline__ void hit(const T& tr, int inst, float t, float u, float v, float md) const {
+		rec->t = t;
+		rec->u = u;
+		rec->v = v;
+		rec->max_dim = md;
+		rec->inst = inst;
+		rec->place = tr.place;
+		if (T::NESTED && tr.place < 0) {
+			rec->depth = tr.L + 1;
+			for (int k = 1; k <= tr.L; ++k) rec->path[k - 1] = tr.lv_inst[k];
+			rec->path[tr.L] = inst;
+		}
+	}
+};
+
+// Register cap of the kernel: 64 for flat scenes (spheres, lights, bilinear
+// patches in one level), where more resident warps hide the walk's memory
+// latency (4M rays against the heightfield: 1.06 ms; 1.13 at 80 registers,
+// 1.37 at 128), 128 for the larger variants, whose bicubic bisection spills
+// below that (300,000 mixed rays against instanced patches and spheres:
+// 2.04 ms; 2.30 at 184, 2.80 at 72).
 template <unsigned F>
 struct TraceKernelRegs {
-	static constexpr int value = F == FEAT_FLAT ? 64 : 255;
+	static constexpr int value = F == FEAT_FLAT ? 64 : 128;
 };
 
 template <unsigned F>
@@ -33,22 +63,28 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
                                                                    uint32_t n, unsigned* status) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
+	HitRec rec;
+	rec.inst = -1;
 	WorldRayD wr;
 	wr.o = ld3(rays.o, i);
 	wr.d = ld3(rays.d, i);
-	wr.odx = ld3(rays.odx, i);
-	wr.ody = ld3(rays.ody, i);
-	wr.ddx = ld3(rays.ddx, i);
-	wr.ddy = ld3(rays.ddy, i);
 	wr.time = __ldg(rays.time + i);
 	wr.occl = rays.type ? (__ldg(rays.type + i) == 32) : false;
-
-	HitRec rec;
-	unsigned err = trace_ray<F>(sc, wr, &rec);
-	const bool hit = rec.obj >= 0;
+	unsigned err;
+	{
+		Trav<F, StreamIO> tr;
+		tr.io.rays = &rays;
+		tr.io.rec = &rec;
+		tr.io.i = i;
+		tr.init(sc, wr.o, wr.d, wr.time, wr.occl);
+		tr.walk(sc);
+		err = tr.err;
+	}
+	const bool hit = rec.inst >= 0;
 	if (hits.hit) hits.hit[i] = hit ? 1 : 0;
-	if (hits.id) hits.id[i] = hit ? rec.id : 0ull;
+	if (hits.id) hits.id[i] = hit ? hit_id(sc, rec) : 0ull;
 	if (hits.t) hits.t[i] = (hit && !wr.occl) ? rec.t : INFINITY;
+	if (hit && !wr.occl && hits.want_geometry) hit_surface(sc, &rec);
 	if (hit && !wr.occl && hits.want_geometry == WANT_UV && (rec.kind == OBJ_BILINEAR || rec.kind == OBJ_BICUBIC)) {
 		// a patch's u, v are the bisection's own: no geometry to evaluate
 		hits.uv[2 * (size_t)i] = rec.u;

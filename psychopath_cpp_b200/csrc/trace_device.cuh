@@ -1,5 +1,5 @@
 /*
- * Device-side ray traversal of the uploaded scene: one ray per thread.
+ * Device-side ray traversal of the uploaded scene.
  *
  * The reference traces ray *streams* breadth-first (accel/bvh4.cpp:163-236,
  * object/patch_utils.hpp:18-200); every per-ray decision there depends only
@@ -8,11 +8,17 @@
  * one order-dependent case, two candidates at exactly the same t, resolves
  * to whichever is found first; child boxes are visited nearest-first here.
  *
- * Per-ray state: the ray in the current instance space, a node stack,
- * a level stack for nested assemblies (element id prefix, inherited shader,
- * merged motion transforms, as the reference's xform_stack /
- * surface_shader_stack / element_id, tracer/tracer.cpp:125-219), and the
- * path bits of the patch bisection (PatchWork, patch_run).
+ * What a lane carries from step to step is small and meant for registers:
+ * the ray in the current space, the next tree reference (`cur`), the stack
+ * depth and the placement it is in.  Everything an assembly instance adds
+ * on the way down (merged motion transforms, the inherited shader, the
+ * element id prefix: the reference's xform_stack, surface_shader_stack and
+ * element_id, tracer/tracer.cpp:125-219) depends on the path of instances
+ * alone and is laid out once per scene, one DevPlace per unrolled assembly
+ * instance.  Scenes that unroll to more than PSY_MAX_PLACES keep a level
+ * stack in local memory instead.  (With the merged frames, the hit record,
+ * the level stack and a copy of the ray in a lane's local memory the
+ * 1280x720x4 many-light frame took PSY_OLD ms; now PSY_NEW.)
  */
 #ifndef PSY_TRACE_DEVICE_CUH
 #define PSY_TRACE_DEVICE_CUH
@@ -34,13 +40,6 @@ struct WorldRayD {
 	bool occl;
 };
 
-// Ray in the current instance space (Ray, basics/ray.hpp:24-37).  Its
-// width parameters are kept apart (ray_width_of): only patch leaves need
-// them, so they are computed on first use in each space.
-struct LocalRay {
-	V3 o, d, dinv;
-};
-
 __device__ __forceinline__ M44 load_m44_dev(const float* p) {
 	M44 m;
 	const float4* q = reinterpret_cast<const float4*>(p);
@@ -55,41 +54,32 @@ __device__ __forceinline__ M44 load_m44_dev(const float* p) {
 	return m;
 }
 
-// WorldRay::update_ray (basics/ray.hpp:207-305): with and without transform.
-__device__ __forceinline__ LocalRay make_local(const WorldRayD& wr) {
-	LocalRay r;
-	r.o = wr.o;
-	r.d = wr.d;
-	r.dinv = recip3(r.d);
-	return r;
-}
-
-__device__ __forceinline__ LocalRay make_local_x(const WorldRayD& wr, const M44& t) {
-	LocalRay r;
-	r.o = pos_to(t, wr.o);
-	r.d = dir_to(t, wr.d);
-	r.dinv = recip3(r.d);
-	return r;
-}
-
-// The width parameters update_ray computes beside the local ray `r` (made
-// from wr with transform t, or none).  Computed once per space a ray meets
-// a patch in.
-__device__ __forceinline__ RayWidth ray_width_of(const WorldRayD& wr, const LocalRay& r, const M44* t) {
-	if (!t) return ray_width_params(r.o, r.d, wr.odx, wr.ody, wr.ddx, wr.ddy);
-	return ray_width_params(r.o, r.d, dir_to(*t, wr.odx), dir_to(*t, wr.ody), dir_to(*t, wr.ddx), dir_to(*t, wr.ddy));
-}
-
-// Merged motion-transform sequence of a level (the reference's xform_stack frame).
+// A sequence of motion matrices (16 floats each, 16-byte aligned): a
+// placement's merged frame, an instance's transforms or a frame in local
+// memory.  count 0 = no transform (identity).
 struct Frame {
-	int count;  // 0 = no transform (identity)
-	M44 m[PSY_MAX_MOTION];
+	const float* m;
+	int count;
 };
 
-__device__ __forceinline__ M44 frame_at_index_lerp(const Frame& f, float alpha) {
+__device__ __forceinline__ M44 load_m44(const float* p) {
+	M44 m;
+	const float4* q = reinterpret_cast<const float4*>(p);
+#pragma unroll
+	for (int r = 0; r < 4; ++r) {
+		const float4 v = q[r];
+		m.m[r][0] = v.x;
+		m.m[r][1] = v.y;
+		m.m[r][2] = v.z;
+		m.m[r][3] = v.w;
+	}
+	return m;
+}
+
+__device__ __forceinline__ M44 frame_at(const Frame& f, float alpha) {
 	const SeqPos sp = seq_pos(alpha, f.count);
-	if (sp.single) return f.m[sp.i0];
-	return m44_lerp(sp.nalpha, f.m[sp.i0], f.m[sp.i0 + 1]);
+	if (sp.single) return load_m44(f.m + 16 * sp.i0);
+	return m44_lerp(sp.nalpha, load_m44(f.m + 16 * sp.i0), load_m44(f.m + 16 * (sp.i0 + 1)));
 }
 
 __device__ __forceinline__ M44 seq_lerp_global(const float* xs, int count, float alpha) {
@@ -98,35 +88,39 @@ __device__ __forceinline__ M44 seq_lerp_global(const float* xs, int count, float
 	return m44_lerp(sp.nalpha, load_m44_dev(xs + 16 * sp.i0), load_m44_dev(xs + 16 * (sp.i0 + 1)));
 }
 
+// Room for one merged frame in local memory.
+struct alignas(16) FrameBuf {
+	float m[PSY_MAX_MOTION * 16];
+};
+
 // merge() of transform sequences (math/transform.hpp:241-272): parent `a`
-// with instance transforms `b` (global, count nb), written into `dst`.
-// Returns false if the result needs more than PSY_MAX_MOTION samples.  The
-// three cases of the reference (equal counts, more parent samples, more
-// instance samples) share one loop with one matrix product.  (Outlined, so
-// that its frames pass through memory, this and the other traversal helpers
-// cost 11% of the many-light render's traversal time.)
-__device__ __forceinline__ bool frame_merge(const Frame& a, const float* b, int nb, Frame* dst) {
+// with instance transforms `b`, written into `dst`.  Returns the merged
+// sequence; its count is -1 if it needs more than PSY_MAX_MOTION samples.
+// The three cases of the reference (equal counts, more parent samples, more
+// instance samples) share one loop with one matrix product.
+__device__ __forceinline__ Frame frame_merge(const Frame& a, const float* b, int nb, FrameBuf* dst) {
 	const int na = a.count;
-	if (na > PSY_MAX_MOTION || nb > PSY_MAX_MOTION) return false;
+	Frame out{dst->m, -1};
+	if (na > PSY_MAX_MOTION || nb > PSY_MAX_MOTION) return out;
 	const int n = na > nb ? na : nb;
 	const float inv_s = n > 1 ? 1.0f / (float)(n - 1) : 0.0f;
 #pragma unroll 1
 	for (int i = 0; i < n; ++i) {
 		M44 r;
 		if (na == nb) {
-			r = m44_mul(a.m[i], load_m44_dev(b + 16 * i));
+			r = m44_mul(load_m44(a.m + 16 * i), load_m44_dev(b + 16 * i));
 		} else if (na > nb) {
-			if (nb == 0) r = a.m[i];
-			else r = m44_mul(a.m[i], seq_lerp_global(b, nb, (float)i * inv_s));
+			if (nb == 0) r = load_m44(a.m + 16 * i);
+			else r = m44_mul(load_m44(a.m + 16 * i), seq_lerp_global(b, nb, (float)i * inv_s));
 		} else {
 			// the reference multiplies instance * lerped-parent in this case
 			if (na == 0) r = load_m44_dev(b + 16 * i);
-			else r = m44_mul(load_m44_dev(b + 16 * i), frame_at_index_lerp(a, (float)i * inv_s));
+			else r = m44_mul(load_m44_dev(b + 16 * i), frame_at(a, (float)i * inv_s));
 		}
-		dst->m[i] = r;
+		for (int k = 0; k < 16; ++k) dst->m[16 * i + k] = r.m[k / 4][k % 4];
 	}
-	dst->count = n;
-	return true;
+	out.count = n;
+	return out;
 }
 
 // ---------------------------------------------------------------------
@@ -255,19 +249,6 @@ struct Patch {
 	V3 p[NV];
 };
 
-template <int NV>
-__device__ __forceinline__ Box patch_bound(const Patch<NV>& q) {
-	Box b;
-	b.lo = q.p[0];
-	b.hi = q.p[0];
-#pragma unroll
-	for (int i = 1; i < NV; ++i) {
-		b.lo = vmin3(b.lo, q.p[i]);
-		b.hi = vmax3(b.hi, q.p[i]);
-	}
-	return b;
-}
-
 __device__ __forceinline__ float patch_ulen(const Patch<4>& q) { return longest_axis(q.p[0] - q.p[1]); }
 __device__ __forceinline__ float patch_vlen(const Patch<4>& q) { return longest_axis(q.p[0] - q.p[2]); }
 __device__ __forceinline__ float patch_ulen(const Patch<16>& q) { return longest_axis(q.p[0] - q.p[3]); }
@@ -279,17 +260,11 @@ __device__ __forceinline__ void patch_load(const float* src, Patch<NV>* q) {
 	for (int i = 0; i < NV; ++i) q->p[i] = V3(__ldg(src + i * 3), __ldg(src + i * 3 + 1), __ldg(src + i * 3 + 2));
 }
 
-// Result of a patch leaf hit, consumed by the shading epilogue.
-struct PatchHit {
-	float t, u, v, max_dim;
-};
-
 // Splits of a patch at the middle of u or v (Bilinear::split_u / split_v,
 // object/bilinear.hpp:59-82; Bicubic::split_u / split_v, de Casteljau at 0.5
 // per row or column, object/bicubic.hpp:74-108), with the reference's float
 // operations.  patch_split leaves the second half in `p` and writes the
-// first half to `f`; patch_half_u / patch_half_v keep one half in place and
-// give the same values for it.
+// first half to `f`.
 __device__ __forceinline__ void patch_split(Patch<4>& p, Patch<4>& f, bool along_u) {
 	if (along_u) {
 		const V3 m01 = (p.p[0] + p.p[1]) * 0.5f;
@@ -311,29 +286,6 @@ __device__ __forceinline__ void patch_split(Patch<4>& p, Patch<4>& f, bool along
 		p.p[1] = m13;
 	}
 }
-__device__ __forceinline__ void patch_half_u(Patch<4>& p, bool second) {
-	const V3 m01 = (p.p[0] + p.p[1]) * 0.5f;
-	const V3 m23 = (p.p[2] + p.p[3]) * 0.5f;
-	if (second) {
-		p.p[0] = m01;
-		p.p[2] = m23;
-	} else {
-		p.p[1] = m01;
-		p.p[3] = m23;
-	}
-}
-__device__ __forceinline__ void patch_half_v(Patch<4>& p, bool second) {
-	const V3 m02 = (p.p[0] + p.p[2]) * 0.5f;
-	const V3 m13 = (p.p[1] + p.p[3]) * 0.5f;
-	if (second) {
-		p.p[0] = m02;
-		p.p[1] = m13;
-	} else {
-		p.p[2] = m02;
-		p.p[3] = m13;
-	}
-}
-
 // One de Casteljau split at 0.5 of the control points a,b,c,d of a row or a
 // column: a..d become the second half, fa..fd the first.
 __device__ __forceinline__ void bezier_split(V3& a, V3& b, V3& c, V3& d, V3& fa, V3& fb, V3& fc, V3& fd) {
@@ -351,24 +303,6 @@ __device__ __forceinline__ void bezier_split(V3& a, V3& b, V3& c, V3& d, V3& fa,
 	b = q1;
 	c = q2;
 }
-// The same split keeping one half in place.
-__device__ __forceinline__ void bezier_half(V3& a, V3& b, V3& c, V3& d, bool second) {
-	const V3 tmp = (b + c) * 0.5f;
-	const V3 q2 = (d + c) * 0.5f;
-	const V3 q1 = (tmp + q2) * 0.5f;
-	const V3 a1 = (a + b) * 0.5f;
-	const V3 a2 = (tmp + a1) * 0.5f;
-	const V3 a3 = (a2 + q1) * 0.5f;
-	if (second) {
-		a = a3;
-		b = q1;
-		c = q2;
-	} else {
-		b = a1;
-		c = a2;
-		d = a3;
-	}
-}
 __device__ __forceinline__ void patch_split(Patch<16>& p, Patch<16>& f, bool along_u) {
 	if (along_u) {
 #pragma unroll
@@ -381,82 +315,113 @@ __device__ __forceinline__ void patch_split(Patch<16>& p, Patch<16>& f, bool alo
 			bezier_split(p.p[c], p.p[c + 4], p.p[c + 8], p.p[c + 12], f.p[c], f.p[c + 4], f.p[c + 8], f.p[c + 12]);
 	}
 }
-__device__ __forceinline__ void patch_half_u(Patch<16>& p, bool second) {
-#pragma unroll
-	for (int r = 0; r < 4; ++r) bezier_half(p.p[r * 4], p.p[r * 4 + 1], p.p[r * 4 + 2], p.p[r * 4 + 3], second);
-}
-__device__ __forceinline__ void patch_half_v(Patch<16>& p, bool second) {
-#pragma unroll
-	for (int c = 0; c < 4; ++c) bezier_half(p.p[c], p.p[c + 4], p.p[c + 8], p.p[c + 12], second);
-}
-
-// The 24 floats of a BBox4 record (six 128-bit loads).
-__device__ __forceinline__ void load_box4(const float4* q, float* b) {
-#pragma unroll
-	for (int i = 0; i < 6; ++i) {
-		const float4 v = __ldg(q + i);
-		b[i * 4 + 0] = v.x;
-		b[i * 4 + 1] = v.y;
-		b[i * 4 + 2] = v.z;
-		b[i * 4 + 3] = v.w;
-	}
-}
-
-// Path of a node in the bisection tree: one bit per split level.
-struct Bits128 {
-	uint64_t lo, hi;
-	__device__ __forceinline__ bool get(int i) const { return i < 64 ? ((lo >> i) & 1ull) : ((hi >> (i - 64)) & 1ull); }
-	__device__ __forceinline__ void set(int i, bool v) {
-		if (i < 64) lo = v ? (lo | (1ull << i)) : (lo & ~(1ull << i));
-		else hi = v ? (hi | (1ull << (i - 64))) : (hi & ~(1ull << (i - 64)));
-	}
-	// keep bits [0, n)
-	__device__ __forceinline__ void truncate(int n) {
-		if (n <= 0) { lo = 0; hi = 0; }
-		else if (n < 64) { lo &= (1ull << n) - 1ull; hi = 0; }
-		else if (n < 128) { hi &= (1ull << (n - 64)) - 1ull; }
-	}
-	// highest set bit below n, or -1
-	__device__ __forceinline__ int highest_below(int n) const {
-		Bits128 t = *this;
-		t.truncate(n);
-		if (t.hi) return 64 + 63 - __clzll((long long)t.hi);
-		if (t.lo) return 63 - __clzll((long long)t.lo);
-		return -1;
-	}
-	__device__ __forceinline__ int popc() const { return __popcll(lo) + __popcll(hi); }
+// ---------------------------------------------------------------------
+// Slab tests
+// ---------------------------------------------------------------------
+// min and max of the bisection: the reference's orders (a op b ? a : b,
+// std::min / std::max), or, for operands that are never NaN (clean patches
+// and rays: RAY_ODD), single instructions.  Without NaN the two differ in
+// the sign of a zero at most, which no comparison that follows can tell.
+template <bool CLEAN>
+struct MinMax {
+	__device__ static __forceinline__ float vlo(float a, float b) { return CLEAN ? fminf(a, b) : vmin(a, b); }
+	__device__ static __forceinline__ float vhi(float a, float b) { return CLEAN ? fmaxf(a, b) : vmax(a, b); }
+	__device__ static __forceinline__ float slo(float a, float b) { return CLEAN ? fminf(a, b) : smin(a, b); }
+	__device__ static __forceinline__ float shi(float a, float b) { return CLEAN ? fmaxf(a, b) : smax(a, b); }
+	__device__ static __forceinline__ float axis(V3 v) { return shi(shi(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); }
 };
+
+template <int NV, bool CLEAN>
+__device__ __forceinline__ Box patch_bound(const Patch<NV>& q) {
+	typedef MinMax<CLEAN> M;
+	Box b;
+	b.lo = q.p[0];
+	b.hi = q.p[0];
+#pragma unroll
+	for (int i = 1; i < NV; ++i) {
+		b.lo = V3(M::vlo(b.lo.x, q.p[i].x), M::vlo(b.lo.y, q.p[i].y), M::vlo(b.lo.z, q.p[i].z));
+		b.hi = V3(M::vhi(b.hi.x, q.p[i].x), M::vhi(b.hi.y, q.p[i].y), M::vhi(b.hi.z, q.p[i].z));
+	}
+	return b;
+}
 
 // Bounds of a sub-patch (each time sample) and the ray's test against them:
 // the top of the loop of intersect_rays_with_patch (object/patch_utils.hpp).
-template <int NV, int TSC>
-__device__ __forceinline__ bool patch_node_test(const Patch<NV> (&q)[TSC], float t_nalpha, const LocalRay& r,
-                                                float max_t, float* max_dim, float* h0, float* h1) {
+template <int NV, int TSC, bool CLEAN>
+__device__ __forceinline__ bool patch_node_test(const Patch<NV> (&q)[TSC], float t_nalpha, V3 o, V3 dinv, float max_t,
+                                                float* max_dim, float* h0, float* h1) {
+	typedef MinMax<CLEAN> M;
 	Box bb[TSC];
 	float md = 0.0f;
 #pragma unroll
 	for (int k = 0; k < TSC; ++k) {
-		bb[k] = patch_bound<NV>(q[k]);
-		const float ld = longest_axis(bb[k].hi - bb[k].lo);
-		md = (k == 0) ? ld : smax(md, ld);
+		bb[k] = patch_bound<NV, CLEAN>(q[k]);
+		const float ld = M::axis(bb[k].hi - bb[k].lo);
+		md = (k == 0) ? ld : M::shi(md, ld);
 	}
 	*max_dim = md;
-	const bool h = (TSC == 1) ? box_hit(bb[0], r.o, r.dinv, max_t, h0, h1)
-	                          : box_hit(box_lerp(t_nalpha, bb[0], bb[TSC - 1]), r.o, r.dinv, max_t, h0, h1);
-	// A NaN far distance comes from 0 * inf: the ray runs exactly along a
-	// box face (a zero direction component, the origin on the face).  The
-	// reference's std::min/max slab test then reports a hit with h0 = 0 and
-	// h1 = NaN, and every sub-box is again NaN or a plain miss, so none of
-	// the subtree's leaves can be taken (their t = (h0 + h1) / 2 is NaN)
-	// while the reference still walks all of it, millions of nodes deep
-	// for a camera ray through the image centre.  Treating it as a miss
-	// gives the same hits.
-	return h && !(*h1 != *h1);
+	const Box b = (TSC == 1) ? bb[0] : box_lerp(t_nalpha, bb[0], bb[TSC - 1]);
+	if (!CLEAN) {
+		const bool h = box_hit(b, o, dinv, max_t, h0, h1);
+		// A NaN far distance comes from 0 * inf: the ray runs exactly along a
+		// box face (a zero direction component, the origin on the face).  The
+		// reference's std::min/max slab test then reports a hit with h0 = 0 and
+		// h1 = NaN, and every sub-box is again NaN or a plain miss, so none of
+		// the subtree's leaves can be taken (their t = (h0 + h1) / 2 is NaN)
+		// while the reference still walks all of it, millions of nodes deep
+		// for a camera ray through the image centre.  Treating it as a miss
+		// gives the same hits.
+		return h && !(*h1 != *h1);
+	}
+	const float x0 = (b.lo.x - o.x) * dinv.x, x1 = (b.hi.x - o.x) * dinv.x;
+	const float y0 = (b.lo.y - o.y) * dinv.y, y1 = (b.hi.y - o.y) * dinv.y;
+	const float z0 = (b.lo.z - o.z) * dinv.z, z1 = (b.hi.z - o.z) * dinv.z;
+	*h0 = fmaxf(fmaxf(0.0f, fminf(z0, z1)), fmaxf(fminf(x0, x1), fminf(y0, y1)));
+	*h1 = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1)) * BBOX_MAXT_ADJUST;
+	return *h0 <= fminf(max_t, *h1);
+}
+
+// ---------------------------------------------------------------------
+// Patch bisection
+// ---------------------------------------------------------------------
+// Ray::min_width (basics/ray.hpp:132-153) with the parts that do not change
+// along the ray taken out of the bisection: the two flip distances cost an
+// IEEE division each.
+struct RayFlip {
+	float ax, ay;          // owx - fwx, owy - fwy
+	float tflipx, tflipy;
+	float dwx, dwy, fwx, fwy;
+};
+
+__device__ __forceinline__ RayFlip ray_flip(const RayWidth& w) {
+	RayFlip f;
+	f.ax = w.owx - w.fwx;
+	f.ay = w.owy - w.fwy;
+	f.tflipx = f.ax / w.dwx;
+	f.tflipy = f.ay / w.dwy;
+	f.dwx = w.dwx; f.dwy = w.dwy;
+	f.fwx = w.fwx; f.fwy = w.fwy;
+	return f;
+}
+
+__device__ __forceinline__ float flip_min_width(const RayFlip& w, float tnear, float tfar) {
+	float minx, miny;
+	if (tnear < w.tflipx && tfar > w.tflipx) minx = w.fwx;
+	else minx = smin(fabsf(w.ax + (w.dwx * tnear)) + w.fwx, fabsf(w.ax + (w.dwx * tfar)) + w.fwx);
+	if (tnear < w.tflipy && tfar > w.tflipy) miny = w.fwy;
+	else miny = smin(fabsf(w.ay + (w.dwy * tnear)) + w.fwy, fabsf(w.ay + (w.dwy * tfar)) + w.fwy);
+	return smin(minx, miny);
 }
 
 // Pending first halves a bisection can hold: at most one per second half
 // on the path, and the path has at most PSY_SPLIT_STACK - 1 of those.
 #define PSY_PATCH_PEND PSY_SPLIT_STACK
+
+// A bisection ends with an error (ERRF_BISECT) after this many loop
+// iterations.  The walk is finite (a leaf is forced at 63 second halves or
+// depth 127), but a ray the reference would bisect for hours must not hold
+// a wave: far above any bisection of a real scene.
+#define PSY_PATCH_MAX_STEPS (1u << 24)
 
 // Per-ray bisection of one patch with TSC time samples (TSC = 1 or 2):
 // intersect_rays_with_patch for a single ray (object/patch_utils.hpp:18-200).
@@ -469,57 +434,42 @@ __device__ __forceinline__ bool patch_node_test(const Patch<NV> (&q)[TSC], float
 // first halves (control points and uv range) if both are, and dropped if
 // its box is missed (box_hit only gets stricter as the ray's max t
 // shrinks, so the reference would find it missed later as well).  When a
-// subtree ends, the deepest pending first half is popped and tested again
-// with the current max t.  The stack holds only the halves that are
-// pending, so it is written once per split that hits both halves; the path
-// bits (1 = second half) give the reference's stack index (its forced leaf
-// at 63: the population count of the path) and the depth to resume at.
-// Control points and uv ranges are those of the reference's walk, so the
-// visiting order and the leaf results are the same.
+// subtree ends, the last pending first half is popped and tested again
+// with the current max t.  A node carries its depth and the number of
+// second halves on its path: the reference's stack index, its forced leaf
+// at 63.  Control points and uv ranges are those of the reference's walk, so
+// the visiting order and the leaf results are the same.
 //
 // The bisection can stop after any number of loop iterations and resume
 // later from its cursor (the node at the top of the loop, whose box the ray
-// hits, with its path bits and uv range) and its stack, so that a lane can
-// leave a long bisection to run with the other lanes of its warp.
-// patch_run works on a cursor the caller holds as a local (kept in
-// registers) and copies back only when it stops short of the end.
+// hits) and its stack, so that a lane can leave a long bisection to run
+// with the other lanes of its warp.  patch_run works on a cursor the caller
+// holds as a local (kept in registers) and copies back only when it stops
+// short of the end.
 template <int NV, int TSC>
 struct PatchCursor {
 	Patch<NV> cur[TSC];        // the node at the top of the loop
-	Bits128 path, dirs, pend;  // dirs bit: 1 = split along u
-	int depth;                 // splits from the root
 	float u0, u1, v0, v1;
-	float t_nalpha, max_dim, h0, h1;
-	bool found;
-	unsigned steps;  // loop iterations taken (bounded: PSY_PATCH_MAX_STEPS)
-	int sp;          // pending first halves on the stack
+	float max_dim, h0, h1;     // its test
+	float t_nalpha;
+	int depth, seconds;        // splits from the root, second halves among them
+	int sp;                    // pending first halves on the stack
+	unsigned steps;            // loop iterations taken (bounded: PSY_PATCH_MAX_STEPS)
 };
 
-// A bisection ends with an error (ERRF_BISECT) after this many loop
-// iterations.  The walk is finite (a leaf is forced at 63 second halves or
-// depth 127), but a ray the reference would bisect for hours must not hold
-// a wave: far above any bisection of a real scene.
-#define PSY_PATCH_MAX_STEPS (1u << 24)
-
-// Sub-patches stored on the current path (with their uv ranges).
+// The pending first halves.
 template <int NV, int TSC>
 struct PatchStore {
 	Patch<NV> pend[PSY_PATCH_PEND][TSC];
-	float penduv[PSY_PATCH_PEND][4];
-};
-
-// A suspended bisection in a lane's traversal state.
-template <int NV, int TSC>
-struct PatchWork {
-	PatchCursor<NV, TSC> c;
-	PatchStore<NV, TSC> st;
+	float4 uv[PSY_PATCH_PEND];
+	int2 at[PSY_PATCH_PEND];   // depth, second halves
 };
 
 // The root's test: sets up `pc` and returns true when the ray hits the
 // patch's box.
-template <int NV, int TSC>
-__device__ __forceinline__ bool patch_begin(PatchCursor<NV, TSC>& pc, const float* verts, float time,
-                                            const LocalRay& r, float max_t) {
+template <int NV, int TSC, bool CLEAN>
+__device__ __forceinline__ bool patch_begin(PatchCursor<NV, TSC>& pc, const float* verts, float time, V3 o, V3 dinv,
+                                            float max_t) {
 #pragma unroll
 	for (int k = 0; k < TSC; ++k) patch_load<NV>(verts + k * NV * 3, &pc.cur[k]);
 	pc.t_nalpha = 0.0f;
@@ -530,47 +480,39 @@ __device__ __forceinline__ bool patch_begin(PatchCursor<NV, TSC>& pc, const floa
 		const float t_time = time * (float)(TSC - 1);
 		pc.t_nalpha = t_time - (float)(int)t_time;
 	}
-	if (!patch_node_test<NV, TSC>(pc.cur, pc.t_nalpha, r, max_t, &pc.max_dim, &pc.h0, &pc.h1)) return false;
-	pc.path = Bits128{0, 0};
-	pc.dirs = Bits128{0, 0};
-	pc.pend = Bits128{0, 0};
+	if (!patch_node_test<NV, TSC, CLEAN>(pc.cur, pc.t_nalpha, o, dinv, max_t, &pc.max_dim, &pc.h0, &pc.h1)) return false;
+	pc.u0 = pc.v0 = 0.0f;
+	pc.u1 = pc.v1 = 1.0f;
 	pc.depth = 0;
-	pc.u0 = 0.0f;
-	pc.u1 = 1.0f;
-	pc.v0 = 0.0f;
-	pc.v1 = 1.0f;
-	pc.found = false;
-	pc.steps = 0;
+	pc.seconds = 0;
 	pc.sp = 0;
+	pc.steps = 0;
 	return true;
 }
 
+enum : int { PATCH_MORE = 0, PATCH_DONE = 1, PATCH_BLOCKED = 2 };
+
 // Runs up to `units` iterations of the bisection loop (a leaf test or a
-// split, with the resume that follows it).  Returns true when the
-// bisection has ended; pc.found then says whether a leaf was taken (the
-// closest one in *hit, with *max_t lowered to it; for occlusion rays the
-// first one).  Otherwise `pc` is the node to carry on from.  A bisection
-// that exceeds PSY_PATCH_MAX_STEPS iterations ends without a hit and sets
-// ERRF_BISECT in *err.
-template <int NV, int TSC>
-__device__ __forceinline__ bool patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV, TSC>& ps, const float* verts,
-                                          const LocalRay& r, const RayWidth& rw, float* max_t, bool occl,
-                                          float dice_rate, float min_upoly, PatchHit* hit, int& units,
-                                          unsigned* err) {
+// split, with the resume that follows it).  Returns PATCH_DONE when the
+// bisection has ended, PATCH_BLOCKED when an occlusion ray took a leaf
+// (that ends it), PATCH_MORE when `pc` is the node to carry on from.
+// `leaf(t, u, v, max_dim)` is called for every leaf taken, each closer than
+// the last, with *max_t lowered to it.  A bisection that exceeds
+// PSY_PATCH_MAX_STEPS iterations ends and sets ERRF_BISECT in *err.
+template <int NV, int TSC, bool CLEAN, class LEAF>
+__device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV, TSC>& ps, V3 o, V3 dinv,
+                                         const RayFlip& rw, float* max_t, bool occl, float dice_rate, float min_upoly,
+                                         int& units, unsigned* err, LEAF leaf) {
 	Patch<NV>(&cur)[TSC] = pc.cur;
 	const float t_nalpha = pc.t_nalpha;
 	float &max_dim = pc.max_dim, &h0 = pc.h0, &h1 = pc.h1;
-	Bits128 &path = pc.path, &dirs = pc.dirs, &pend = pc.pend;
-	int& depth = pc.depth;
 	float &u0 = pc.u0, &u1 = pc.u1, &v0 = pc.v0, &v1 = pc.v1;
-	bool& found = pc.found;
 	while (true) {
-		if (units == 0) return false;
+		if (units == 0) return PATCH_MORE;
 		--units;
 		if (++pc.steps > PSY_PATCH_MAX_STEPS) {
-			found = false;
 			*err |= ERRF_BISECT;
-			return true;
+			return PATCH_DONE;
 		}
 		// `cur` is a node whose box the ray hits; max_dim, h0, h1 are its test
 		// A NaN width (from NaN ray differentials: a grazing hit makes the
@@ -579,19 +521,14 @@ __device__ __forceinline__ bool patch_run(PatchCursor<NV, TSC>& pc, PatchStore<N
 		// reference's std::max, no sub-patch is ever small enough, and its
 		// bisection does not end.  Here it counts as zero width: the leaves
 		// stop at min_upoly, as for a ray with zero differentials.
-		const float wm = ray_min_width(rw, h0, h1) * dice_rate;
+		const float wm = flip_min_width(rw, h0, h1) * dice_rate;
 		const float width = (wm != wm) ? min_upoly : smax(wm, min_upoly);
-		bool entered = false;
-		if (max_dim <= width || path.popc() == PSY_SPLIT_STACK - 1 || depth == 127) {
+		if (max_dim <= width || pc.seconds == PSY_SPLIT_STACK - 1 || pc.depth == 127) {
 			const float tt = (h0 + h1) * 0.5f;
 			if (tt > 0.0f && tt < *max_t) {
-				found = true;
-				if (occl) return true;
-				*max_t = tt;
-				hit->t = tt;
-				hit->u = (u0 + u1) * 0.5f;
-				hit->v = (v0 + v1) * 0.5f;
-				hit->max_dim = max_dim;
+				if (!occl) *max_t = tt;
+				leaf(tt, (u0 + u1) * 0.5f, (v0 + v1) * 0.5f, max_dim);
+				if (occl) return PATCH_BLOCKED;
 			}
 		} else {
 			const bool along_u = patch_ulen(cur[0]) > patch_vlen(cur[0]);
@@ -599,100 +536,160 @@ __device__ __forceinline__ bool patch_run(PatchCursor<NV, TSC>& pc, PatchStore<N
 #pragma unroll
 			for (int k = 0; k < TSC; ++k) patch_split(cur[k], first[k], along_u);
 			float smd, sh0, sh1, fmd, fh0, fh1;
-			const bool s_hit = patch_node_test<NV, TSC>(cur, t_nalpha, r, *max_t, &smd, &sh0, &sh1);
-			const bool f_hit = patch_node_test<NV, TSC>(first, t_nalpha, r, *max_t, &fmd, &fh0, &fh1);
-			dirs.set(depth, along_u);
+			const bool s_hit = patch_node_test<NV, TSC, CLEAN>(cur, t_nalpha, o, dinv, *max_t, &smd, &sh0, &sh1);
+			const bool f_hit = patch_node_test<NV, TSC, CLEAN>(first, t_nalpha, o, dinv, *max_t, &fmd, &fh0, &fh1);
 			const float mid = along_u ? (u0 + u1) * 0.5f : (v0 + v1) * 0.5f;
 			if (s_hit) {
-				path.set(depth, true);
-				pend.set(depth, f_hit);
+				++pc.depth;
 				if (f_hit) {
-					// the first half waits on the stack with its uv range
+					// the first half waits on the stack
 					const int q = pc.sp++;
 #pragma unroll
 					for (int k = 0; k < TSC; ++k) ps.pend[q][k] = first[k];
-					ps.penduv[q][0] = u0;
-					ps.penduv[q][1] = along_u ? mid : u1;
-					ps.penduv[q][2] = v0;
-					ps.penduv[q][3] = along_u ? v1 : mid;
+					ps.uv[q] = make_float4(u0, along_u ? mid : u1, v0, along_u ? v1 : mid);
+					ps.at[q] = make_int2(pc.depth, pc.seconds);
 				}
+				++pc.seconds;
 				if (along_u) u0 = mid; else v0 = mid;
 				max_dim = smd;
 				h0 = sh0;
 				h1 = sh1;
-				entered = true;
-			} else if (f_hit) {
-				path.set(depth, false);
+				continue;
+			}
+			if (f_hit) {
+				++pc.depth;
 #pragma unroll
 				for (int k = 0; k < TSC; ++k) cur[k] = first[k];
 				if (along_u) u1 = mid; else v1 = mid;
 				max_dim = fmd;
 				h0 = fh0;
 				h1 = fh1;
-				entered = true;
-			}
-			if (entered) {
-				++depth;
 				continue;
 			}
 		}
-		// resume at the deepest pending first half (the top of the stack)
-		// whose box is still hit
+		// resume at the last pending first half whose box is still hit
 		while (true) {
-			const int j = pend.highest_below(depth);
-			if (j < 0) return true;
-			pend.set(j, false);
-			path.set(j, false);
-			depth = j + 1;
-			path.truncate(depth);
-			dirs.truncate(depth);
-			pend.truncate(depth);
+			if (pc.sp == 0) return PATCH_DONE;
 			const int q = --pc.sp;
 #pragma unroll
 			for (int k = 0; k < TSC; ++k) cur[k] = ps.pend[q][k];
-			u0 = ps.penduv[q][0]; u1 = ps.penduv[q][1]; v0 = ps.penduv[q][2]; v1 = ps.penduv[q][3];
-			if (patch_node_test<NV, TSC>(cur, t_nalpha, r, *max_t, &max_dim, &h0, &h1)) break;
+			const float4 w = ps.uv[q];
+			u0 = w.x; u1 = w.y; v0 = w.z; v1 = w.w;
+			pc.depth = ps.at[q].x;
+			pc.seconds = ps.at[q].y;
+			if (patch_node_test<NV, TSC, CLEAN>(cur, t_nalpha, o, dinv, *max_t, &max_dim, &h0, &h1)) break;
 		}
 	}
 }
 
-// The whole bisection of one patch in one call, its state in the caller's
-// frame.  Returns true when a leaf was taken.
+// The leaf a whole bisection ended with.
+struct PatchHit {
+	float t, u, v, max_dim;
+};
+
+// The whole bisection of one patch in one call, with the reference's own
+// minima and maxima: rays or patches whose slab tests can meet NaN.  Not
+// inlined: next to no ray comes here.  Returns true when a leaf was taken.
 template <int NV, int TSC>
-__device__ bool patch_whole(const float* verts, float time, const LocalRay& r, const RayWidth& rw,
-                                            float* max_t, bool occl, float dice_rate, float min_upoly,
-                                            PatchHit* hit, unsigned* err) {
+static __device__ __noinline__ bool patch_whole(const float* verts, float time, V3 o, V3 dinv, const RayFlip& rw,
+                                                float max_t, bool occl, float dice_rate, float min_upoly,
+                                                PatchStore<NV, TSC>& ps, PatchHit* hit, unsigned* err) {
 	PatchCursor<NV, TSC> pc;
-	PatchStore<NV, TSC> ps;
-	if (!patch_begin<NV, TSC>(pc, verts, time, r, *max_t)) return false;
+	if (!patch_begin<NV, TSC, false>(pc, verts, time, o, dinv, max_t)) return false;
 	int units = 0x7fffffff;
-	patch_run<NV, TSC>(pc, ps, verts, r, rw, max_t, occl, dice_rate, min_upoly, hit, units, err);
-	return pc.found;
+	bool found = false;
+	unsigned e = 0;
+	patch_run<NV, TSC, false>(pc, ps, o, dinv, rw, &max_t, occl, dice_rate, min_upoly, units, &e,
+	                          [&](float t, float u, float v, float md) {
+		                          found = true;
+		                          *hit = PatchHit{t, u, v, md};
+	                          });
+	*err |= e;
+	return found && !(e & ERRF_BISECT);
 }
 
 // ---------------------------------------------------------------------
 // Whole-scene traversal
 // ---------------------------------------------------------------------
+// The closest hit as the traversal leaves it.  Object, kind, shader and
+// element id follow from the instance and where it was met: the placement,
+// or (place < 0) the path of instances from the root.
 struct HitRec {
 	float t;
 	float u, v, max_dim;
-	int obj;          // global object index, -1 = miss
-	int kind;
-	int shader;       // innermost bound shader, -1 = none
-	uint64_t id;
-	int depth;        // number of instances on the path
-	int path[PSY_MAX_LEVELS];  // global instance indices, root first
+	int inst;                  // global instance index, -1 = miss
+	int place;                 // its assembly's placement, -1 = scene without placements
+	int depth;                 // instances on the path (place < 0)
+	int path[PSY_MAX_LEVELS];  // global instance indices, root first (place < 0)
+	int obj, kind, shader;     // set by hit_surface
 };
 
-struct Level {
-	int asmb;
-	int stack_base;
-	int shader;
-	int inst;         // global instance that entered this level (-1 for the root)
-	uint64_t id;
-	int id_bits;      // id bits of this level's assembly
-	int inst_base;
-};
+// Element id of the hit (Intersection::id): the local instance index of
+// every level, pushed with that assembly's bits.
+__device__ __forceinline__ uint64_t hit_id(const DevScene& sc, const HitRec& h) {
+	if (h.place >= 0) {
+		const DevPlace& p = sc.places[h.place];
+		return id_push(p.id, (uint64_t)(h.inst - p.inst_base), p.id_bits);
+	}
+	uint64_t id = 0;
+	int asmb = 0;
+	for (int k = 0; k < h.depth; ++k) {
+		id = id_push(id, (uint64_t)(h.path[k] - sc.assemblies[asmb].inst_base), sc.assemblies[asmb].id_bits);
+		asmb = sc.instances[h.path[k]].data;
+	}
+	return id;
+}
+
+// The shader bound to the hit: the innermost one on the path.
+__device__ __forceinline__ int hit_shader(const DevScene& sc, const HitRec& h) {
+	const int own = sc.instances[h.inst].shader;
+	if (own >= 0) return own;
+	if (h.place >= 0) return sc.places[h.place].shader;
+	for (int k = h.depth - 2; k >= 0; --k) {
+		const int s = sc.instances[h.path[k]].shader;
+		if (s >= 0) return s;
+	}
+	return -1;
+}
+
+// The object hit, its kind and its shader.
+__device__ __forceinline__ void hit_surface(const DevScene& sc, HitRec* h) {
+	h->obj = sc.instances[h->inst].data;
+	h->kind = sc.objects[h->obj].kind;
+	h->shader = hit_shader(sc, *h);
+}
+
+// Transform from world space into the hit object's space at the ray time
+// (the Intersection::space of the reference).  Returns false when the path
+// carries no transform (identity).
+template <unsigned F>
+__device__ bool hit_space(const DevScene& sc, const HitRec& rec, float time, M44* out, unsigned* err) {
+	if (!(F & FEAT_XFORM)) return false;
+	Frame f{nullptr, 0};
+	FrameBuf buf[2];
+	int b = 0;
+	auto merge = [&](const DevInstance& inst) {
+		if (inst.xform_count == 0) return true;
+		f = frame_merge(f, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &buf[b]);
+		b ^= 1;
+		if (f.count < 0) {
+			*err |= ERRF_MOTION;
+			return false;
+		}
+		return true;
+	};
+	if (rec.place >= 0) {
+		const DevPlace& p = sc.places[rec.place];
+		f = Frame{sc.place_frames + (size_t)p.frame * 16, p.frame_count};
+		if (!merge(sc.instances[rec.inst])) return false;
+	} else {
+		for (int k = 0; k < rec.depth; ++k)
+			if (!merge(sc.instances[rec.path[k]])) return false;
+	}
+	if (f.count == 0) return false;
+	*out = frame_at(f, time);
+	return true;
+}
 
 // Patch kind of a bisection in progress: bilinear or bicubic, one or two
 // time samples.
@@ -702,540 +699,532 @@ enum : int { PM_NONE = 0, PM_BILINEAR1, PM_BILINEAR2, PM_BICUBIC1, PM_BICUBIC2 }
 template <unsigned F>
 struct PatchBuf {
 	static constexpr int TS = (F & FEAT_PATCH_MOTION) ? 2 : 1;
-	static constexpr size_t b4 = (F & FEAT_BILINEAR) ? sizeof(PatchWork<4, TS>) : 0;
-	static constexpr size_t b16 = (F & FEAT_BICUBIC) ? sizeof(PatchWork<16, TS>) : 0;
+	template <int NV>
+	struct Work {
+		PatchCursor<NV, TS> c;
+		PatchStore<NV, TS> st;
+	};
+	static constexpr size_t b4 = (F & FEAT_BILINEAR) ? sizeof(Work<4>) : 0;
+	static constexpr size_t b16 = (F & FEAT_BICUBIC) ? sizeof(Work<16>) : 0;
 	static constexpr size_t m = b4 > b16 ? b4 : b16;
 	static constexpr size_t bytes = m > 16 ? m : 16;
 };
 
-// Traversal state of one ray.  trace_init sets it up.  A lane that runs
-// its ray alone calls trace_step (to the next object leaf and its test)
-// until it returns false; the wave kernels advance it in pieces instead
-// (walk_nodes, leaf_visit, patch_step, each returning false once the ray
-// is finished).  rec and err then hold the result.  Kernels can refill a
-// lane with a new ray between pieces.
-template <unsigned F>
-struct TraceState {
-	WorldRayD wr;
-	float max_t;
-	unsigned err;
-	HitRec rec;
-	Level lv[PSY_MAX_LEVELS];
-	Frame frames[PSY_MAX_LEVELS];   // merged frames of transformed levels
-	int lvl_frame[PSY_MAX_LEVELS];  // frame used by each level, -1 = none
-	LocalRay lvr[PSY_MAX_LEVELS];   // ray of each enclosing level, kept while a transformed child is traversed
-	int node_stack[PSY_NODE_STACK];
-	int nsp, L;
-	int leaf;                       // leaf popped by walk_nodes, for leaf_visit
-	LocalRay r;                     // the ray in the current level's space
-	RayWidth rw;                    // width parameters of r, valid when rw_ok
-	bool rw_ok;
-	// a patch leaf whose bisection is in progress (pmode != PM_NONE): its
-	// vertices, ray and widths, the hit record's fields, the bisection
-	int pmode;
-	int p_obj, p_kind, p_shader, p_gi;
-	uint64_t p_id;
-	const float* pverts;
-	LocalRay pr;
-	RayWidth prw;
-	PatchHit ph;
-	alignas(16) unsigned char pbuf[PatchBuf<F>::bytes];
-	template <int NV, int TSC>
-	__device__ __forceinline__ PatchWork<NV, TSC>& work() {
-		static_assert(sizeof(PatchWork<NV, TSC>) <= sizeof(pbuf), "patch work buffer");
-		return *reinterpret_cast<PatchWork<NV, TSC>*>(pbuf);
-	}
+// References beyond those of the tree: the end of a level on the stack
+// (REF_LEVEL, or REF_LEVEL_RAY when the enclosing level's ray is to be
+// restored), and no reference (take the next one from the stack).
+static constexpr int REF_LEVEL = (int)0xf0000000;
+static constexpr int REF_LEVEL_RAY = (int)0xf0000001;
+static constexpr int REF_NONE = REF_EMPTY;
+
+enum : unsigned {
+	RAY_OCCL = 1u,   // occlusion ray: ends at the first hit
+	RAY_ODD = 2u,    // a slab test of the ray in its current space can meet NaN or inf - inf
+	RAY_HIT = 4u,    // a hit was recorded
+	RAY_WIDTH = 8u   // the width parameters are those of the current space
 };
 
-// F is a mask of FEAT_* scene features; code for absent features is not
-// compiled into the variant, which keeps the flat-scene kernels small.
-template <unsigned F>
-__device__ __forceinline__ void trace_init(const DevScene& sc, TraceState<F>& s, const WorldRayD& wr) {
-	s.wr = wr;
-	s.err = 0;
-	s.max_t = wr.occl ? 1.0f : INFINITY;
-	s.rec.obj = -1;
-	s.rec.t = INFINITY;
-	s.rec.depth = 0;
-	s.nsp = 0;
-	s.L = 0;
-	s.lv[0].asmb = 0;
-	s.lv[0].stack_base = 0;
-	s.lv[0].shader = -1;
-	s.lv[0].inst = -1;
-	s.lv[0].id = 0;
-	s.lv[0].id_bits = sc.assemblies[0].id_bits;
-	s.lv[0].inst_base = sc.assemblies[0].inst_base;
-	s.lvl_frame[0] = -1;
-	s.r = make_local(wr);
-	s.rw_ok = false;
-	s.pmode = PM_NONE;
-	const int root = sc.assemblies[0].root;
-	if (root != REF_EMPTY) s.node_stack[s.nsp++] = root;
-}
+// Traversal state of one ray.  IO gives the world ray (origin, direction,
+// differentials: read again where an instance or a patch needs them) and
+// takes the hits.  The members above the line are meant for registers, the
+// ones below live in local memory.
+template <unsigned F, class IO>
+struct Trav {
+	V3 o, d, dinv;      // the ray in the current space
+	float max_t, time;
+	int cur;            // next reference
+	int sp, L;          // stack entries, assembly levels entered
+	int place;          // current placement (scenes with placements)
+	int pmode;          // bisection in progress (PM_*)
+	unsigned flags, err;
+	IO io;
+	// ---
+	uint2 stack[PSY_NODE_STACK + PSY_MAX_LEVELS];  // reference, distance of its box (as bits)
+	RayFlip rw;                                    // width parameters of the current space (RAY_WIDTH)
+	float lvr[PSY_MAX_LEVELS][9];                  // ray of each enclosing level (REF_LEVEL_RAY)
+	// scenes without placements: the entered instances and merged frames
+	int lv_inst[PSY_MAX_LEVELS], lv_frame[PSY_MAX_LEVELS], lv_count[PSY_MAX_LEVELS];
+	FrameBuf frames[PSY_MAX_LEVELS];
+	// the bisection in progress: its instance, ray and widths, its cursor and stack
+	int p_inst;
+	V3 p_o, p_dinv;
+	RayFlip p_rw;
+	alignas(16) unsigned char pbuf[PatchBuf<F>::bytes];
 
-// Records the hit on an object of the current level (Intersection fields
-// the traversal knows).  Returns false when the ray is finished: an
-// occlusion ray stops at its first hit.
-template <unsigned F>
-__device__ __forceinline__ bool trace_record(TraceState<F>& s, int obj, int kind, uint64_t id, int shader, int gi,
-                                             const PatchHit& ph) {
-	HitRec& rec = s.rec;
-	rec.obj = obj;
-	rec.kind = kind;
-	rec.id = id;
-	rec.shader = shader;
-	if (s.wr.occl) return false;
-	rec.t = ph.t;
-	rec.u = ph.u;
-	rec.v = ph.v;
-	rec.max_dim = ph.max_dim;
-	const int L = s.L;
-	rec.depth = L + 1;
-	for (int k = 1; k <= L; ++k) rec.path[k - 1] = s.lv[k].inst;
-	rec.path[L] = gi;
-	return true;
-}
+	static constexpr bool NESTED = (F & FEAT_NESTED) != 0;
+	static constexpr bool XFORM = (F & FEAT_XFORM) != 0;
+	static constexpr int TS = PatchBuf<F>::TS;
 
-// An inner node: tests the child boxes (BBox4::intersect_ray,
-// basics/bbox.hpp:566-595) and pushes the hit children, nearest on top.
-// Returns false when the node stack overflows (the ray ends with an error).
-template <unsigned F>
-__device__ __forceinline__ bool node_visit(const DevScene& sc, TraceState<F>& s, int ref) {
-	const WorldRayD& wr = s.wr;
-	const DevNode* nd = sc.nodes + ref;
-	float b[24];
-	load_box4(reinterpret_cast<const float4*>(nd->b), b);
-	const int4 ch = __ldg(reinterpret_cast<const int4*>(nd->child));
-	const int4 meta = __ldg(reinterpret_cast<const int4*>(&nd->nchild));
-	const int nch = meta.x;
-	const int ts = meta.y;
-	if (ts > 1) {
-		// motion: lerp the boxes of the two time samples around the ray
-		// time (sample 0 is in the node, later ones in node_extra)
-		const SeqPos sp = seq_pos(wr.time, ts);
-		auto extra = [&](int k) {
-			return reinterpret_cast<const float4*>(sc.node_extra + (size_t)(meta.z + k - 1) * 24);
-		};
-		if (sp.single) {
-			if (sp.i0 != 0) load_box4(extra(sp.i0), b);
-		} else {
-			float e1[24];
-			load_box4(extra(sp.i0 + 1), e1);
-			if (sp.i0 != 0) load_box4(extra(sp.i0), b);
-			const float ia = one_minus(sp.nalpha);
-#pragma unroll
-			for (int i = 0; i < 24; ++i) b[i] = (b[i] * ia) + (e1[i] * sp.nalpha);
+	template <int NV>
+	__device__ __forceinline__ typename PatchBuf<F>::template Work<NV>& work() {
+		return *reinterpret_cast<typename PatchBuf<F>::template Work<NV>*>(pbuf);
+	}
+
+	// the same room as that of a patch with one time sample
+	typedef PatchBuf<F & ~FEAT_PATCH_MOTION> Still;
+	template <int NV>
+	__device__ __forceinline__ typename Still::template Work<NV>& still_work() {
+		return *reinterpret_cast<typename Still::template Work<NV>*>(pbuf);
+	}
+
+	__device__ __forceinline__ static bool odd_ray(V3 o, V3 d, V3 dinv) {
+		// zero direction components (infinite reciprocals), infinities and NaN
+		const float s = (fabsf(o.x) + fabsf(o.y) + fabsf(o.z)) + (fabsf(d.x) + fabsf(d.y) + fabsf(d.z));
+		const float r = fmaxf(fmaxf(fabsf(dinv.x), fabsf(dinv.y)), fabsf(dinv.z));
+		return !(s < INFINITY) || !(r < INFINITY);
+	}
+
+	__device__ __forceinline__ void set_ray(V3 no, V3 nd) {
+		o = no;
+		d = nd;
+		dinv = recip3(nd);
+		flags &= ~(RAY_ODD | RAY_WIDTH);
+		if (odd_ray(o, d, dinv)) flags |= RAY_ODD;
+	}
+
+	__device__ __forceinline__ void init(const DevScene& sc, V3 wo, V3 wd, float t, bool occl) {
+		flags = occl ? RAY_OCCL : 0u;
+		set_ray(wo, wd);
+		time = t;
+		max_t = occl ? 1.0f : INFINITY;
+		cur = __ldg(sc.asmb_root);
+		sp = 0;
+		L = 0;
+		place = 0;
+		pmode = PM_NONE;
+		err = 0;
+		if (NESTED && !sc.places) {
+			place = -1;
+			lv_frame[0] = -1;
+			lv_count[0] = 0;
 		}
 	}
-	// slab tests of the four children; every array index below is a
-	// compile-time constant so the node stays in registers
-	const bool ds0 = s.r.dinv.x < 0.0f, ds1 = s.r.dinv.y < 0.0f, ds2 = s.r.dinv.z < 0.0f;
-	const int chv[4] = {ch.x, ch.y, ch.z, ch.w};
-	float tk[4];
-	int ck[4], sk[4];
-	int nhit = 0;
-#pragma unroll
-	for (int c = 0; c < 4; ++c) {
-		const float x0 = b[0 * 4 + c], x1 = b[1 * 4 + c];
-		const float y0 = b[2 * 4 + c], y1 = b[3 * 4 + c];
-		const float z0 = b[4 * 4 + c], z1 = b[5 * 4 + c];
-		const float xlo = ((ds0 ? x1 : x0) - s.r.o.x) * s.r.dinv.x;
-		const float xhi = ((ds0 ? x0 : x1) - s.r.o.x) * s.r.dinv.x;
-		const float ylo = ((ds1 ? y1 : y0) - s.r.o.y) * s.r.dinv.y;
-		const float yhi = ((ds1 ? y0 : y1) - s.r.o.y) * s.r.dinv.y;
-		const float zlo = ((ds2 ? z1 : z0) - s.r.o.z) * s.r.dinv.z;
-		const float zhi = ((ds2 ? z0 : z1) - s.r.o.z) * s.r.dinv.z;
-		const float mins = vmax(vmax(xlo, ylo), vmax(zlo, 0.0f));
-		const float maxs = vmax(vmin(vmin(xhi, yhi), zhi), -INFINITY) * BBOX_MAXT_ADJUST;
-		const bool h = c < nch && mins < s.max_t && mins <= maxs;
-		// a hit has mins < max_t <= inf, so inf marks the misses
-		tk[c] = h ? mins : INFINITY;
-		ck[c] = chv[c];
-		sk[c] = c;
-		nhit += h ? 1 : 0;
-	}
-	// nearest first, ties in child order (a stable sort by distance)
-	auto cswap = [&](int a, int bb) {
-		if (tk[bb] < tk[a] || (tk[bb] == tk[a] && sk[bb] < sk[a])) {
-			const float t = tk[a]; tk[a] = tk[bb]; tk[bb] = t;
-			const int c = ck[a]; ck[a] = ck[bb]; ck[bb] = c;
-			const int q = sk[a]; sk[a] = sk[bb]; sk[bb] = q;
-		}
-	};
-	if (s.nsp + nhit > PSY_NODE_STACK) {
-		s.err |= ERRF_STACK;
-		return false;
-	}
-	if (wr.occl) {
-		// an occlusion ray stops at any hit, so the order it meets the
-		// children in does not matter: push the hit ones unsorted
-#pragma unroll
-		for (int c = 3; c >= 0; --c)
-			if (tk[c] != INFINITY) s.node_stack[s.nsp++] = ck[c];
-		return true;
-	}
-	cswap(0, 1);
-	cswap(2, 3);
-	cswap(0, 2);
-	cswap(1, 3);
-	cswap(1, 2);
-	if (nhit > 3) s.node_stack[s.nsp++] = ck[3];
-	if (nhit > 2) s.node_stack[s.nsp++] = ck[2];
-	if (nhit > 1) s.node_stack[s.nsp++] = ck[1];
-	if (nhit > 0) s.node_stack[s.nsp++] = ck[0];
-	return true;
-}
 
-// Leaves the finished levels, restoring the ray of the enclosing level.
-template <unsigned F>
-__device__ __forceinline__ void leave_levels(TraceState<F>& s) {
-	constexpr bool NESTED = (F & FEAT_NESTED) != 0;
-	while (NESTED && s.L > 0 && s.nsp == s.lv[s.L].stack_base) {
-		const bool changed = s.lvl_frame[s.L] != s.lvl_frame[s.L - 1];
-		--s.L;
-		if (changed) {
-			s.r = s.lvr[s.L];
-			s.rw_ok = false;
+	// The merged motion frame of the current level.
+	__device__ __forceinline__ Frame level_frame(const DevScene& sc) const {
+		if (place >= 0) {
+			const int4 p = __ldg(reinterpret_cast<const int4*>(sc.places + place));
+			return Frame{sc.place_frames + (size_t)p.z * 16, p.w};
 		}
+		return Frame{lv_count[L] ? frames[lv_frame[L]].m : nullptr, lv_count[L]};
 	}
-}
 
-// Enters the assembly of instance `inst` (global index gi, element id
-// `id`, inherited shader): merges its transforms into the level's frame,
-// moves the ray into its space and pushes its root.  Returns false when the
-// node stack overflows.
-template <unsigned F>
-__device__ __forceinline__ bool enter_assembly(const DevScene& sc, TraceState<F>& s, const DevInstance& inst, int gi,
-                                               uint64_t id, int shader) {
-	constexpr bool XFORM = (F & FEAT_XFORM) != 0;
-	const WorldRayD& wr = s.wr;
-	Frame none;
-	none.count = 0;
-	const int L = s.L;
-	const Frame& parent = s.lvl_frame[L] >= 0 ? s.frames[s.lvl_frame[L]] : none;
-	if (L + 1 >= PSY_MAX_LEVELS) {
-		s.err |= ERRF_LEVELS;
-		return true;
+	// Records a hit on instance gi.  Returns false when the ray is finished
+	// (an occlusion ray).
+	__device__ __forceinline__ bool record(int gi, float t, float u, float v, float md) {
+		flags |= RAY_HIT;
+		io.hit(*this, gi, t, u, v, md);
+		return (flags & RAY_OCCL) == 0;
 	}
-	const DevAssembly as = sc.assemblies[inst.data];
-	if (as.root == REF_EMPTY) return true;
-	if (XFORM && inst.xform_count > 0) {
-		if (!frame_merge(parent, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &s.frames[L + 1])) {
-			s.err |= ERRF_MOTION;
-			return true;
-		}
-		s.lvl_frame[L + 1] = L + 1;
-		s.lvr[L] = s.r;
-		s.r = make_local_x(wr, frame_at_index_lerp(s.frames[L + 1], wr.time));
-		s.rw_ok = false;
-	} else {
-		s.lvl_frame[L + 1] = s.lvl_frame[L];
-	}
-	s.L = L + 1;
-	Level& nl = s.lv[L + 1];
-	nl.asmb = inst.data;
-	nl.stack_base = s.nsp;
-	nl.shader = shader;
-	nl.inst = gi;
-	nl.id = id;
-	nl.id_bits = as.id_bits;
-	nl.inst_base = as.inst_base;
-	if (s.nsp + 1 > PSY_NODE_STACK) {
-		s.err |= ERRF_STACK;
-		return false;
-	}
-	s.node_stack[s.nsp++] = as.root;
-	return true;
-}
 
-// The test of object instance `inst` of the current level (global index
-// gi, element id `id`, bound shader).  With RESUME a patch whose box the
-// ray hits only starts its bisection (patch_step carries it on); without,
-// the bisection runs here.  Returns false when the ray is finished (an
-// occlusion ray's hit).
-template <unsigned F, bool RESUME>
-__device__ __forceinline__ bool object_test(const DevScene& sc, TraceState<F>& s, const DevInstance& inst, int gi,
-                                            uint64_t id, int shader) {
-	constexpr bool XFORM = (F & FEAT_XFORM) != 0;
-	const WorldRayD& wr = s.wr;
-	Frame none;
-	none.count = 0;
-	const int L = s.L;
-	LocalRay lr = s.r;
-	M44 om;  // the object's own transform at the ray time
-	const bool oxf = XFORM && inst.xform_count > 0;
-	if (oxf) {
-		const Frame& parent = s.lvl_frame[L] >= 0 ? s.frames[s.lvl_frame[L]] : none;
-		Frame nf;
-		if (!frame_merge(parent, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &nf)) {
-			s.err |= ERRF_MOTION;
-			return true;
-		}
-		om = frame_at_index_lerp(nf, wr.time);
-		lr = make_local_x(wr, om);
-	}
-	const DevObject ob = sc.objects[inst.data];
-	// width parameters for patches: the object's own, or the level's (cached)
-	auto width = [&]() -> RayWidth {
-		if (oxf) return ray_width_of(wr, lr, &om);
-		if (!s.rw_ok) {
-			if (XFORM && s.lvl_frame[L] >= 0) {
-				const M44 lm = frame_at_index_lerp(s.frames[s.lvl_frame[L]], wr.time);
-				s.rw = ray_width_of(wr, s.r, &lm);
-			} else {
-				s.rw = ray_width_of(wr, s.r, nullptr);
+	// Takes the next reference from the stack into `cur`, leaving finished
+	// levels on the way.  An inner node whose box begins beyond max_t is
+	// passed over: none of its children could be hit.  Returns false when the
+	// stack is empty (the ray is finished).
+	__device__ __forceinline__ bool pop(const DevScene& sc) {
+		while (cur == REF_NONE) {
+			if (sp == 0) return false;
+			const uint2 e = stack[--sp];
+			const int ref = (int)e.x;
+			if (ref >= 0) {
+				if (__uint_as_float(e.y) < max_t) cur = ref;
+				continue;
 			}
-			s.rw_ok = true;
-		}
-		return s.rw;
-	};
-	// a patch with RESUME: test the root box here, bisect in patch_step
-	auto begin_patch = [&](const float* v) {
-		int pm = PM_NONE;
-		if constexpr ((F & FEAT_BILINEAR) != 0) {
-			if (ob.kind == OBJ_BILINEAR) {
-				if constexpr ((F & FEAT_PATCH_MOTION) != 0) {
-					if (ob.n0 != 1)
-						pm = patch_begin<4, 2>(s.template work<4, 2>().c, v, wr.time, lr, s.max_t) ? PM_BILINEAR2 : -1;
+			if (NESTED && ref >= REF_LEVEL && ref <= REF_LEVEL_RAY) {
+				--L;
+				if (place >= 0) place = (int)e.y;
+				if (XFORM && ref == REF_LEVEL_RAY) {
+					o = V3(lvr[L][0], lvr[L][1], lvr[L][2]);
+					d = V3(lvr[L][3], lvr[L][4], lvr[L][5]);
+					dinv = V3(lvr[L][6], lvr[L][7], lvr[L][8]);
+					flags &= ~(RAY_ODD | RAY_WIDTH);
+					if (odd_ray(o, d, dinv)) flags |= RAY_ODD;
 				}
-				if (pm == PM_NONE) pm = patch_begin<4, 1>(s.template work<4, 1>().c, v, wr.time, lr, s.max_t) ? PM_BILINEAR1 : -1;
+				continue;
 			}
+			cur = ref;
+		}
+		return true;
+	}
+
+	// The distances of a node's four children in the reference's own order of
+	// operations (BBox4::intersect_ray, basics/bbox.hpp:566-595, SSE min/max
+	// semantics), infinity for a miss: rays and boxes with infinities or NaN.
+	static __device__ __noinline__ float4 odd_node(const DevScene& sc, int ref, V3 o, V3 dinv, float time, float max_t) {
+		const DevNode* nd = sc.nodes + (ref & REF_NODE_MASK);
+		float b[24];
+		for (int i = 0; i < 24; ++i) b[i] = nd->b[i];
+		if (nd->ts > 1) {
+			const SeqPos q = seq_pos(time, nd->ts);
+			const float* x0 = q.i0 ? sc.node_extra + (size_t)(nd->extra + q.i0 - 1) * 24 : nd->b;
+			const float* x1 = q.single ? x0 : sc.node_extra + (size_t)(nd->extra + q.i0) * 24;
+			const float ia = one_minus(q.nalpha);
+			for (int i = 0; i < 24; ++i) b[i] = q.single ? x0[i] : (x0[i] * ia) + (x1[i] * q.nalpha);
+		}
+		const bool ds0 = dinv.x < 0.0f, ds1 = dinv.y < 0.0f, ds2 = dinv.z < 0.0f;
+		float tk[4];
+		for (int c = 0; c < 4; ++c) {
+			const float xlo = ((ds0 ? b[4 + c] : b[c]) - o.x) * dinv.x;
+			const float xhi = ((ds0 ? b[c] : b[4 + c]) - o.x) * dinv.x;
+			const float ylo = ((ds1 ? b[12 + c] : b[8 + c]) - o.y) * dinv.y;
+			const float yhi = ((ds1 ? b[8 + c] : b[12 + c]) - o.y) * dinv.y;
+			const float zlo = ((ds2 ? b[20 + c] : b[16 + c]) - o.z) * dinv.z;
+			const float zhi = ((ds2 ? b[16 + c] : b[20 + c]) - o.z) * dinv.z;
+			const float mins = vmax(vmax(xlo, ylo), vmax(zlo, 0.0f));
+			const float maxs = vmax(vmin(vmin(xhi, yhi), zhi), -INFINITY) * BBOX_MAXT_ADJUST;
+			tk[c] = c < nd->nchild && mins < max_t && mins <= maxs ? mins : INFINITY;
+		}
+		return make_float4(tk[0], tk[1], tk[2], tk[3]);
+	}
+
+	// An inner node (cur): tests the child boxes, leaves the nearest hit child
+	// in `cur` (REF_NONE when none is hit) and the others on the stack,
+	// nearest on top, ties in child order.  Returns false when the node stack
+	// overflows (the ray ends with an error).
+	__device__ __forceinline__ bool node_step(const DevScene& sc) {
+		const int ref = cur;
+		const DevNode* nd = sc.nodes + (ref & REF_NODE_MASK);
+		float t0, t1, t2, t3;
+		if ((flags & RAY_ODD) || (ref & REF_NODE_ODD)) {
+			const float4 t = odd_node(sc, ref, o, dinv, time, max_t);
+			t0 = t.x; t1 = t.y; t2 = t.z; t3 = t.w;
+		} else {
+			// the near and far planes by the direction's signs
+			const char* base = reinterpret_cast<const char*>(nd);
+			const int sx = dinv.x < 0.0f ? 16 : 0, sy = dinv.y < 0.0f ? 16 : 0, sz = dinv.z < 0.0f ? 16 : 0;
+			auto row = [](const char* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
+			float4 xn = row(base + sx), xf = row(base + 16 - sx);
+			float4 yn = row(base + 32 + sy), yf = row(base + 48 - sy);
+			float4 zn = row(base + 64 + sz), zf = row(base + 80 - sz);
+			if (ref & REF_NODE_MOVING) {
+				// lerp the boxes of the two time samples around the ray time
+				// (sample 0 is in the node, later ones in node_extra)
+				const int4 meta = __ldg(reinterpret_cast<const int4*>(&nd->nchild));
+				const SeqPos q = seq_pos(time, meta.y);
+				auto extra = [&](int k) { return reinterpret_cast<const char*>(sc.node_extra + (size_t)(meta.z + k - 1) * 24); };
+				if (q.i0 != 0) {
+					const char* e = extra(q.i0);
+					xn = row(e + sx); xf = row(e + 16 - sx);
+					yn = row(e + 32 + sy); yf = row(e + 48 - sy);
+					zn = row(e + 64 + sz); zf = row(e + 80 - sz);
+				}
+				if (!q.single) {
+					const char* e = extra(q.i0 + 1);
+					const float al = q.nalpha, ia = one_minus(q.nalpha);
+					auto lerp4 = [&](float4 a, float4 b) {
+						return make_float4((a.x * ia) + (b.x * al), (a.y * ia) + (b.y * al), (a.z * ia) + (b.z * al),
+						                   (a.w * ia) + (b.w * al));
+					};
+					xn = lerp4(xn, row(e + sx)); xf = lerp4(xf, row(e + 16 - sx));
+					yn = lerp4(yn, row(e + 32 + sy)); yf = lerp4(yf, row(e + 48 - sy));
+					zn = lerp4(zn, row(e + 64 + sz)); zf = lerp4(zf, row(e + 80 - sz));
+				}
+			}
+			auto slab = [&](float nx, float fx, float ny, float fy, float nz, float fz) {
+				const float mins = fmaxf(fmaxf((nx - o.x) * dinv.x, (ny - o.y) * dinv.y), fmaxf((nz - o.z) * dinv.z, 0.0f));
+				const float maxs = fminf(fminf((fx - o.x) * dinv.x, (fy - o.y) * dinv.y), (fz - o.z) * dinv.z) * BBOX_MAXT_ADJUST;
+				return mins < max_t && mins <= maxs ? mins : INFINITY;
+			};
+			// a hit has mins < max_t <= inf, so inf marks the misses (absent
+			// children have inverted infinite boxes)
+			t0 = slab(xn.x, xf.x, yn.x, yf.x, zn.x, zf.x);
+			t1 = slab(xn.y, xf.y, yn.y, yf.y, zn.y, zf.y);
+			t2 = slab(xn.z, xf.z, yn.z, yf.z, zn.z, zf.z);
+			t3 = slab(xn.w, xf.w, yn.w, yf.w, zn.w, zf.w);
+		}
+		const int4 ch = __ldg(reinterpret_cast<const int4*>(nd->child));
+		const bool h0 = t0 < INFINITY, h1 = t1 < INFINITY, h2 = t2 < INFINITY, h3 = t3 < INFINITY;
+		if (flags & RAY_OCCL) {
+			// any blocker ends the ray: the order is that of the children, and
+			// max_t does not shrink
+			t0 = h0 ? 0.0f : t0;
+			t1 = h1 ? 0.0f : t1;
+			t2 = h2 ? 0.0f : t2;
+			t3 = h3 ? 0.0f : t3;
+		}
+		const int nhit = (h0 ? 1 : 0) + (h1 ? 1 : 0) + (h2 ? 1 : 0) + (h3 ? 1 : 0);
+		if (sp - L + nhit > PSY_NODE_STACK) {
+			err |= ERRF_STACK;
+			return false;
+		}
+		// each child's place in the order: how many come before it
+		const int l01 = t1 < t0, l02 = t2 < t0, l03 = t3 < t0, l12 = t2 < t1, l13 = t3 < t1, l23 = t3 < t2;
+		const int r0 = l01 + l02 + l03, r1 = 1 - l01 + l12 + l13, r2 = 2 - l02 - l12 + l23, r3 = 3 - l03 - l13 - l23;
+		const int top = sp + nhit - 1;
+		int next = REF_NONE;
+		auto put = [&](bool h, int r, int ref_c, float t) {
+			if (!h) return;
+			if (r == 0) next = ref_c;
+			else stack[top - r] = make_uint2((unsigned)ref_c, __float_as_uint(t));
+		};
+		put(h0, r0, ch.x, t0);
+		put(h1, r1, ch.y, t1);
+		put(h2, r2, ch.z, t2);
+		put(h3, r3, ch.w, t3);
+		if (nhit > 0) sp = top;
+		cur = next;
+		return true;
+	}
+
+	// A leaf (cur) of class LEAF_ENTER: enters the assembly of the instance,
+	// moves the ray into its space and goes to its root.  Returns false when
+	// the node stack overflows.
+	__device__ __forceinline__ bool enter(const DevScene& sc) {
+		const int gi = cur & REF_LEAF_MASK;
+		const int4 m = __ldg(reinterpret_cast<const int4*>(&sc.leaves[gi].data));  // rank, transforms, assembly
+		cur = REF_NONE;
+		Frame f;
+		int child = -1, root;
+		if (place >= 0) {
+			child = __ldg(&sc.places[place].child_base) + m.x;
+			const int4 p = __ldg(reinterpret_cast<const int4*>(sc.places + child));
+			root = p.x;
+			f = Frame{sc.place_frames + (size_t)p.z * 16, p.w};
+			if (root != REF_EMPTY && f.count < 0) {
+				err |= ERRF_MOTION;
+				return true;
+			}
+		} else {
+			root = __ldg(sc.asmb_root + m.z);
+			if (root != REF_EMPTY) {
+				const Frame parent = level_frame(sc);
+				f = parent;
+				lv_inst[L + 1] = gi;
+				lv_frame[L + 1] = lv_frame[L];
+				if (XFORM && m.y > 0) {
+					const DevInstance inst = sc.instances[gi];
+					f = frame_merge(parent, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &frames[L + 1]);
+					if (f.count < 0) {
+						err |= ERRF_MOTION;
+						return true;
+					}
+					lv_frame[L + 1] = L + 1;
+				}
+				lv_count[L + 1] = f.count;
+			}
+		}
+		if (root == REF_EMPTY) return true;
+		if (sp - L + 1 > PSY_NODE_STACK) {
+			err |= ERRF_STACK;
+			return false;
+		}
+		const bool moved = XFORM && m.y > 0;
+		stack[sp++] = make_uint2((unsigned)(moved ? REF_LEVEL_RAY : REF_LEVEL), (unsigned)place);
+		if (moved) {
+			lvr[L][0] = o.x; lvr[L][1] = o.y; lvr[L][2] = o.z;
+			lvr[L][3] = d.x; lvr[L][4] = d.y; lvr[L][5] = d.z;
+			lvr[L][6] = dinv.x; lvr[L][7] = dinv.y; lvr[L][8] = dinv.z;
+			const M44 t = frame_at(f, time);
+			set_ray(pos_to(t, io.origin()), dir_to(t, io.direction()));
+		}
+		++L;
+		place = child;
+		cur = root;
+		return true;
+	}
+
+	// The transform of an object instance that carries its own, at the ray
+	// time.  Returns false when it needs more motion samples than supported.
+	__device__ __forceinline__ bool object_frame(const DevScene& sc, const DevInstance& inst, M44* om) {
+		FrameBuf buf;
+		const Frame f = frame_merge(level_frame(sc), sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &buf);
+		if (f.count < 0) {
+			err |= ERRF_MOTION;
+			return false;
+		}
+		*om = frame_at(f, time);
+		return true;
+	}
+
+	// A leaf of class LEAF_SPHERE: a sphere or sphere light at rest in its
+	// assembly's space, whole in its leaf record.
+	__device__ __forceinline__ bool sphere_leaf(const DevScene& sc) {
+		const int gi = cur & REF_LEAF_MASK;
+		cur = REF_NONE;
+		const float4 g = __ldg(reinterpret_cast<const float4*>(sc.leaves[gi].sphere));
+		const float t = sphere_t(o, d, V3(g.x, g.y, g.z), g.w, max_t);
+		if (!(t >= 0.0f)) return true;
+		if (!(flags & RAY_OCCL)) max_t = t;
+		return record(gi, t, 0.0f, 0.0f, 0.0f);
+	}
+
+	// A leaf of class LEAF_SIMPLE: moving or transformed spheres and sphere
+	// lights, rectangle lights.
+	__device__ __forceinline__ bool simple_leaf(const DevScene& sc) {
+		const int gi = cur & REF_LEAF_MASK;
+		cur = REF_NONE;
+		const DevInstance inst = sc.instances[gi];
+		const DevObject ob = sc.objects[inst.data];
+		V3 lo = o, ld = d, li = dinv;
+		if (XFORM && inst.xform_count > 0) {
+			M44 om;
+			if (!object_frame(sc, inst, &om)) return true;
+			lo = pos_to(om, io.origin());
+			ld = dir_to(om, io.direction());
+			li = recip3(ld);
+		}
+		float t;
+		if (ob.kind == OBJ_RECT_LIGHT) {
+			float dx, dy;
+			rect_light_at(sc, ob, time, &dx, &dy, nullptr);
+			t = rect_light_t(lo, ld, li, dx, dy, max_t);
+		} else {
+			V3 cent;
+			float radi;
+			float col[3];
+			if (ob.kind == OBJ_SPHERE) sphere_at(sc, ob, time, &cent, &radi);
+			else light_at(sc, ob, time, &cent, &radi, col);
+			t = sphere_t(lo, ld, cent, radi, max_t);
+		}
+		if (!(t >= 0.0f)) return true;
+		if (!(flags & RAY_OCCL)) max_t = t;
+		return record(gi, t, 0.0f, 0.0f, 0.0f);
+	}
+
+	// Width parameters for the patch of instance at transform `om` (oxf: its
+	// own; else the level's, kept for the next patch in the same space).
+	__device__ __forceinline__ RayFlip widths(const DevScene& sc, bool oxf, M44& om, V3 lo, V3 ld) {
+		if (!oxf && (flags & RAY_WIDTH)) return rw;
+		V3 odx, ody, ddx, ddy;
+		io.differentials(&odx, &ody, &ddx, &ddy);
+		bool xf = oxf;
+		if (XFORM && !oxf) {
+			const Frame f = level_frame(sc);
+			if (f.count > 0) {
+				om = frame_at(f, time);
+				xf = true;
+			}
+		}
+		if (xf) {
+			odx = dir_to(om, odx);
+			ody = dir_to(om, ody);
+			ddx = dir_to(om, ddx);
+			ddy = dir_to(om, ddy);
+		}
+		const RayFlip w = ray_flip(ray_width_params(lo, ld, odx, ody, ddx, ddy));
+		if (!oxf) {
+			rw = w;
+			flags |= RAY_WIDTH;
+		}
+		return w;
+	}
+
+	// A leaf of class LEAF_PATCH.  WHOLE: the bisection runs here, to its end.
+	// Otherwise the patch's box is tested and its bisection set up (pmode) for
+	// patch_step to carry on.  Rays and patches whose tests can meet NaN are
+	// bisected whole in either case.  Returns false when the ray is finished.
+	template <bool WHOLE>
+	__device__ __forceinline__ bool patch_leaf(const DevScene& sc) {
+		const int gi = cur & REF_LEAF_MASK;
+		cur = REF_NONE;
+		const int4 m = __ldg(reinterpret_cast<const int4*>(&sc.leaves[gi].data));  // vertices, transforms, -, kind
+		V3 lo = o, ld = d, li = dinv;
+		bool odd = (flags & RAY_ODD) != 0 || (m.w & LEAF_PATCH_ODD) != 0;
+		M44 om;
+		const bool oxf = XFORM && m.y > 0;
+		if (oxf) {
+			if (!object_frame(sc, sc.instances[gi], &om)) return true;
+			lo = pos_to(om, io.origin());
+			ld = dir_to(om, io.direction());
+			li = recip3(ld);
+			odd = odd_ray(lo, ld, li) || (m.w & LEAF_PATCH_ODD) != 0;
+		}
+		const float* v = sc.fpool + m.x;
+		const int pm = m.w & 7;  // PM_*
+		const bool occl = (flags & RAY_OCCL) != 0;
+		const float dr = sc.dice_rate, mu = sc.min_upoly_size;
+		bool live = true, in = false;
+		// one patch kind: its bisection state and the number of its time samples
+		auto one = [&](auto& w) {
+			constexpr int NV = sizeof(w.c.cur[0]) / sizeof(V3), N = sizeof(w.c.cur) / sizeof(w.c.cur[0]);
+			if (odd) {
+				PatchHit ph;
+				const RayFlip f = widths(sc, oxf, om, lo, ld);
+				if (!patch_whole<NV, N>(v, time, lo, li, f, max_t, occl, dr, mu, w.st, &ph, &err)) return;
+				if (!occl) max_t = ph.t;
+				live = record(gi, ph.t, ph.u, ph.v, ph.max_dim);
+				return;
+			}
+			PatchCursor<NV, N> pc;
+			in = patch_begin<NV, N, true>(pc, v, time, lo, li, max_t);
+			if (!in) return;
+			if constexpr (WHOLE) {
+				const RayFlip f = widths(sc, oxf, om, lo, ld);
+				int units = 0x7fffffff;
+				live = patch_run<NV, N, true>(pc, w.st, lo, li, f, &max_t, occl, dr, mu, units, &err,
+				                              [&](float t, float u, float v2, float md) { record(gi, t, u, v2, md); }) !=
+				       PATCH_BLOCKED;
+			} else {
+				w.c = pc;
+			}
+		};
+		if constexpr ((F & FEAT_BILINEAR) != 0) {
+			if (pm == PM_BILINEAR1) one(still_work<4>());
+			else if (TS == 2 && pm == PM_BILINEAR2) one(work<4>());
 		}
 		if constexpr ((F & FEAT_BICUBIC) != 0) {
-			if (ob.kind == OBJ_BICUBIC) {
-				if constexpr ((F & FEAT_PATCH_MOTION) != 0) {
-					if (ob.n0 != 1)
-						pm = patch_begin<16, 2>(s.template work<16, 2>().c, v, wr.time, lr, s.max_t) ? PM_BICUBIC2 : -1;
-				}
-				if (pm == PM_NONE) pm = patch_begin<16, 1>(s.template work<16, 1>().c, v, wr.time, lr, s.max_t) ? PM_BICUBIC1 : -1;
-			}
+			if (pm == PM_BICUBIC1) one(still_work<16>());
+			else if (TS == 2 && pm == PM_BICUBIC2) one(work<16>());
 		}
-		if (pm > PM_NONE) {
-			s.pmode = pm;
-			s.pverts = v;
-			s.pr = lr;
-			s.prw = width();
-			s.p_obj = inst.data;
-			s.p_kind = ob.kind;
-			s.p_id = id;
-			s.p_shader = shader;
-			s.p_gi = gi;
+		if (!WHOLE && in) {
+			p_rw = widths(sc, oxf, om, lo, ld);
+			pmode = pm;
+			p_inst = gi;
+			p_o = lo;
+			p_dinv = li;
 		}
-	};
-	bool hit = false;
-	PatchHit ph;
-	ph.u = ph.v = ph.max_dim = 0.0f;
-	float max_t = s.max_t;
-	const float* v = sc.fpool + ob.data;
-	if (ob.kind == OBJ_SPHERE || ob.kind == OBJ_SPHERE_LIGHT) {
-		V3 cent;
-		float radi;
-		if (ob.kind == OBJ_SPHERE) {
-			sphere_at(sc, ob, wr.time, &cent, &radi);
-		} else {
-			float col[3];
-			light_at(sc, ob, wr.time, &cent, &radi, col);
-		}
-		const float t = sphere_t(lr.o, lr.d, cent, radi, max_t);
-		if (t >= 0.0f) {
-			hit = true;
-			ph.t = t;
-			if (!wr.occl) max_t = t;
-		}
-	} else if (ob.kind == OBJ_RECT_LIGHT) {
-		float dx, dy;
-		rect_light_at(sc, ob, wr.time, &dx, &dy, nullptr);
-		const float t = rect_light_t(lr.o, lr.d, lr.dinv, dx, dy, max_t);
-		if (t >= 0.0f) {
-			hit = true;
-			ph.t = t;
-			if (!wr.occl) max_t = t;
-		}
-	} else if constexpr (!RESUME) {
-		// the bisection runs here, to its end
-		if ((F & FEAT_BILINEAR) && ob.kind == OBJ_BILINEAR) {
-			const RayWidth w = width();
-			if ((F & FEAT_PATCH_MOTION) && ob.n0 != 1)
-				hit = patch_whole<4, 2>(v, wr.time, lr, w, &max_t, wr.occl, sc.dice_rate, sc.min_upoly_size, &ph,
-				                             &s.err);
-			else
-				hit = patch_whole<4, 1>(v, wr.time, lr, w, &max_t, wr.occl, sc.dice_rate, sc.min_upoly_size, &ph,
-				                             &s.err);
-		} else if ((F & FEAT_BICUBIC) && ob.kind == OBJ_BICUBIC) {
-			const RayWidth w = width();
-			if ((F & FEAT_PATCH_MOTION) && ob.n0 != 1)
-				hit = patch_whole<16, 2>(v, wr.time, lr, w, &max_t, wr.occl, sc.dice_rate, sc.min_upoly_size, &ph,
-				                             &s.err);
-			else
-				hit = patch_whole<16, 1>(v, wr.time, lr, w, &max_t, wr.occl, sc.dice_rate, sc.min_upoly_size, &ph,
-				                             &s.err);
-		}
-	} else {
-		begin_patch(v);
+		return live;
 	}
-	s.max_t = max_t;
-	if (hit) return trace_record<F>(s, inst.data, ob.kind, id, shader, gi, ph);
-	return true;
-}
 
-// One step of a lane that runs its ray alone: traverse to the next object
-// leaf and test it, a patch's whole bisection included.  The closest hit
-// does not depend on the order objects are tested in (a sub-patch's box
-// lies inside its parent's, so max_t pruning only drops leaves that could
-// not be closer), except for exact ties.  Returns false when the ray is
-// finished.
-template <unsigned F>
-__device__ __forceinline__ bool trace_step(const DevScene& sc, TraceState<F>& s) {
-	constexpr bool NESTED = (F & FEAT_NESTED) != 0;
-	while (true) {
-		leave_levels<F>(s);
-		if (s.nsp == 0) return false;
-		const int ref = s.node_stack[--s.nsp];
-		if (ref >= 0) {
-			if (!node_visit<F>(sc, s, ref)) return false;
-			continue;
+	// Carries the bisection in progress on for up to `units` iterations of its
+	// loop (`units` is left at the iterations not used).  Returns false when
+	// the ray is finished (an occlusion ray's hit).
+	__device__ __forceinline__ bool patch_step(const DevScene& sc, int& units) {
+		int r = PATCH_DONE;
+		const bool occl = (flags & RAY_OCCL) != 0;
+		const float dr = sc.dice_rate, mu = sc.min_upoly_size;
+		const RayFlip w = p_rw;
+		const V3 lo = p_o, li = p_dinv;
+		// the cursor runs as a local copy (registers) and goes back to the
+		// state only when the bisection stops short of its end
+		auto run = [&](auto& pw) {
+			auto pc = pw.c;
+			r = patch_run<sizeof(pc.cur[0]) / sizeof(V3), sizeof(pc.cur) / sizeof(pc.cur[0]), true>(
+			    pc, pw.st, lo, li, w, &max_t, occl, dr, mu, units, &err,
+			    [&](float t, float u, float v, float md) { record(p_inst, t, u, v, md); });
+			if (r == PATCH_MORE) pw.c = pc;
+		};
+		if constexpr ((F & FEAT_BILINEAR) != 0) {
+			if (pmode == PM_BILINEAR1) run(still_work<4>());
+			else if (TS == 2 && pmode == PM_BILINEAR2) run(work<4>());
 		}
-		// leaf: one instance of the current level's assembly
-		const int local = leaf_instance(ref);
-		const int gi = s.lv[s.L].inst_base + local;
-		const DevInstance inst = sc.instances[gi];
-		const uint64_t id = id_push(s.lv[s.L].id, (uint64_t)local, s.lv[s.L].id_bits);
-		const int shader = inst.shader >= 0 ? inst.shader : s.lv[s.L].shader;
-		if (NESTED && inst.kind == INST_ASSEMBLY) {
-			if (!enter_assembly<F>(sc, s, inst, gi, id, shader)) return false;
-			continue;
+		if constexpr ((F & FEAT_BICUBIC) != 0) {
+			if (pmode == PM_BICUBIC1) run(still_work<16>());
+			else if (TS == 2 && pmode == PM_BICUBIC2) run(work<16>());
 		}
-		return object_test<F, false>(sc, s, inst, gi, id, shader);
+		if (r == PATCH_MORE) return true;
+		pmode = PM_NONE;
+		return r != PATCH_BLOCKED;
 	}
-}
 
-// The walk cut into pieces for kernels that group their lanes by the work
-// they do next: up to `nodes` inner-node visits, stopping at a leaf, which
-// is popped into s.leaf for leaf_visit.  Returns WALK_DONE when the ray is
-// finished, WALK_LEAF at a leaf, WALK_MORE when the visits ran out; `nodes`
-// is left at the visits not used.
-enum : int { WALK_DONE = 0, WALK_LEAF = 1, WALK_MORE = 2 };
-
-template <unsigned F>
-__device__ __forceinline__ int walk_nodes(const DevScene& sc, TraceState<F>& s, int& nodes) {
-	while (true) {
-		leave_levels<F>(s);
-		if (s.nsp == 0) return WALK_DONE;
-		const int ref = s.node_stack[s.nsp - 1];
-		if (ref < 0) {
-			--s.nsp;
-			s.leaf = ref;
-			return WALK_LEAF;
-		}
-		if (nodes == 0) return WALK_MORE;
-		--nodes;
-		--s.nsp;
-		if (!node_visit<F>(sc, s, ref)) return WALK_DONE;
-	}
-}
-
-// The leaf popped by walk_nodes: an assembly instance is entered, an object
-// instance tested (a patch starts its bisection).  Returns false when the
-// ray is finished.
-template <unsigned F>
-__device__ __forceinline__ bool leaf_visit(const DevScene& sc, TraceState<F>& s) {
-	constexpr bool NESTED = (F & FEAT_NESTED) != 0;
-	const int local = leaf_instance(s.leaf);
-	const int gi = s.lv[s.L].inst_base + local;
-	const DevInstance inst = sc.instances[gi];
-	const uint64_t id = id_push(s.lv[s.L].id, (uint64_t)local, s.lv[s.L].id_bits);
-	const int shader = inst.shader >= 0 ? inst.shader : s.lv[s.L].shader;
-	if (NESTED && inst.kind == INST_ASSEMBLY) return enter_assembly<F>(sc, s, inst, gi, id, shader);
-	return object_test<F, true>(sc, s, inst, gi, id, shader);
-}
-
-// Work kinds of the wave kernels' lanes: idle, node visits, a leaf visit of
-// one of three classes, a bisection in progress.  Leaf visits are told
-// apart by class so that the lanes of a warp step run one branch of
-// leaf_visit together: assembly entries (transform merge, ray transform),
-// simple objects (spheres, sphere and rectangle lights), patches (root box,
-// ray widths, bisection set-up).
-enum : int { KIND_IDLE = 0, KIND_NODES = 1, LEAF_ENTER = 2, LEAF_SIMPLE = 3, LEAF_PATCH = 4, KIND_PATCH = 5 };
-
-// The class of the leaf walk_nodes stopped at (s.leaf).
-template <unsigned F>
-__device__ __forceinline__ int leaf_class(const DevScene& sc, const TraceState<F>& s) {
-	constexpr bool NESTED = (F & FEAT_NESTED) != 0;
-	const int gi = s.lv[s.L].inst_base + leaf_instance(s.leaf);
-	const int2 kd = __ldg(reinterpret_cast<const int2*>(sc.instances + gi));  // kind, data
-	if (NESTED && kd.x == INST_ASSEMBLY) return LEAF_ENTER;
-	const int ok = __ldg(&sc.objects[kd.y].kind);
-	return (ok == OBJ_BICUBIC || ok == OBJ_BILINEAR) ? LEAF_PATCH : LEAF_SIMPLE;
-}
-
-// Carries the bisection in progress on for up to `units` iterations of its
-// loop (`units` is left at the iterations not used).  Returns false when
-// the ray is finished (an occlusion ray's hit).
-template <unsigned F>
-__device__ __forceinline__ bool patch_step(const DevScene& sc, TraceState<F>& s, int& units) {
-	constexpr int TS = PatchBuf<F>::TS;
-	bool done = false, found = false;
-	float max_t = s.max_t;
-	const bool occl = s.wr.occl;
-	const float dr = sc.dice_rate, mu = sc.min_upoly_size;
-	// the cursor runs as a local copy (registers) and goes back to the
-	// state only when the bisection stops short of its end
-	auto run = [&](auto& pw) {
-		auto pc = pw.c;
-		done = patch_run(pc, pw.st, s.pverts, s.pr, s.prw, &max_t, occl, dr, mu, &s.ph, units, &s.err);
-		if (!done) pw.c = pc;
-		found = pc.found;
-	};
-	if constexpr ((F & FEAT_BILINEAR) != 0) {
-		if (s.pmode == PM_BILINEAR1) run(s.template work<4, 1>());
-		else if (TS == 2 && s.pmode == PM_BILINEAR2) run(s.template work<4, TS>());
-	}
-	if constexpr ((F & FEAT_BICUBIC) != 0) {
-		if (s.pmode == PM_BICUBIC1) run(s.template work<16, 1>());
-		else if (TS == 2 && s.pmode == PM_BICUBIC2) run(s.template work<16, TS>());
-	}
-	s.max_t = max_t;
-	if (!done) return true;
-	s.pmode = PM_NONE;
-	if (found) return trace_record<F>(s, s.p_obj, s.p_kind, s.p_id, s.p_shader, s.p_gi, s.ph);
-	return true;
-}
-
-// Traces one ray through the scene. Returns the device error flags.
-template <unsigned F>
-__device__ unsigned trace_ray(const DevScene& sc, const WorldRayD& wr, HitRec* rec) {
-	TraceState<F> s;
-	trace_init<F>(sc, s, wr);
-	while (trace_step<F>(sc, s)) {
-	}
-	*rec = s.rec;
-	return s.err;
-}
-
-// Transform from world space into the hit object's space at the ray time
-// (the Intersection::space of the reference), rebuilt from the hit path.
-// Returns false when the path carries no transform (identity).
-template <unsigned F>
-__device__ bool hit_space(const DevScene& sc, const HitRec& rec, float time, M44* out, unsigned* err) {
-	if (!(F & FEAT_XFORM)) return false;
-	Frame f;
-	f.count = 0;
-	for (int k = 0; k < rec.depth; ++k) {
-		const DevInstance inst = sc.instances[rec.path[k]];
-		if (inst.xform_count > 0) {
-			Frame g;
-			if (!frame_merge(f, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &g)) {
-				*err |= ERRF_MOTION;
-				return false;
-			}
-			f = g;
+	// A lane that runs its ray alone: the whole walk.  The closest hit does
+	// not depend on the order objects are tested in (a sub-patch's box lies
+	// inside its parent's, so max_t pruning only drops leaves that could not
+	// be closer), except for exact ties.
+	__device__ __forceinline__ void walk(const DevScene& sc) {
+		bool live = pop(sc);
+		while (live) {
+			while (live && cur >= 0) live = node_step(sc) && pop(sc);
+			if (!live) return;
+			const int cls = leaf_class(cur);
+			if (NESTED && cls == LEAF_ENTER) live = enter(sc);
+			else if (cls == LEAF_SPHERE) live = sphere_leaf(sc);
+			else if ((F & (FEAT_BILINEAR | FEAT_BICUBIC)) && cls == LEAF_PATCH) live = patch_leaf<true>(sc);
+			else live = simple_leaf(sc);
+			live = live && pop(sc);
 		}
 	}
-	if (f.count == 0) return false;
-	*out = frame_at_index_lerp(f, time);
-	return true;
-}
+};
 
 }  // namespace psy
 
