@@ -282,8 +282,9 @@ def run_render_ours(args, rank, local, pg, world):
     rays_per_render = int(integ.stats.rays)
     occl_per_render = int(integ.stats.occlusion_rays)
     launches_per_render = int(integ.stats.launches)
-    # every wave launches one closest-hit and one occlusion traversal per segment
-    trace_launches_per_render = int(integ.stats.waves) * 2 * RENDER_PATH_LENGTH
+    # every wave launches one traversal per segment (closest-hit rays and the
+    # last vertex's shadow rays) and one for the last shadow rays
+    trace_launches_per_render = int(integ.stats.waves) * (RENDER_PATH_LENGTH + 1)
     counters = ctx.trace_counters()
     paths = w * h * RENDER_SPP
     if pg:

@@ -41,6 +41,12 @@ struct HaltonDev {
 	const double* cmul;
 };
 
+// A block of the adjoint gathers its gradient in shared memory, in 64 bits
+// where that fits 32 KB (a block sums the paths of a whole wave's share, and
+// 32-bit sums of so many terms lost 8e-6 of the gradient), in 32 bits up to
+// twice as many parameters, else it adds to the output directly.
+enum : int { GRAD_GLOBAL = 0, GRAD_SMEM32, GRAD_SMEM64 };
+
 // Parameters of one render (PathTraceIntegrator's settings and its film).
 struct RenderParams {
 	uint32_t width, height, spp, seed, path_length;
@@ -59,7 +65,7 @@ struct RenderParams {
 	const float* dl_dxyz;    // adjoint: dL / d(film sums), width * height * 3
 	float* grad;             // adjoint: gradient accumulator, param_count floats
 	int param_count;
-	int grad_in_smem;        // adjoint: accumulate per block in shared memory first
+	int grad_in_smem;        // adjoint: where a block accumulates (GRAD_*)
 };
 
 // Largest path_length of the adjoint (vertex records per path).
@@ -76,19 +82,11 @@ struct WaveRange {
 // Path state of one wave, structure of arrays (PTState,
 // integrator/path_trace_integrator.hpp:49-63).
 struct PathSoA {
-	uint32_t* smp;      // sampler offset
-	uint32_t* dimstep;  // next sampler dimension | step << 16
-	float* wl;
-	float* time;
-	float* last_pdf;
-	float4* col;
+	uint4* head;        // sampler offset, next sampler dimension | step << 16, wavelength, last pdf (as bits)
+	float4* col;        // radiance so far; of a finished path, its sample
 	float4* fcol;
-	float4* lcol;       // between the shadow ray and its result: the light's contribution
-	float* hit;         // stored intersection, 16 floats per path
-	float* pray;        // previous ray, 16 floats per path
-	float* hitx;        // GTR hits: world dpdu, dpdv, dndu, dndv, 12 floats per path
+	float4* lcol;       // between a shadow ray and its result: the light's contribution
 	float* sample;      // film sample XYZ, 3 floats per path
-	uint16_t* rid;      // render of the path (batches)
 	// adjoint pass only
 	float4* adj;        // dL / d(sample spectrum) per hero wavelength
 	float4* valb;       // albedo spectrum of each parameterised vertex, PSY_ADJ_MAX_VERTS per path
@@ -101,9 +99,9 @@ struct PathSoA {
 
 // Rays and hits of a wave by queue position (cap = the wave's path capacity).
 struct WaveBufs {
-	float4* ray[2];     // [0] camera / bounce rays, [1] shadow rays: 5 planes of cap float4
+	float4* ray[3];     // camera / bounce rays (two, taken in turn) and shadow rays: 5 planes of cap float4
 	float4* hit_f;      // t, u, v, max_dim
-	int4* hit_i;        // 3 planes: obj, kind | depth << 8, shader, path[0]; path[1..4]; path[5..7]
+	int4* hit_i;        // 3 planes: instance, placement, depth, path[0]; path[1..4]; path[5..7]
 	uint8_t* occl;      // shadow ray result: 1 = blocked (or no shadow ray)
 	int cap;
 };

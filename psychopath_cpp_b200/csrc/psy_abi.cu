@@ -162,19 +162,11 @@ static int wave_set(psy_ctx* ctx, const char* prefix, uint64_t P, uint32_t path_
 		return ctx->scratch_buffer((pre + name).c_str(), bytes, &rc);
 	};
 	PathSoA& ps = ws->ps;
-	ps.smp = (uint32_t*)buf("smp", P * 4);
-	ps.dimstep = (uint32_t*)buf("dimstep", P * 4);
-	ps.wl = (float*)buf("wl", P * 4);
-	ps.time = (float*)buf("time", P * 4);
-	ps.last_pdf = (float*)buf("lpdf", P * 4);
+	ps.head = (uint4*)buf("head", P * 16);
 	ps.col = (float4*)buf("col", P * 16);
 	ps.fcol = (float4*)buf("fcol", P * 16);
 	ps.lcol = (float4*)buf("lcol", P * 16);
-	ps.hit = (float*)buf("hit", P * 64);
-	ps.pray = (float*)buf("pray", P * 64);
-	ps.hitx = (float*)buf("hitx", P * 48);
 	ps.sample = (float*)buf("sample", P * 12);
-	ps.rid = (uint16_t*)buf("rid", P * 2);
 	ps.adj = nullptr;
 	ps.valb = nullptr;
 	ps.vpid = nullptr;
@@ -202,12 +194,12 @@ static int wave_set(psy_ctx* ctx, const char* prefix, uint64_t P, uint32_t path_
 	wb.cap = (int)P;
 	wb.ray[0] = (float4*)buf("ray0", P * 80);
 	wb.ray[1] = (float4*)buf("ray1", P * 80);
+	wb.ray[2] = (float4*)buf("ray2", P * 80);
 	wb.hit_f = (float4*)buf("hitf", P * 16);
 	wb.hit_i = (int4*)buf("hiti", P * 48);
 	wb.occl = (uint8_t*)buf("occl", P);
-	if (!ps.smp || !ps.dimstep || !ps.wl || !ps.time || !ps.last_pdf || !ps.col || !ps.fcol || !ps.lcol ||
-	    !ps.hit || !ps.pray || !ps.hitx || !ps.sample || !ps.rid || !wq.q0 || !wq.q1 || !wq.counters || !wq.rays || !wb.ray[0] ||
-	    !wb.ray[1] || !wb.hit_f || !wb.hit_i || !wb.occl)
+	if (!ps.head || !ps.col || !ps.fcol || !ps.lcol || !ps.sample || !wq.q0 || !wq.q1 || !wq.counters || !wq.rays ||
+	    !wb.ray[0] || !wb.ray[1] || !wb.ray[2] || !wb.hit_f || !wb.hit_i || !wb.occl)
 		return rc ? rc : PSY_ERR_OOM;
 	return PSY_OK;
 }
@@ -255,8 +247,8 @@ static int render_single(psy_ctx* ctx, const psy_render_desc* desc, const Render
 	ctx->last_counts = ws.wq.rays;
 	uint32_t launches = 0, waves = 0;
 	for (uint64_t base = 0; base < total; base += P) {
-		// each wave launches 2 * path_length traversal kernels
-		if (ctx->profiling && (rc = timer_reserve(ctx, 2 * (int)rp.path_length))) return rc;
+		// each wave launches path_length + 1 traversal kernels
+		if (ctx->profiling && (rc = timer_reserve(ctx, (int)rp.path_length + 1))) return rc;
 		WaveRange wv;
 		wv.base = base;
 		wv.paths = (int)((total - base) < P ? (total - base) : P);
@@ -474,7 +466,7 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 			ctx->batch_graph_key = key;
 		} else {
 			// the launch count of the captured sequence
-			for (size_t i = 0; i < waves.size(); ++i) launches += 2 + 4 * max_len;
+			for (size_t i = 0; i < waves.size(); ++i) launches += 5 + 2 * max_len;
 		}
 		if ((rc = ctx_cuda(ctx, cudaGraphLaunch(ctx->batch_graph, st), "psy_render_batch: graph launch"))) return rc;
 	} else {
@@ -997,7 +989,8 @@ int psy_render_adjoint(psy_ctx* ctx, const psy_render_desc* desc, const psy_diff
 	if ((rc = diff_params(ctx, diff, "psy_render_adjoint", &rp))) return rc;
 	rp.dl_dxyz = dl_dxyz;
 	rp.grad = grad;
-	rp.grad_in_smem = (size_t)rp.param_count * sizeof(float) <= 32768 ? 1 : 0;
+	const size_t pc = (size_t)rp.param_count;
+	rp.grad_in_smem = pc * sizeof(double) <= 32768 ? GRAD_SMEM64 : pc * sizeof(float) <= 32768 ? GRAD_SMEM32 : GRAD_GLOBAL;
 	return render_single(ctx, desc, rp, true, stats, (cudaStream_t)stream);
 }
 

@@ -24,7 +24,7 @@ cudaError_t launch_render_wave(const DevScene& sc, const HaltonDev& hd, const Re
 	w.sc = sc;
 	w.rp = rp;
 	block = valid_block(block);
-	const size_t gsmem = (rp.grad && rp.grad_in_smem) ? sizeof(float) * (size_t)rp.param_count : 0;
+	const size_t gsmem = (rp.grad && rp.grad_in_smem) ? (rp.grad_in_smem == GRAD_SMEM64 ? sizeof(double) : sizeof(float)) * (size_t)rp.param_count : 0;
 	const uint32_t L = rp.path_length;
 	switch (feature_variant(sc.features)) {
 		case FEAT_FLAT: launch_wave<PlainWave, FEAT_FLAT>(w, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
@@ -72,7 +72,8 @@ __global__ void light_sample_kernel(DevScene sc, LightQuerySoADev q, LightSample
 	lq.id = 0;
 	lq.selection_pdf = 1.0f;
 	lq.light_sample_pdf = 1.0f;
-	light_tree_sample(sc, &lq, ident_inv);
+	light_tree_pick<FEAT_ALL>(sc, &lq);
+	light_emit<FEAT_ALL>(sc, &lq, ident_inv);
 	if (!lq.valid) {
 		atomicOr(status, ERRF_NOLIGHT);
 		return;

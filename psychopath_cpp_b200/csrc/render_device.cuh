@@ -786,11 +786,15 @@ static __device__ __noinline__ void rect_light_sample(const DevScene& sc, const 
 // small.
 static __device__ __noinline__ M44 m44_inverse_dev(const M44& a, const RcpTable& rt) { return m44_inverse(a, rt); }
 
-// LightTree::sample starting at the root assembly's tree.
-static __device__ void light_tree_sample(const DevScene& sc, LightQuery* q, float ident_inv) {
+// LightTree::sample starting at the root assembly's tree, in two parts: the
+// walk to a light (q->obj, -1 when there is none), and its sample.
+template <unsigned F>
+static __device__ __forceinline__ void light_tree_pick(const DevScene& sc, LightQuery* q) {
+	constexpr bool NESTED = (F & FEAT_NESTED) != 0, XFORM = (F & FEAT_XFORM) != 0;
 	q->valid = false;
+	q->obj = -1;
 	int asmb = 0;
-	for (int level = 0; level < 16; ++level) {
+	for (int level = 0; level < (NESTED ? 16 : 1); ++level) {
 		const DevAssembly as = sc.assemblies[asmb];
 		if (as.light_root < 0) return;
 		int node = as.light_root;
@@ -835,7 +839,7 @@ static __device__ void light_tree_sample(const DevScene& sc, LightQuery* q, floa
 		const int local = leaf;
 		const DevInstance inst = sc.instances[as.inst_base + local];
 		q->id = id_push(q->id, (uint64_t)local, as.id_bits);
-		if (inst.xform_count > 0) {
+		if (XFORM && inst.xform_count > 0) {
 			const M44 X = seq_lerp_global(sc.xforms + (size_t)inst.xform * 16, inst.xform_count, q->time);
 			q->pos = pos_to(X, q->pos);
 			q->nor = normalized(dir_transpose(m44_inverse_dev(X, sc.rcp), q->nor));
@@ -846,25 +850,33 @@ static __device__ void light_tree_sample(const DevScene& sc, LightQuery* q, floa
 			const DevObject ob = sc.objects[inst.data];
 			if (ob.kind != OBJ_SPHERE_LIGHT && ob.kind != OBJ_RECT_LIGHT) return;
 			q->obj = inst.data;
-			float p = 1.0f;
-			V3 tl;
-			if (ob.kind == OBJ_SPHERE_LIGHT)
-				sphere_light_sample(sc, ob, q->pos, q->u, q->v, q->wavelength, q->time, &tl, &p, &q->spec);
-			else
-				rect_light_sample(sc, ob, q->pos, q->u, q->v, q->wavelength, q->time, &tl, &p, &q->spec);
-			// xform.dir_from: the reference inverts the accumulated transform,
-			// which is the identity when no instance carried one
-			if (q->has_xform) q->to_light = dir_to(m44_inverse_dev(q->xform, sc.rcp), tl);
-			else q->to_light = tl * ident_inv;
 			q->selection_pdf *= (tot_prob * (float)as.light_count);
-			q->light_sample_pdf = p;
-			q->valid = true;
 			return;
 		}
+		if (!NESTED) return;
 		const DevAssembly sub = sc.assemblies[inst.data];
 		q->selection_pdf *= (tot_prob * (float)as.light_count) / (float)sub.light_count;
 		asmb = inst.data;
 	}
+}
+
+template <unsigned F>
+static __device__ __forceinline__ void light_emit(const DevScene& sc, LightQuery* q, float ident_inv) {
+	constexpr bool XFORM = (F & FEAT_XFORM) != 0;
+	if (q->obj < 0) return;
+	const DevObject ob = sc.objects[q->obj];
+	float p = 1.0f;
+	V3 tl;
+	if (ob.kind == OBJ_SPHERE_LIGHT)
+		sphere_light_sample(sc, ob, q->pos, q->u, q->v, q->wavelength, q->time, &tl, &p, &q->spec);
+	else
+		rect_light_sample(sc, ob, q->pos, q->u, q->v, q->wavelength, q->time, &tl, &p, &q->spec);
+	// xform.dir_from: the reference inverts the accumulated transform,
+	// which is the identity when no instance carried one
+	if (XFORM && q->has_xform) q->to_light = dir_to(m44_inverse_dev(q->xform, sc.rcp), tl);
+	else q->to_light = tl * ident_inv;
+	q->light_sample_pdf = p;
+	q->valid = true;
 }
 
 // ---------------------------------------------------------------------

@@ -5,24 +5,31 @@
  * The reference renders a bucket as a stream of paths and loops
  *   generate one ray per live path -> Tracer::trace -> update -> partition.
  * Here a wave of paths lives in HBM as SoA state and the loop is split into
- * kernels that each do one kind of work, so the traversal kernels carry no
- * shading state and the shading kernels no traversal state:
+ * kernels that each do one kind of work, so the traversal kernel carries no
+ * shading state and the shading kernel no traversal state:
  *
- *   camera_gen            camera rays of every path of the wave
- *   trace<closest>        Tracer::trace of the ray buffer (closest hits)
- *   shade_hit             update_path after a camera / bounce ray, then
- *                         next_ray_for_path's shadow step: light-tree sample
- *                         and shadow ray; live paths are compacted into the
- *                         next queue (ballot + popc, one atomic per warp)
- *   trace<occlusion>      Tracer::trace of the shadow rays
- *   shade_shadow          update_path after the shadow ray, then the bounce
- *                         ray (the path stays at its queue position)
- *   ... trace<closest> -> shade_hit -> ... for path_length bounces.
+ *   camera_gen   camera rays of every path of the wave
+ *   trace        Tracer::trace of the closest-hit rays and of the shadow rays
+ *                of the last vertex, in one launch
+ *   shade        update_path with both results, then next_ray_for_path's two
+ *                steps at the new vertex: light sample with its shadow ray,
+ *                and the bounce ray; live paths are compacted into the next
+ *                queue (ballot + popc, one atomic per warp)
+ *   ... trace -> shade for path_length vertices, then the last shadow rays
+ *   finish       their results, every sample's spectrum to XYZ, film sums
  *
- * Rays and hits are stored by queue position (coalesced), path state by
- * path slot.  Finished paths write their film sample
- * (Color_XYZ(col) * XYZ_NORM_FAC); a per-wave reduction adds each pixel's
- * samples in sample order.
+ * The reference traces the shadow ray before it generates the bounce ray;
+ * the bounce does not depend on the result (only the path's radiance does,
+ * which is added to in the same order here), so both leave a vertex together
+ * and nothing of the vertex is stored.  (As kernels of their own, hit and
+ * shadow shading wrote and read 176 bytes of vertex a path and step, and a
+ * small frame waited for twice as many launches: 80x60 preview 525 -> 455 us,
+ * 320x240x16 render 2.55 -> 2.26 ms.)
+ *
+ * Rays and hits are stored by queue position (coalesced), path state by path
+ * slot.  Finished paths leave their spectrum in the path state; a per-wave
+ * reduction adds each pixel's samples (Color_XYZ(col) * XYZ_NORM_FAC) in
+ * sample order.
  *
  * The same kernels serve two modes.  PlainWave renders one scene and takes
  * the scene and render parameters as kernel parameters.  BatchWave renders
@@ -138,73 +145,31 @@ struct WaveIO {
 	}
 };
 
-// World-space shading data of the stored intersection (the PTState::inter
-// and prev_ray the reference keeps per path).
-struct StoredHit {
+// World-space shading data of a path vertex (the PTState::inter and prev_ray
+// of the reference).
+struct Vertex {
 	V3 p, n, off;       // geo.p, geo.n (after transformed_from), signed ray-origin offset
-	float t;
+	V3 d;               // direction of the ray that met it
+	V3 odx, ody;        // that ray's origin differentials transferred to the hit
 	float bf;           // 1 when the hit was back-facing
 	float col[3];       // closure colour (Lambert)
 	int pid;            // differentiable renders: the shader's first albedo weight (>= 0), -2 - q when its
 	                    // RGB albedo is scaled by params[q], or -1 (not parameterised)
 	int gtr;            // the GTR shader of the hit, or -1 (Lambert)
-	V3 d, odx, ody, ddx, ddy;  // previous ray
-	V3 dpdu, dpdv, dndu, dndv; // GTR hits: geo's derivatives in world space (transformed_from)
+};
+// What the GTR closure reads besides: geo's derivatives in world space
+// (transformed_from) and the direction differentials of the ray.
+struct GtrVertex {
+	V3 ddx, ddy, dpdu, dpdv, dndu, dndv;
 };
 
-__device__ __forceinline__ void load_hit(const PathSoA& ps, int s, StoredHit* h) {
-	const float4* g = reinterpret_cast<const float4*>(ps.hit) + (size_t)s * 4;
-	const float4 a = g[0], b = g[1], c = g[2], d = g[3];
-	h->p = V3(a.x, a.y, a.z);
-	h->n = V3(a.w, b.x, b.y);
-	h->off = V3(b.z, b.w, c.x);
-	h->t = c.y;
-	h->col[0] = c.z; h->col[1] = c.w; h->col[2] = d.x;
-	h->bf = d.y;
-	h->pid = __float_as_int(d.z);
-	h->gtr = __float_as_int(d.w);
-	if (h->gtr >= 0) {
-		const float4* x = reinterpret_cast<const float4*>(ps.hitx) + (size_t)s * 3;
-		const float4 u = x[0], v = x[1], w = x[2];
-		h->dpdu = V3(u.x, u.y, u.z);
-		h->dpdv = V3(u.w, v.x, v.y);
-		h->dndu = V3(v.z, v.w, w.x);
-		h->dndv = V3(w.y, w.z, w.w);
-	}
-	const float4* r = reinterpret_cast<const float4*>(ps.pray) + (size_t)s * 4;
-	const float4 e = r[0], f = r[1], gg = r[2], hh = r[3];
-	h->d = V3(e.x, e.y, e.z);
-	h->odx = V3(e.w, f.x, f.y);
-	h->ody = V3(f.z, f.w, gg.x);
-	h->ddx = V3(gg.y, gg.z, gg.w);
-	h->ddy = V3(hh.x, hh.y, hh.z);
-}
-
-__device__ __forceinline__ void store_hit(const PathSoA& ps, int s, const StoredHit& h) {
-	float4* g = reinterpret_cast<float4*>(ps.hit) + (size_t)s * 4;
-	g[0] = make_float4(h.p.x, h.p.y, h.p.z, h.n.x);
-	g[1] = make_float4(h.n.y, h.n.z, h.off.x, h.off.y);
-	g[2] = make_float4(h.off.z, h.t, h.col[0], h.col[1]);
-	g[3] = make_float4(h.col[2], h.bf, __int_as_float(h.pid), __int_as_float(h.gtr));
-	if (h.gtr >= 0) {
-		float4* x = reinterpret_cast<float4*>(ps.hitx) + (size_t)s * 3;
-		x[0] = make_float4(h.dpdu.x, h.dpdu.y, h.dpdu.z, h.dpdv.x);
-		x[1] = make_float4(h.dpdv.y, h.dpdv.z, h.dndu.x, h.dndu.y);
-		x[2] = make_float4(h.dndu.z, h.dndv.x, h.dndv.y, h.dndv.z);
-	}
-	float4* r = reinterpret_cast<float4*>(ps.pray) + (size_t)s * 4;
-	r[0] = make_float4(h.d.x, h.d.y, h.d.z, h.odx.x);
-	r[1] = make_float4(h.odx.y, h.odx.z, h.ody.x, h.ody.y);
-	r[2] = make_float4(h.ody.z, h.ddx.x, h.ddx.y, h.ddx.z);
-	r[3] = make_float4(h.ddy.x, h.ddy.y, h.ddy.z, 0.0f);
-}
-
-// Intersection -> stored hit: DifferentialGeometry::transformed_from(space)
-// (basics/differential_geometry.hpp:20-40) and the offset of
-// path_trace_integrator.cpp:141-145.
+// Intersection -> vertex: DifferentialGeometry::transformed_from(space)
+// (basics/differential_geometry.hpp:20-40), the offset of
+// path_trace_integrator.cpp:141-145 and the transferred differentials of
+// propagate_differentials.
 template <unsigned F>
-__device__ void make_stored(const DevScene& sc, const HitRec& rec, const WorldRayD& wr, float ident_inv,
-                            StoredHit* sh, int* closure, float* emit_col, float* light_pdf, unsigned* err) {
+__device__ __forceinline__ void make_vertex(const DevScene& sc, const HitRec& rec, const WorldRayD& wr, float ident_inv,
+                                            Vertex* sh, GtrVertex* gv, int* closure, float* light_pdf, unsigned* err) {
 	M44 space;
 	const bool xf = hit_space<F>(sc, rec, wr.time, &space, err);
 	V3 lo = wr.o, ld = wr.d;
@@ -215,7 +180,7 @@ __device__ void make_stored(const DevScene& sc, const HitRec& rec, const WorldRa
 	HitInfo h;
 	hit_geometry(sc, rec, wr.time, lo, ld, false, &h);
 	*closure = h.closure;
-	emit_col[0] = h.col[0]; emit_col[1] = h.col[1]; emit_col[2] = h.col[2];
+	sh->col[0] = h.col[0]; sh->col[1] = h.col[1]; sh->col[2] = h.col[2];
 	*light_pdf = h.light_pdf;
 	if (h.closure != CLOSURE_LAMBERT && h.closure != CLOSURE_GTR) return;
 	M44 inv;
@@ -234,34 +199,33 @@ __device__ void make_stored(const DevScene& sc, const HitRec& rec, const WorldRa
 	if (h.closure == CLOSURE_GTR) {
 		// the rest of DifferentialGeometry::transformed_from (basics/differential_geometry.hpp:20-40)
 		sh->gtr = rec.shader;
-		sh->dpdu = dir_to(inv, h.geo.dpdu);
-		sh->dpdv = dir_to(inv, h.geo.dpdv);
-		sh->dndu = nor_from(nx, h.geo.dndu) * il;
-		sh->dndv = nor_from(nx, h.geo.dndv) * il;
+		gv->dpdu = dir_to(inv, h.geo.dpdu);
+		gv->dpdv = dir_to(inv, h.geo.dpdv);
+		gv->dndu = nor_from(nx, h.geo.dndu) * il;
+		gv->dndv = nor_from(nx, h.geo.dndv) * il;
+		gv->ddx = wr.ddx;
+		gv->ddy = wr.ddy;
 	}
 	V3 off = dir_to(inv, h.offset);
 	if (h.backfacing) off = off * -1.0f;
 	sh->off = off;
 	sh->bf = h.backfacing ? 1.0f : 0.0f;
-	sh->t = rec.t;
-	sh->col[0] = h.col[0]; sh->col[1] = h.col[1]; sh->col[2] = h.col[2];
 	sh->d = wr.d;
-	sh->odx = wr.odx;
-	sh->ody = wr.ody;
-	sh->ddx = wr.ddx;
-	sh->ddy = wr.ddy;
+	const V3 nn = normalized(sh->n);
+	sh->odx = transfer_origin_differential(rec.t, nn, wr.d, wr.odx, wr.ddx);
+	sh->ody = transfer_origin_differential(rec.t, nn, wr.d, wr.ody, wr.ddy);
 }
 
-// LambertClosure::propagate_differentials (shading/surface_closure.hpp:306-320).
-__device__ __forceinline__ void propagate_differentials(const StoredHit& h, WorldRayD* out) {
+// The outgoing ray's differentials (LambertClosure::propagate_differentials,
+// shading/surface_closure.hpp:306-320).
+__device__ __forceinline__ void propagate_differentials(const Vertex& h, WorldRayD* out) {
 	const float len = length(out->d);
-	const V3 nn = normalized(h.n);
 	V3 x, y;
 	coordinate_system(out->d, &x, &y);
 	x = normalized(x);
 	y = normalized(y);
-	out->odx = transfer_origin_differential(h.t, nn, h.d, h.odx, h.ddx);
-	out->ody = transfer_origin_differential(h.t, nn, h.d, h.ody, h.ddy);
+	out->odx = h.odx;
+	out->ody = h.ody;
 	out->ddx = (x * 0.15f) / len;
 	out->ddy = (y * 0.15f) / len;
 }
@@ -270,16 +234,15 @@ __device__ __forceinline__ void propagate_differentials(const StoredHit& h, Worl
 // origin differentials transferred to the hit, normal differentials turned
 // into half-vector differentials, direction differentials reflected about
 // the half vector, then clamped (clamp_dd).
-static __device__ __noinline__ void gtr_propagate_differentials(const StoredHit& h, WorldRayD* out) {
-	V3 nn = normalized(h.n);
-	const V3 hh = normalized(normalized(h.d * -1.0f) + normalized(out->d));
-	out->odx = transfer_origin_differential(h.t, nn, h.d, h.odx, h.ddx);
-	out->ody = transfer_origin_differential(h.t, nn, h.d, h.ody, h.ddy);
+static __device__ __noinline__ void gtr_direction_differentials(const GtrVertex& g, V3 n, V3 d, V3 odx, V3 ody, V3 out,
+                                                                V3* oddx, V3* oddy) {
+	V3 nn = normalized(n);
+	const V3 hh = normalized(normalized(d * -1.0f) + normalized(out));
 	float dux, dvx, duy, dvy;
-	uv_differentials(out->odx, h.dpdu, h.dpdv, &dux, &dvx);
-	uv_differentials(out->ody, h.dpdu, h.dpdv, &duy, &dvy);
-	V3 dndx = (h.dndu * dux) + (h.dndv * dvx);
-	V3 dndy = (h.dndu * duy) + (h.dndv * dvy);
+	uv_differentials(odx, g.dpdu, g.dpdv, &dux, &dvx);
+	uv_differentials(ody, g.dpdu, g.dpdv, &duy, &dvy);
+	V3 dndx = (g.dndu * dux) + (g.dndv * dvx);
+	V3 dndy = (g.dndu * duy) + (g.dndv * dvy);
 	if (dot(nn, hh) < 0.0f) {
 		nn = nn * -1.0f;
 		dndx = dndx * -1.0f;
@@ -290,23 +253,20 @@ static __device__ __noinline__ void gtr_propagate_differentials(const StoredHit&
 	const M44 xf = axis_angle(axis, angle);
 	const V3 dhdx = dir_to(xf, dndx);
 	const V3 dhdy = dir_to(xf, dndy);
-	out->ddx = reflect_dd(hh, dhdx, h.d, h.ddx);
-	out->ddy = reflect_dd(hh, dhdy, h.d, h.ddy);
-	const float len_d = length(out->d);
-	const float len_dx = length(out->ddx);
-	const float len_dy = length(out->ddy);
-	if ((len_dx / len_d) > 0.9f) out->ddx = out->ddx * ((0.9f * len_d) / len_dx);
-	if ((len_dy / len_d) > 0.9f) out->ddy = out->ddy * ((0.9f * len_d) / len_dy);
+	V3 ddx = reflect_dd(hh, dhdx, d, g.ddx);
+	V3 ddy = reflect_dd(hh, dhdy, d, g.ddy);
+	const float len_d = length(out);
+	const float len_dx = length(ddx);
+	const float len_dy = length(ddy);
+	if ((len_dx / len_d) > 0.9f) ddx = ddx * ((0.9f * len_d) / len_dx);
+	if ((len_dy / len_d) > 0.9f) ddy = ddy * ((0.9f * len_d) / len_dy);
+	*oddx = ddx;
+	*oddy = ddy;
 }
-
-__device__ __forceinline__ void finish_path(const PathSoA& ps, int slot, const Spec& col, float wl) {
-	float xyz[3];
-	spec_to_xyz(col, wl, xyz);
-	float3 o;
-	o.x = xyz[0] * XYZ_NORM_FAC;
-	o.y = xyz[1] * XYZ_NORM_FAC;
-	o.z = xyz[2] * XYZ_NORM_FAC;
-	reinterpret_cast<float3*>(ps.sample)[slot] = o;
+__device__ __forceinline__ void gtr_propagate_differentials(const Vertex& h, const GtrVertex& g, WorldRayD* out) {
+	out->odx = h.odx;
+	out->ody = h.ody;
+	gtr_direction_differentials(g, h.n, h.d, h.odx, h.ody, out->d, &out->ddx, &out->ddy);
 }
 
 // ---------------------------------------------------------------------
@@ -358,7 +318,7 @@ __device__ __forceinline__ int emission_param(const RenderParams& rp, int obj) {
 
 // lambert_eval with the albedo taken from parameters when the stored hit's
 // shader has them.
-__device__ __forceinline__ Spec lambert_eval_p(const RenderParams& rp, const StoredHit& sh, V3 out, float wl) {
+__device__ __forceinline__ Spec lambert_eval_p(const RenderParams& rp, const Vertex& sh, V3 out, float wl) {
 	if (sh.pid == -1) return lambert_eval(sh.col, sh.d, out, sh.n, wl);
 	if (sh.pid < -1) {
 		Spec f = lambert_eval(sh.col, sh.d, out, sh.n, wl);
@@ -385,7 +345,10 @@ static __device__ void grad_add(const RenderParams& rp, float* sg, const PathSoA
                          int lp, float wl) {
 	const float4 u4 = ps.adj[slot];
 	const float ub[4] = {u4.x * B.e[0], u4.y * B.e[1], u4.z * B.e[2], u4.w * B.e[3]};
-	float* g = rp.grad_in_smem ? sg : rp.grad;
+	auto add = [&](int k, float v) {
+		if (rp.grad_in_smem == GRAD_SMEM64) atomicAdd(reinterpret_cast<double*>(sg) + k, (double)v);
+		else atomicAdd((rp.grad_in_smem ? sg : rp.grad) + k, v);
+	};
 	const float scale = lp >= 0 ? rp.params[lp] : 1.0f;
 	if (nv > PSY_ADJ_MAX_VERTS) nv = PSY_ADJ_MAX_VERTS;
 	float a[PSY_ADJ_MAX_VERTS][4];
@@ -403,7 +366,7 @@ static __device__ void grad_add(const RenderParams& rp, float* sg, const PathSoA
 				if (pid[v] != -1) q *= a[v][j];
 			d += q;
 		}
-		atomicAdd(g + lp, d);
+		add(lp, d);
 	}
 	for (int v = 0; v < nv; ++v) {
 		if (pid[v] == -1) continue;
@@ -416,13 +379,13 @@ static __device__ void grad_add(const RenderParams& rp, float* sg, const PathSoA
 		if (pid[v] < -1) {
 			// scaled RGB albedo: its derivative is the upsampled colour
 			const float4 u = ps.vdsc[slot * PSY_ADJ_MAX_VERTS + v];
-			atomicAdd(g + (-2 - pid[v]), ((q[0] * u.x + q[1] * u.y) + q[2] * u.z) + q[3] * u.w);
+			add(-2 - pid[v], ((q[0] * u.x + q[1] * u.y) + q[2] * u.z) + q[3] * u.w);
 			continue;
 		}
 		for (int k = 0; k < 4; ++k) {
 			float d = 0.0f;
 			for (int j = 0; j < 4; ++j) d += q[j] * albedo_basis(k, wavelength_n(wl, j));
-			atomicAdd(g + pid[v] + k, d);
+			add(pid[v] + k, d);
 		}
 	}
 }
@@ -431,21 +394,17 @@ static __device__ void grad_add(const RenderParams& rp, float* sg, const PathSoA
 // global gradient at the end.
 __device__ __forceinline__ void grad_begin(const RenderParams& rp, float* sg) {
 	if (!rp.grad || !rp.grad_in_smem) return;
-	for (int i = threadIdx.x; i < rp.param_count; i += blockDim.x) sg[i] = 0.0f;
+	const int words = rp.param_count * (rp.grad_in_smem == GRAD_SMEM64 ? 2 : 1);
+	for (int i = threadIdx.x; i < words; i += blockDim.x) sg[i] = 0.0f;
 	__syncthreads();
 }
 __device__ __forceinline__ void grad_end(const RenderParams& rp, float* sg) {
 	if (!rp.grad || !rp.grad_in_smem) return;
 	__syncthreads();
-	for (int i = threadIdx.x; i < rp.param_count; i += blockDim.x)
-		if (sg[i] != 0.0f) atomicAdd(rp.grad + i, sg[i]);
-}
-
-// Warp-wide work fetch: lane 0 takes the next 32 queue positions.
-__device__ __forceinline__ int fetch32(int* work) {
-	int base = 0;
-	if ((threadIdx.x & 31) == 0) base = atomicAdd(work, 32);
-	return __shfl_sync(0xffffffffu, base, 0);
+	for (int i = threadIdx.x; i < rp.param_count; i += blockDim.x) {
+		const float v = rp.grad_in_smem == GRAD_SMEM64 ? (float)reinterpret_cast<double*>(sg)[i] : sg[i];
+		if (v != 0.0f) atomicAdd(rp.grad + i, v);
+	}
 }
 
 // ---------------------------------------------------------------------
@@ -478,14 +437,7 @@ __global__ void __launch_bounds__(256) camera_gen_kernel(W w, HaltonDev hd, Wave
 	WorldRayD wr;
 	camera_ray(w.scene(rid), rx, ry, dx, dy, samp_c, samp_a, samp_b, &wr);
 	store_ray(wb.ray[0], wb.cap, slot, wr, rid << 1);
-	if (W::BATCH) ps.rid[slot] = (uint16_t)rid;
-	ps.smp[slot] = smp;
-	ps.dimstep[slot] = dim;  // step 0
-	ps.wl[slot] = wl;
-	ps.time[slot] = wr.time;
-	ps.last_pdf[slot] = 0.0f;
-	ps.col[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-	ps.fcol[slot] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+	ps.head[slot] = make_uint4(smp, dim, __float_as_uint(wl), __float_as_uint(0.0f));  // step 0
 	if (!W::BATCH && rp.dl_dxyz) {
 		// d(film sum)/d(col) of finish_path: XYZ_NORM_FAC / 4 * CIE(lambda_j)
 		const float* g = rp.dl_dxyz + 3 * pixel;
@@ -502,8 +454,9 @@ __global__ void __launch_bounds__(256) camera_gen_kernel(W w, HaltonDev hd, Wave
 // ---------------------------------------------------------------------
 // Traversal of a ray buffer (Tracer::trace, tracer/tracer.cpp:38-121)
 // ---------------------------------------------------------------------
-// n_dev == nullptr: n_host rays.  OCCL: occlusion rays, the result (1 =
-// blocked or no ray) goes to wb.occl by position.
+// `parts`: TRACE_CLOSEST, TRACE_OCCL or both, n rays each (n_dev == nullptr:
+// n_host), the closest-hit rays first.  A shadow ray's result (1 = blocked or
+// no ray) goes to wb.occl by position.
 //
 // Persistent warps with per-lane ray replacement: a lane whose ray is
 // finished takes the next ray of the queue between traversal steps instead
@@ -545,18 +498,43 @@ struct TraceCfg {
 // (root box, ray widths, bisection set-up).
 enum : int { KIND_IDLE = 0, KIND_NODES, KIND_ENTER, KIND_SIMPLE, KIND_BEGIN, KIND_PATCH, KIND_COUNT };
 
-template <class W, unsigned F, bool OCCL>
-__global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS) trace_wave_kernel(W w, WaveBufs wb, const float4* __restrict__ rb,
-                                                         const int* n_dev, int n_host, int* work,
-                                                         unsigned long long* counts, unsigned* status) {
+enum : unsigned { TRACE_CLOSEST = 1u, TRACE_OCCL = 2u };
+
+template <class W, unsigned F>
+__global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS)
+    trace_wave_kernel(W w, WaveBufs wb, const float4* __restrict__ rc, const float4* __restrict__ ro, const int* n_dev,
+                      int n_host, unsigned parts, int* work, unsigned long long* counts, unsigned* status) {
 	const int n = n_dev ? *n_dev : n_host;
+	const int nc = (parts & TRACE_CLOSEST) ? n : 0;
+	const unsigned total = (unsigned)nc + ((parts & TRACE_OCCL) ? (unsigned)n : 0u);
+	// traversal counters of the block: closest-hit rays, occlusion rays
+	__shared__ unsigned long long s_counts[2 * TC_COUNT];
+	if (threadIdx.x < 2 * TC_COUNT) s_counts[threadIdx.x] = 0ull;
+	__syncthreads();
 	const int lane = threadIdx.x & 31;
 	const unsigned lt_mask = (1u << lane) - 1u;
 	unsigned err = 0;
 	// per-lane work counters (TC_*), and the warp's own (lane 0 keeps them)
 	unsigned rays = 0, c_nodes = 0, c_leaves = 0, c_iters = 0, c_warp = 0, c_lanes = 0;
+	bool c_occl = nc == 0, w_occl = nc == 0;  // the kind of ray they are of
+	auto flush = [&]() {
+		unsigned long long* c = s_counts + (c_occl ? TC_COUNT : 0);
+		if (rays) atomicAdd(c + TC_RAYS, (unsigned long long)rays);
+		if (c_nodes) atomicAdd(c + TC_NODES, (unsigned long long)c_nodes);
+		if (c_leaves) atomicAdd(c + TC_LEAVES, (unsigned long long)c_leaves);
+		if (c_iters) atomicAdd(c + TC_PATCH_ITERS, (unsigned long long)c_iters);
+		rays = c_nodes = c_leaves = c_iters = 0;
+	};
+	auto flush_warp = [&]() {
+		unsigned long long* c = s_counts + (w_occl ? TC_COUNT : 0);
+		if (lane == 0 && c_warp) {
+			atomicAdd(c + TC_WARP_STEPS, (unsigned long long)c_warp);
+			atomicAdd(c + TC_LANE_STEPS, (unsigned long long)c_lanes);
+		}
+		c_warp = c_lanes = 0;
+	};
 	Trav<F, WaveIO> tr;
-	tr.io.rb = rb;
+	tr.io.rb = rc;
 	tr.io.wb = &wb;
 	tr.io.i = -1;
 	tr.pmode = PM_NONE;
@@ -566,27 +544,39 @@ __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS) t
 	while (true) {
 		const unsigned idle = __ballot_sync(0xffffffffu, tr.io.i < 0);
 		if (more && (__popc(idle) >= TraceCfg<F>::REFILL_MIN || idle == 0xffffffffu)) {
-			int base = 0;
-			if (lane == 0) base = atomicAdd(work, __popc(idle));
+			unsigned base = 0;
+			if (lane == 0) base = (unsigned)atomicAdd(work, __popc(idle));
 			base = __shfl_sync(0xffffffffu, base, 0);
-			if (base + __popc(idle) >= n) more = false;
+			if (base + __popc(idle) >= total) more = false;
+			if (!w_occl && base >= (unsigned)nc) {
+				flush_warp();
+				w_occl = true;
+			}
 			if (tr.io.i < 0) {
-				const int k = base + __popc(idle & lt_mask);
-				if (k < n) {
+				const unsigned q = base + __popc(idle & lt_mask);
+				if (q < total) {
+					const bool occl = q >= (unsigned)nc;
+					const int k = (int)(occl ? q - (unsigned)nc : q);
+					const float4* rb = occl ? ro : rc;
+					if (occl != c_occl) {
+						flush();
+						c_occl = occl;
+					}
 					const int tag = __float_as_int(rb[4 * (size_t)wb.cap + k].w);
 					if (tag & 1) {
-						// no ray: a shadow step without a light sample, or a
-						// path of a shorter render in a batch that has ended
-						if (OCCL) wb.occl[k] = 1;
+						// no ray: a shadow step without a light sample, or the
+						// last vertex of a path
+						if (occl) wb.occl[k] = 1;
 					} else {
 						rid = tag >> 1;
+						tr.io.rb = rb;
 						tr.io.i = k;
-						const float4 a = rb[k], b = rb[wb.cap + k];
-						tr.init(w.scene(rid), V3(a.x, a.y, a.z), V3(b.x, b.y, b.z), a.w, OCCL);
+						const float4 a = rb[k], b = rb[(size_t)wb.cap + k];
+						tr.init(w.scene(rid), V3(a.x, a.y, a.z), V3(b.x, b.y, b.z), a.w, occl);
 						++rays;
 						if (tr.cur == REF_EMPTY) {
 							// an empty scene
-							if (OCCL) wb.occl[k] = 0;
+							if (occl) wb.occl[k] = 0;
 							else wb.hit_i[k] = make_int4(-1, 0, 0, 0);
 							tr.io.i = -1;
 						}
@@ -647,184 +637,194 @@ __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS) t
 			}
 			if (!live) {
 				err |= tr.err;
-				if (OCCL) wb.occl[tr.io.i] = (tr.flags & RAY_HIT) ? 1 : 0;
+				if (tr.flags & RAY_OCCL) wb.occl[tr.io.i] = (tr.flags & RAY_HIT) ? 1 : 0;
 				else if (!(tr.flags & RAY_HIT)) wb.hit_i[tr.io.i] = make_int4(-1, 0, 0, 0);
 				tr.io.i = -1;
 			}
 		}
 	}
-	unsigned long long c[4] = {rays, c_nodes, c_leaves, c_iters};
-#pragma unroll
-	for (int k = 0; k < 4; ++k)
-		for (int o = 16; o > 0; o >>= 1) c[k] += __shfl_down_sync(0xffffffffu, c[k], o);
-	if (lane == 0) {
-		if (c[0]) atomicAdd(counts + TC_RAYS, c[0]);
-		if (c[1]) atomicAdd(counts + TC_NODES, c[1]);
-		if (c[2]) atomicAdd(counts + TC_LEAVES, c[2]);
-		if (c[3]) atomicAdd(counts + TC_PATCH_ITERS, c[3]);
-		if (c_warp) atomicAdd(counts + TC_WARP_STEPS, (unsigned long long)c_warp);
-		if (c_lanes) atomicAdd(counts + TC_LANE_STEPS, (unsigned long long)c_lanes);
-	}
+	flush();
+	flush_warp();
+	__syncthreads();
+	if (threadIdx.x < 2 * TC_COUNT && s_counts[threadIdx.x]) atomicAdd(counts + threadIdx.x, s_counts[threadIdx.x]);
 	if (err) atomicOr(status, err);
 }
 
 // ---------------------------------------------------------------------
-// After a camera (CAMERA) or bounce ray: update_path
-// (path_trace_integrator.cpp:251-272 and 273-302), then the shadow step of
-// next_ray_for_path (path_trace_integrator.cpp:126-184).
+// A path's step from vertex to vertex: update_path with the shadow ray's
+// result of the last vertex (path_trace_integrator.cpp:235-249) and with the
+// camera (CAMERA) or bounce ray's (251-272, 273-302), then next_ray_for_path's
+// shadow step (126-184) and bounce step (185-223) at the vertex met.
 //
-// Registers are capped at PSY_SHADE_MAXNREG a thread.  The kernel waits on
-// memory (path state, light-tree nodes, light and shader records) through
-// long dependent chains, and with the compiler's choice of about 225
-// registers only 8 warps fit an SM; at 32 registers 64 fit, and the spills
-// stay in L1.  Measured (640x360x4 many-light frame / flat 20,000- and
-// 50,000-primitive renders): 95.2 -> 84.4 ms and 45.2 -> 23.1 and
-// 96.5 -> 47.5 ms for the whole render, with caps of 168, 128, 96, 64, 48
-// and 40 registers in between.
+// The block works in phases that its warps enter together: surface, light
+// tree walk, light sample and shadow ray, bounce.  The kernel's code is some
+// hundred KB, and warps spread over all of it miss in the instruction cache
+// (25 of 35 stall cycles an instruction, with 64 warps an SM each on its
+// own); in phase they share the lines.
 // ---------------------------------------------------------------------
-#ifndef PSY_SHADE_MAXNREG
-#define PSY_SHADE_MAXNREG 32
-#endif
+//
+// 512 threads and 40 registers (3 blocks an SM; the spills stay in L1): the
+// 512x384x16 frame with 50,000 primitives takes 13.98 ms, 14.23 with 2
+// blocks of 64 registers, 14.30 with 4 of 32, 14.81 with 4 blocks of 256
+// threads, 17.49 with 8 of 128 (one kernel each for hit and shadow shading,
+// warps on their own: 18.23).
+#define PSY_SHADE_BLOCK 512
+#define PSY_SHADE_MIN_BLOCKS 3
 template <class W, bool CAMERA, unsigned F>
-__global__ void __maxnreg__(PSY_SHADE_MAXNREG) shade_hit_kernel(W w, HaltonDev hd, PathSoA ps, WaveBufs wb,
-                                                        const int* __restrict__ q_in, const int* n_dev, int n_host,
-                                                        int* q_out, int* n_out, int* work, unsigned* status) {
-	extern __shared__ float sgrad[];
+__global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
+    shade_kernel(W w, HaltonDev hd, PathSoA ps, WaveBufs wb, const float4* __restrict__ rin, float4* __restrict__ rout,
+                 float4* __restrict__ rshadow, const int* __restrict__ q_in, const int* n_dev, int n_host, int* q_out,
+                 int* n_out, unsigned* status) {
+	extern __shared__ __align__(16) float sgrad[];
 	if (!W::BATCH) grad_begin(w.render(0), sgrad);
 	const int lane = threadIdx.x & 31;
 	const int n = n_dev ? *n_dev : n_host;
 	unsigned err = 0;
-	while (true) {
-		const int base = fetch32(work);
-		if (base >= n) break;
-		const int i = base + lane;
-		bool live = false;
-		int slot = -1;
-		WorldRayD sray;
-		int stag = 1;
-		WorldRayD wr;
-		const int tag = i < n ? load_ray(wb.ray[0], wb.cap, i, &wr) : 1;
-		// (tag & 1): the path ended at its own path length before this step
-		// (a shorter render of a batch) and is only waiting in the queue
-		if (i < n && !(tag & 1)) {
-			slot = q_in ? q_in[i] : i;
-			const int rid = tag >> 1;
+	for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+		const int i = base + (int)threadIdx.x;
+		bool live = false, gtr = false, delta = false;
+		int slot = 0, rid = 0;
+		uint32_t smp = 0, dim = 0, step = 0;
+		float wl = 0.0f, time = 0.0f;
+		Vertex sh;
+		GtrVertex gv;
+		// ---- the results of the last vertex's rays
+		if (i < n) {
+			slot = CAMERA ? i : q_in[i];
+			const int tag = __float_as_int(rin[4 * (size_t)wb.cap + i].w);
+			rid = tag >> 1;
 			const DevScene& sc = w.scene(rid);
 			const RenderParams& rp = w.render(rid);
-			const uint32_t smp = ps.smp[slot];
-			const uint32_t ds = ps.dimstep[slot];
-			uint32_t dim = ds & 0xffffu;
-			uint32_t step = ds >> 16;
-			const float wl = ps.wl[slot];
-			const float time = ps.time[slot];
-			const float last_pdf = ps.last_pdf[slot];
-			Spec col = sp(ps.col[slot]);
-			const Spec fcol = sp(ps.fcol[slot]);
-			HitRec rec;
-			load_rec(wb, i, &rec);
-			bool done = false;
-			StoredHit sh;
-			if (rec.inst >= 0) {
-				hit_surface(sc, &rec);
-				int closure;
-				float ecol[3], lpdf;
-				make_stored<F>(sc, rec, wr, rp.ident_inv, &sh, &closure, ecol, &lpdf, &err);
-				const int vtx = (int)(step >> 1);  // index of this path vertex
-				if (closure == CLOSURE_EMIT) {
-					done = true;
-					Spec e = rgb_to_spec(ecol, wl);
-					const int lp = emission_param(rp, rec.obj);
-					if (lp >= 0)
-						for (int k = 0; k < 4; ++k) e.e[k] *= rp.params[lp];
-					Spec C;
-					if (!CAMERA && last_pdf != 0.0f) {
-						const float mis_inv_pdf = power_heuristic(last_pdf, lpdf) / last_pdf;
-						for (int k = 0; k < 4; ++k) C.e[k] = ((fcol.e[k] * last_pdf) * e.e[k]) * mis_inv_pdf;
-					} else {
-						for (int k = 0; k < 4; ++k) C.e[k] = fcol.e[k] * e.e[k];
-					}
-					for (int k = 0; k < 4; ++k) col.e[k] += C.e[k];
-					if (!W::BATCH && rp.grad) {
-						// the same contribution without its parameterised factors
-						const Spec e0 = rgb_to_spec(ecol, wl);
-						const Spec fx = sp(ps.fexcl[slot]);
-						Spec B;
-						if (!CAMERA && last_pdf != 0.0f) {
-							const float mis_inv_pdf = power_heuristic(last_pdf, lpdf) / last_pdf;
-							for (int k = 0; k < 4; ++k) B.e[k] = ((fx.e[k] * last_pdf) * e0.e[k]) * mis_inv_pdf;
-						} else {
-							for (int k = 0; k < 4; ++k) B.e[k] = fx.e[k] * e0.e[k];
-						}
-						grad_add(rp, sgrad, ps, slot, vtx, B, lp, wl);
-					}
-				} else if (closure != CLOSURE_LAMBERT && closure != CLOSURE_GTR) {
-					done = true;  // closures outside the supported set end the path
-				} else {
-					sh.pid = (rp.params && rec.shader >= 0) ? rp.shader_param[rec.shader] : -1;
-					if (!W::BATCH && rp.grad && vtx < PSY_ADJ_MAX_VERTS) {
-						Spec a = Spec{};
-						if (sh.pid >= 0) {
-							a = albedo_spec(rp.params + sh.pid, wl);
-						} else if (sh.pid < -1) {
-							const Spec up = rgb_to_spec(sh.col, wl);
-							const float q = rp.params[-2 - sh.pid];
-							for (int k = 0; k < 4; ++k) a.e[k] = up.e[k] * q;
-							ps.vdsc[slot * PSY_ADJ_MAX_VERTS + vtx] = f4(up);
-						}
-						ps.vpid[slot * PSY_ADJ_MAX_VERTS + vtx] = sh.pid;
-						ps.valb[slot * PSY_ADJ_MAX_VERTS + vtx] = f4(a);
-					}
+			const uint4 head = ps.head[slot];
+			smp = head.x;
+			dim = head.y & 0xffffu;
+			step = head.y >> 16;
+			wl = __uint_as_float(head.z);
+			const float last_pdf = __uint_as_float(head.w);
+			Spec col = Spec{};
+			if (!CAMERA) {
+				col = sp(ps.col[slot]);
+				if (wb.occl[i] == 0) {
+					const Spec c = sp(ps.lcol[slot]);
+					for (int k = 0; k < 4; ++k) col.e[k] += c.e[k];
+					if (!W::BATCH && rp.grad)
+						grad_add(rp, sgrad, ps, slot, (int)(step >> 1), sp(ps.nee_base[slot]), ps.nee_param[slot], wl);
 				}
-			} else {
-				done = true;
-				const Spec bg = rgb_to_spec(sc.background, wl);
-				for (int k = 0; k < 4; ++k) col.e[k] += fcol.e[k] * bg.e[k];
 			}
-			step++;
-			if (step == rp.path_length * 2) done = true;
-			const bool gtr = !done && sh.gtr >= 0;
-			const Gtr gp = gtr ? gtr_of(sc.shaders[sh.gtr]) : Gtr{};
-			if (done) {
-				finish_path(ps, slot, col, wl);
-			} else if (gtr && gtr_is_delta(gp)) {
+			if (!(tag & 1)) {  // (tag & 1): the last vertex sent no bounce ray
+				WorldRayD wr;
+				load_ray(rin, wb.cap, i, &wr);
+				time = wr.time;
+				HitRec rec;
+				load_rec(wb, i, &rec);
+				const Spec fcol = CAMERA ? Spec{{1.0f, 1.0f, 1.0f, 1.0f}} : sp(ps.fcol[slot]);
+				if (rec.inst >= 0) {
+					hit_surface(sc, &rec);
+					int closure;
+					float lpdf;
+					make_vertex<F>(sc, rec, wr, rp.ident_inv, &sh, &gv, &closure, &lpdf, &err);
+					const int vtx = (int)(step >> 1);  // index of this path vertex
+					if (closure == CLOSURE_EMIT) {
+						const Spec e0 = rgb_to_spec(sh.col, wl);
+						Spec e = e0;
+						const int lp = emission_param(rp, rec.obj);
+						if (lp >= 0)
+							for (int k = 0; k < 4; ++k) e.e[k] *= rp.params[lp];
+						const bool mis = !CAMERA && last_pdf != 0.0f;
+						const float mis_inv_pdf = mis ? power_heuristic(last_pdf, lpdf) / last_pdf : 0.0f;
+						Spec C;
+						for (int k = 0; k < 4; ++k)
+							C.e[k] = mis ? ((fcol.e[k] * last_pdf) * e.e[k]) * mis_inv_pdf : fcol.e[k] * e.e[k];
+						for (int k = 0; k < 4; ++k) col.e[k] += C.e[k];
+						if (!W::BATCH && rp.grad) {
+							// the same contribution without its parameterised factors
+							const Spec fx = sp(ps.fexcl[slot]);
+							Spec B;
+							for (int k = 0; k < 4; ++k)
+								B.e[k] = mis ? ((fx.e[k] * last_pdf) * e0.e[k]) * mis_inv_pdf : fx.e[k] * e0.e[k];
+							grad_add(rp, sgrad, ps, slot, vtx, B, lp, wl);
+						}
+					} else if (closure == CLOSURE_LAMBERT || closure == CLOSURE_GTR) {
+						// (closures outside the supported set end the path)
+						live = true;
+						sh.pid = (rp.params && rec.shader >= 0) ? rp.shader_param[rec.shader] : -1;
+						gtr = sh.gtr >= 0;
+						delta = gtr && gtr_is_delta(gtr_of(sc.shaders[sh.gtr]));
+						if (!W::BATCH && rp.grad && vtx < PSY_ADJ_MAX_VERTS) {
+							Spec a = Spec{};
+							if (sh.pid >= 0) {
+								a = albedo_spec(rp.params + sh.pid, wl);
+							} else if (sh.pid < -1) {
+								const Spec up = rgb_to_spec(sh.col, wl);
+								const float q = rp.params[-2 - sh.pid];
+								for (int k = 0; k < 4; ++k) a.e[k] = up.e[k] * q;
+								ps.vdsc[slot * PSY_ADJ_MAX_VERTS + vtx] = f4(up);
+							}
+							ps.vpid[slot * PSY_ADJ_MAX_VERTS + vtx] = sh.pid;
+							ps.valb[slot * PSY_ADJ_MAX_VERTS + vtx] = f4(a);
+						}
+					}
+				} else {
+					const Spec bg = rgb_to_spec(sc.background, wl);
+					for (int k = 0; k < 4; ++k) col.e[k] += fcol.e[k] * bg.e[k];
+				}
+			}
+			ps.col[slot] = f4(col);
+		}
+		// ---- the live paths' places in the next queue (ballot compaction)
+		const unsigned m = __ballot_sync(0xffffffffu, live);
+		int j = 0;
+		if (lane == 0 && m) j = atomicAdd(n_out, __popc(m));
+		j = __shfl_sync(0xffffffffu, j, 0) + __popc(m & ((1u << lane) - 1u));
+		if (live) q_out[j] = slot;
+		__syncthreads();
+		// ---- light tree walk
+		LightQuery q;
+		q.obj = -1;
+		q.valid = false;
+		q.has_xform = false;
+		if (live && !delta) {
+			const DevScene& sc = w.scene(rid);
+			q.n = sampler_get(hd, smp, dim);
+			q.u = sampler_get(hd, smp, dim + 1);
+			q.v = sampler_get(hd, smp, dim + 2);
+			q.pos = sh.p;
+			// lq_nor = geo.n, flipped for back-facing hits
+			q.nor = (sh.bf != 0.0f) ? sh.n * -1.0f : sh.n;
+			q.d = sh.d;
+			q.wavelength = wl;
+			q.time = time;
+			q.id = 0;
+			q.selection_pdf = 1.0f;
+			q.light_sample_pdf = 1.0f;
+			q.gtr = gtr;
+			if (gtr) q.gp = gtr_of(sc.shaders[sh.gtr]);
+			light_tree_pick<F>(sc, &q);
+		}
+		__syncthreads();
+		// ---- light sample and shadow ray
+		if (live) {
+			const DevScene& sc = w.scene(rid);
+			const RenderParams& rp = w.render(rid);
+			float4 contrib = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+			if (delta) {
 				// a delta closure takes no light sample and no sampler draws;
 				// the reference traces the step's ray again, and its result
 				// adds nothing (path_trace_integrator.cpp:131-184, 235-249)
-				sray = wr;
-				sray.occl = true;
-				stag = rid << 1;
-				ps.dimstep[slot] = (dim & 0xffffu) | (step << 16);
-				ps.col[slot] = f4(col);
-				ps.lcol[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+				const size_t cap = wb.cap;
+				for (int k = 0; k < 4; ++k) rshadow[k * cap + j] = rin[k * cap + i];
+				float4 last = rin[4 * cap + i];
+				last.w = __int_as_float(rid << 1);
+				rshadow[4 * cap + j] = last;
 				if (!W::BATCH && rp.grad) {
 					ps.nee_param[slot] = -1;
 					ps.nee_base[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 				}
-				store_hit(ps, slot, sh);
-				live = true;
 			} else {
-				// shadow step: light-tree sample and shadow ray
-				LightQuery q;
-				q.n = sampler_get(hd, smp, dim++);
-				q.u = sampler_get(hd, smp, dim++);
-				q.v = sampler_get(hd, smp, dim++);
-				q.pos = sh.p;
-				// lq_nor = geo.n, flipped for back-facing hits
-				q.nor = (sh.bf != 0.0f) ? sh.n * -1.0f : sh.n;
-				q.d = sh.d;
-				q.wavelength = wl;
-				q.time = time;
-				q.has_xform = false;
-				q.id = 0;
-				q.obj = -1;
-				q.selection_pdf = 1.0f;
-				q.light_sample_pdf = 1.0f;
-				q.gtr = gtr;
-				q.gp = gp;
-				light_tree_sample(sc, &q, rp.ident_inv);
-				float4 contrib = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+				light_emit<F>(sc, &q, rp.ident_inv);
+				dim += 3;
 				if (q.valid) {
-					const float bsdf_pdf = gtr ? gtr_pdf(gp, sh.d, q.to_light, sh.n) : lambert_pdf(sh.d, q.to_light, sh.n);
+					const float bsdf_pdf = gtr ? gtr_pdf(q.gp, sh.d, q.to_light, sh.n) : lambert_pdf(sh.d, q.to_light, sh.n);
 					const float mis_inv_pdf = power_heuristic(q.light_sample_pdf, bsdf_pdf) / q.light_sample_pdf;
 					const float lc = (float)rp.light_count;
 					Spec lcol;
@@ -833,15 +833,17 @@ __global__ void __maxnreg__(PSY_SHADE_MAXNREG) shade_hit_kernel(W w, HaltonDev h
 					if (lp >= 0)
 						for (int k = 0; k < 4; ++k) lcol.e[k] *= rp.params[lp];
 					if (!W::BATCH && rp.grad) ps.nee_param[slot] = lp;
+					WorldRayD sray;
 					sray.o = sh.p + sh.off;
 					sray.d = (q.to_light - sh.off) * 0.9995f;
 					sray.time = time;
-					sray.occl = true;
-					if (gtr) gtr_propagate_differentials(sh, &sray);
+					if (gtr) gtr_propagate_differentials(sh, gv, &sray);
 					else propagate_differentials(sh, &sray);
+					store_ray(rshadow, wb.cap, j, sray, rid << 1);
 					// the light's contribution if the shadow ray is not blocked
 					// (update_path, shadow result: path_trace_integrator.cpp:235-249)
-					const Spec fac = gtr ? gtr_eval(gp, sh.d, sray.d, sh.n, wl) : lambert_eval_p(rp, sh, sray.d, wl);
+					const Spec fac = gtr ? gtr_eval(q.gp, sh.d, sray.d, sh.n, wl) : lambert_eval_p(rp, sh, sray.d, wl);
+					const Spec fcol = CAMERA ? Spec{{1.0f, 1.0f, 1.0f, 1.0f}} : sp(ps.fcol[slot]);
 					Spec c;
 					for (int k = 0; k < 4; ++k) c.e[k] = (fcol.e[k] * lcol.e[k]) * fac.e[k];
 					contrib = f4(c);
@@ -855,130 +857,108 @@ __global__ void __maxnreg__(PSY_SHADE_MAXNREG) shade_hit_kernel(W w, HaltonDev h
 							b.e[k] = (fx.e[k] * (((q.spec.e[k] * mis_inv_pdf) * lc) / q.selection_pdf)) * f0.e[k];
 						ps.nee_base[slot] = f4(b);
 					}
-					stag = rid << 1;
 				} else {
 					err |= ERRF_NOLIGHT;
-					sray.o = V3(0.0f); sray.d = V3(0.0f, 0.0f, 1.0f); sray.time = time;
-					sray.odx = sray.ody = sray.ddx = sray.ddy = V3(0.0f);
-					stag = (rid << 1) | 1;
+					rshadow[4 * (size_t)wb.cap + j] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float((rid << 1) | 1));
 				}
-				ps.dimstep[slot] = (dim & 0xffffu) | (step << 16);
-				ps.col[slot] = f4(col);
-				ps.lcol[slot] = contrib;
-				store_hit(ps, slot, sh);
-				live = true;
 			}
+			ps.lcol[slot] = contrib;
 		}
-		// ballot compaction of the live paths into the next queue
-		const unsigned m = __ballot_sync(0xffffffffu, live);
-		int out_base = 0;
-		if (lane == 0 && m) out_base = atomicAdd(n_out, __popc(m));
-		out_base = __shfl_sync(0xffffffffu, out_base, 0);
+		__syncthreads();
+		// ---- bounce
 		if (live) {
-			const int j = out_base + __popc(m & ((1u << lane) - 1u));
-			q_out[j] = slot;
-			store_ray(wb.ray[1], wb.cap, j, sray, stag);
+			const RenderParams& rp = w.render(rid);
+			step += 2;
+			float pdf = 0.0f;
+			if (step == rp.path_length * 2) {
+				// the path's last vertex: only its shadow ray is left
+				rout[4 * (size_t)wb.cap + j] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float((rid << 1) | 1));
+			} else {
+				Spec fcol = CAMERA ? Spec{{1.0f, 1.0f, 1.0f, 1.0f}} : sp(ps.fcol[slot]);
+				// The reference passes two sampler.next() calls as arguments; g++
+				// evaluates them right to left, so the second draw is `si` and the
+				// first `sj`.
+				const float sj = sampler_get(hd, smp, dim++);
+				const float si = sampler_get(hd, smp, dim++);
+				WorldRayD wr;
+				wr.o = sh.p + sh.off;
+				wr.time = time;
+				V3 out;
+				Spec filter;
+				if (gtr) {
+					const Gtr gp = gtr_of(w.scene(rid).shaders[sh.gtr]);
+					gtr_sample(gp, sh.d, sh.n, si, sj, wl, &out, &filter, &pdf);
+					wr.d = out;
+					gtr_propagate_differentials(sh, gv, &wr);
+				} else {
+					V3 nn = normalized(sh.n);
+					if (dot(nn, sh.d) > 0.0f) nn = nn * -1.0f;
+					const V3 dir = cosine_sample_hemisphere(si, sj);
+					pdf = dir.z * (float)PSY_INV_PI_D;
+					out = zup_to_vec(dir, nn);
+					filter = lambert_eval_p(rp, sh, out, wl);
+					wr.d = out;
+					propagate_differentials(sh, &wr);
+				}
+				store_ray(rout, wb.cap, j, wr, rid << 1);
+				if (!delta) {
+					if (pdf < 0.00001f) pdf = 0.00001f;
+					for (int k = 0; k < 4; ++k) fcol.e[k] *= filter.e[k] / pdf;
+				} else {
+					for (int k = 0; k < 4; ++k) fcol.e[k] *= filter.e[k];
+				}
+				if (!W::BATCH && rp.grad) {
+					// the path weight without the parameterised albedos
+					Spec fx = sp(ps.fexcl[slot]);
+					const float cs = gtr ? 0.0f : lambert_cos(sh.d, out, sh.n);
+					for (int k = 0; k < 4; ++k) fx.e[k] *= (sh.pid != -1 ? cs : filter.e[k]) / (delta ? 1.0f : pdf);
+					ps.fexcl[slot] = f4(fx);
+				}
+				if (delta) pdf = 0.0f;  // last_pdf 0: the next emitter hit takes no MIS weight
+				ps.fcol[slot] = f4(fcol);
+			}
+			ps.head[slot] = make_uint4(smp, (dim & 0xffffu) | (step << 16), __float_as_uint(wl), __float_as_uint(pdf));
 		}
+		__syncthreads();
 	}
 	if (!W::BATCH) grad_end(w.render(0), sgrad);
 	if (err) atomicOr(status, err);
 }
 
-// ---------------------------------------------------------------------
-// After the shadow ray: update_path (path_trace_integrator.cpp:235-249),
-// then the bounce step of next_ray_for_path (path_trace_integrator.cpp:185-223).
-// Paths keep their queue position.
-// ---------------------------------------------------------------------
+// The shadow rays of the wave's last vertices.
 template <class W>
-__global__ void __launch_bounds__(256) shade_shadow_kernel(W w, HaltonDev hd, PathSoA ps, WaveBufs wb,
-                                                           const int* __restrict__ q_in, const int* n_dev, int* work) {
-	extern __shared__ float sgrad[];
+__global__ void __launch_bounds__(256) shade_last_kernel(W w, PathSoA ps, WaveBufs wb, const int* __restrict__ q_in,
+                                                         const int* n_dev) {
+	extern __shared__ __align__(16) float sgrad[];
 	if (!W::BATCH) grad_begin(w.render(0), sgrad);
 	const int n = *n_dev;
-	while (true) {
-		const int base = fetch32(work);
-		if (base >= n) break;
-		const int i = base + (threadIdx.x & 31);
-		if (i >= n) continue;
+	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+		if (wb.occl[i] != 0) continue;
 		const int slot = q_in[i];
-		const int rid = W::BATCH ? (int)ps.rid[slot] : 0;
-		const uint32_t smp = ps.smp[slot];
-		const uint32_t ds = ps.dimstep[slot];
-		uint32_t dim = ds & 0xffffu;
-		uint32_t step = ds >> 16;
-		const float wl = ps.wl[slot];
 		Spec col = sp(ps.col[slot]);
-		const RenderParams& rp = w.render(rid);
-		if (wb.occl[i] == 0) {
-			const Spec c = sp(ps.lcol[slot]);
-			for (int k = 0; k < 4; ++k) col.e[k] += c.e[k];
-			if (!W::BATCH && rp.grad)
-				grad_add(rp, sgrad, ps, slot, (int)(step >> 1) + 1, sp(ps.nee_base[slot]), ps.nee_param[slot], wl);
-		}
-		step++;
-		if (step == rp.path_length * 2) {
-			finish_path(ps, slot, col, wl);
-			// paths of longer renders in the same batch keep going: leave a
-			// "no ray" mark so later steps pass over this queue position
-			WorldRayD none;
-			none.o = none.d = none.odx = none.ody = none.ddx = none.ddy = V3(0.0f);
-			none.time = 0.0f;
-			store_ray(wb.ray[0], wb.cap, i, none, (rid << 1) | 1);
-			continue;
-		}
-		StoredHit sh;
-		load_hit(ps, slot, &sh);
-		Spec fcol = sp(ps.fcol[slot]);
-		// The reference passes two sampler.next() calls as arguments; g++
-		// evaluates them right to left, so the second draw is `si` and the
-		// first `sj`.
-		const float sj = sampler_get(hd, smp, dim++);
-		const float si = sampler_get(hd, smp, dim++);
-		WorldRayD wr;
-		wr.o = sh.p + sh.off;
-		wr.time = ps.time[slot];
-		wr.occl = false;
-		V3 out;
-		float pdf;
-		Spec filter;
-		bool delta = false;
-		if (sh.gtr >= 0) {
-			const Gtr gp = gtr_of(w.scene(rid).shaders[sh.gtr]);
-			gtr_sample(gp, sh.d, sh.n, si, sj, wl, &out, &filter, &pdf);
-			delta = gtr_is_delta(gp);
-			wr.d = out;
-			gtr_propagate_differentials(sh, &wr);
-		} else {
-			V3 nn = normalized(sh.n);
-			if (dot(nn, sh.d) > 0.0f) nn = nn * -1.0f;
-			const V3 dir = cosine_sample_hemisphere(si, sj);
-			pdf = dir.z * (float)PSY_INV_PI_D;
-			out = zup_to_vec(dir, nn);
-			filter = lambert_eval_p(rp, sh, out, wl);
-			wr.d = out;
-			propagate_differentials(sh, &wr);
-		}
-		if (!delta) {
-			if (pdf < 0.00001f) pdf = 0.00001f;
-			for (int k = 0; k < 4; ++k) fcol.e[k] *= filter.e[k] / pdf;
-		} else {
-			for (int k = 0; k < 4; ++k) fcol.e[k] *= filter.e[k];
-			pdf = 0.0f;  // last_pdf 0: the next emitter hit takes no MIS weight
-		}
-		if (!W::BATCH && rp.grad) {
-			// the path weight without the parameterised albedos
-			Spec fx = sp(ps.fexcl[slot]);
-			const float cs = sh.gtr >= 0 ? 0.0f : lambert_cos(sh.d, out, sh.n);
-			for (int k = 0; k < 4; ++k) fx.e[k] *= (sh.pid != -1 ? cs : filter.e[k]) / (delta ? 1.0f : pdf);
-			ps.fexcl[slot] = f4(fx);
-		}
-		store_ray(wb.ray[0], wb.cap, i, wr, rid << 1);
-		ps.dimstep[slot] = (dim & 0xffffu) | (step << 16);
+		const Spec c = sp(ps.lcol[slot]);
+		for (int k = 0; k < 4; ++k) col.e[k] += c.e[k];
 		ps.col[slot] = f4(col);
-		ps.fcol[slot] = f4(fcol);
-		ps.last_pdf[slot] = pdf;
+		if (!W::BATCH && w.render(0).grad) {
+			const uint4 head = ps.head[slot];
+			grad_add(w.render(0), sgrad, ps, slot, (int)(head.y >> 17), sp(ps.nee_base[slot]), ps.nee_param[slot],
+			         __uint_as_float(head.z));
+		}
 	}
 	if (!W::BATCH) grad_end(w.render(0), sgrad);
+}
+
+// The finished paths' film samples: Color_XYZ(col) * XYZ_NORM_FAC.
+static __global__ void __launch_bounds__(256) sample_xyz_kernel(PathSoA ps, int paths) {
+	const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+	if (slot >= paths) return;
+	float xyz[3];
+	spec_to_xyz(sp(ps.col[slot]), __uint_as_float(ps.head[slot].z), xyz);
+	float3 o;
+	o.x = xyz[0] * XYZ_NORM_FAC;
+	o.y = xyz[1] * XYZ_NORM_FAC;
+	o.z = xyz[2] * XYZ_NORM_FAC;
+	reinterpret_cast<float3*>(ps.sample)[slot] = o;
 }
 
 // Adds each pixel's samples, in sample order, to its render's film; rejects
@@ -1025,7 +1005,7 @@ static int persistent_grid(K kernel, int block) {
 struct WaveGrids {
 	int block = 0;
 	int trace_b = 0;  // traversal block size
-	int trace_c, trace_o, shade_c, shade_b, shadow;
+	int trace, shade_c, shade_b, last;
 };
 
 template <class W, unsigned F>
@@ -1037,21 +1017,18 @@ static const WaveGrids& grids_for(int block) {
 		WaveGrids n;
 		n.block = block;
 		n.trace_b = TraceCfg<F>::launch_block(block);
-		n.trace_c = persistent_grid(trace_wave_kernel<W, F, false>, n.trace_b);
-		n.trace_o = persistent_grid(trace_wave_kernel<W, F, true>, n.trace_b);
-		n.shade_c = persistent_grid(shade_hit_kernel<W, true, F>, block);
-		n.shade_b = persistent_grid(shade_hit_kernel<W, false, F>, block);
-		n.shadow = persistent_grid(shade_shadow_kernel<W>, block);
+		n.trace = persistent_grid(trace_wave_kernel<W, F>, n.trace_b);
+		n.shade_c = persistent_grid(shade_kernel<W, true, F>, PSY_SHADE_BLOCK);
+		n.shade_b = persistent_grid(shade_kernel<W, false, F>, PSY_SHADE_BLOCK);
+		n.last = persistent_grid(shade_last_kernel<W>, 256);
 		g[k] = n;
 	}
 	return g[k];
 }
 
-// Counters per wave: [0] camera trace work, [1] camera shade work, [2]
-// live paths after the camera step; then per bounce eight: [0] shadow trace
-// work, [1] shadow shade work, [2] bounce trace work, [3] bounce shade work,
-// [4] live paths after the bounce.
-inline int wave_counter_count(uint32_t path_length) { return 4 + 8 * (int)path_length; }
+// Counters per wave, two a stage (vertices 0 .. path_length, the last stage
+// being the last shadow rays): traversal work, live paths after the stage.
+inline int wave_counter_count(uint32_t path_length) { return 2 * ((int)path_length + 1); }
 
 template <class W, unsigned F>
 void launch_wave(const W& w, uint32_t path_length, const HaltonDev& hd, const WaveRange& wv,
@@ -1068,37 +1045,36 @@ void launch_wave(const W& w, uint32_t path_length, const HaltonDev& hd, const Wa
 	int* c = wq.counters;
 	cudaMemsetAsync(c, 0, sizeof(int) * wave_counter_count(path_length), st);
 	camera_gen_kernel<W><<<(P + block - 1) / block, block, 0, st>>>(w, hd, wv, ps, wb);
-	tstart();
-	trace_wave_kernel<W, F, false><<<g.trace_c, g.trace_b, 0, st>>>(w, wb, wb.ray[0], nullptr, P, c + 0, wq.rays, status);
-	tstop();
-	// camera hit -> shadow rays of the live paths into queue 0
-	int* q = wq.q0;
-	int* n = c + 2;
-	shade_hit_kernel<W, true, F><<<g.shade_c, block, gsmem, st>>>(w, hd, ps, wb, nullptr, nullptr, P, q, n, c + 1,
-	                                                             status);
-	*launches += 3;
-	c += 4;
-	for (uint32_t b = 0; b < path_length; ++b) {
+	const float4* rin = wb.ray[0];
+	float4 *rout = wb.ray[2], *rshadow = wb.ray[1];
+	int *q = nullptr, *n = nullptr;  // the stage's queue (null: every path of the wave)
+	auto grid = [&](int full, int threads) {
+		const int need = (P + threads - 1) / threads;
+		return need < full ? need : full;
+	};
+	for (uint32_t v = 0; v <= path_length; ++v, c += 2) {
+		const unsigned parts = v == 0 ? TRACE_CLOSEST : v == path_length ? TRACE_OCCL : TRACE_CLOSEST | TRACE_OCCL;
 		tstart();
-		trace_wave_kernel<W, F, true><<<g.trace_o, g.trace_b, 0, st>>>(w, wb, wb.ray[1], n, 0, c + 0, wq.rays + TC_COUNT,
-		                                                          status);
-		tstop();
-		shade_shadow_kernel<W><<<g.shadow, block, gsmem, st>>>(w, hd, ps, wb, q, n, c + 1);
-		*launches += 2;
-		if (b + 1 == path_length) break;  // the last shadow step ends every path
-		tstart();
-		trace_wave_kernel<W, F, false><<<g.trace_c, g.trace_b, 0, st>>>(w, wb, wb.ray[0], n, 0, c + 2, wq.rays, status);
+		trace_wave_kernel<W, F><<<g.trace, g.trace_b, 0, st>>>(w, wb, rin, rshadow, n, P, parts, c, wq.rays, status);
 		tstop();
 		int* q2 = (q == wq.q0) ? wq.q1 : wq.q0;
-		int* n2 = c + 4;
-		shade_hit_kernel<W, false, F><<<g.shade_b, block, gsmem, st>>>(w, hd, ps, wb, q, n, 0, q2, n2, c + 3, status);
-		*launches += 2;
+		if (v == path_length)
+			shade_last_kernel<W><<<grid(g.last, 256), 256, gsmem, st>>>(w, ps, wb, q, n);
+		else if (v == 0)
+			shade_kernel<W, true, F><<<grid(g.shade_c, PSY_SHADE_BLOCK), PSY_SHADE_BLOCK, gsmem, st>>>(
+			    w, hd, ps, wb, rin, rout, rshadow, nullptr, nullptr, P, q2, c + 1, status);
+		else
+			shade_kernel<W, false, F><<<grid(g.shade_b, PSY_SHADE_BLOCK), PSY_SHADE_BLOCK, gsmem, st>>>(
+			    w, hd, ps, wb, rin, rout, rshadow, q, n, 0, q2, c + 1, status);
+		float4* t = const_cast<float4*>(rin);
+		rin = rout;
+		rout = t;
 		q = q2;
-		n = n2;
-		c += 8;
+		n = c + 1;
 	}
+	sample_xyz_kernel<<<(P + 255) / 256, 256, 0, st>>>(ps, P);
 	film_reduce_kernel<W><<<(wv.pixels + 127) / 128, 128, 0, st>>>(w, wv, ps);
-	++*launches;
+	*launches += 5 + 2 * path_length;
 }
 
 }  // namespace psy

