@@ -541,9 +541,15 @@ __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS)
 	tr.cur = REF_NONE;
 	int rid = 0;
 	bool more = true;  // the queue may still hold rays (warp-uniform)
+	// a queue too short to fill every lane is spread over all warps: each
+	// runs on fewer lanes, whose rays wait less for one another
+	const unsigned warps = gridDim.x * (blockDim.x >> 5);
+	const unsigned per = (total + warps - 1) / warps;
+	const unsigned use = per < 32u ? (1u << per) - 1u : 0xffffffffu;
+	const int refill = min(TraceCfg<F>::REFILL_MIN, __popc(use));
 	while (true) {
-		const unsigned idle = __ballot_sync(0xffffffffu, tr.io.i < 0);
-		if (more && (__popc(idle) >= TraceCfg<F>::REFILL_MIN || idle == 0xffffffffu)) {
+		const unsigned idle = __ballot_sync(0xffffffffu, tr.io.i < 0) & use;
+		if (more && (__popc(idle) >= refill || idle == use)) {
 			unsigned base = 0;
 			if (lane == 0) base = (unsigned)atomicAdd(work, __popc(idle));
 			base = __shfl_sync(0xffffffffu, base, 0);
@@ -552,7 +558,7 @@ __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS)
 				flush_warp();
 				w_occl = true;
 			}
-			if (tr.io.i < 0) {
+			if (tr.io.i < 0 && ((use >> lane) & 1u)) {
 				const unsigned q = base + __popc(idle & lt_mask);
 				if (q < total) {
 					const bool occl = q >= (unsigned)nc;
@@ -992,6 +998,13 @@ __global__ void film_reduce_kernel(W w, WaveRange wv, PathSoA ps) {
 // ---------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------
+static int sm_count() {
+	int dev = 0, sms = 1;
+	cudaGetDevice(&dev);
+	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+	return sms;
+}
+
 // Persistent grid: resident blocks of `kernel` at `block` threads x SMs.
 template <typename K>
 static int persistent_grid(K kernel, int block) {
@@ -1005,7 +1018,7 @@ static int persistent_grid(K kernel, int block) {
 struct WaveGrids {
 	int block = 0;
 	int trace_b = 0;  // traversal block size
-	int trace, shade_c, shade_b, last;
+	int trace, shade_c, shade_b, last, sms;
 };
 
 template <class W, unsigned F>
@@ -1021,6 +1034,7 @@ static const WaveGrids& grids_for(int block) {
 		n.shade_c = persistent_grid(shade_kernel<W, true, F>, PSY_SHADE_BLOCK);
 		n.shade_b = persistent_grid(shade_kernel<W, false, F>, PSY_SHADE_BLOCK);
 		n.last = persistent_grid(shade_last_kernel<W>, 256);
+		n.sms = sm_count();
 		g[k] = n;
 	}
 	return g[k];
@@ -1052,6 +1066,12 @@ void launch_wave(const W& w, uint32_t path_length, const HaltonDev& hd, const Wa
 		const int need = (P + threads - 1) / threads;
 		return need < full ? need : full;
 	};
+	// shading blocks: smaller ones for waves that would leave SMs without any
+	// (80x60 preview: 443 us with 512-thread blocks on 10 SMs, 345 with 64 and
+	// the rays spread over all warps)
+	int sb = PSY_SHADE_BLOCK;
+	while (sb > 64 && (P + sb - 1) / sb < 2 * g.sms) sb >>= 1;
+	const int per = PSY_SHADE_BLOCK / sb;
 	for (uint32_t v = 0; v <= path_length; ++v, c += 2) {
 		const unsigned parts = v == 0 ? TRACE_CLOSEST : v == path_length ? TRACE_OCCL : TRACE_CLOSEST | TRACE_OCCL;
 		tstart();
@@ -1061,10 +1081,10 @@ void launch_wave(const W& w, uint32_t path_length, const HaltonDev& hd, const Wa
 		if (v == path_length)
 			shade_last_kernel<W><<<grid(g.last, 256), 256, gsmem, st>>>(w, ps, wb, q, n);
 		else if (v == 0)
-			shade_kernel<W, true, F><<<grid(g.shade_c, PSY_SHADE_BLOCK), PSY_SHADE_BLOCK, gsmem, st>>>(
+			shade_kernel<W, true, F><<<grid(g.shade_c * per, sb), sb, gsmem, st>>>(
 			    w, hd, ps, wb, rin, rout, rshadow, nullptr, nullptr, P, q2, c + 1, status);
 		else
-			shade_kernel<W, false, F><<<grid(g.shade_b, PSY_SHADE_BLOCK), PSY_SHADE_BLOCK, gsmem, st>>>(
+			shade_kernel<W, false, F><<<grid(g.shade_b * per, sb), sb, gsmem, st>>>(
 			    w, hd, ps, wb, rin, rout, rshadow, q, n, 0, q2, c + 1, status);
 		float4* t = const_cast<float4*>(rin);
 		rin = rout;

@@ -60,9 +60,11 @@ struct TraceKernelRegs {
 
 template <unsigned F>
 __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc, RaySoA rays, HitSoA hits,
-                                                                   uint32_t n, unsigned* status) {
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
+                                                                   uint32_t n, int lanes, unsigned* status) {
+	// `lanes` rays a warp (a power of two)
+	const int lane = threadIdx.x & 31;
+	const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (uint32_t)lanes + (uint32_t)lane;
+	if (lane >= lanes || i >= n) return;
 	HitRec rec;
 	rec.inst = -1;
 	WorldRayD wr;
@@ -148,13 +150,20 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
 cudaError_t launch_trace(const DevScene& sc, const RaySoA& rays, const HitSoA& hits, uint32_t n, unsigned* status,
                          cudaStream_t stream) {
 	if (n == 0) return cudaSuccess;
+	// A short stream is spread over the SMs, and its warps run on fewer lanes,
+	// whose rays wait less for one another: at least 8 warps an SM as long as
+	// there are rays (1021 rays against a flat scene: 51 us in 8 blocks of 128
+	// threads, 23 so).
 	const int block = 128;
-	const uint32_t grid = (n + block - 1) / block;
+	const uint32_t warps = 8 * 148;
+	int lanes = 32;
+	while (lanes > 1 && n / (uint32_t)lanes < warps) lanes >>= 1;
+	const uint32_t grid = (uint32_t)((((uint64_t)n + lanes - 1) / lanes * 32 + block - 1) / block);
 	switch (feature_variant(sc.features)) {
-		case FEAT_FLAT: trace_kernel<FEAT_FLAT><<<grid, block, 0, stream>>>(sc, rays, hits, n, status); break;
-		case FEAT_STILL_BICUBIC: trace_kernel<FEAT_STILL_BICUBIC><<<grid, block, 0, stream>>>(sc, rays, hits, n, status); break;
-		case FEAT_STILL: trace_kernel<FEAT_STILL><<<grid, block, 0, stream>>>(sc, rays, hits, n, status); break;
-		default: trace_kernel<FEAT_ALL><<<grid, block, 0, stream>>>(sc, rays, hits, n, status); break;
+		case FEAT_FLAT: trace_kernel<FEAT_FLAT><<<grid, block, 0, stream>>>(sc, rays, hits, n, lanes, status); break;
+		case FEAT_STILL_BICUBIC: trace_kernel<FEAT_STILL_BICUBIC><<<grid, block, 0, stream>>>(sc, rays, hits, n, lanes, status); break;
+		case FEAT_STILL: trace_kernel<FEAT_STILL><<<grid, block, 0, stream>>>(sc, rays, hits, n, lanes, status); break;
+		default: trace_kernel<FEAT_ALL><<<grid, block, 0, stream>>>(sc, rays, hits, n, lanes, status); break;
 	}
 	return cudaGetLastError();
 }

@@ -1,0 +1,68 @@
+"""Launch shapes and scene forms that the traversal picks by size: short
+streams and waves, and scenes that unroll to more placements than are laid
+out."""
+import numpy as np
+import pytest
+
+from psychopath_cpp_b200 import api, scenes
+from psychopath_cpp_b200.scene import Assembly, Sphere
+from tests import parity
+
+pytestmark = pytest.mark.gpu
+FIELDS = ("hit", "t", "uv", "p", "n", "dpdu", "backfacing", "offset", "space", "closure", "closure_color")
+
+
+def equal(a, b):
+    return all(np.array_equal(a[k], b[k], equal_nan=a[k].dtype.kind == "f") for k in a)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 1183, 1184, 2367, 2368, 9473, 37887, 37888])
+def test_short_stream_is_the_stream_s_beginning(ctx, n):
+    ctx.upload(scenes.plain_scene(3))
+    rays = parity.random_rays(40000, (-6, -6, 0.01), (6, 6, 3), seed=5, occl_frac=0.3)
+    whole = api.Tracer(ctx).trace(rays, fields=FIELDS + ("id",))
+    part = api.Tracer(ctx).trace({k: v[:n] for k, v in rays.items()}, fields=FIELDS + ("id",))
+    assert equal(part, {k: v[:n] for k, v in whole.items()})
+
+
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (17, 3, 1), (8, 8, 1), (13, 5, 2), (61, 47, 3), (160, 120, 2)])
+def test_wave_length_does_not_change_the_film(ctx, w, h, spp):
+    sc = scenes.plain_scene(4, res=(w, h), spp=spp)
+    ctx.upload(sc)
+    x, c = api.PathTraceIntegrator(ctx, w, h, spp, path_length=3).integrate()
+    y, d = api.PathTraceIntegrator(ctx, w, h, spp, path_length=3, stream_paths=spp * max(1, w * h // 3)).integrate()
+    assert np.array_equal(c, d) and np.array_equal(x, y)
+
+
+def overgrown(sc):
+    """`sc` with a far-away nest of some 270,000 assembly instances."""
+    inner = Assembly()
+    inner.add_object("s", Sphere([0.0, 0.0, 0.0], 0.5))
+    inner.add_instance("s")
+    for level in range(3):
+        outer = Assembly()
+        outer.add_assembly("in", inner)
+        for k in range(65):
+            outer.add_instance("in", [scenes.placement((0, 0, 1), 0.0, (2.0 * k, 0.0, 100.0 * level))])
+        inner = outer
+    sc.root.add_assembly("nest", inner)
+    sc.root.add_instance("nest", [scenes.placement((0, 0, 1), 0.0, (1e5, 1e5, 1e5))])
+    return sc
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_scene_without_placements_gives_the_same_hits(ctx, seed):
+    """A scene past the placements' limit keeps a level stack per ray; with
+    the nest out of every ray's way its hits and its film are those of the
+    scene without the nest."""
+    make = lambda: scenes.many_light_scene(seed, res=(48, 27), spp=2, n_patches=40, n_groups=20, n_lights=30)
+    rays = parity.random_rays(20000, (-4, -4, -0.5), (4, 4, 5), seed=seed, occl_frac=0.3)
+    got = []
+    for sc in (make(), overgrown(make())):
+        ctx.upload(sc)
+        hits = api.Tracer(ctx).trace(rays, fields=FIELDS)
+        film, counts = api.PathTraceIntegrator(ctx, 48, 27, 2, path_length=4).integrate()
+        got.append((hits, film, counts))
+    assert 0 < got[0][0]["hit"].sum() < len(rays["time"])
+    assert equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
