@@ -84,24 +84,25 @@ __device__ __forceinline__ int load_ray(const float4* rb, int cap, int i, WorldR
 // Hit planes: 0: t, u, v, max_dim (float4)   1: instance, placement, depth,
 // path[0]   2: path[1..4]   3: path[5..7] (int4).  The path is written and
 // read in scenes without placements only, as far as the hit's depth.
-__device__ __forceinline__ void load_rec(const WaveBufs& wb, int i, HitRec* h) {
+__device__ __forceinline__ void load_rec(const WaveBufs& wb, int i, HitRec* h, HitPath* hp) {
 	const int4 a = wb.hit_i[i];
 	h->inst = a.x;
 	if (a.x < 0) return;
 	const float4 f = wb.hit_f[i];
 	h->t = f.x; h->u = f.y; h->v = f.z; h->max_dim = f.w;
 	h->place = a.y;
+	hp->depth = 0;
 	if (a.y >= 0) return;
-	h->depth = a.z;
-	h->path[0] = a.w;
+	hp->depth = a.z;
+	hp->path[0] = a.w;
 	const int cap = wb.cap;
-	if (h->depth > 1) {
+	if (hp->depth > 1) {
 		const int4 b = wb.hit_i[cap + i];
-		h->path[1] = b.x; h->path[2] = b.y; h->path[3] = b.z; h->path[4] = b.w;
+		hp->path[1] = b.x; hp->path[2] = b.y; hp->path[3] = b.z; hp->path[4] = b.w;
 	}
-	if (h->depth > 5) {
+	if (hp->depth > 5) {
 		const int4 c = wb.hit_i[2 * cap + i];
-		h->path[5] = c.x; h->path[6] = c.y; h->path[7] = c.z;
+		hp->path[5] = c.x; hp->path[6] = c.y; hp->path[7] = c.z;
 	}
 }
 
@@ -136,7 +137,7 @@ struct WaveIO {
 			return;
 		}
 		int p[PSY_MAX_LEVELS] = {};
-		for (int k = 1; k <= tr.L; ++k) p[k - 1] = tr.lv_inst[k];
+		for (int k = 1; k <= tr.L; ++k) p[k - 1] = tr.mem->lv_inst[k];
 		p[tr.L] = inst;
 		const int cap = wb->cap;
 		wb->hit_i[i] = make_int4(inst, -1, tr.L + 1, p[0]);
@@ -168,10 +169,10 @@ struct GtrVertex {
 // path_trace_integrator.cpp:141-145 and the transferred differentials of
 // propagate_differentials.
 template <unsigned F>
-__device__ __forceinline__ void make_vertex(const DevScene& sc, const HitRec& rec, const WorldRayD& wr, float ident_inv,
+__device__ __forceinline__ void make_vertex(const DevScene& sc, const HitRec& rec, const HitPath& path, const WorldRayD& wr, float ident_inv,
                                             Vertex* sh, GtrVertex* gv, int* closure, float* light_pdf, unsigned* err) {
 	M44 space;
-	const bool xf = hit_space<F>(sc, rec, wr.time, &space, err);
+	const bool xf = hit_space<F>(sc, rec, path, wr.time, &space, err);
 	V3 lo = wr.o, ld = wr.d;
 	if (xf) {
 		lo = pos_to(space, wr.o);
@@ -533,7 +534,9 @@ __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS)
 		}
 		c_warp = c_lanes = 0;
 	};
+	TravMem<F> mem;
 	Trav<F, WaveIO> tr;
+	tr.mem = &mem;
 	tr.io.rb = rc;
 	tr.io.wb = &wb;
 	tr.io.i = -1;
@@ -722,13 +725,14 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 				load_ray(rin, wb.cap, i, &wr);
 				time = wr.time;
 				HitRec rec;
-				load_rec(wb, i, &rec);
+				HitPath path;
+				load_rec(wb, i, &rec, &path);
 				const Spec fcol = CAMERA ? Spec{{1.0f, 1.0f, 1.0f, 1.0f}} : sp(ps.fcol[slot]);
 				if (rec.inst >= 0) {
-					hit_surface(sc, &rec);
+					hit_surface(sc, &rec, path);
 					int closure;
 					float lpdf;
-					make_vertex<F>(sc, rec, wr, rp.ident_inv, &sh, &gv, &closure, &lpdf, &err);
+					make_vertex<F>(sc, rec, path, wr, rp.ident_inv, &sh, &gv, &closure, &lpdf, &err);
 					const int vtx = (int)(step >> 1);  // index of this path vertex
 					if (closure == CLOSURE_EMIT) {
 						const Spec e0 = rgb_to_spec(sh.col, wl);

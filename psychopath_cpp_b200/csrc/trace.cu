@@ -22,6 +22,7 @@ __device__ __forceinline__ void st3(float* p, uint32_t i, V3 v) {
 struct StreamIO {
 	const RaySoA* rays;
 	HitRec* rec;
+	HitPath* path;
 	uint32_t i;
 	__device__ __forceinline__ V3 origin() const { return ld3(rays->o, i); }
 	__device__ __forceinline__ V3 direction() const { return ld3(rays->d, i); }
@@ -40,9 +41,9 @@ struct StreamIO {
 		rec->inst = inst;
 		rec->place = tr.place;
 		if (T::NESTED && tr.place < 0) {
-			rec->depth = tr.L + 1;
-			for (int k = 1; k <= tr.L; ++k) rec->path[k - 1] = tr.lv_inst[k];
-			rec->path[tr.L] = inst;
+			path->depth = tr.L + 1;
+			for (int k = 1; k <= tr.L; ++k) path->path[k - 1] = tr.mem->lv_inst[k];
+			path->path[tr.L] = inst;
 		}
 	}
 };
@@ -66,6 +67,7 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
 	const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (uint32_t)lanes + (uint32_t)lane;
 	if (lane >= lanes || i >= n) return;
 	HitRec rec;
+	HitPath path;
 	rec.inst = -1;
 	WorldRayD wr;
 	wr.o = ld3(rays.o, i);
@@ -74,9 +76,12 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
 	wr.occl = rays.type ? (__ldg(rays.type + i) == 32) : false;
 	unsigned err;
 	{
+		TravMem<F> mem;
 		Trav<F, StreamIO> tr;
+		tr.mem = &mem;
 		tr.io.rays = &rays;
 		tr.io.rec = &rec;
+		tr.io.path = &path;
 		tr.io.i = i;
 		tr.init(sc, wr.o, wr.d, wr.time, wr.occl);
 		tr.walk(sc);
@@ -84,16 +89,16 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
 	}
 	const bool hit = rec.inst >= 0;
 	if (hits.hit) hits.hit[i] = hit ? 1 : 0;
-	if (hits.id) hits.id[i] = hit ? hit_id(sc, rec) : 0ull;
+	if (hits.id) hits.id[i] = hit ? hit_id(sc, rec, path) : 0ull;
 	if (hits.t) hits.t[i] = (hit && !wr.occl) ? rec.t : INFINITY;
-	if (hit && !wr.occl && hits.want_geometry) hit_surface(sc, &rec);
+	if (hit && !wr.occl && hits.want_geometry) hit_surface(sc, &rec, path);
 	if (hit && !wr.occl && hits.want_geometry == WANT_UV && (rec.kind == OBJ_BILINEAR || rec.kind == OBJ_BICUBIC)) {
 		// a patch's u, v are the bisection's own: no geometry to evaluate
 		hits.uv[2 * (size_t)i] = rec.u;
 		hits.uv[2 * (size_t)i + 1] = rec.v;
 	} else if (hit && !wr.occl && hits.want_geometry) {
 		M44 space;
-		const bool xf = hit_space<F>(sc, rec, wr.time, &space, &err);
+		const bool xf = hit_space<F>(sc, rec, path, wr.time, &space, &err);
 		V3 lo = wr.o, ld = wr.d;
 		if (xf) {
 			lo = pos_to(space, wr.o);

@@ -315,6 +315,41 @@ __device__ __forceinline__ void patch_split(Patch<16>& p, Patch<16>& f, bool alo
 			bezier_split(p.p[c], p.p[c + 4], p.p[c + 8], p.p[c + 12], f.p[c], f.p[c + 4], f.p[c + 8], f.p[c + 12]);
 	}
 }
+// Four floats as two packed pairs.
+struct Quad {
+	unsigned long long a, b;
+};
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+	unsigned long long r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+	return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& x, float& y) {
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ void load_axis(const char* p, Quad& lo, Quad& hi) {
+	asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(lo.a), "=l"(lo.b), "=l"(hi.a), "=l"(hi.b) : "l"(p));
+}
+__device__ __forceinline__ void lerp_quad(Quad& a, const Quad& b, unsigned long long ia, unsigned long long al) {
+	a.a = add2(mul2(a.a, ia), mul2(b.a, al));
+	a.b = add2(mul2(a.b, ia), mul2(b.b, al));
+}
+__device__ __forceinline__ void planes(const Quad& q, float no, float di, float* t) {
+	const unsigned long long n = pack2(no, no), d = pack2(di, di);
+	unpack2(mul2(add2(q.a, n), d), t[0], t[1]);
+	unpack2(mul2(add2(q.b, n), d), t[2], t[3]);
+}
+
 // ---------------------------------------------------------------------
 // Slab tests
 // ---------------------------------------------------------------------
@@ -619,51 +654,54 @@ struct HitRec {
 	float u, v, max_dim;
 	int inst;                  // global instance index, -1 = miss
 	int place;                 // its assembly's placement, -1 = scene without placements
-	int depth;                 // instances on the path (place < 0)
-	int path[PSY_MAX_LEVELS];  // global instance indices, root first (place < 0)
 	int obj, kind, shader;     // set by hit_surface
+};
+// The path to a hit without placement: global instance indices, root first.
+struct HitPath {
+	int depth;
+	int path[PSY_MAX_LEVELS];
 };
 
 // Element id of the hit (Intersection::id): the local instance index of
 // every level, pushed with that assembly's bits.
-__device__ __forceinline__ uint64_t hit_id(const DevScene& sc, const HitRec& h) {
+__device__ __forceinline__ uint64_t hit_id(const DevScene& sc, const HitRec& h, const HitPath& hp) {
 	if (h.place >= 0) {
 		const DevPlace& p = sc.places[h.place];
 		return id_push(p.id, (uint64_t)(h.inst - p.inst_base), p.id_bits);
 	}
 	uint64_t id = 0;
 	int asmb = 0;
-	for (int k = 0; k < h.depth; ++k) {
-		id = id_push(id, (uint64_t)(h.path[k] - sc.assemblies[asmb].inst_base), sc.assemblies[asmb].id_bits);
-		asmb = sc.instances[h.path[k]].data;
+	for (int k = 0; k < hp.depth; ++k) {
+		id = id_push(id, (uint64_t)(hp.path[k] - sc.assemblies[asmb].inst_base), sc.assemblies[asmb].id_bits);
+		asmb = sc.instances[hp.path[k]].data;
 	}
 	return id;
 }
 
 // The shader bound to the hit: the innermost one on the path.
-__device__ __forceinline__ int hit_shader(const DevScene& sc, const HitRec& h) {
+__device__ __forceinline__ int hit_shader(const DevScene& sc, const HitRec& h, const HitPath& hp) {
 	const int own = sc.instances[h.inst].shader;
 	if (own >= 0) return own;
 	if (h.place >= 0) return sc.places[h.place].shader;
-	for (int k = h.depth - 2; k >= 0; --k) {
-		const int s = sc.instances[h.path[k]].shader;
+	for (int k = hp.depth - 2; k >= 0; --k) {
+		const int s = sc.instances[hp.path[k]].shader;
 		if (s >= 0) return s;
 	}
 	return -1;
 }
 
 // The object hit, its kind and its shader.
-__device__ __forceinline__ void hit_surface(const DevScene& sc, HitRec* h) {
+__device__ __forceinline__ void hit_surface(const DevScene& sc, HitRec* h, const HitPath& hp) {
 	h->obj = sc.instances[h->inst].data;
 	h->kind = sc.objects[h->obj].kind;
-	h->shader = hit_shader(sc, *h);
+	h->shader = hit_shader(sc, *h, hp);
 }
 
 // Transform from world space into the hit object's space at the ray time
 // (the Intersection::space of the reference).  Returns false when the path
 // carries no transform (identity).
 template <unsigned F>
-__device__ bool hit_space(const DevScene& sc, const HitRec& rec, float time, M44* out, unsigned* err) {
+__device__ bool hit_space(const DevScene& sc, const HitRec& rec, const HitPath& hp, float time, M44* out, unsigned* err) {
 	if (!(F & FEAT_XFORM)) return false;
 	Frame f{nullptr, 0};
 	FrameBuf buf[2];
@@ -683,8 +721,8 @@ __device__ bool hit_space(const DevScene& sc, const HitRec& rec, float time, M44
 		f = Frame{sc.place_frames + (size_t)p.frame * 16, p.frame_count};
 		if (!merge(sc.instances[rec.inst])) return false;
 	} else {
-		for (int k = 0; k < rec.depth; ++k)
-			if (!merge(sc.instances[rec.path[k]])) return false;
+		for (int k = 0; k < hp.depth; ++k)
+			if (!merge(sc.instances[hp.path[k]])) return false;
 	}
 	if (f.count == 0) return false;
 	*out = frame_at(f, time);
@@ -724,21 +762,13 @@ enum : unsigned {
 	RAY_WIDTH = 8u   // the width parameters are those of the current space
 };
 
-// Traversal state of one ray.  IO gives the world ray (origin, direction,
-// differentials: read again where an instance or a patch needs them) and
-// takes the hits.  The members above the line are meant for registers, the
-// ones below live in local memory.
-template <unsigned F, class IO>
-struct Trav {
-	V3 o, d, dinv;      // the ray in the current space
-	float max_t, time;
-	int cur;            // next reference
-	int sp, L;          // stack entries, assembly levels entered
-	int place;          // current placement (scenes with placements)
-	int pmode;          // bisection in progress (PM_*)
-	unsigned flags, err;
-	IO io;
-	// ---
+// The parts of a ray's traversal state that are indexed at run time or too
+// large for registers.  They are a variable of their own: one struct with
+// the walk's scalars would keep those in local memory too, since the
+// compiler does not take a variable with a run-time index apart (1280x720x4
+// many-light frame 149 ms so, 141 apart).
+template <unsigned F>
+struct TravMem {
 	uint2 stack[PSY_NODE_STACK + PSY_MAX_LEVELS];  // reference, distance of its box (as bits)
 	RayFlip rw;                                    // width parameters of the current space (RAY_WIDTH)
 	float lvr[PSY_MAX_LEVELS][9];                  // ray of each enclosing level (REF_LEVEL_RAY)
@@ -750,6 +780,22 @@ struct Trav {
 	V3 p_o, p_dinv;
 	RayFlip p_rw;
 	alignas(16) unsigned char pbuf[PatchBuf<F>::bytes];
+};
+
+// Traversal state of one ray.  IO gives the world ray (origin, direction,
+// differentials: read again where an instance or a patch needs them) and
+// takes the hits.
+template <unsigned F, class IO>
+struct Trav {
+	V3 o, d, dinv;      // the ray in the current space
+	float max_t, time;
+	int cur;            // next reference
+	int sp, L;          // stack entries, assembly levels entered
+	int place;          // current placement (scenes with placements)
+	int pmode;          // bisection in progress (PM_*)
+	unsigned flags, err;
+	IO io;
+	TravMem<F>* mem;
 
 	static constexpr bool NESTED = (F & FEAT_NESTED) != 0;
 	static constexpr bool XFORM = (F & FEAT_XFORM) != 0;
@@ -757,14 +803,14 @@ struct Trav {
 
 	template <int NV>
 	__device__ __forceinline__ typename PatchBuf<F>::template Work<NV>& work() {
-		return *reinterpret_cast<typename PatchBuf<F>::template Work<NV>*>(pbuf);
+		return *reinterpret_cast<typename PatchBuf<F>::template Work<NV>*>(mem->pbuf);
 	}
 
 	// the same room as that of a patch with one time sample
 	typedef PatchBuf<F & ~FEAT_PATCH_MOTION> Still;
 	template <int NV>
 	__device__ __forceinline__ typename Still::template Work<NV>& still_work() {
-		return *reinterpret_cast<typename Still::template Work<NV>*>(pbuf);
+		return *reinterpret_cast<typename Still::template Work<NV>*>(mem->pbuf);
 	}
 
 	__device__ __forceinline__ static bool odd_ray(V3 o, V3 d, V3 dinv) {
@@ -795,8 +841,8 @@ struct Trav {
 		err = 0;
 		if (NESTED && !sc.places) {
 			place = -1;
-			lv_frame[0] = -1;
-			lv_count[0] = 0;
+			mem->lv_frame[0] = -1;
+			mem->lv_count[0] = 0;
 		}
 	}
 
@@ -806,7 +852,7 @@ struct Trav {
 			const int4 p = __ldg(reinterpret_cast<const int4*>(sc.places + place));
 			return Frame{sc.place_frames + (size_t)p.z * 16, p.w};
 		}
-		return Frame{lv_count[L] ? frames[lv_frame[L]].m : nullptr, lv_count[L]};
+		return Frame{mem->lv_count[L] ? mem->frames[mem->lv_frame[L]].m : nullptr, mem->lv_count[L]};
 	}
 
 	// Records a hit on instance gi.  Returns false when the ray is finished
@@ -824,7 +870,7 @@ struct Trav {
 	__device__ __forceinline__ bool pop(const DevScene& sc) {
 		while (cur == REF_NONE) {
 			if (sp == 0) return false;
-			const uint2 e = stack[--sp];
+			const uint2 e = mem->stack[--sp];
 			const int ref = (int)e.x;
 			if (ref >= 0) {
 				if (__uint_as_float(e.y) < max_t) cur = ref;
@@ -834,9 +880,9 @@ struct Trav {
 				--L;
 				if (place >= 0) place = (int)e.y;
 				if (XFORM && ref == REF_LEVEL_RAY) {
-					o = V3(lvr[L][0], lvr[L][1], lvr[L][2]);
-					d = V3(lvr[L][3], lvr[L][4], lvr[L][5]);
-					dinv = V3(lvr[L][6], lvr[L][7], lvr[L][8]);
+					o = V3(mem->lvr[L][0], mem->lvr[L][1], mem->lvr[L][2]);
+					d = V3(mem->lvr[L][3], mem->lvr[L][4], mem->lvr[L][5]);
+					dinv = V3(mem->lvr[L][6], mem->lvr[L][7], mem->lvr[L][8]);
 					flags &= ~(RAY_ODD | RAY_WIDTH);
 					if (odd_ray(o, d, dinv)) flags |= RAY_ODD;
 				}
@@ -885,54 +931,56 @@ struct Trav {
 		const int ref = cur;
 		const DevNode* nd = sc.nodes + (ref & REF_NODE_MASK);
 		float t0, t1, t2, t3;
+		const int4 ch = __ldg(reinterpret_cast<const int4*>(nd->child));
 		if ((flags & RAY_ODD) || (ref & REF_NODE_ODD)) {
 			const float4 t = odd_node(sc, ref, o, dinv, time, max_t);
 			t0 = t.x; t1 = t.y; t2 = t.z; t3 = t.w;
 		} else {
-			// the near and far planes by the direction's signs
 			const char* base = reinterpret_cast<const char*>(nd);
-			const int sx = dinv.x < 0.0f ? 16 : 0, sy = dinv.y < 0.0f ? 16 : 0, sz = dinv.z < 0.0f ? 16 : 0;
-			auto row = [](const char* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
-			float4 xn = row(base + sx), xf = row(base + 16 - sx);
-			float4 yn = row(base + 32 + sy), yf = row(base + 48 - sy);
-			float4 zn = row(base + 64 + sz), zf = row(base + 80 - sz);
-			if (ref & REF_NODE_MOVING) {
-				// lerp the boxes of the two time samples around the ray time
-				// (sample 0 is in the node, later ones in node_extra)
-				const int4 meta = __ldg(reinterpret_cast<const int4*>(&nd->nchild));
-				const SeqPos q = seq_pos(time, meta.y);
-				auto extra = [&](int k) { return reinterpret_cast<const char*>(sc.node_extra + (size_t)(meta.z + k - 1) * 24); };
-				if (q.i0 != 0) {
-					const char* e = extra(q.i0);
-					xn = row(e + sx); xf = row(e + 16 - sx);
-					yn = row(e + 32 + sy); yf = row(e + 48 - sy);
-					zn = row(e + 64 + sz); zf = row(e + 80 - sz);
+			float tn[4], tf[4];
+			{
+				Quad xl, xh, yl, yh, zl, zh;
+				load_axis(base, xl, xh);
+				load_axis(base + 32, yl, yh);
+				load_axis(base + 64, zl, zh);
+				if (ref & REF_NODE_MOVING) {
+					const int4 meta = __ldg(reinterpret_cast<const int4*>(&nd->nchild));
+					const SeqPos q = seq_pos(time, meta.y);
+					auto extra = [&](int k) { return reinterpret_cast<const char*>(sc.node_extra + (size_t)(meta.z + k - 1) * 24); };
+					if (q.i0 != 0) {
+						const char* e = extra(q.i0);
+						load_axis(e, xl, xh);
+						load_axis(e + 32, yl, yh);
+						load_axis(e + 64, zl, zh);
+					}
+					if (!q.single) {
+						const char* e = extra(q.i0 + 1);
+						const unsigned long long al = pack2(q.nalpha, q.nalpha), ia = pack2(one_minus(q.nalpha), one_minus(q.nalpha));
+						Quad a, b;
+						load_axis(e, a, b);
+						lerp_quad(xl, a, ia, al); lerp_quad(xh, b, ia, al);
+						load_axis(e + 32, a, b);
+						lerp_quad(yl, a, ia, al); lerp_quad(yh, b, ia, al);
+						load_axis(e + 64, a, b);
+						lerp_quad(zl, a, ia, al); lerp_quad(zh, b, ia, al);
+					}
 				}
-				if (!q.single) {
-					const char* e = extra(q.i0 + 1);
-					const float al = q.nalpha, ia = one_minus(q.nalpha);
-					auto lerp4 = [&](float4 a, float4 b) {
-						return make_float4((a.x * ia) + (b.x * al), (a.y * ia) + (b.y * al), (a.z * ia) + (b.z * al),
-						                   (a.w * ia) + (b.w * al));
-					};
-					xn = lerp4(xn, row(e + sx)); xf = lerp4(xf, row(e + 16 - sx));
-					yn = lerp4(yn, row(e + 32 + sy)); yf = lerp4(yf, row(e + 48 - sy));
-					zn = lerp4(zn, row(e + 64 + sz)); zf = lerp4(zf, row(e + 80 - sz));
-				}
+				float l[4], h[4];
+				planes(xl, -o.x, dinv.x, l); planes(xh, -o.x, dinv.x, h);
+#pragma unroll
+				for (int c = 0; c < 4; ++c) { tn[c] = fminf(l[c], h[c]); tf[c] = fmaxf(l[c], h[c]); }
+				planes(yl, -o.y, dinv.y, l); planes(yh, -o.y, dinv.y, h);
+#pragma unroll
+				for (int c = 0; c < 4; ++c) { tn[c] = fmaxf(tn[c], fminf(l[c], h[c])); tf[c] = fminf(tf[c], fmaxf(l[c], h[c])); }
+				planes(zl, -o.z, dinv.z, l); planes(zh, -o.z, dinv.z, h);
+#pragma unroll
+				for (int c = 0; c < 4; ++c) { tn[c] = fmaxf(fmaxf(tn[c], fminf(l[c], h[c])), 0.0f); tf[c] = fminf(tf[c], fmaxf(l[c], h[c])) * BBOX_MAXT_ADJUST; }
 			}
-			auto slab = [&](float nx, float fx, float ny, float fy, float nz, float fz) {
-				const float mins = fmaxf(fmaxf((nx - o.x) * dinv.x, (ny - o.y) * dinv.y), fmaxf((nz - o.z) * dinv.z, 0.0f));
-				const float maxs = fminf(fminf((fx - o.x) * dinv.x, (fy - o.y) * dinv.y), (fz - o.z) * dinv.z) * BBOX_MAXT_ADJUST;
-				return mins < max_t && mins <= maxs ? mins : INFINITY;
-			};
-			// a hit has mins < max_t <= inf, so inf marks the misses (absent
-			// children have inverted infinite boxes)
-			t0 = slab(xn.x, xf.x, yn.x, yf.x, zn.x, zf.x);
-			t1 = slab(xn.y, xf.y, yn.y, yf.y, zn.y, zf.y);
-			t2 = slab(xn.z, xf.z, yn.z, yf.z, zn.z, zf.z);
-			t3 = slab(xn.w, xf.w, yn.w, yf.w, zn.w, zf.w);
+			t0 = tn[0] < max_t && tn[0] <= tf[0] ? tn[0] : INFINITY;
+			t1 = tn[1] < max_t && tn[1] <= tf[1] ? tn[1] : INFINITY;
+			t2 = tn[2] < max_t && tn[2] <= tf[2] && ch.z != REF_EMPTY ? tn[2] : INFINITY;
+			t3 = tn[3] < max_t && tn[3] <= tf[3] && ch.w != REF_EMPTY ? tn[3] : INFINITY;
 		}
-		const int4 ch = __ldg(reinterpret_cast<const int4*>(nd->child));
 		const bool h0 = t0 < INFINITY, h1 = t1 < INFINITY, h2 = t2 < INFINITY, h3 = t3 < INFINITY;
 		if (flags & RAY_OCCL) {
 			// any blocker ends the ray: the order is that of the children, and
@@ -955,7 +1003,7 @@ struct Trav {
 		auto put = [&](bool h, int r, int ref_c, float t) {
 			if (!h) return;
 			if (r == 0) next = ref_c;
-			else stack[top - r] = make_uint2((unsigned)ref_c, __float_as_uint(t));
+			else mem->stack[top - r] = make_uint2((unsigned)ref_c, __float_as_uint(t));
 		};
 		put(h0, r0, ch.x, t0);
 		put(h1, r1, ch.y, t1);
@@ -989,18 +1037,18 @@ struct Trav {
 			if (root != REF_EMPTY) {
 				const Frame parent = level_frame(sc);
 				f = parent;
-				lv_inst[L + 1] = gi;
-				lv_frame[L + 1] = lv_frame[L];
+				mem->lv_inst[L + 1] = gi;
+				mem->lv_frame[L + 1] = mem->lv_frame[L];
 				if (XFORM && m.y > 0) {
 					const DevInstance inst = sc.instances[gi];
-					f = frame_merge(parent, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &frames[L + 1]);
+					f = frame_merge(parent, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &mem->frames[L + 1]);
 					if (f.count < 0) {
 						err |= ERRF_MOTION;
 						return true;
 					}
-					lv_frame[L + 1] = L + 1;
+					mem->lv_frame[L + 1] = L + 1;
 				}
-				lv_count[L + 1] = f.count;
+				mem->lv_count[L + 1] = f.count;
 			}
 		}
 		if (root == REF_EMPTY) return true;
@@ -1009,11 +1057,11 @@ struct Trav {
 			return false;
 		}
 		const bool moved = XFORM && m.y > 0;
-		stack[sp++] = make_uint2((unsigned)(moved ? REF_LEVEL_RAY : REF_LEVEL), (unsigned)place);
+		mem->stack[sp++] = make_uint2((unsigned)(moved ? REF_LEVEL_RAY : REF_LEVEL), (unsigned)place);
 		if (moved) {
-			lvr[L][0] = o.x; lvr[L][1] = o.y; lvr[L][2] = o.z;
-			lvr[L][3] = d.x; lvr[L][4] = d.y; lvr[L][5] = d.z;
-			lvr[L][6] = dinv.x; lvr[L][7] = dinv.y; lvr[L][8] = dinv.z;
+			mem->lvr[L][0] = o.x; mem->lvr[L][1] = o.y; mem->lvr[L][2] = o.z;
+			mem->lvr[L][3] = d.x; mem->lvr[L][4] = d.y; mem->lvr[L][5] = d.z;
+			mem->lvr[L][6] = dinv.x; mem->lvr[L][7] = dinv.y; mem->lvr[L][8] = dinv.z;
 			const M44 t = frame_at(f, time);
 			set_ray(pos_to(t, io.origin()), dir_to(t, io.direction()));
 		}
@@ -1084,7 +1132,7 @@ struct Trav {
 	// Width parameters for the patch of instance at transform `om` (oxf: its
 	// own; else the level's, kept for the next patch in the same space).
 	__device__ __forceinline__ RayFlip widths(const DevScene& sc, bool oxf, M44& om, V3 lo, V3 ld) {
-		if (!oxf && (flags & RAY_WIDTH)) return rw;
+		if (!oxf && (flags & RAY_WIDTH)) return mem->rw;
 		V3 odx, ody, ddx, ddy;
 		io.differentials(&odx, &ody, &ddx, &ddy);
 		bool xf = oxf;
@@ -1103,7 +1151,7 @@ struct Trav {
 		}
 		const RayFlip w = ray_flip(ray_width_params(lo, ld, odx, ody, ddx, ddy));
 		if (!oxf) {
-			rw = w;
+			mem->rw = w;
 			flags |= RAY_WIDTH;
 		}
 		return w;
@@ -1167,11 +1215,11 @@ struct Trav {
 			else if (TS == 2 && pm == PM_BICUBIC2) one(work<16>());
 		}
 		if (!WHOLE && in) {
-			p_rw = widths(sc, oxf, om, lo, ld);
+			mem->p_rw = widths(sc, oxf, om, lo, ld);
 			pmode = pm;
-			p_inst = gi;
-			p_o = lo;
-			p_dinv = li;
+			mem->p_inst = gi;
+			mem->p_o = lo;
+			mem->p_dinv = li;
 		}
 		return live;
 	}
@@ -1183,15 +1231,15 @@ struct Trav {
 		int r = PATCH_DONE;
 		const bool occl = (flags & RAY_OCCL) != 0;
 		const float dr = sc.dice_rate, mu = sc.min_upoly_size;
-		const RayFlip w = p_rw;
-		const V3 lo = p_o, li = p_dinv;
+		const RayFlip w = mem->p_rw;
+		const V3 lo = mem->p_o, li = mem->p_dinv;
 		// the cursor runs as a local copy (registers) and goes back to the
 		// state only when the bisection stops short of its end
 		auto run = [&](auto& pw) {
 			auto pc = pw.c;
 			r = patch_run<sizeof(pc.cur[0]) / sizeof(V3), sizeof(pc.cur) / sizeof(pc.cur[0]), true>(
 			    pc, pw.st, lo, li, w, &max_t, occl, dr, mu, units, &err,
-			    [&](float t, float u, float v, float md) { record(p_inst, t, u, v, md); });
+			    [&](float t, float u, float v, float md) { record(mem->p_inst, t, u, v, md); });
 			if (r == PATCH_MORE) pw.c = pc;
 		};
 		if constexpr ((F & FEAT_BILINEAR) != 0) {
