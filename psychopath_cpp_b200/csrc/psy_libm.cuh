@@ -248,7 +248,9 @@ PSY_LM_HD float lm_asinf(float x) {
 	}
 
 #ifdef __CUDACC__
-__device__ __constant__ static const uint64_t psy_lm_exp2_tab_dev[32] = PSY_LM_EXP2_TABLE;
+// in global memory: the lanes of a warp look up different entries, which
+// constant memory serves one after another
+__device__ static const uint64_t psy_lm_exp2_tab_dev[32] = PSY_LM_EXP2_TABLE;
 #endif
 static const uint64_t psy_lm_exp2_tab_host[32] = PSY_LM_EXP2_TABLE;
 
@@ -264,7 +266,7 @@ PSY_LM_HD float lm_expf(float x) {
 	kd -= shift;
 	const double r = z - kd;
 #ifdef __CUDA_ARCH__
-	uint64_t t = psy_lm_exp2_tab_dev[ki % 32];
+	uint64_t t = __ldg((const unsigned long long*)&psy_lm_exp2_tab_dev[ki % 32]);
 #else
 	uint64_t t = psy_lm_exp2_tab_host[ki % 32];
 #endif

@@ -41,6 +41,7 @@ enum : unsigned {
 	FEAT_BICUBIC = 4u,       // bicubic patches
 	FEAT_PATCH_MOTION = 8u,  // patches with two time samples
 	FEAT_BILINEAR = 16u,     // bilinear patches
+	FEAT_GTR = 32u,          // GTR shaders (shading only)
 	FEAT_FLAT = 16u,         // spheres, lights and bilinear patches in one level
 	FEAT_STILL_BICUBIC = 7u, // levels, transforms, bicubic patches (no bilinear, no patch motion)
 	FEAT_STILL = 23u,        // everything but patch motion
@@ -51,6 +52,7 @@ enum : unsigned {
 // FEAT_FLAT, FEAT_STILL_BICUBIC, FEAT_STILL, FEAT_ALL: smaller variants
 // leave out the code of absent features).
 inline unsigned feature_variant(unsigned f) {
+	f &= (unsigned)FEAT_ALL;
 	if ((f & ~FEAT_FLAT) == 0u) return FEAT_FLAT;
 	if ((f & ~FEAT_STILL_BICUBIC) == 0u) return FEAT_STILL_BICUBIC;
 	if ((f & ~FEAT_STILL) == 0u) return FEAT_STILL;

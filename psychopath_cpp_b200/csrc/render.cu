@@ -6,12 +6,12 @@
 
 namespace psy {
 
-extern template void launch_wave<PlainWave, FEAT_FLAT>(const PlainWave&, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
-extern template void launch_wave<PlainWave, FEAT_STILL_BICUBIC>(const PlainWave&, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
-extern template void launch_wave<PlainWave, FEAT_STILL>(const PlainWave&, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
-extern template void launch_wave<PlainWave, FEAT_ALL>(const PlainWave&, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
-extern template void launch_wave<BatchWave, FEAT_FLAT>(const BatchWave&, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
-extern template void launch_wave<BatchWave, FEAT_ALL>(const BatchWave&, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
+extern template void launch_wave<PlainWave, FEAT_FLAT>(const PlainWave&, int, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
+extern template void launch_wave<PlainWave, FEAT_STILL_BICUBIC>(const PlainWave&, int, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
+extern template void launch_wave<PlainWave, FEAT_STILL>(const PlainWave&, int, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
+extern template void launch_wave<PlainWave, FEAT_ALL>(const PlainWave&, int, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
+extern template void launch_wave<BatchWave, FEAT_FLAT>(const BatchWave&, int, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
+extern template void launch_wave<BatchWave, FEAT_ALL>(const BatchWave&, int, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
 
 int render_counter_count(uint32_t path_length) { return wave_counter_count(path_length); }
 
@@ -26,11 +26,12 @@ cudaError_t launch_render_wave(const DevScene& sc, const HaltonDev& hd, const Re
 	block = valid_block(block);
 	const size_t gsmem = (rp.grad && rp.grad_in_smem) ? (rp.grad_in_smem == GRAD_SMEM64 ? sizeof(double) : sizeof(float)) * (size_t)rp.param_count : 0;
 	const uint32_t L = rp.path_length;
+	const int mode = shade_mode(sc.features, rp.grad != nullptr);
 	switch (feature_variant(sc.features)) {
-		case FEAT_FLAT: launch_wave<PlainWave, FEAT_FLAT>(w, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
-		case FEAT_STILL_BICUBIC: launch_wave<PlainWave, FEAT_STILL_BICUBIC>(w, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
-		case FEAT_STILL: launch_wave<PlainWave, FEAT_STILL>(w, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
-		default: launch_wave<PlainWave, FEAT_ALL>(w, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
+		case FEAT_FLAT: launch_wave<PlainWave, FEAT_FLAT>(w, mode, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
+		case FEAT_STILL_BICUBIC: launch_wave<PlainWave, FEAT_STILL_BICUBIC>(w, mode, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
+		case FEAT_STILL: launch_wave<PlainWave, FEAT_STILL>(w, mode, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
+		default: launch_wave<PlainWave, FEAT_ALL>(w, mode, L, hd, wv, ps, wb, wq, status, block, gsmem, st, launches, timer); break;
 	}
 	return cudaGetLastError();
 }
@@ -43,11 +44,12 @@ cudaError_t launch_batch_wave(const DevScene* scenes, const RenderParams* render
 	w.scenes = scenes;
 	w.renders = renders;
 	w.count = count;
+	const int mode = shade_mode(features, false);
 	block = valid_block(block);
 	if (feature_variant(features) == FEAT_FLAT)
-		launch_wave<BatchWave, FEAT_FLAT>(w, max_path_length, hd, wv, ps, wb, wq, status, block, 0, st, launches, nullptr);
+		launch_wave<BatchWave, FEAT_FLAT>(w, mode, max_path_length, hd, wv, ps, wb, wq, status, block, 0, st, launches, nullptr);
 	else
-		launch_wave<BatchWave, FEAT_ALL>(w, max_path_length, hd, wv, ps, wb, wq, status, block, 0, st, launches, nullptr);
+		launch_wave<BatchWave, FEAT_ALL>(w, mode, max_path_length, hd, wv, ps, wb, wq, status, block, 0, st, launches, nullptr);
 	return cudaGetLastError();
 }
 
@@ -72,7 +74,7 @@ __global__ void light_sample_kernel(DevScene sc, LightQuerySoADev q, LightSample
 	lq.id = 0;
 	lq.selection_pdf = 1.0f;
 	lq.light_sample_pdf = 1.0f;
-	light_tree_pick<FEAT_ALL>(sc, &lq);
+	light_tree_pick<FEAT_ALL, false>(sc, &lq);
 	light_emit<FEAT_ALL>(sc, &lq, ident_inv);
 	if (!lq.valid) {
 		atomicOr(status, ERRF_NOLIGHT);

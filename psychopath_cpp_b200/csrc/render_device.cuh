@@ -174,9 +174,34 @@ __device__ __forceinline__ V3 uniform_sample_sphere(float u, float v) {
 }
 
 // sphere_lambert (utils/monte_carlo.hpp:207-233).
-static __device__ __noinline__ float sphere_lambert_partial(float nlcos, float rcos) {
+// The cosine tests: |cos a - cos b| <= |a - b|, so where nlcos lies 1e-3 off
+// a limit's cosine (0, +-sin r), the angle lies as far off the limit; rsin is
+// off sin r by at most 2.5e-4 (the rounding of rcos^2) and the arc cosines
+// of the angle tests by less than 1e-6, so both tests agree there.  They
+// spare the arc cosines, and where the cap lies wholly above or below the
+// horizon (most nodes of a light tree walk) all arc functions.  An nlcos past
+// +-1 by rounding (its arc cosine is NaN) takes the angle tests.
+enum : int { CAP_ABOVE, CAP_MOSTLY_ABOVE, CAP_MOSTLY_BELOW, CAP_BELOW, CAP_UNSURE };
+__device__ __forceinline__ int cap_case(float nlcos, float rsin2) {
+	const float rsin = sqrtf(rsin2), m = 1e-3f;
+	if (nlcos > rsin + m) return nlcos <= 1.0f ? CAP_ABOVE : CAP_UNSURE;
+	if (nlcos < -(rsin + m)) return nlcos >= -1.0f ? CAP_BELOW : CAP_UNSURE;
+	if (nlcos > m && nlcos < rsin - m) return CAP_MOSTLY_ABOVE;
+	if (nlcos < -m && nlcos > m - rsin) return CAP_MOSTLY_BELOW;
+	return CAP_UNSURE;
+}
+
+// A cap that the horizon cuts, or may (c: cap_case).
+static __device__ __noinline__ float sphere_lambert_cut(float nlcos, float rcos, float rsin2, int c) {
+	if (c == CAP_UNSURE) {
+		const float nl = lm_acosf(nlcos);
+		const float r = lm_acosf(rcos);
+		if ((double)nl < (PSY_HPI_D - (double)r)) return nlcos * rsin2;
+		if ((double)nl < PSY_HPI_D) c = CAP_MOSTLY_ABOVE;
+		else if ((double)nl < (PSY_HPI_D + (double)r)) c = CAP_MOSTLY_BELOW;
+		else return 0.0f;
+	}
 	const float nlsin = (float)sqrt(1.0 - (double)(nlcos * nlcos));
-	const float rsin2 = (float)(1.0 - (double)(rcos * rcos));
 	const float rsin = sqrtf(rsin2);
 	const float ysin = rcos / nlsin;
 	const float ycos2 = (float)(1.0 - (double)(ysin * ysin));
@@ -184,32 +209,8 @@ static __device__ __noinline__ float sphere_lambert_partial(float nlcos, float r
 	const float g = (float)(((((-2.0 * (double)nlsin) * (double)rcos) * (double)ycos) + PSY_HPI_D) -
 	                        (double)lm_asinf(ysin) + (double)(ysin * ycos));
 	const float h = nlcos * ((ycos * sqrtf(rsin2 - ycos2)) + (rsin2 * lm_asinf(ycos / rsin)));
-	const float nl = lm_acosf(nlcos);
-	const float r = lm_acosf(rcos);
-	if ((double)nl < (PSY_HPI_D - (double)r)) return nlcos * rsin2;
-	if ((double)nl < PSY_HPI_D) return (nlcos * rsin2) + g - h;
-	if ((double)nl < (PSY_HPI_D + (double)r)) return (float)((double)(g + h) * PSY_INV_PI_D);
-	return 0.0f;
-}
-
-// The same with the two plain cases taken first: the whole cap above the
-// horizon (nl < pi/2 - r: nlcos * rsin2) and all of it below (nl >= pi/2 +
-// r: 0).  Their angle tests are decided on the cosines where those are well
-// apart: |cos a - cos b| <= |a - b|, so nlcos above sin r by 1e-3 puts nl
-// below pi/2 - r by as much, while rsin is off by at most 2.5e-4 (the
-// rounding of rcos^2) and the arc cosines by less than 1e-6.  A light tree
-// walk mostly meets these cases (small lights above or below the surface),
-// and they need none of the four arc functions.  (With the children's
-// records side by side, the spectral grid place found once and the sampler's
-// divisions by multiplication: 1.2M-path render 3.42 -> 2.99 ms, 3.1M paths
-// under 100 lights 22.5 -> 20.7 ms.)  An nlcos past +-1 by
-// rounding (its arc cosine is NaN) goes through the full form.
-__device__ __forceinline__ float sphere_lambert(float nlcos, float rcos) {
-	const float rsin2 = (float)(1.0 - (double)(rcos * rcos));
-	const float lim = sqrtf(rsin2) + 1e-3f;
-	if (nlcos > lim && nlcos <= 1.0f) return nlcos * rsin2;
-	if (nlcos < -lim && nlcos >= -1.0f) return 0.0f;
-	return sphere_lambert_partial(nlcos, rcos);
+	if (c == CAP_MOSTLY_ABOVE) return (nlcos * rsin2) + g - h;
+	return (float)((double)(g + h) * PSY_INV_PI_D);
 }
 
 __device__ __forceinline__ float power_heuristic(float a, float b) {
@@ -640,9 +641,20 @@ __device__ __forceinline__ Box light_node_box(const DevScene& sc, const DevLight
 
 // LightTree's node_prob (accel/light_tree.cpp:6-28) for a box centre seen
 // along d from the query point, half diagonal squared r2, and e_isa = energy
-// / r2.  nn is the query's normal, unit and facing it (the Lambert closure's
-// estimate takes it so for every node).
-__device__ __forceinline__ float light_prob(const LightQuery& q, V3 nn, V3 d, float r2, float e_isa) {
+// / r2, in two parts: what is quick, and (`cut`: cap_case, else -1) the caps
+// that the horizon cuts.  nn is the query's normal, unit and facing it (the
+// Lambert closure's estimate takes it so for every node).
+struct LightProb {
+	float est, e_isa;
+	float nlcos, rcos, rsin2;
+	int cut;
+};
+
+template <bool GTR>
+__device__ __forceinline__ LightProb light_prob(const LightQuery& q, V3 nn, V3 d, float r2, float e_isa) {
+	LightProb p;
+	p.e_isa = e_isa;
+	p.cut = -1;
 	const float dist2 = length2(d);
 	float cos_theta_max;
 	if (dist2 <= r2) {
@@ -652,20 +664,31 @@ __device__ __forceinline__ float light_prob(const LightQuery& q, V3 nn, V3 d, fl
 		const float sin_theta_max2 = q2 < 1.0f ? q2 : 1.0f;
 		cos_theta_max = sqrtf(1.0f - sin_theta_max2);
 	}
-	float est;
-	if (q.gtr) est = gtr_estimate(q.gp, q.d, d, cos_theta_max, q.nor);
-	else est = cos_theta_max < 0.0f ? 1.0f : sphere_lambert(dot(nn, normalized(d)), cos_theta_max);
-	const float approx_contrib = 0.0f < est ? est : 0.0f;
-	return e_isa * approx_contrib;
+	if (GTR && q.gtr) {
+		p.est = gtr_estimate(q.gp, q.d, d, cos_theta_max, q.nor);
+		return p;
+	}
+	p.est = 1.0f;
+	if (cos_theta_max < 0.0f) return p;
+	p.nlcos = dot(nn, normalized(d));
+	p.rcos = cos_theta_max;
+	p.rsin2 = (float)(1.0 - (double)(p.rcos * p.rcos));
+	const int c = cap_case(p.nlcos, p.rsin2);
+	p.est = c == CAP_ABOVE ? p.nlcos * p.rsin2 : 0.0f;
+	if (c != CAP_ABOVE && c != CAP_BELOW) p.cut = c;
+	return p;
 }
+__device__ __forceinline__ float light_prob_value(const LightProb& p) { return p.e_isa * (0.0f < p.est ? p.est : 0.0f); }
 
-// node_prob of a node whose bounds move: they are interpolated at the query's time.
-static __device__ __noinline__ float light_prob_moving(const DevScene& sc, const LightQuery& q, V3 nn, int index) {
+// The box of a node whose bounds move, at the query's time.
+static __device__ __noinline__ void light_moving(const DevScene& sc, V3 pos, float time, int index, V3* d, float* r2,
+                                                 float* e_isa) {
 	const DevLightNode nd = sc.light_nodes[index];
-	const Box bbox = light_node_box(sc, nd, q.time);
+	const Box bbox = light_node_box(sc, nd, time);
 	const float r = box_diagonal(bbox) * 0.5f;
-	const float r2 = r * r;
-	return light_prob(q, nn, box_center(bbox) - q.pos, r2, nd.energy * (1.0f / r2));
+	*r2 = r * r;
+	*e_isa = nd.energy * (1.0f / *r2);
+	*d = box_center(bbox) - pos;
 }
 
 // SphereLight::sample; returns the colour scale and writes the shadow vector and pdf.
@@ -788,7 +811,7 @@ static __device__ __noinline__ M44 m44_inverse_dev(const M44& a, const RcpTable&
 
 // LightTree::sample starting at the root assembly's tree, in two parts: the
 // walk to a light (q->obj, -1 when there is none), and its sample.
-template <unsigned F>
+template <unsigned F, bool GTR>
 static __device__ __forceinline__ void light_tree_pick(const DevScene& sc, LightQuery* q) {
 	constexpr bool NESTED = (F & FEAT_NESTED) != 0, XFORM = (F & FEAT_XFORM) != 0;
 	q->valid = false;
@@ -810,10 +833,27 @@ static __device__ __forceinline__ void light_tree_pick(const DevScene& sc, Light
 			const float4* pr = reinterpret_cast<const float4*>(sc.light_pairs + node);
 			const float4 a = __ldg(pr), b = __ldg(pr + 1), c = __ldg(pr + 2);
 			const int2 ch = __ldg(reinterpret_cast<const int2*>(pr + 3));
-			float p1 = a.w < 0.0f ? light_prob_moving(sc, *q, nn, sc.light_nodes[node].c1)
-			                      : light_prob(*q, nn, V3(a.x, a.y, a.z) - q->pos, a.w, c.x);
-			float p2 = b.w < 0.0f ? light_prob_moving(sc, *q, nn, sc.light_nodes[node].c2)
-			                      : light_prob(*q, nn, V3(b.x, b.y, b.z) - q->pos, b.w, c.y);
+			V3 d1 = V3(a.x, a.y, a.z) - q->pos, d2 = V3(b.x, b.y, b.z) - q->pos;
+			float r1 = a.w, r2 = b.w, e1 = c.x, e2 = c.y;
+			if (r1 < 0.0f) light_moving(sc, q->pos, q->time, sc.light_nodes[node].c1, &d1, &r1, &e1);
+			if (r2 < 0.0f) light_moving(sc, q->pos, q->time, sc.light_nodes[node].c2, &d2, &r2, &e2);
+			LightProb l1 = light_prob<GTR>(*q, nn, d1, r1, e1);
+			LightProb l2 = light_prob<GTR>(*q, nn, d2, r2, e2);
+			// cut caps one after the other, a lane's first with the other
+			// lanes' first whichever child it is: most have one at most
+			while (l1.cut >= 0 || l2.cut >= 0) {
+				const bool first = l1.cut >= 0;
+				const float est = sphere_lambert_cut(first ? l1.nlcos : l2.nlcos, first ? l1.rcos : l2.rcos,
+				                                     first ? l1.rsin2 : l2.rsin2, first ? l1.cut : l2.cut);
+				if (first) {
+					l1.est = est;
+					l1.cut = -1;
+				} else {
+					l2.est = est;
+					l2.cut = -1;
+				}
+			}
+			float p1 = light_prob_value(l1), p2 = light_prob_value(l2);
 			const float total = p1 + p2;
 			if (total <= 0.0f) {
 				p1 = 0.5f;

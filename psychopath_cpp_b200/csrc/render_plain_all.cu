@@ -4,5 +4,5 @@
 #include "render_wave.cuh"
 
 namespace psy {
-template void launch_wave<PlainWave, FEAT_ALL>(const PlainWave&, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
+template void launch_wave<PlainWave, FEAT_ALL>(const PlainWave&, int, uint32_t, const HaltonDev&, const WaveRange&, const PathSoA&, const WaveBufs&, const WaveQueues&, unsigned*, int, size_t, cudaStream_t, uint32_t*, const LaunchTimer*);
 }  // namespace psy

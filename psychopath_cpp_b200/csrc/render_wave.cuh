@@ -168,7 +168,7 @@ struct GtrVertex {
 // (basics/differential_geometry.hpp:20-40), the offset of
 // path_trace_integrator.cpp:141-145 and the transferred differentials of
 // propagate_differentials.
-template <unsigned F>
+template <unsigned F, bool GTR>
 __device__ __forceinline__ void make_vertex(const DevScene& sc, const HitRec& rec, const HitPath& path, const WorldRayD& wr, float ident_inv,
                                             Vertex* sh, GtrVertex* gv, int* closure, float* light_pdf, unsigned* err) {
 	M44 space;
@@ -179,11 +179,11 @@ __device__ __forceinline__ void make_vertex(const DevScene& sc, const HitRec& re
 		ld = dir_to(space, wr.d);
 	}
 	HitInfo h;
-	hit_geometry(sc, rec, wr.time, lo, ld, false, &h);
+	hit_geometry<GTR>(sc, rec, wr.time, lo, ld, false, &h);
 	*closure = h.closure;
 	sh->col[0] = h.col[0]; sh->col[1] = h.col[1]; sh->col[2] = h.col[2];
 	*light_pdf = h.light_pdf;
-	if (h.closure != CLOSURE_LAMBERT && h.closure != CLOSURE_GTR) return;
+	if (h.closure != CLOSURE_LAMBERT && !(GTR && h.closure == CLOSURE_GTR)) return;
 	M44 inv;
 	if (xf) {
 		inv = m44_inverse_dev(space, sc.rcp);
@@ -197,7 +197,7 @@ __device__ __forceinline__ void make_vertex(const DevScene& sc, const HitRec& re
 	const float il = 1.0f / length(n);
 	sh->n = n * il;
 	sh->gtr = -1;
-	if (h.closure == CLOSURE_GTR) {
+	if (GTR && h.closure == CLOSURE_GTR) {
 		// the rest of DifferentialGeometry::transformed_from (basics/differential_geometry.hpp:20-40)
 		sh->gtr = rec.shader;
 		gv->dpdu = dir_to(inv, h.geo.dpdu);
@@ -672,20 +672,26 @@ __global__ void __launch_bounds__(TraceCfg<F>::BLOCK, TraceCfg<F>::MIN_BLOCKS)
 // own); in phase they share the lines.
 // ---------------------------------------------------------------------
 //
-// 512 threads and 40 registers (3 blocks an SM; the spills stay in L1): the
-// 512x384x16 frame with 50,000 primitives takes 13.98 ms, 14.23 with 2
-// blocks of 64 registers, 14.30 with 4 of 32, 14.81 with 4 blocks of 256
-// threads, 17.49 with 8 of 128 (one kernel each for hit and shadow shading,
-// warps on their own: 18.23).
+// 512 threads, 2 blocks an SM (64 registers; the spills stay in L1), or 3 (40)
+// in the adjoint pass, which keeps more of a vertex.  Fewer threads a block
+// lose the phases' order: while hit and shadow shading had just been joined,
+// the 512x384x16 frame with 50,000 primitives took 13.98 ms with 3 x 512,
+// 14.23 with 2, 14.30 with 4, 14.81 with 4 x 256, 17.49 with 8 x 128.  Without
+// the GTR code 2 and 3 blocks take 12.4 ms, the GTR frame 0.75 and 0.79, the
+// differentiable step 7.63 and 7.37.
 #define PSY_SHADE_BLOCK 512
-#define PSY_SHADE_MIN_BLOCKS 3
-template <class W, bool CAMERA, unsigned F>
-__global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
+constexpr int shade_min_blocks(unsigned mode) { return (mode & 2u) ? 3 : 2; }
+
+enum : unsigned { SHADE_GTR = 1u, SHADE_ADJOINT = 2u };
+
+template <class W, bool CAMERA, unsigned F, unsigned MODE>
+__global__ void __launch_bounds__(PSY_SHADE_BLOCK, shade_min_blocks(MODE))
     shade_kernel(W w, HaltonDev hd, PathSoA ps, WaveBufs wb, const float4* __restrict__ rin, float4* __restrict__ rout,
                  float4* __restrict__ rshadow, const int* __restrict__ q_in, const int* n_dev, int n_host, int* q_out,
                  int* n_out, unsigned* status) {
 	extern __shared__ __align__(16) float sgrad[];
-	if (!W::BATCH) grad_begin(w.render(0), sgrad);
+	constexpr bool GTR = (MODE & SHADE_GTR) != 0, ADJOINT = !W::BATCH && (MODE & SHADE_ADJOINT) != 0;
+	if (ADJOINT) grad_begin(w.render(0), sgrad);
 	const int lane = threadIdx.x & 31;
 	const int n = n_dev ? *n_dev : n_host;
 	unsigned err = 0;
@@ -716,7 +722,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 				if (wb.occl[i] == 0) {
 					const Spec c = sp(ps.lcol[slot]);
 					for (int k = 0; k < 4; ++k) col.e[k] += c.e[k];
-					if (!W::BATCH && rp.grad)
+					if (ADJOINT)
 						grad_add(rp, sgrad, ps, slot, (int)(step >> 1), sp(ps.nee_base[slot]), ps.nee_param[slot], wl);
 				}
 			}
@@ -732,7 +738,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 					hit_surface(sc, &rec, path);
 					int closure;
 					float lpdf;
-					make_vertex<F>(sc, rec, path, wr, rp.ident_inv, &sh, &gv, &closure, &lpdf, &err);
+					make_vertex<F, GTR>(sc, rec, path, wr, rp.ident_inv, &sh, &gv, &closure, &lpdf, &err);
 					const int vtx = (int)(step >> 1);  // index of this path vertex
 					if (closure == CLOSURE_EMIT) {
 						const Spec e0 = rgb_to_spec(sh.col, wl);
@@ -746,7 +752,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 						for (int k = 0; k < 4; ++k)
 							C.e[k] = mis ? ((fcol.e[k] * last_pdf) * e.e[k]) * mis_inv_pdf : fcol.e[k] * e.e[k];
 						for (int k = 0; k < 4; ++k) col.e[k] += C.e[k];
-						if (!W::BATCH && rp.grad) {
+						if (ADJOINT) {
 							// the same contribution without its parameterised factors
 							const Spec fx = sp(ps.fexcl[slot]);
 							Spec B;
@@ -754,13 +760,13 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 								B.e[k] = mis ? ((fx.e[k] * last_pdf) * e0.e[k]) * mis_inv_pdf : fx.e[k] * e0.e[k];
 							grad_add(rp, sgrad, ps, slot, vtx, B, lp, wl);
 						}
-					} else if (closure == CLOSURE_LAMBERT || closure == CLOSURE_GTR) {
+					} else if (closure == CLOSURE_LAMBERT || (GTR && closure == CLOSURE_GTR)) {
 						// (closures outside the supported set end the path)
 						live = true;
 						sh.pid = (rp.params && rec.shader >= 0) ? rp.shader_param[rec.shader] : -1;
-						gtr = sh.gtr >= 0;
+						gtr = GTR && sh.gtr >= 0;
 						delta = gtr && gtr_is_delta(gtr_of(sc.shaders[sh.gtr]));
-						if (!W::BATCH && rp.grad && vtx < PSY_ADJ_MAX_VERTS) {
+						if (ADJOINT && vtx < PSY_ADJ_MAX_VERTS) {
 							Spec a = Spec{};
 							if (sh.pid >= 0) {
 								a = albedo_spec(rp.params + sh.pid, wl);
@@ -809,7 +815,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 			q.light_sample_pdf = 1.0f;
 			q.gtr = gtr;
 			if (gtr) q.gp = gtr_of(sc.shaders[sh.gtr]);
-			light_tree_pick<F>(sc, &q);
+			light_tree_pick<F, GTR>(sc, &q);
 		}
 		__syncthreads();
 		// ---- light sample and shadow ray
@@ -826,7 +832,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 				float4 last = rin[4 * cap + i];
 				last.w = __int_as_float(rid << 1);
 				rshadow[4 * cap + j] = last;
-				if (!W::BATCH && rp.grad) {
+				if (ADJOINT) {
 					ps.nee_param[slot] = -1;
 					ps.nee_base[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 				}
@@ -842,7 +848,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 					const int lp = emission_param(rp, q.obj);
 					if (lp >= 0)
 						for (int k = 0; k < 4; ++k) lcol.e[k] *= rp.params[lp];
-					if (!W::BATCH && rp.grad) ps.nee_param[slot] = lp;
+					if (ADJOINT) ps.nee_param[slot] = lp;
 					WorldRayD sray;
 					sray.o = sh.p + sh.off;
 					sray.d = (q.to_light - sh.off) * 0.9995f;
@@ -857,7 +863,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 					Spec c;
 					for (int k = 0; k < 4; ++k) c.e[k] = (fcol.e[k] * lcol.e[k]) * fac.e[k];
 					contrib = f4(c);
-					if (!W::BATCH && rp.grad) {
+					if (ADJOINT) {
 						// without the light's scale and the albedos of parameterised vertices
 						const Spec fx = sp(ps.fexcl[slot]);
 						const float cs = gtr ? 0.0f : lambert_cos(sh.d, sray.d, sh.n);
@@ -917,7 +923,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 				} else {
 					for (int k = 0; k < 4; ++k) fcol.e[k] *= filter.e[k];
 				}
-				if (!W::BATCH && rp.grad) {
+				if (ADJOINT) {
 					// the path weight without the parameterised albedos
 					Spec fx = sp(ps.fexcl[slot]);
 					const float cs = gtr ? 0.0f : lambert_cos(sh.d, out, sh.n);
@@ -931,7 +937,7 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, PSY_SHADE_MIN_BLOCKS)
 		}
 		__syncthreads();
 	}
-	if (!W::BATCH) grad_end(w.render(0), sgrad);
+	if (ADJOINT) grad_end(w.render(0), sgrad);
 	if (err) atomicOr(status, err);
 }
 
@@ -1019,10 +1025,18 @@ static int persistent_grid(K kernel, int block) {
 	return sms * (b < 1 ? 1 : b);
 }
 
+// The compiled shading modes: Lambert and emission only (the closures of most
+// scenes: without the GTR code and its vertex data there is less to spill),
+// all closures, and the adjoint pass.  One kernel for all three: 512x384x16
+// frame with 50,000 primitives 13.7 ms, 12.4 so (together with
+// light_tree_pick's cut caps).
+static constexpr int SHADE_MODES = 3;
+inline int shade_mode(unsigned features, bool adjoint) { return adjoint ? 2 : (features & FEAT_GTR) ? 1 : 0; }
+
 struct WaveGrids {
 	int block = 0;
 	int trace_b = 0;  // traversal block size
-	int trace, shade_c, shade_b, last, sms;
+	int trace, shade_c[SHADE_MODES], shade_b[SHADE_MODES], last, sms;
 };
 
 template <class W, unsigned F>
@@ -1035,8 +1049,14 @@ static const WaveGrids& grids_for(int block) {
 		n.block = block;
 		n.trace_b = TraceCfg<F>::launch_block(block);
 		n.trace = persistent_grid(trace_wave_kernel<W, F>, n.trace_b);
-		n.shade_c = persistent_grid(shade_kernel<W, true, F>, PSY_SHADE_BLOCK);
-		n.shade_b = persistent_grid(shade_kernel<W, false, F>, PSY_SHADE_BLOCK);
+		n.shade_c[0] = persistent_grid(shade_kernel<W, true, F, 0u>, PSY_SHADE_BLOCK);
+		n.shade_b[0] = persistent_grid(shade_kernel<W, false, F, 0u>, PSY_SHADE_BLOCK);
+		n.shade_c[1] = persistent_grid(shade_kernel<W, true, F, SHADE_GTR>, PSY_SHADE_BLOCK);
+		n.shade_b[1] = persistent_grid(shade_kernel<W, false, F, SHADE_GTR>, PSY_SHADE_BLOCK);
+		if constexpr (!W::BATCH) {
+			n.shade_c[2] = persistent_grid(shade_kernel<W, true, F, SHADE_GTR | SHADE_ADJOINT>, PSY_SHADE_BLOCK);
+			n.shade_b[2] = persistent_grid(shade_kernel<W, false, F, SHADE_GTR | SHADE_ADJOINT>, PSY_SHADE_BLOCK);
+		}
 		n.last = persistent_grid(shade_last_kernel<W>, 256);
 		n.sms = sm_count();
 		g[k] = n;
@@ -1049,7 +1069,7 @@ static const WaveGrids& grids_for(int block) {
 inline int wave_counter_count(uint32_t path_length) { return 2 * ((int)path_length + 1); }
 
 template <class W, unsigned F>
-void launch_wave(const W& w, uint32_t path_length, const HaltonDev& hd, const WaveRange& wv,
+void launch_wave(const W& w, int mode, uint32_t path_length, const HaltonDev& hd, const WaveRange& wv,
                         const PathSoA& ps, const WaveBufs& wb, const WaveQueues& wq, unsigned* status, int block,
                         size_t gsmem, cudaStream_t st, uint32_t* launches, const LaunchTimer* tm) {
 	const WaveGrids& g = grids_for<W, F>(block);
@@ -1084,12 +1104,20 @@ void launch_wave(const W& w, uint32_t path_length, const HaltonDev& hd, const Wa
 		int* q2 = (q == wq.q0) ? wq.q1 : wq.q0;
 		if (v == path_length)
 			shade_last_kernel<W><<<grid(g.last, 256), 256, gsmem, st>>>(w, ps, wb, q, n);
-		else if (v == 0)
-			shade_kernel<W, true, F><<<grid(g.shade_c * per, sb), sb, gsmem, st>>>(
-			    w, hd, ps, wb, rin, rout, rshadow, nullptr, nullptr, P, q2, c + 1, status);
-		else
-			shade_kernel<W, false, F><<<grid(g.shade_b * per, sb), sb, gsmem, st>>>(
-			    w, hd, ps, wb, rin, rout, rshadow, q, n, 0, q2, c + 1, status);
+		else {
+			auto shade = [&](auto first, auto later) {
+				if (v == 0)
+					first<<<grid(g.shade_c[mode] * per, sb), sb, gsmem, st>>>(w, hd, ps, wb, rin, rout, rshadow, nullptr, nullptr,
+					                                                         P, q2, c + 1, status);
+				else
+					later<<<grid(g.shade_b[mode] * per, sb), sb, gsmem, st>>>(w, hd, ps, wb, rin, rout, rshadow, q, n, 0, q2,
+					                                                         c + 1, status);
+			};
+			if (mode == 0) shade(shade_kernel<W, true, F, 0u>, shade_kernel<W, false, F, 0u>);
+			else if (mode == 1) shade(shade_kernel<W, true, F, SHADE_GTR>, shade_kernel<W, false, F, SHADE_GTR>);
+			else if constexpr (!W::BATCH)
+				shade(shade_kernel<W, true, F, SHADE_GTR | SHADE_ADJOINT>, shade_kernel<W, false, F, SHADE_GTR | SHADE_ADJOINT>);
+		}
 		float4* t = const_cast<float4*>(rin);
 		rin = rout;
 		rout = t;

@@ -967,6 +967,7 @@ struct Builder {
 			ds.fresnel = desc->shaders[s].fresnel;
 			if (ds.kind < 0 || ds.kind > 2) return fail("unknown shader kind");
 			if (ds.kind == SHADER_GTR) {
+				out->features |= FEAT_GTR;
 				// GTRClosure::validate (shading/surface_closure.hpp:352-372)
 				float r = std::max(0.0f, std::min(0.9999f, ds.roughness));
 				float t = std::max(0.0001f, ds.tail_shape);

@@ -194,6 +194,7 @@ __device__ __forceinline__ void closure_of_shader(const DevScene& sc, int shader
 // sphere's u, v, which come with them) cost more than the rest of a hit's
 // geometry and are left out unless `derivs` asks for them or the closure is
 // the one that reads them (GTR).
+template <bool GTR>
 static __device__ __forceinline__ void hit_geometry(const DevScene& sc, const HitRec& rec, float time, V3 lo, V3 ld, bool derivs, HitInfo* h) {
 	const DevObject ob = sc.objects[rec.obj];
 	const float t = rec.t;
@@ -208,7 +209,7 @@ static __device__ __forceinline__ void hit_geometry(const DevScene& sc, const Hi
 		h->backfacing = dot(g.n, normalized(ld)) > 0.0f;
 		h->offset = g.n * 0.000001f;
 		closure_of_shader(sc, rec.shader, h);
-		if (!derivs && h->closure != CLOSURE_GTR) return;
+		if (!derivs && !(GTR && h->closure == CLOSURE_GTR)) return;
 		const V3 unit_p = g.n;
 		const V3 p = unit_p * radi;
 		const float lat_cos = unit_p.z;
@@ -276,7 +277,7 @@ static __device__ __forceinline__ void hit_geometry(const DevScene& sc, const Hi
 		g.v = rec.v;
 		const float* verts = sc.fpool + ob.data;
 		closure_of_shader(sc, rec.shader, h);
-		derivs = derivs || h->closure == CLOSURE_GTR;
+		derivs = derivs || (GTR && h->closure == CLOSURE_GTR);
 		if (ob.kind == OBJ_BILINEAR) {
 			Patch<4> q;
 			patch_at<4>(verts, ob.n0, time, &q);

@@ -107,7 +107,7 @@ __global__ void __maxnreg__(TraceKernelRegs<F>::value) trace_kernel(DevScene sc,
 			space = m44_identity();
 		}
 		HitInfo h;
-		hit_geometry(sc, rec, wr.time, lo, ld, hits.want_geometry != WANT_POINT, &h);
+		hit_geometry<true>(sc, rec, wr.time, lo, ld, hits.want_geometry != WANT_POINT, &h);
 		if (hits.uv) {
 			hits.uv[2 * (size_t)i] = h.geo.u;
 			hits.uv[2 * (size_t)i + 1] = h.geo.v;

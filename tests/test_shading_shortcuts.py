@@ -53,6 +53,12 @@ def test_sphere_lambert_plain_cases(near):
     lim = np.sqrt(rsin2) + F(1e-3)
     above, below = nlcos > lim, nlcos < -lim
     nl, r = np.arccos(nlcos.astype(np.float64)), np.arccos(rcos.astype(np.float64))
+    rsin, m = np.sqrt(rsin2), F(1e-3)
+    mostly_above = (nlcos > m) & (nlcos < rsin - m)
+    mostly_below = (nlcos < -m) & (nlcos > m - rsin)
     assert above.sum() > 1000 and below.sum() > 1000
+    for mostly, lo, hi in ((mostly_above, np.pi / 2 - r, np.pi / 2 + 0 * r), (mostly_below, np.pi / 2 + 0 * r, np.pi / 2 + r)):
+        assert mostly.sum() > 1000 or near > 0.999
+        assert np.all(nl[mostly] > lo[mostly] + 1e-4) and np.all(nl[mostly] < hi[mostly] - 1e-4)
     assert np.all(nl[above] < np.pi / 2 - r[above] - 1e-4)
     assert np.all(nl[below] > np.pi / 2 + r[below] + 1e-4)
