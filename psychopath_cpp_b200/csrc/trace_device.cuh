@@ -260,34 +260,24 @@ __device__ __forceinline__ void patch_load(const float* src, Patch<NV>* q) {
 	for (int i = 0; i < NV; ++i) q->p[i] = V3(__ldg(src + i * 3), __ldg(src + i * 3 + 1), __ldg(src + i * 3 + 2));
 }
 
-// Splits of a patch at the middle of u or v (Bilinear::split_u / split_v,
-// object/bilinear.hpp:59-82; Bicubic::split_u / split_v, de Casteljau at 0.5
-// per row or column, object/bicubic.hpp:74-108), with the reference's float
-// operations.  patch_split leaves the second half in `p` and writes the
-// first half to `f`.
-__device__ __forceinline__ void patch_split(Patch<4>& p, Patch<4>& f, bool along_u) {
-	if (along_u) {
-		const V3 m01 = (p.p[0] + p.p[1]) * 0.5f;
-		const V3 m23 = (p.p[2] + p.p[3]) * 0.5f;
-		f.p[0] = p.p[0];
-		f.p[1] = m01;
-		f.p[2] = p.p[2];
-		f.p[3] = m23;
-		p.p[0] = m01;
-		p.p[2] = m23;
-	} else {
-		const V3 m02 = (p.p[0] + p.p[2]) * 0.5f;
-		const V3 m13 = (p.p[1] + p.p[3]) * 0.5f;
-		f.p[0] = p.p[0];
-		f.p[1] = p.p[1];
-		f.p[2] = m02;
-		f.p[3] = m13;
-		p.p[0] = m02;
-		p.p[1] = m13;
-	}
+// A split of a patch at the middle of its first direction (Bilinear::split_u,
+// object/bilinear.hpp:59-82; Bicubic::split_u, de Casteljau at 0.5 per row,
+// object/bicubic.hpp:74-108), with the reference's float operations: the
+// second half is left in `p`, the first goes to `f`.  split_v is the same on
+// the transposed patch.
+__device__ __forceinline__ void patch_split(Patch<4>& p, Patch<4>& f) {
+	const V3 m01 = (p.p[0] + p.p[1]) * 0.5f;
+	const V3 m23 = (p.p[2] + p.p[3]) * 0.5f;
+	f.p[0] = p.p[0];
+	f.p[1] = m01;
+	f.p[2] = p.p[2];
+	f.p[3] = m23;
+	p.p[0] = m01;
+	p.p[2] = m23;
 }
-// One de Casteljau split at 0.5 of the control points a,b,c,d of a row or a
-// column: a..d become the second half, fa..fd the first.
+
+// One de Casteljau split at 0.5 of the control points a,b,c,d of a row: a..d
+// become the second half, fa..fd the first.
 __device__ __forceinline__ void bezier_split(V3& a, V3& b, V3& c, V3& d, V3& fa, V3& fb, V3& fc, V3& fd) {
 	const V3 tmp = (b + c) * 0.5f;
 	const V3 q2 = (d + c) * 0.5f;
@@ -303,18 +293,32 @@ __device__ __forceinline__ void bezier_split(V3& a, V3& b, V3& c, V3& d, V3& fa,
 	b = q1;
 	c = q2;
 }
-__device__ __forceinline__ void patch_split(Patch<16>& p, Patch<16>& f, bool along_u) {
-	if (along_u) {
+__device__ __forceinline__ void patch_split(Patch<16>& p, Patch<16>& f) {
 #pragma unroll
-		for (int r = 0; r < 4; ++r)
-			bezier_split(p.p[r * 4], p.p[r * 4 + 1], p.p[r * 4 + 2], p.p[r * 4 + 3], f.p[r * 4], f.p[r * 4 + 1],
-			             f.p[r * 4 + 2], f.p[r * 4 + 3]);
-	} else {
-#pragma unroll
-		for (int c = 0; c < 4; ++c)
-			bezier_split(p.p[c], p.p[c + 4], p.p[c + 8], p.p[c + 12], f.p[c], f.p[c + 4], f.p[c + 8], f.p[c + 12]);
-	}
+	for (int r = 0; r < 4; ++r)
+		bezier_split(p.p[r * 4], p.p[r * 4 + 1], p.p[r * 4 + 2], p.p[r * 4 + 3], f.p[r * 4], f.p[r * 4 + 1],
+		             f.p[r * 4 + 2], f.p[r * 4 + 3]);
 }
+
+// Exchanges the patch's two directions where `t` says so, by selection.
+__device__ __forceinline__ void swap_if(bool t, float& a, float& b) {
+	const float x = t ? b : a, y = t ? a : b;
+	a = x;
+	b = y;
+}
+__device__ __forceinline__ void swap_if(bool t, V3& a, V3& b) {
+	swap_if(t, a.x, b.x);
+	swap_if(t, a.y, b.y);
+	swap_if(t, a.z, b.z);
+}
+__device__ __forceinline__ void patch_transpose_if(bool t, Patch<4>& p) { swap_if(t, p.p[1], p.p[2]); }
+__device__ __forceinline__ void patch_transpose_if(bool t, Patch<16>& p) {
+#pragma unroll
+	for (int r = 0; r < 4; ++r)
+#pragma unroll
+		for (int c = r + 1; c < 4; ++c) swap_if(t, p.p[r * 4 + c], p.p[c * 4 + r]);
+}
+
 // Four floats as two packed pairs.
 struct Quad {
 	unsigned long long a, b;
@@ -481,12 +485,19 @@ __device__ __forceinline__ float flip_min_width(const RayFlip& w, float tnear, f
 // with the other lanes of its warp.  patch_run works on a cursor the caller
 // holds as a local (kept in registers) and copies back only when it stops
 // short of the end.
+//
+// A node may be kept transposed (`tr`): a patch to be split along its second
+// direction is transposed by selection first, so that the lanes of a warp
+// split along either direction in one piece of code (300,000 mixed rays
+// against bicubic ground: 1.91 -> 1.68 ms, 4M rays against the heightfield
+// 1.02 -> 0.97).
 template <int NV, int TSC>
 struct PatchCursor {
 	Patch<NV> cur[TSC];        // the node at the top of the loop
-	float u0, u1, v0, v1;
+	float a0, a1, b0, b1;      // its range along its first and second direction (u and v, or v and u if tr)
 	float max_dim, h0, h1;     // its test
 	float t_nalpha;
+	bool tr;
 	int depth, seconds;        // splits from the root, second halves among them
 	int sp;                    // pending first halves on the stack
 	unsigned steps;            // loop iterations taken (bounded: PSY_PATCH_MAX_STEPS)
@@ -496,8 +507,8 @@ struct PatchCursor {
 template <int NV, int TSC>
 struct PatchStore {
 	Patch<NV> pend[PSY_PATCH_PEND][TSC];
-	float4 uv[PSY_PATCH_PEND];
-	int2 at[PSY_PATCH_PEND];   // depth, second halves
+	float4 ab[PSY_PATCH_PEND];
+	int2 at[PSY_PATCH_PEND];   // depth * 2 + tr, second halves
 };
 
 // The root's test: sets up `pc` and returns true when the ray hits the
@@ -516,8 +527,9 @@ __device__ __forceinline__ bool patch_begin(PatchCursor<NV, TSC>& pc, const floa
 		pc.t_nalpha = t_time - (float)(int)t_time;
 	}
 	if (!patch_node_test<NV, TSC, CLEAN>(pc.cur, pc.t_nalpha, o, dinv, max_t, &pc.max_dim, &pc.h0, &pc.h1)) return false;
-	pc.u0 = pc.v0 = 0.0f;
-	pc.u1 = pc.v1 = 1.0f;
+	pc.a0 = pc.b0 = 0.0f;
+	pc.a1 = pc.b1 = 1.0f;
+	pc.tr = false;
 	pc.depth = 0;
 	pc.seconds = 0;
 	pc.sp = 0;
@@ -541,7 +553,21 @@ __device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV
 	Patch<NV>(&cur)[TSC] = pc.cur;
 	const float t_nalpha = pc.t_nalpha;
 	float &max_dim = pc.max_dim, &h0 = pc.h0, &h1 = pc.h1;
-	float &u0 = pc.u0, &u1 = pc.u1, &v0 = pc.v0, &v1 = pc.v1;
+	float &a0 = pc.a0, &a1 = pc.a1, &b0 = pc.b0, &b1 = pc.b1;
+	// (where NaN can occur, the order of a bound's minima matters: the
+	// patch's own)
+	auto test = [&](const Patch<NV>(&q)[TSC], float* md, float* t0, float* t1) {
+		if constexpr (CLEAN) {
+			return patch_node_test<NV, TSC, true>(q, t_nalpha, o, dinv, *max_t, md, t0, t1);
+		} else {
+			Patch<NV> own[TSC];
+			for (int k = 0; k < TSC; ++k) {
+				own[k] = q[k];
+				patch_transpose_if(pc.tr, own[k]);
+			}
+			return patch_node_test<NV, TSC, false>(own, t_nalpha, o, dinv, *max_t, md, t0, t1);
+		}
+	};
 	while (true) {
 		if (units == 0) return PATCH_MORE;
 		--units;
@@ -562,18 +588,28 @@ __device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV
 			const float tt = (h0 + h1) * 0.5f;
 			if (tt > 0.0f && tt < *max_t) {
 				if (!occl) *max_t = tt;
-				leaf(tt, (u0 + u1) * 0.5f, (v0 + v1) * 0.5f, max_dim);
+				const float a = (a0 + a1) * 0.5f, b = (b0 + b1) * 0.5f;
+				leaf(tt, pc.tr ? b : a, pc.tr ? a : b, max_dim);
 				if (occl) return PATCH_BLOCKED;
 			}
 		} else {
-			const bool along_u = patch_ulen(cur[0]) > patch_vlen(cur[0]);
+			// the longer direction is split, the second one on a tie (split_u
+			// only if u is strictly longer)
+			const float la = patch_ulen(cur[0]), lb = patch_vlen(cur[0]);
+			const bool turn = pc.tr ? la < lb : !(la > lb);
+			pc.tr = pc.tr != turn;
+			swap_if(turn, a0, b0);
+			swap_if(turn, a1, b1);
 			Patch<NV> first[TSC];
 #pragma unroll
-			for (int k = 0; k < TSC; ++k) patch_split(cur[k], first[k], along_u);
+			for (int k = 0; k < TSC; ++k) {
+				patch_transpose_if(turn, cur[k]);
+				patch_split(cur[k], first[k]);
+			}
 			float smd, sh0, sh1, fmd, fh0, fh1;
-			const bool s_hit = patch_node_test<NV, TSC, CLEAN>(cur, t_nalpha, o, dinv, *max_t, &smd, &sh0, &sh1);
-			const bool f_hit = patch_node_test<NV, TSC, CLEAN>(first, t_nalpha, o, dinv, *max_t, &fmd, &fh0, &fh1);
-			const float mid = along_u ? (u0 + u1) * 0.5f : (v0 + v1) * 0.5f;
+			const bool s_hit = test(cur, &smd, &sh0, &sh1);
+			const bool f_hit = test(first, &fmd, &fh0, &fh1);
+			const float mid = (a0 + a1) * 0.5f;
 			if (s_hit) {
 				++pc.depth;
 				if (f_hit) {
@@ -581,11 +617,11 @@ __device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV
 					const int q = pc.sp++;
 #pragma unroll
 					for (int k = 0; k < TSC; ++k) ps.pend[q][k] = first[k];
-					ps.uv[q] = make_float4(u0, along_u ? mid : u1, v0, along_u ? v1 : mid);
-					ps.at[q] = make_int2(pc.depth, pc.seconds);
+					ps.ab[q] = make_float4(a0, mid, b0, b1);
+					ps.at[q] = make_int2(pc.depth * 2 + (pc.tr ? 1 : 0), pc.seconds);
 				}
 				++pc.seconds;
-				if (along_u) u0 = mid; else v0 = mid;
+				a0 = mid;
 				max_dim = smd;
 				h0 = sh0;
 				h1 = sh1;
@@ -595,7 +631,7 @@ __device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV
 				++pc.depth;
 #pragma unroll
 				for (int k = 0; k < TSC; ++k) cur[k] = first[k];
-				if (along_u) u1 = mid; else v1 = mid;
+				a1 = mid;
 				max_dim = fmd;
 				h0 = fh0;
 				h1 = fh1;
@@ -608,11 +644,13 @@ __device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV
 			const int q = --pc.sp;
 #pragma unroll
 			for (int k = 0; k < TSC; ++k) cur[k] = ps.pend[q][k];
-			const float4 w = ps.uv[q];
-			u0 = w.x; u1 = w.y; v0 = w.z; v1 = w.w;
-			pc.depth = ps.at[q].x;
-			pc.seconds = ps.at[q].y;
-			if (patch_node_test<NV, TSC, CLEAN>(cur, t_nalpha, o, dinv, *max_t, &max_dim, &h0, &h1)) break;
+			const float4 w = ps.ab[q];
+			a0 = w.x; a1 = w.y; b0 = w.z; b1 = w.w;
+			const int2 at = ps.at[q];
+			pc.depth = at.x >> 1;
+			pc.tr = (at.x & 1) != 0;
+			pc.seconds = at.y;
+			if (test(cur, &max_dim, &h0, &h1)) break;
 		}
 	}
 }
