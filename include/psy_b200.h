@@ -332,6 +332,14 @@ typedef struct psy_light_sample_soa {
 int psy_light_sample(psy_ctx* ctx, const psy_light_query_soa* q, uint32_t n, const psy_light_sample_soa* out,
                      void* stream);
 
+/*
+ * The same with host arrays, one row a query (synchronous): rows of 15
+ * floats (n, u, v, pos xyz, nor xyz, d xyz, wavelength, time, unused) in,
+ * rows of 14 floats (to_light xyz, spec x4, the query's wavelength,
+ * selection_pdf, light_pdf, 4 zeros) and ids (may be NULL) out.
+ */
+int psy_light_sample_rows(psy_ctx* ctx, const float* rows, uint32_t n, float* out, uint64_t* ids);
+
 /* ------------------------------------------------------------------ */
 /* Rendering                                                            */
 /* ------------------------------------------------------------------ */

@@ -151,7 +151,7 @@ EXPORTED = ["psy_ctx_create", "psy_ctx_destroy", "psy_last_error", "psy_version"
             "psy_scene_stats_get", "psy_build_bvh4", "psy_build_light_tree", "psy_trace", "psy_trace_host", "psy_sync",
             "psy_trace_host_noalloc", "psy_render_batch", "psy_batch_autotune", "psy_render_diff",
             "psy_render_adjoint", "psy_profile_enable", "psy_profile_read", "psy_profile_counters",
-            "psy_light_sample", "psy_render", "psy_film_srgb8", "psy_math_check", "psy_file_parse",
+            "psy_light_sample", "psy_light_sample_rows", "psy_render", "psy_film_srgb8", "psy_math_check", "psy_file_parse",
             "psy_file_scene_desc", "psy_file_render_settings", "psy_file_free"]
 
 _lib = None
@@ -195,6 +195,8 @@ def load():
     if hasattr(L, "psy_trace_host_noalloc"):
         L.psy_trace_host_noalloc.argtypes = [C.c_void_p, C.POINTER(RaySoA), C.c_uint32, C.POINTER(HitSoA),
                                              C.c_void_p]
+    if hasattr(L, "psy_light_sample_rows"):
+        L.psy_light_sample_rows.argtypes = [C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p, C.c_void_p]
     if hasattr(L, "psy_light_sample"):
         L.psy_light_sample.argtypes = [C.c_void_p, C.POINTER(LightQuerySoA), C.c_uint32,
                                        C.POINTER(LightSampleSoA), C.c_void_p]

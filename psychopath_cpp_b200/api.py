@@ -403,31 +403,11 @@ class LightTree:
         """q: (n, 15) float32 rows n u v pos(3) nor(3) d(3) wavelength time (pad).
         Returns (out (n, 14) in the oracle's layout: to_light(3) spec(4)
         hero selection_pdf light_pdf light_count pad(3), ids (n,))."""
-        torch = _torch()
-        dev = torch.device("cuda", self.ctx.device)
         q = np.ascontiguousarray(q, np.float32).reshape(-1, 15)
         n = q.shape[0]
-        cols = {"n": q[:, 0], "u": q[:, 1], "v": q[:, 2], "pos": q[:, 3:6], "nor": q[:, 6:9], "d": q[:, 9:12],
-                "wavelength": q[:, 12], "time": q[:, 13]}
-        dq = {k: torch.from_numpy(np.ascontiguousarray(v)).to(dev) for k, v in cols.items()}
-        out = {"to_light": torch.zeros((n, 3), dtype=torch.float32, device=dev),
-               "spec": torch.zeros((n, 4), dtype=torch.float32, device=dev),
-               "selection_pdf": torch.zeros(n, dtype=torch.float32, device=dev),
-               "light_pdf": torch.zeros(n, dtype=torch.float32, device=dev),
-               "id": torch.zeros(n, dtype=torch.int64, device=dev)}
-        qs = _abi.LightQuerySoA(*[C.c_void_p(dq[k].data_ptr()) for k in
-                                  ("n", "u", "v", "pos", "nor", "d", "wavelength", "time")])
-        os_ = _abi.LightSampleSoA(*[C.c_void_p(out[k].data_ptr()) for k in
-                                    ("to_light", "spec", "selection_pdf", "light_pdf", "id")])
-        self.ctx.check(self.ctx.L.psy_light_sample(self.ctx.h, C.byref(qs), n, C.byref(os_), None))
-        self.ctx.sync()
-        res = np.zeros((n, 14), np.float32)
-        res[:, 0:3] = out["to_light"].cpu().numpy()
-        res[:, 3:7] = out["spec"].cpu().numpy()
-        res[:, 7] = q[:, 12]
-        res[:, 8] = out["selection_pdf"].cpu().numpy()
-        res[:, 9] = out["light_pdf"].cpu().numpy()
-        return res, out["id"].cpu().numpy().view(np.uint64)
+        res, ids = np.empty((n, 14), np.float32), np.empty(n, np.uint64)
+        self.ctx.check(self.ctx.L.psy_light_sample_rows(self.ctx.h, _ptr(q), n, _ptr(res), _ptr(ids)))
+        return res, ids
 
 
 class PathTraceIntegrator:

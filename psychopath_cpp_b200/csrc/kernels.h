@@ -156,6 +156,9 @@ cudaError_t launch_batch_wave(const DevScene* scenes, const RenderParams* render
                               const WaveBufs& wb, const WaveQueues& wq, unsigned* status, int block,
                               cudaStream_t st, uint32_t* launches);
 
+cudaError_t launch_light_rows(const DevScene& sc, const float* rows, float* out, uint64_t* ids, uint32_t n,
+                              float ident_inv, unsigned* status, cudaStream_t st);
+
 cudaError_t launch_light_sample(const DevScene& sc, const LightQuerySoADev& q, const LightSampleSoADev& o, uint32_t n,
                                 float ident_inv, unsigned* status, cudaStream_t st);
 

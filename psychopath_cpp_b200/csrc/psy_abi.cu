@@ -956,6 +956,33 @@ int psy_light_sample(psy_ctx* ctx, const psy_light_query_soa* q, uint32_t n, con
 	                "light sample launch");
 }
 
+int psy_light_sample_rows(psy_ctx* ctx, const float* rows, uint32_t n, float* out, uint64_t* ids) {
+	if (!ctx) return PSY_ERR_ARG;
+	if (!ctx->has_scene) return ctx_fail(ctx, PSY_ERR_NO_SCENE, "psy_light_sample_rows: no scene uploaded");
+	if (n == 0) return PSY_OK;
+	if (!rows || !out) return ctx_fail(ctx, PSY_ERR_ARG, "psy_light_sample_rows: rows and out are required");
+	if (ctx->dev.assemblies == nullptr || ctx->host->assemblies[0].light_root < 0)
+		return ctx_fail(ctx, PSY_ERR_ARG, "psy_light_sample_rows: the scene has no lights");
+	cudaSetDevice(ctx->device);
+	int rc;
+	// ids, rows and samples in one buffer: one copy in, two out
+	const size_t id_bytes = (size_t)n * sizeof(uint64_t), row_bytes = (size_t)n * 15 * sizeof(float);
+	const size_t out_bytes = (size_t)n * 14 * sizeof(float);
+	char* buf = static_cast<char*>(ctx->scratch_buffer("light_rows", id_bytes + row_bytes + out_bytes, &rc));
+	if (!buf) return rc;
+	uint64_t* d_ids = reinterpret_cast<uint64_t*>(buf);
+	float* d_rows = reinterpret_cast<float*>(buf + id_bytes);
+	float* d_out = reinterpret_cast<float*>(buf + id_bytes + row_bytes);
+	cudaStream_t st = ctx->host_stream();
+	if ((rc = ctx_cuda(ctx, cudaMemcpyAsync(d_rows, rows, row_bytes, cudaMemcpyHostToDevice, st), "H2D queries"))) return rc;
+	if ((rc = ctx_cuda(ctx, launch_light_rows(ctx->dev, d_rows, d_out, d_ids, n, ctx->ident_inv, ctx->d_status, st),
+	                   "light sample launch")))
+		return rc;
+	if ((rc = ctx_cuda(ctx, cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, st), "D2H samples"))) return rc;
+	if (ids && (rc = ctx_cuda(ctx, cudaMemcpyAsync(ids, d_ids, id_bytes, cudaMemcpyDeviceToHost, st), "D2H ids"))) return rc;
+	return ctx->check_status(st);
+}
+
 int psy_render(psy_ctx* ctx, const psy_render_desc* desc, float* xyz, uint32_t* counts, psy_render_stats* stats,
                void* stream) {
 	if (!ctx || !desc || !xyz) return PSY_ERR_ARG;

@@ -56,6 +56,54 @@ cudaError_t launch_batch_wave(const DevScene* scenes, const RenderParams* render
 // ---------------------------------------------------------------------
 // Batched LightTree::sample queries (psy_light_sample)
 // ---------------------------------------------------------------------
+// One LightTree::sample query of a Lambert surface.
+__device__ __forceinline__ void light_query(const DevScene& sc, LightQuery* lq, float ident_inv) {
+	lq->has_xform = false;
+	lq->gtr = false;
+	lq->id = 0;
+	lq->selection_pdf = 1.0f;
+	lq->light_sample_pdf = 1.0f;
+	light_tree_pick<FEAT_ALL, false>(sc, lq);
+	light_emit<FEAT_ALL>(sc, lq, ident_inv);
+}
+
+// Queries and samples as rows (psy_light_sample_rows).
+__global__ void light_rows_kernel(DevScene sc, const float* __restrict__ rows, float* __restrict__ out,
+                                  uint64_t* __restrict__ ids, uint32_t n, float ident_inv, unsigned* status) {
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n) return;
+	const float* r = rows + 15 * (size_t)i;
+	float* o = out + 14 * (size_t)i;
+	LightQuery lq;
+	lq.n = r[0];
+	lq.u = r[1];
+	lq.v = r[2];
+	lq.pos = V3(r[3], r[4], r[5]);
+	lq.nor = V3(r[6], r[7], r[8]);
+	lq.d = V3(r[9], r[10], r[11]);
+	lq.wavelength = r[12];
+	lq.time = r[13];
+	light_query(sc, &lq, ident_inv);
+	if (!lq.valid) atomicOr(status, ERRF_NOLIGHT);
+	// (a query without a sample ends the call with an error)
+	o[0] = lq.valid ? lq.to_light.x : 0.0f;
+	o[1] = lq.valid ? lq.to_light.y : 0.0f;
+	o[2] = lq.valid ? lq.to_light.z : 0.0f;
+	for (int k = 0; k < 4; ++k) o[3 + k] = lq.valid ? lq.spec.e[k] : 0.0f;
+	o[7] = lq.wavelength;
+	o[8] = lq.valid ? lq.selection_pdf : 0.0f;
+	o[9] = lq.valid ? lq.light_sample_pdf : 0.0f;
+	for (int k = 10; k < 14; ++k) o[k] = 0.0f;
+	ids[i] = lq.valid ? lq.id : 0ull;
+}
+
+cudaError_t launch_light_rows(const DevScene& sc, const float* rows, float* out, uint64_t* ids, uint32_t n,
+                              float ident_inv, unsigned* status, cudaStream_t st) {
+	if (n == 0) return cudaSuccess;
+	light_rows_kernel<<<(n + 127) / 128, 128, 0, st>>>(sc, rows, out, ids, n, ident_inv, status);
+	return cudaGetLastError();
+}
+
 __global__ void light_sample_kernel(DevScene sc, LightQuerySoADev q, LightSampleSoADev o, uint32_t n, float ident_inv,
                                     unsigned* status) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -69,13 +117,7 @@ __global__ void light_sample_kernel(DevScene sc, LightQuerySoADev q, LightSample
 	lq.d = V3(q.d[3 * i], q.d[3 * i + 1], q.d[3 * i + 2]);
 	lq.wavelength = q.wavelength[i];
 	lq.time = q.time[i];
-	lq.has_xform = false;
-	lq.gtr = false;
-	lq.id = 0;
-	lq.selection_pdf = 1.0f;
-	lq.light_sample_pdf = 1.0f;
-	light_tree_pick<FEAT_ALL, false>(sc, &lq);
-	light_emit<FEAT_ALL>(sc, &lq, ident_inv);
+	light_query(sc, &lq, ident_inv);
 	if (!lq.valid) {
 		atomicOr(status, ERRF_NOLIGHT);
 		return;

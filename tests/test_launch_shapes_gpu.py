@@ -66,3 +66,37 @@ def test_scene_without_placements_gives_the_same_hits(ctx, seed):
     assert 0 < got[0][0]["hit"].sum() < len(rays["time"])
     assert equal(got[0][0], got[1][0])
     assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1000])
+def test_light_sample_rows_match_the_device_form(ctx, n):
+    """psy_light_sample_rows (host rows) against psy_light_sample (device
+    arrays) on the same queries."""
+    import ctypes as C
+
+    import torch
+
+    from psychopath_cpp_b200 import _abi
+    ctx.upload(scenes.batch_scene(5, (64, 64), 1, 20, 37))
+    rng = np.random.default_rng(n)
+    q = np.zeros((n, 15), np.float32)
+    q[:, 0:3] = rng.random((n, 3))
+    q[:, 3:6] = rng.uniform(-4, 4, (n, 3))
+    for k in (6, 9):
+        v = rng.normal(size=(n, 3))
+        q[:, k:k + 3] = v / np.linalg.norm(v, axis=1, keepdims=True)
+    q[:, 12] = rng.uniform(380, 700, n)
+    q[:, 13] = rng.random(n)
+    rows, ids = api.LightTree(ctx).sample(q)
+    cols = [torch.from_numpy(np.ascontiguousarray(q[:, c])).cuda()
+            for c in (0, 1, 2, slice(3, 6), slice(6, 9), slice(9, 12), 12, 13)]
+    out = [torch.zeros(s, dtype=t, device="cuda") for s, t in
+           (((n, 3), torch.float32), ((n, 4), torch.float32), (n, torch.float32), (n, torch.float32), (n, torch.int64))]
+    qs = _abi.LightQuerySoA(*[C.c_void_p(t.data_ptr()) for t in cols])
+    ss = _abi.LightSampleSoA(*[C.c_void_p(t.data_ptr()) for t in out])
+    ctx.check(ctx.L.psy_light_sample(ctx.h, C.byref(qs), n, C.byref(ss), None))
+    ctx.sync()
+    want = np.zeros((n, 14), np.float32)
+    want[:, 0:3], want[:, 3:7] = out[0].cpu().numpy(), out[1].cpu().numpy()
+    want[:, 7], want[:, 8], want[:, 9] = q[:, 12], out[2].cpu().numpy(), out[3].cpu().numpy()
+    assert np.array_equal(rows, want) and np.array_equal(ids, out[4].cpu().numpy().view(np.uint64))
