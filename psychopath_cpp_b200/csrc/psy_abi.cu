@@ -7,6 +7,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/psy_b200.h"
@@ -154,54 +155,54 @@ struct WaveSet {
 	WaveQueues wq;
 };
 
-static int wave_set(psy_ctx* ctx, const char* prefix, uint64_t P, uint32_t path_length, WaveSet* ws,
+static int wave_set(psy_ctx* ctx, const char* prefix, uint64_t P, uint32_t path_length, bool paths_in_hits, WaveSet* ws,
                     bool adjoint = false) {
-	int rc = PSY_OK;
-	std::string pre(prefix);
-	auto buf = [&](const char* name, size_t bytes) -> void* {
-		return ctx->scratch_buffer((pre + name).c_str(), bytes, &rc);
-	};
+	// one device buffer for all of them (allocating them one by one was most
+	// of a new context's first render)
 	PathSoA& ps = ws->ps;
-	ps.head = (uint4*)buf("head", P * 16);
-	ps.col = (float4*)buf("col", P * 16);
-	ps.fcol = (float4*)buf("fcol", P * 16);
-	ps.lcol = (float4*)buf("lcol", P * 16);
-	ps.sample = (float*)buf("sample", P * 12);
-	ps.adj = nullptr;
-	ps.valb = nullptr;
-	ps.vpid = nullptr;
-	ps.nee_param = nullptr;
-	ps.vdsc = nullptr;
-	ps.fexcl = nullptr;
-	ps.nee_base = nullptr;
-	if (adjoint) {
-		ps.adj = (float4*)buf("adj", P * 16);
-		ps.valb = (float4*)buf("valb", P * 16 * PSY_ADJ_MAX_VERTS);
-		ps.vpid = (int*)buf("vpid", P * 4 * PSY_ADJ_MAX_VERTS);
-		ps.nee_param = (int*)buf("neep", P * 4);
-		ps.vdsc = (float4*)buf("vdsc", P * 16 * PSY_ADJ_MAX_VERTS);
-		ps.fexcl = (float4*)buf("fexcl", P * 16);
-		ps.nee_base = (float4*)buf("neeb", P * 16);
-		if (!ps.adj || !ps.valb || !ps.vpid || !ps.nee_param || !ps.vdsc || !ps.fexcl || !ps.nee_base)
-			return rc ? rc : PSY_ERR_OOM;
-	}
 	WaveQueues& wq = ws->wq;
-	wq.q0 = (int*)buf("q0", P * 4);
-	wq.q1 = (int*)buf("q1", P * 4);
-	wq.counters = (int*)buf("counters", sizeof(int) * render_counter_count(path_length));
-	wq.rays = (unsigned long long*)buf("rays", 2 * TC_COUNT * sizeof(unsigned long long));
 	WaveBufs& wb = ws->wb;
+	std::memset(ws, 0, sizeof(*ws));
 	wb.cap = (int)P;
-	wb.ray[0] = (float4*)buf("ray0", P * 80);
-	wb.ray[1] = (float4*)buf("ray1", P * 80);
-	wb.ray[2] = (float4*)buf("ray2", P * 80);
-	wb.hit_f = (float4*)buf("hitf", P * 16);
-	wb.hit_i = (int4*)buf("hiti", P * 48);
-	wb.occl = (uint8_t*)buf("occl", P);
-	if (!ps.head || !ps.col || !ps.fcol || !ps.lcol || !ps.sample || !wq.q0 || !wq.q1 || !wq.counters || !wq.rays ||
-	    !wb.ray[0] || !wb.ray[1] || !wb.ray[2] || !wb.hit_f || !wb.hit_i || !wb.occl)
-		return rc ? rc : PSY_ERR_OOM;
-	return PSY_OK;
+	char* base = nullptr;
+	size_t at = 0;
+	auto place = [&](auto** p, size_t bytes) {
+		*p = base ? reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(base + at) : nullptr;
+		at += (bytes + 255) / 256 * 256;
+	};
+	auto layout = [&]() {
+		at = 0;
+		place(&ps.head, P * 16);
+		place(&ps.col, P * 16);
+		place(&ps.fcol, P * 16);
+		place(&ps.lcol, P * 16);
+		place(&ps.sample, P * 12);
+		if (adjoint) {
+			place(&ps.adj, P * 16);
+			place(&ps.valb, P * 16 * PSY_ADJ_MAX_VERTS);
+			place(&ps.vpid, P * 4 * PSY_ADJ_MAX_VERTS);
+			place(&ps.nee_param, P * 4);
+			place(&ps.vdsc, P * 16 * PSY_ADJ_MAX_VERTS);
+			place(&ps.fexcl, P * 16);
+			place(&ps.nee_base, P * 16);
+		}
+		place(&wq.q0, P * 4);
+		place(&wq.q1, P * 4);
+		place(&wq.counters, sizeof(int) * render_counter_count(path_length));
+		for (float4*& r : wb.ray) place(&r, P * 80);
+		place(&wb.hit_f, P * 16);
+		place(&wb.hit_i, P * (paths_in_hits ? 48 : 16));
+		place(&wb.occl, P);
+	};
+	layout();
+	int rc = PSY_OK;
+	base = static_cast<char*>(ctx->scratch_buffer((std::string(prefix) + "wave").c_str(), at, &rc));
+	if (!base) return rc ? rc : PSY_ERR_OOM;
+	layout();
+	// the counters outlive the wave's buffers (psy_profile_counters)
+	wq.rays = static_cast<unsigned long long*>(
+	    ctx->scratch_buffer((std::string(prefix) + "rays").c_str(), 2 * TC_COUNT * sizeof(unsigned long long), &rc));
+	return wq.rays ? PSY_OK : (rc ? rc : PSY_ERR_OOM);
 }
 
 // Profiling: makes room for `pairs` more traversal-launch timings.  The
@@ -241,7 +242,7 @@ static int render_single(psy_ctx* ctx, const psy_render_desc* desc, const Render
 	if (P < desc->spp) P = desc->spp;
 	if (P > total) P = total;
 	WaveSet ws;
-	if ((rc = wave_set(ctx, "r_", P, rp.path_length, &ws, adjoint))) return rc;
+	if ((rc = wave_set(ctx, "r_", P, rp.path_length, ctx->dev.places == nullptr, &ws, adjoint))) return rc;
 	if ((rc = ctx_cuda(ctx, cudaMemsetAsync(ws.wq.rays, 0, 2 * TC_COUNT * sizeof(unsigned long long), st), "memset")))
 		return rc;
 	ctx->last_counts = ws.wq.rays;
@@ -340,6 +341,7 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 	uint64_t total = 0, pixels = 0;
 	uint32_t max_len = 1, max_spp = 1;
 	unsigned features = 0;
+	bool paths_in_hits = false;
 	int rc;
 	for (uint32_t i = 0; i < b->count; ++i) {
 		psy_ctx* sc = b->scenes[i];
@@ -359,6 +361,7 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 		if (rps[i].path_length > max_len) max_len = rps[i].path_length;
 		if (rps[i].spp > max_spp) max_spp = rps[i].spp;
 		features |= sc->dev.features;
+		if (!sc->dev.places) paths_in_hits = true;
 	}
 	uint64_t P = b->stream_paths ? b->stream_paths : (ctx->tuned_stream_paths ? ctx->tuned_stream_paths : (1u << 21));
 	if (P > (1ull << 26)) P = 1ull << 26;
@@ -366,7 +369,7 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 	if (P > total) P = total;
 	const int block = (int)(b->block_size ? b->block_size : (ctx->tuned_block ? ctx->tuned_block : 128));
 	WaveSet ws;
-	if ((rc = wave_set(ctx, "b_", P, max_len, &ws))) return rc;
+	if ((rc = wave_set(ctx, "b_", P, max_len, paths_in_hits, &ws))) return rc;
 	DevScene* d_scs = static_cast<DevScene*>(ctx->scratch_buffer("b_scenes", sizeof(DevScene) * b->count, &rc));
 	if (!d_scs) return rc;
 	RenderParams* d_rps = static_cast<RenderParams*>(ctx->scratch_buffer("b_renders", sizeof(RenderParams) * b->count, &rc));
