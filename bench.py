@@ -282,25 +282,34 @@ def run_render_ours(args, rank, local, pg, world):
     rays_per_render = int(integ.stats.rays)
     occl_per_render = int(integ.stats.occlusion_rays)
     launches_per_render = int(integ.stats.launches)
-    # every wave launches one traversal per segment (closest-hit rays and the
-    # last vertex's shadow rays) and one for the last shadow rays
-    trace_launches_per_render = int(integ.stats.waves) * (RENDER_PATH_LENGTH + 1)
     counters = ctx.trace_counters()
     paths = w * h * RENDER_SPP
     if pg:
         pg.barrier()
     torch.cuda.synchronize(dev)
     start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    # the traversal kernels (the dominant ones) are timed by the library with
-    # CUDA events on the render stream around each of their launches
-    ctx.check(ctx.L.psy_profile_enable(ctx.h, 1))
     with ClockSampler(local) as clk:
         start.record(stream)
         for _ in range(args.steps):
             integ.integrate_device(xyz, cnt, sp, with_stats=False)
         end.record(stream)
         torch.cuda.synchronize(dev)
+    # the traversal kernels (the dominant ones) are timed by the library with
+    # CUDA events on the render stream around each of their launches, in
+    # renders of their own (a profiled render keeps one wave in flight)
+    profiled = max(1, min(args.steps, 2))
+    ctx.check(ctx.L.psy_profile_enable(ctx.h, 1))
+    integ.integrate_device(xyz, cnt, sp, with_stats=True)
+    profiled_waves = int(integ.stats.waves)
     trace_ms, trace_launches = C.c_double(), C.c_uint32()
+    ctx.check(ctx.L.psy_profile_read(ctx.h, C.byref(trace_ms), C.byref(trace_launches)))
+    p0, p1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    p0.record(stream)
+    for _ in range(profiled):
+        integ.integrate_device(xyz, cnt, sp, with_stats=False)
+    p1.record(stream)
+    torch.cuda.synchronize(dev)
+    profiled_ms = p0.elapsed_time(p1)
     ctx.check(ctx.L.psy_profile_read(ctx.h, C.byref(trace_ms), C.byref(trace_launches)))
     ctx.check(ctx.L.psy_profile_enable(ctx.h, 0))
     ctx.sync(sp)
@@ -315,13 +324,15 @@ def run_render_ours(args, rank, local, pg, world):
     # roofline of the traversal kernels: their algorithmic bytes (80 B per
     # closest-hit ray, 64 B per occlusion ray) over their own launch time
     closest = rays_per_render - occl_per_render
-    trace_bytes = (closest * BYTES_PER_CLOSEST_RAY + occl_per_render * BYTES_PER_OCCLUSION_RAY) * args.steps
+    trace_bytes = (closest * BYTES_PER_CLOSEST_RAY + occl_per_render * BYTES_PER_OCCLUSION_RAY) * profiled
     n_trace = int(trace_launches.value)
-    if n_trace != trace_launches_per_render * args.steps:
-        raise RuntimeError("timed %d traversal launches, expected %d x %d steps" %
-                           (n_trace, trace_launches_per_render, args.steps))
+    # every wave launches one traversal per segment (closest-hit rays and the
+    # last vertex's shadow rays) and one for the last shadow rays
+    if n_trace != profiled_waves * (RENDER_PATH_LENGTH + 1) * profiled:
+        raise RuntimeError("timed %d traversal launches, expected %d x %d x %d steps" %
+                           (n_trace, profiled_waves, RENDER_PATH_LENGTH + 1, profiled))
     achieved = trace_bytes / (trace_ms.value * 1e-3) / 1e9 if trace_ms.value > 0 else 0.0
-    traffic = TRAFFIC_BYTES_PER_RAY * rays_per_render * args.steps / n_trace
+    traffic = TRAFFIC_BYTES_PER_RAY * rays_per_render * profiled / n_trace
     # end to end: the public call plus the device->host read of the film each step
     h_xyz = torch.empty(w * h * 3, dtype=torch.float32, pin_memory=True)
     h_cnt = torch.empty(w * h, dtype=torch.int32, pin_memory=True)
@@ -343,7 +354,7 @@ def run_render_ours(args, rank, local, pg, world):
         "warmup": args.warmup, "ms_per_step": round(ms, 3), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded many-light scene)",
         "config": {"workload": render_workload_name(), "paths_per_step": paths, "path_length": RENDER_PATH_LENGTH,
-                   "stream_paths": args.stream_paths or "auto (2^21)",
+                   "stream_paths": args.stream_paths or "auto (2^22 in flight)",
                    "parallelism": "replicas" if world > 1 else "single",
                    "l2": "per-path state (~200 B x 2M paths in flight) larger than L2"},
         "mrays_per_s": round(mrays, 2), "rays_per_path": round(rbar, 4),
@@ -352,7 +363,7 @@ def run_render_ours(args, rank, local, pg, world):
                      "kernel": "trace_wave_kernel (closest-hit and occlusion traversal)",
                      "algorithmic_bytes_per_launch": round(trace_bytes / n_trace),
                      "avg_launch_ms": round(trace_ms.value / n_trace, 4), "launches_timed": n_trace,
-                     "share_of_step": round(trace_ms.value / args.steps / ms, 3), "peak_source": peak_kind,
+                     "share_of_step": round(trace_ms.value / profiled_ms, 3), "peak_source": peak_kind,
                      "basis": "80 B per closest-hit ray, 64 B per occlusion ray; traffic: DRAM bytes per launch "
                               "scaled from one ncu capture by rays (profiles/)"},
         "e2e": {"value": round(world * paths / (e2e_ms * 1e-3), 1), "unit": "paths/s",

@@ -348,7 +348,7 @@ typedef struct psy_render_desc {
 	uint32_t spp;             /* samples per pixel */
 	uint32_t seed;            /* sampler seed (RenderSettings Seed) */
 	uint32_t path_length;     /* max path segments (PathTraceIntegrator::path_length, default 4) */
-	uint32_t stream_paths;    /* paths in flight per wave, 0 = automatic */
+	uint32_t stream_paths;    /* paths per wave, one wave after another; 0 = automatic (up to 2^22 in flight, in two waves) */
 	uint32_t block_size;      /* threads per block for the wavefront kernels, 0 = automatic */
 } psy_render_desc;
 
@@ -497,7 +497,8 @@ typedef struct psy_batch_desc {
 	const psy_render_desc* renders;   /* per render: width, height, spp, seed, path_length */
 	float* const* xyz;                /* per render: device film, width*height*3 floats, accumulated */
 	uint32_t* const* counts;          /* per render: device sample counts, or NULL; the array may be NULL */
-	uint32_t stream_paths;            /* paths per wave; 0 = the context's tuned value, else 2^21 */
+	uint32_t stream_paths;            /* paths per wave, one wave after another; 0 = the context's tuned value, else
+	                                     2^22, in flight in two waves */
 	uint32_t block_size;              /* 64, 128 or 256 threads per block; 0 = tuned value, else 128 */
 	uint32_t use_graph;               /* 1: launch through a CUDA graph captured once and reused while
 	                                     the batch's launch parameters stay the same */

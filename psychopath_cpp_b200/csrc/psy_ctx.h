@@ -44,6 +44,9 @@ struct psy_ctx {
 	cudaGraphExec_t batch_graph = nullptr;
 	std::vector<uint8_t> batch_graph_key;
 	cudaStream_t capture_stream = nullptr;
+	// the second of two waves in flight (WavePair)
+	cudaStream_t side_stream = nullptr;
+	cudaEvent_t fork_event = nullptr, join_event = nullptr;
 	uint32_t tuned_stream_paths = 0;
 	uint32_t tuned_block = 0;
 	// optional timing of the traversal launches (psy_profile_enable)

@@ -484,13 +484,13 @@ struct TraceCfg {
 // next, so that the lanes doing the same work run together instead of one
 // lane's long bisection or transformed-instance entry holding up the others.
 // (2, 4 or 8 node visits: within 1%; 16 bisection iterations: 2% better than
-// 8 on the many-light frame.  Warps that follow one kind of work per block,
+// 8 on the many-light frame, 32 another 1% in flat scenes.  Warps that follow one kind of work per block,
 // which paid while a step's code and state did not fit the caches, cost 5%.)
 #ifndef PSY_WALK_NODES
 #define PSY_WALK_NODES 4
 #endif
 #ifndef PSY_PATCH_UNITS
-#define PSY_PATCH_UNITS 16
+#define PSY_PATCH_UNITS 32
 #endif
 // Kinds of work of a lane: idle, inner nodes, a leaf visit of one of three
 // classes, a bisection in progress.  Leaf visits are told apart so that the

@@ -25,7 +25,8 @@ def test_short_stream_is_the_stream_s_beginning(ctx, n):
     assert equal(part, {k: v[:n] for k, v in whole.items()})
 
 
-@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (17, 3, 1), (8, 8, 1), (13, 5, 2), (61, 47, 3), (160, 120, 2)])
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (17, 3, 1), (8, 8, 1), (13, 5, 2), (61, 47, 3), (160, 120, 2), (419, 313, 1),
+                                     (311, 223, 3)])
 def test_wave_length_does_not_change_the_film(ctx, w, h, spp):
     sc = scenes.plain_scene(4, res=(w, h), spp=spp)
     ctx.upload(sc)
@@ -100,3 +101,46 @@ def test_light_sample_rows_match_the_device_form(ctx, n):
     want[:, 0:3], want[:, 3:7] = out[0].cpu().numpy(), out[1].cpu().numpy()
     want[:, 7], want[:, 8], want[:, 9] = q[:, 12], out[2].cpu().numpy(), out[3].cpu().numpy()
     assert np.array_equal(rows, want) and np.array_equal(ids, out[4].cpu().numpy().view(np.uint64))
+
+
+def test_batch_with_two_waves_in_flight_equals_plain_renders(ctx):
+    entries = []
+    for k, (w, h, spp) in enumerate([(301, 157, 2), (64, 48, 5), (233, 129, 3)]):
+        c = api.Context(0)
+        c.upload(scenes.batch_scene(k, (w, h), spp, 60 + 40 * k, 3 + k))
+        entries.append({"scene": c, "width": w, "height": h, "spp": spp, "seed": 7 + k})
+    b = api.BatchRenderer(ctx, entries)
+    assert b.paths >= 1 << 17
+    b.render()
+    for e, (x, c) in zip(entries, b.images()):
+        y, d = api.PathTraceIntegrator(e["scene"], e["width"], e["height"], e["spp"], seed=e["seed"],
+                                       stream_paths=4096).integrate()
+        assert np.array_equal(c, d) and np.array_equal(x, y)
+
+
+def test_adjoint_with_two_waves_in_flight(ctx):
+    """The gradient does not depend on the waves but for the order of its
+    32-bit sums: at most some hundred blocks' sums are added to a parameter in
+    either run, each rounding by half an ulp of the running total."""
+    import torch
+    w, h, spp = 256, 192, 4
+    sc = scenes.adjoint_scene(2, res=(w, h), spp=spp)
+    ctx.upload(sc)
+    shaders, objects, ns, no = api.flat_indices(sc)
+    sp, op, count = np.full(ns, -1, np.int32), np.full(no, -1, np.int32), 0
+    for name, sh in sc.root.shaders.items():
+        if name.startswith("mat"):
+            sp[shaders[id(sh)]] = count
+            count += 4
+    for name in sc.root.objects:
+        if name.startswith("light"):
+            op[objects[(0, name)]] = count
+            count += 1
+    params = torch.full((count,), 0.6, device="cuda")
+    dl = torch.rand(h * w * 3, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    g = [api.DiffRenderer(ctx, w, h, spp, sp, op, count, stream_paths=s).adjoint(params, dl).double()
+         for s in (0, 50000)]
+    assert w * h * spp >= 1 << 17
+    # 8 launches of at most 3 * 148 blocks, twice: 7104 additions of 2^-24
+    bound = 7104 * 2.0 ** -24
+    assert torch.all((g[0] - g[1]).abs() <= bound * g[1].abs().clamp_min(float(g[1].abs().max()) * 1e-3))
