@@ -174,6 +174,10 @@ __device__ __forceinline__ V3 uniform_sample_sphere(float u, float v) {
 }
 
 // sphere_lambert (utils/monte_carlo.hpp:207-233).
+// (The reference takes 1 - x of a float x in double and rounds to float.  The
+// double difference is exact but for x below 2^-29 or beyond 2^53, where it
+// rounds like the float one, so the float subtraction gives the same bits.)
+//
 // The cosine tests: |cos a - cos b| <= |a - b|, so where nlcos lies 1e-3 off
 // a limit's cosine (0, +-sin r), the angle lies as far off the limit; rsin is
 // off sin r by at most 2.5e-4 (the rounding of rcos^2) and the arc cosines
@@ -183,11 +187,13 @@ __device__ __forceinline__ V3 uniform_sample_sphere(float u, float v) {
 // +-1 by rounding (its arc cosine is NaN) takes the angle tests.
 enum : int { CAP_ABOVE, CAP_MOSTLY_ABOVE, CAP_MOSTLY_BELOW, CAP_BELOW, CAP_UNSURE };
 __device__ __forceinline__ int cap_case(float nlcos, float rsin2) {
-	const float rsin = sqrtf(rsin2), m = 1e-3f;
-	if (nlcos > rsin + m) return nlcos <= 1.0f ? CAP_ABOVE : CAP_UNSURE;
-	if (nlcos < -(rsin + m)) return nlcos >= -1.0f ? CAP_BELOW : CAP_UNSURE;
-	if (nlcos > m && nlcos < rsin - m) return CAP_MOSTLY_ABOVE;
-	if (nlcos < -m && nlcos > m - rsin) return CAP_MOSTLY_BELOW;
+	// (on squares: the margin is far above their rounding)
+	const float m = 1e-3f;
+	const float c = fabsf(nlcos), in = c + m, out = c - m;
+	if (out > 0.0f) {
+		if (out * out > rsin2) return c <= 1.0f ? (nlcos > 0.0f ? CAP_ABOVE : CAP_BELOW) : CAP_UNSURE;
+		if (in * in < rsin2) return nlcos > 0.0f ? CAP_MOSTLY_ABOVE : CAP_MOSTLY_BELOW;
+	}
 	return CAP_UNSURE;
 }
 
@@ -204,7 +210,7 @@ static __device__ __noinline__ float sphere_lambert_cut(float nlcos, float rcos,
 	const float nlsin = (float)sqrt(1.0 - (double)(nlcos * nlcos));
 	const float rsin = sqrtf(rsin2);
 	const float ysin = rcos / nlsin;
-	const float ycos2 = (float)(1.0 - (double)(ysin * ysin));
+	const float ycos2 = 1.0f - ysin * ysin;  // (float)(1.0 - (double)..)
 	const float ycos = sqrtf(ycos2);
 	const float g = (float)(((((-2.0 * (double)nlsin) * (double)rcos) * (double)ycos) + PSY_HPI_D) -
 	                        (double)lm_asinf(ysin) + (double)(ysin * ycos));
@@ -672,7 +678,7 @@ __device__ __forceinline__ LightProb light_prob(const LightQuery& q, V3 nn, V3 d
 	if (cos_theta_max < 0.0f) return p;
 	p.nlcos = dot(nn, normalized(d));
 	p.rcos = cos_theta_max;
-	p.rsin2 = (float)(1.0 - (double)(p.rcos * p.rcos));
+	p.rsin2 = 1.0f - p.rcos * p.rcos;  // (float)(1.0 - (double)..)
 	const int c = cap_case(p.nlcos, p.rsin2);
 	p.est = c == CAP_ABOVE ? p.nlcos * p.rsin2 : 0.0f;
 	if (c != CAP_ABOVE && c != CAP_BELOW) p.cut = c;

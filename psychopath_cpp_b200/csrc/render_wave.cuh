@@ -84,11 +84,9 @@ __device__ __forceinline__ int load_ray(const float4* rb, int cap, int i, WorldR
 // Hit planes: 0: t, u, v, max_dim (float4)   1: instance, placement, depth,
 // path[0]   2: path[1..4]   3: path[5..7] (int4).  The path is written and
 // read in scenes without placements only, as far as the hit's depth.
-__device__ __forceinline__ void load_rec(const WaveBufs& wb, int i, HitRec* h, HitPath* hp) {
-	const int4 a = wb.hit_i[i];
+__device__ __forceinline__ void load_rec(const WaveBufs& wb, int i, int4 a, float4 f, HitRec* h, HitPath* hp) {
 	h->inst = a.x;
 	if (a.x < 0) return;
-	const float4 f = wb.hit_f[i];
 	h->t = f.x; h->u = f.y; h->v = f.z; h->max_dim = f.w;
 	h->place = a.y;
 	hp->depth = 0;
@@ -473,7 +471,7 @@ struct TraceCfg {
 	static constexpr bool NESTED = (F & FEAT_NESTED) != 0;
 	static constexpr int BLOCK = 256;                     // launch bound
 	static constexpr int MIN_BLOCKS = NESTED ? 2 : 3;     // 128 and 80 registers a thread
-	static constexpr int REFILL_MIN = NESTED ? 4 : 8;     // idle lanes that trigger a refill while rays remain
+	static constexpr int REFILL_MIN = NESTED ? 4 : 12;    // idle lanes that trigger a refill while rays remain
 	static int launch_block(int render_block) { return NESTED ? BLOCK : render_block; }
 };
 // Each lane's traversal is cut into kinds of work: node visits (up to
@@ -705,35 +703,42 @@ __global__ void __launch_bounds__(PSY_SHADE_BLOCK, shade_min_blocks(MODE))
 		GtrVertex gv;
 		// ---- the results of the last vertex's rays
 		if (i < n) {
+			// (everything that is read by position or slot is asked for first:
+			// one wait for memory instead of one after another.  The hit of an
+			// entry without a ray is not used.)
 			slot = CAMERA ? i : q_in[i];
-			const int tag = __float_as_int(rin[4 * (size_t)wb.cap + i].w);
+			WorldRayD wr;
+			const int tag = load_ray(rin, wb.cap, i, &wr);
+			HitRec rec;
+			HitPath path;
+			const int4 hi = wb.hit_i[i];
+			const float4 hf = wb.hit_f[i];
+			const uint4 head = ps.head[slot];
+			const float4 col4 = CAMERA ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : ps.col[slot];
+			const float4 lcol4 = CAMERA ? col4 : ps.lcol[slot];
+			const float4 fcol4 = CAMERA ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : ps.fcol[slot];
+			const uint8_t blocked = CAMERA ? (uint8_t)1 : wb.occl[i];
 			rid = tag >> 1;
 			const DevScene& sc = w.scene(rid);
 			const RenderParams& rp = w.render(rid);
-			const uint4 head = ps.head[slot];
 			smp = head.x;
 			dim = head.y & 0xffffu;
 			step = head.y >> 16;
 			wl = __uint_as_float(head.z);
 			const float last_pdf = __uint_as_float(head.w);
-			Spec col = Spec{};
+			Spec col = sp(col4);
 			if (!CAMERA) {
-				col = sp(ps.col[slot]);
-				if (wb.occl[i] == 0) {
-					const Spec c = sp(ps.lcol[slot]);
+				if (blocked == 0) {
+					const Spec c = sp(lcol4);
 					for (int k = 0; k < 4; ++k) col.e[k] += c.e[k];
 					if (ADJOINT)
 						grad_add(rp, sgrad, ps, slot, (int)(step >> 1), sp(ps.nee_base[slot]), ps.nee_param[slot], wl);
 				}
 			}
 			if (!(tag & 1)) {  // (tag & 1): the last vertex sent no bounce ray
-				WorldRayD wr;
-				load_ray(rin, wb.cap, i, &wr);
 				time = wr.time;
-				HitRec rec;
-				HitPath path;
-				load_rec(wb, i, &rec, &path);
-				const Spec fcol = CAMERA ? Spec{{1.0f, 1.0f, 1.0f, 1.0f}} : sp(ps.fcol[slot]);
+				load_rec(wb, i, hi, hf, &rec, &path);
+				const Spec fcol = sp(fcol4);
 				if (rec.inst >= 0) {
 					hit_surface(sc, &rec, path);
 					int closure;

@@ -37,6 +37,14 @@ def check_division(pb):
     assert np.array_equal(t, q // np.uint64(pb)) and np.array_equal(r, q % np.uint64(pb))
 
 
+def test_one_minus_a_float_in_double_or_float():
+    rng = np.random.default_rng(3)
+    x = rng.integers(0, 1 << 32, 4000000, dtype=np.uint64).astype(np.uint32).view(F)
+    x = np.concatenate([x[np.isfinite(x)], np.ldexp(F(1.0) + rng.random(200000).astype(F), rng.integers(-60, 61, 200000)).astype(F)])
+    with np.errstate(over="ignore"):
+        assert np.array_equal((1.0 - x.astype(np.float64)).astype(F), F(1.0) - x)
+
+
 @pytest.mark.parametrize("near", [0.0, 0.9, 0.999, 0.9999999])
 def test_sphere_lambert_plain_cases(near):
     """Where the cosine test takes a plain case, the angle test of the full
@@ -50,12 +58,14 @@ def test_sphere_lambert_plain_cases(near):
     k = rcos.size // 2
     nlcos[:k] = np.clip(np.sign(nlcos[:k]) * s[:k] + rng.normal(0.0, 3e-3, k), -1.0, 1.0).astype(F)
     rsin2 = (1.0 - (rcos * rcos).astype(np.float64)).astype(F)
-    lim = np.sqrt(rsin2) + F(1e-3)
-    above, below = nlcos > lim, nlcos < -lim
+    assert np.array_equal(rsin2, F(1.0) - rcos * rcos)  # the kernels subtract in 32 bits
+    m = F(1e-3)
+    inner, outer = np.abs(nlcos) + m, np.abs(nlcos) - m
+    whole = (outer > 0) & (outer * outer > rsin2)
+    above, below = whole & (nlcos > 0), whole & (nlcos < 0)
     nl, r = np.arccos(nlcos.astype(np.float64)), np.arccos(rcos.astype(np.float64))
-    rsin, m = np.sqrt(rsin2), F(1e-3)
-    mostly_above = (nlcos > m) & (nlcos < rsin - m)
-    mostly_below = (nlcos < -m) & (nlcos > m - rsin)
+    cut = (outer > 0) & ~whole & (inner * inner < rsin2)
+    mostly_above, mostly_below = cut & (nlcos > 0), cut & (nlcos < 0)
     assert above.sum() > 1000 and below.sum() > 1000
     for mostly, lo, hi in ((mostly_above, np.pi / 2 - r, np.pi / 2 + 0 * r), (mostly_below, np.pi / 2 + 0 * r, np.pi / 2 + r)):
         assert mostly.sum() > 1000 or near > 0.999
