@@ -98,7 +98,10 @@ struct alignas(16) FrameBuf {
 // sequence; its count is -1 if it needs more than PSY_MAX_MOTION samples.
 // The three cases of the reference (equal counts, more parent samples, more
 // instance samples) share one loop with one matrix product.
-__device__ __forceinline__ Frame frame_merge(const Frame& a, const float* b, int nb, FrameBuf* dst) {
+// Not inlined: placements hold the merged frames of assembly instances, and
+// what is left (transformed object instances, scenes past the placements'
+// limit) would spread a thousand instructions over the walk's code.
+static __device__ __noinline__ Frame frame_merge(Frame a, const float* b, int nb, FrameBuf* dst) {
 	const int na = a.count;
 	Frame out{dst->m, -1};
 	if (na > PSY_MAX_MOTION || nb > PSY_MAX_MOTION) return out;
@@ -1109,17 +1112,20 @@ struct Trav {
 		return true;
 	}
 
-	// The transform of an object instance that carries its own, at the ray
+	// The transform of object instance gi, which carries its own, at the ray
 	// time.  Returns false when it needs more motion samples than supported.
-	__device__ __forceinline__ bool object_frame(const DevScene& sc, const DevInstance& inst, M44* om) {
+	static __device__ __noinline__ bool object_transform(const DevScene& sc, Frame parent, int gi, float time, M44* om) {
 		FrameBuf buf;
-		const Frame f = frame_merge(level_frame(sc), sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &buf);
-		if (f.count < 0) {
-			err |= ERRF_MOTION;
-			return false;
-		}
+		const DevInstance inst = sc.instances[gi];
+		const Frame f = frame_merge(parent, sc.xforms + (size_t)inst.xform * 16, inst.xform_count, &buf);
+		if (f.count < 0) return false;
 		*om = frame_at(f, time);
 		return true;
+	}
+	__device__ __forceinline__ bool object_frame(const DevScene& sc, int gi, M44* om) {
+		if (object_transform(sc, level_frame(sc), gi, time, om)) return true;
+		err |= ERRF_MOTION;
+		return false;
 	}
 
 	// A leaf of class LEAF_SPHERE: a sphere or sphere light at rest in its
@@ -1144,7 +1150,7 @@ struct Trav {
 		V3 lo = o, ld = d, li = dinv;
 		if (XFORM && inst.xform_count > 0) {
 			M44 om;
-			if (!object_frame(sc, inst, &om)) return true;
+			if (!object_frame(sc, gi, &om)) return true;
 			lo = pos_to(om, io.origin());
 			ld = dir_to(om, io.direction());
 			li = recip3(ld);
@@ -1209,7 +1215,7 @@ struct Trav {
 		M44 om;
 		const bool oxf = XFORM && m.y > 0;
 		if (oxf) {
-			if (!object_frame(sc, sc.instances[gi], &om)) return true;
+			if (!object_frame(sc, gi, &om)) return true;
 			lo = pos_to(om, io.origin());
 			ld = dir_to(om, io.direction());
 			li = recip3(ld);
