@@ -345,12 +345,20 @@ class Tracer:
         Intersection fields as numpy arrays."""
         n = len(rays["time"])
         rs, keep = _ray_soa_host(rays)
-        out = {}
-        hs = _abi.HitSoA()
+        # the fields are cut from one block: allocated one by one, arrays of
+        # this size go back to the system on each release, and the next call
+        # pays for their pages again
+        at, places = 0, []
         for f in fields:
             dt, w = HIT_FIELDS[f]
-            arr = np.zeros((n, w) if w > 1 else (n,), dt)
-            out[f] = arr
+            places.append((f, at, dt, w))
+            at += (n * w * np.dtype(dt).itemsize + 63) // 64 * 64
+        block = np.empty(at, np.uint8)  # the call writes every ray's fields
+        out = {}
+        hs = _abi.HitSoA()
+        for f, first, dt, w in places:
+            arr = block[first:first + n * w * np.dtype(dt).itemsize].view(dt)
+            out[f] = arr.reshape(n, w) if w > 1 else arr
             setattr(hs, f, arr.ctypes.data_as(C.c_void_p))
         self.ctx.check(self.ctx.L.psy_trace_host(self.ctx.h, C.byref(rs), n, C.byref(hs)))
         return out
