@@ -462,10 +462,14 @@ __global__ void __launch_bounds__(256) camera_gen_kernel(W w, HaltonDev hd, Wave
 // of idling until the slowest ray of its warp is done.
 //
 // Registers: 128 a thread where a lane's step can be a bicubic split (96
-// floats live), 80 in flat scenes, where more warps hide the walk's latency
-// (1280x720x4 many-light frame: 169 ms with 2 x 256 or 1 x 512 threads an
-// SM, 192 with 6 x 128, 223 with 2 x 512; 512x384x16 with 50,000
-// primitives: 18.2 ms with 3 or 4 x 256, 18.9 with 2).
+// floats live); there more warps only push one another's stacks and cursors
+// out of L1 (1280x720x4 many-light frame: 125.7 ms with 2 x 256 threads an
+// SM, 129.4 with 5 x 128, 135.9 with 3 x 192, 140.7 with 3 x 256).  80 in flat
+// scenes, where more warps hide the walk's latency (512x384x16 with 50,000
+// primitives: 11.10 ms with 3 x 256, 11.15 with 4; 18.2 and 18.9 with 3 and 2
+// before shading was joined).
+// Idle lanes that trigger a refill: 2 of them 135.6 and 11.7 ms, 4 130.1 and
+// 11.5, 8 11.1, 12 10.8 (instanced, flat).
 template <unsigned F>
 struct TraceCfg {
 	static constexpr bool NESTED = (F & FEAT_NESTED) != 0;

@@ -53,7 +53,7 @@ struct StreamIO {
 // latency (4M rays against the heightfield: 1.06 ms; 1.13 at 80 registers,
 // 1.37 at 128), 128 for the larger variants, whose bicubic bisection spills
 // below that (300,000 mixed rays against instanced patches and spheres:
-// 2.04 ms; 2.30 at 184, 2.80 at 72).
+// 1.67 ms; 1.71 at 144, 1.72 at 168, 1.87 at 112, 1.94 at 96).
 template <unsigned F>
 struct TraceKernelRegs {
 	static constexpr int value = F == FEAT_FLAT ? 64 : 128;
