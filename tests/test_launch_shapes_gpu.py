@@ -144,3 +144,25 @@ def test_adjoint_with_two_waves_in_flight(ctx):
     # 8 launches of at most 3 * 148 blocks, twice: 7104 additions of 2^-24
     bound = 7104 * 2.0 ** -24
     assert torch.all((g[0] - g[1]).abs() <= bound * g[1].abs().clamp_min(float(g[1].abs().max()) * 1e-3))
+
+
+@pytest.mark.parametrize("zeros", [1, 2])
+@pytest.mark.parametrize("name", ["plain", "motion"])
+def test_rays_with_zero_components_match_the_oracle(ctx, name, zeros):
+    """Rays whose slab tests can meet 0 * inf (direction components of zero)
+    take the reference's own minima and maxima, out of line; the others single
+    instructions.  Both against the plain-C oracle."""
+    from oracle import port
+    sc = {"plain": scenes.plain_scene, "motion": scenes.motion_patch_scene}[name](6)
+    rays = parity.random_rays(3000, (-4, -4, 0.01), (4, 4, 3), seed=zeros, occl_frac=0.3)
+    rng = np.random.default_rng(zeros)
+    k = np.arange(0, 3000, 2)  # every other ray
+    for _ in range(zeros):
+        rays["d"][k, rng.integers(0, 3, k.size)] = 0.0
+    rays["d"][np.all(rays["d"] == 0.0, axis=1), 2] = -1.0
+    ctx.upload(sc)
+    mine = api.Tracer(ctx).trace(rays, fields=("hit", "id", "t", "uv", "closure"))
+    ref = port.trace(sc, rays)
+    patch = (ref["uv"][:, 0] != 0) & (mine["closure"] == 1)
+    assert 100 < int(mine["hit"].sum()) < 3000
+    parity.assert_parity(parity.compare_trace(ref, mine, rays["type"], uv_mask=patch))
