@@ -71,7 +71,7 @@ PSY_HD int leaf_instance(int ref) { return -(ref + 1); }
 // node's index with what its test needs to know before the node is read, or
 // a leaf's class and global instance index.
 static constexpr int REF_NODE_MOVING = 1 << 30;  // more than one time sample
-static constexpr int REF_NODE_ODD = 1 << 29;     // a box is not finite
+static constexpr int REF_NODE_ODD = 1 << 29;     // a box is not finite, or inverted; or there is one child only
 static constexpr int REF_NODE_MASK = (1 << 29) - 1;
 static constexpr int REF_LEAF_MASK = (1 << 28) - 1;
 static constexpr int REF_MAX_NODES = 1 << 29, REF_MAX_INSTANCES = 1 << 28;
@@ -84,8 +84,10 @@ enum : int {
 PSY_HD int leaf_class(int ref) { return (int)(((unsigned)ref >> 28) & 7u); }
 PSY_HD int class_ref(int cls, int instance) { return (int)(0x80000000u | ((unsigned)cls << 28) | (unsigned)instance); }
 
-// The planes of an absent child's box: inverted, so that no ray hits it, and
-// finite, so that interpolating them stays so.
+// The planes of an absent child's box: finite, so that interpolating them
+// stays so.  They keep nothing out: an absent child is told by its reference
+// (REF_EMPTY), and only children 2 and 3 may be absent in a node that is not
+// REF_NODE_ODD.
 static constexpr float ABSENT_PLANE = 3.0e38f;
 
 struct alignas(16) DevNode {

@@ -9,9 +9,15 @@ namespace psy {
 // ---------------------------------------------------------------------
 // Tree references and absent children (the traversal's node form)
 // ---------------------------------------------------------------------
-__device__ bool finite_planes(const float* b, int nchild) {
-	for (int k = 0; k < 24; ++k)
-		if ((k & 3) < nchild && !(fabsf(b[k]) < 1e37f)) return false;
+// Boxes that the traversal may test with minima and maxima of the two planes
+// of an axis: finite, and not inverted (a sphere of negative radius has an
+// inverted box; by the ray's sign, as the reference tests, no ray hits it).
+__device__ bool plain_boxes(const float* b, int nchild) {
+	for (int axis = 0; axis < 3; ++axis)
+		for (int c = 0; c < nchild; ++c) {
+			const float lo = b[8 * axis + c], hi = b[8 * axis + 4 + c];
+			if (!(fabsf(lo) < 1e37f) || !(fabsf(hi) < 1e37f) || !(lo <= hi)) return false;
+		}
 	return true;
 }
 
@@ -28,9 +34,10 @@ __global__ void node_flags_kernel(DevNode* nodes, float* extra, int n, int* flag
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	DevNode& nd = nodes[i];
-	bool finite = finite_planes(nd.b, nd.nchild);
-	for (int t = 1; t < nd.ts; ++t) finite = finite_planes(extra + (size_t)(nd.extra + t - 1) * 24, nd.nchild) && finite;
-	flags[i] = (nd.ts > 1 ? REF_NODE_MOVING : 0) | (finite ? 0 : REF_NODE_ODD);
+	// (the test of plain nodes takes the first two children for granted)
+	bool plain = nd.nchild >= 2 && plain_boxes(nd.b, nd.nchild);
+	for (int t = 1; t < nd.ts; ++t) plain = plain && plain_boxes(extra + (size_t)(nd.extra + t - 1) * 24, nd.nchild);
+	flags[i] = (nd.ts > 1 ? REF_NODE_MOVING : 0) | (plain ? 0 : REF_NODE_ODD);
 	for (int t = 0; t < nd.ts || t == 0; ++t) {
 		float* b = t == 0 ? nd.b : extra + (size_t)(nd.extra + t - 1) * 24;
 		for (int k = 0; k < 24; ++k)
