@@ -798,7 +798,8 @@ static constexpr int REF_NONE = REF_EMPTY;
 
 enum : unsigned {
 	RAY_OCCL = 1u,   // occlusion ray: ends at the first hit
-	RAY_ODD = 2u,    // a slab test of the ray in its current space can meet NaN or inf - inf
+	RAY_ODD = 2u,    // a slab test of the ray in its current space can meet NaN or inf - inf; or the ray's time lies
+	                 // before the first sample, where the boxes of moving nodes are extrapolated and may be inverted
 	RAY_HIT = 4u,    // a hit was recorded
 	RAY_WIDTH = 8u   // the width parameters are those of the current space
 };
@@ -866,13 +867,13 @@ struct Trav {
 		d = nd;
 		dinv = recip3(nd);
 		flags &= ~(RAY_ODD | RAY_WIDTH);
-		if (odd_ray(o, d, dinv)) flags |= RAY_ODD;
+		if (odd_ray(o, d, dinv) || !(time >= 0.0f)) flags |= RAY_ODD;
 	}
 
 	__device__ __forceinline__ void init(const DevScene& sc, V3 wo, V3 wd, float t, bool occl) {
 		flags = occl ? RAY_OCCL : 0u;
-		set_ray(wo, wd);
 		time = t;
+		set_ray(wo, wd);
 		max_t = occl ? 1.0f : INFINITY;
 		cur = __ldg(sc.asmb_root);
 		sp = 0;
@@ -925,7 +926,7 @@ struct Trav {
 					d = V3(mem->lvr[L][3], mem->lvr[L][4], mem->lvr[L][5]);
 					dinv = V3(mem->lvr[L][6], mem->lvr[L][7], mem->lvr[L][8]);
 					flags &= ~(RAY_ODD | RAY_WIDTH);
-					if (odd_ray(o, d, dinv)) flags |= RAY_ODD;
+					if (odd_ray(o, d, dinv) || !(time >= 0.0f)) flags |= RAY_ODD;
 				}
 				continue;
 			}
@@ -936,7 +937,10 @@ struct Trav {
 
 	// The distances of a node's four children in the reference's own order of
 	// operations (BBox4::intersect_ray, basics/bbox.hpp:566-595, SSE min/max
-	// semantics), infinity for a miss: rays and boxes with infinities or NaN.
+	// semantics), infinity for a miss: rays and boxes with infinities or NaN,
+	// inverted boxes.  0 for a hit before the first time sample: an
+	// extrapolated box need not hold its children's, and its distance on the
+	// stack would prune them.
 	static __device__ __noinline__ float4 odd_node(const DevScene& sc, int ref, V3 o, V3 dinv, float time, float max_t) {
 		const DevNode* nd = sc.nodes + (ref & REF_NODE_MASK);
 		float b[24];
@@ -959,7 +963,7 @@ struct Trav {
 			const float zhi = ((ds2 ? b[16 + c] : b[20 + c]) - o.z) * dinv.z;
 			const float mins = vmax(vmax(xlo, ylo), vmax(zlo, 0.0f));
 			const float maxs = vmax(vmin(vmin(xhi, yhi), zhi), -INFINITY) * BBOX_MAXT_ADJUST;
-			tk[c] = c < nd->nchild && mins < max_t && mins <= maxs ? mins : INFINITY;
+			tk[c] = c < nd->nchild && mins < max_t && mins <= maxs ? (time >= 0.0f ? mins : 0.0f) : INFINITY;
 		}
 		return make_float4(tk[0], tk[1], tk[2], tk[3]);
 	}

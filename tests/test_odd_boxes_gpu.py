@@ -55,3 +55,17 @@ def test_light_whose_radius_changes_sign(ctx):
     rays["time"][:] = 0.25
     got, want = trace(ctx, sc, rays, False), trace(ctx, scenes.plain_scene(6), rays, False)
     assert equal(got, want, rays)
+
+
+@pytest.mark.parametrize("time,hits", [(-0.9, False), (-0.75, False), (0.5, True)])
+def test_boxes_extrapolated_before_the_first_sample(ctx, time, hits):
+    """Lights whose radius, taken on to a time before the first sample, is
+    below zero: their boxes are inverted at that time."""
+    rays = parity.random_rays(20000, (-6, -6, 0.01), (6, 6, 3), seed=5, occl_frac=0.3)
+    rays["time"][:] = time
+    rng = np.random.default_rng(2)
+    sc = scenes.Scene(name="growing")
+    for k in range(30):
+        sc.root.add_object("grow%d" % k, SphereLight([rng.uniform((-5, -5, 0), (5, 5, 2))], [0.5, 1.5], [[1.0] * 3]))
+        sc.root.add_instance("grow%d" % k)
+    assert bool(trace(ctx, sc, rays, False)["hit"].any()) == hits
