@@ -373,6 +373,13 @@ struct MinMax {
 	__device__ static __forceinline__ float axis(V3 v) { return shi(shi(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); }
 };
 
+// How a sub-patch is tested.  Without NaN the reference's minima and maxima
+// are single instructions.  A ray whose slab tests can meet NaN (RAY_ODD: a
+// direction component of zero, the common one, gives 0 * inf on a box's face)
+// takes the reference's own for its slab test alone; only a patch with huge
+// coordinates takes them, in the patch's own order, for its bounds too.
+enum : int { TEST_CLEAN = 0, TEST_ODD_RAY, TEST_ODD_PATCH };
+
 template <int NV, bool CLEAN>
 __device__ __forceinline__ Box patch_bound(const Patch<NV>& q) {
 	typedef MinMax<CLEAN> M;
@@ -389,21 +396,22 @@ __device__ __forceinline__ Box patch_bound(const Patch<NV>& q) {
 
 // Bounds of a sub-patch (each time sample) and the ray's test against them:
 // the top of the loop of intersect_rays_with_patch (object/patch_utils.hpp).
-template <int NV, int TSC, bool CLEAN>
+template <int NV, int TSC, int TEST>
 __device__ __forceinline__ bool patch_node_test(const Patch<NV> (&q)[TSC], float t_nalpha, V3 o, V3 dinv, float max_t,
                                                 float* max_dim, float* h0, float* h1) {
-	typedef MinMax<CLEAN> M;
+	constexpr bool CLEAN_BOUND = TEST != TEST_ODD_PATCH;
+	typedef MinMax<CLEAN_BOUND> M;
 	Box bb[TSC];
 	float md = 0.0f;
 #pragma unroll
 	for (int k = 0; k < TSC; ++k) {
-		bb[k] = patch_bound<NV, CLEAN>(q[k]);
+		bb[k] = patch_bound<NV, CLEAN_BOUND>(q[k]);
 		const float ld = M::axis(bb[k].hi - bb[k].lo);
 		md = (k == 0) ? ld : M::shi(md, ld);
 	}
 	*max_dim = md;
 	const Box b = (TSC == 1) ? bb[0] : box_lerp(t_nalpha, bb[0], bb[TSC - 1]);
-	if (!CLEAN) {
+	if (TEST != TEST_CLEAN) {
 		const bool h = box_hit(b, o, dinv, max_t, h0, h1);
 		// A NaN far distance comes from 0 * inf: the ray runs exactly along a
 		// box face (a zero direction component, the origin on the face).  The
@@ -516,7 +524,7 @@ struct PatchStore {
 
 // The root's test: sets up `pc` and returns true when the ray hits the
 // patch's box.
-template <int NV, int TSC, bool CLEAN>
+template <int NV, int TSC, int TEST>
 __device__ __forceinline__ bool patch_begin(PatchCursor<NV, TSC>& pc, const float* verts, float time, V3 o, V3 dinv,
                                             float max_t) {
 #pragma unroll
@@ -529,7 +537,7 @@ __device__ __forceinline__ bool patch_begin(PatchCursor<NV, TSC>& pc, const floa
 		const float t_time = time * (float)(TSC - 1);
 		pc.t_nalpha = t_time - (float)(int)t_time;
 	}
-	if (!patch_node_test<NV, TSC, CLEAN>(pc.cur, pc.t_nalpha, o, dinv, max_t, &pc.max_dim, &pc.h0, &pc.h1)) return false;
+	if (!patch_node_test<NV, TSC, TEST>(pc.cur, pc.t_nalpha, o, dinv, max_t, &pc.max_dim, &pc.h0, &pc.h1)) return false;
 	pc.a0 = pc.b0 = 0.0f;
 	pc.a1 = pc.b1 = 1.0f;
 	pc.tr = false;
@@ -549,7 +557,7 @@ enum : int { PATCH_MORE = 0, PATCH_DONE = 1, PATCH_BLOCKED = 2 };
 // `leaf(t, u, v, max_dim)` is called for every leaf taken, each closer than
 // the last, with *max_t lowered to it.  A bisection that exceeds
 // PSY_PATCH_MAX_STEPS iterations ends and sets ERRF_BISECT in *err.
-template <int NV, int TSC, bool CLEAN, class LEAF>
+template <int NV, int TSC, int TEST, class LEAF>
 __device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV, TSC>& ps, V3 o, V3 dinv,
                                          const RayFlip& rw, float* max_t, bool occl, float dice_rate, float min_upoly,
                                          int& units, unsigned* err, LEAF leaf) {
@@ -557,18 +565,18 @@ __device__ __forceinline__ int patch_run(PatchCursor<NV, TSC>& pc, PatchStore<NV
 	const float t_nalpha = pc.t_nalpha;
 	float &max_dim = pc.max_dim, &h0 = pc.h0, &h1 = pc.h1;
 	float &a0 = pc.a0, &a1 = pc.a1, &b0 = pc.b0, &b1 = pc.b1;
-	// (where NaN can occur, the order of a bound's minima matters: the
-	// patch's own)
+	// (where a coordinate can be NaN, the order of a bound's minima matters:
+	// the patch's own)
 	auto test = [&](const Patch<NV>(&q)[TSC], float* md, float* t0, float* t1) {
-		if constexpr (CLEAN) {
-			return patch_node_test<NV, TSC, true>(q, t_nalpha, o, dinv, *max_t, md, t0, t1);
+		if constexpr (TEST != TEST_ODD_PATCH) {
+			return patch_node_test<NV, TSC, TEST>(q, t_nalpha, o, dinv, *max_t, md, t0, t1);
 		} else {
 			Patch<NV> own[TSC];
 			for (int k = 0; k < TSC; ++k) {
 				own[k] = q[k];
 				patch_transpose_if(pc.tr, own[k]);
 			}
-			return patch_node_test<NV, TSC, false>(own, t_nalpha, o, dinv, *max_t, md, t0, t1);
+			return patch_node_test<NV, TSC, TEST>(own, t_nalpha, o, dinv, *max_t, md, t0, t1);
 		}
 	};
 	while (true) {
@@ -663,25 +671,47 @@ struct PatchHit {
 	float t, u, v, max_dim;
 };
 
-// The whole bisection of one patch in one call, with the reference's own
-// minima and maxima: rays or patches whose slab tests can meet NaN.  Not
-// inlined: next to no ray comes here.  Returns true when a leaf was taken.
+// patch_begin and patch_run on a cursor in memory, for rays and patches whose
+// tests can meet NaN.  Not inlined: streams along an axis consist of such
+// rays, but the code of all others must not hold theirs, nor have variables
+// of theirs in memory because these functions want an address.
 template <int NV, int TSC>
-static __device__ __noinline__ bool patch_whole(const float* verts, float time, V3 o, V3 dinv, const RayFlip& rw,
-                                                float max_t, bool occl, float dice_rate, float min_upoly,
-                                                PatchStore<NV, TSC>& ps, PatchHit* hit, unsigned* err) {
+static __device__ __noinline__ bool patch_odd_begin(PatchCursor<NV, TSC>& at, const float* verts, float time, V3 o, V3 dinv,
+                                                    float max_t, bool odd_patch) {
 	PatchCursor<NV, TSC> pc;
-	if (!patch_begin<NV, TSC, false>(pc, verts, time, o, dinv, max_t)) return false;
-	int units = 0x7fffffff;
-	bool found = false;
-	unsigned e = 0;
-	patch_run<NV, TSC, false>(pc, ps, o, dinv, rw, &max_t, occl, dice_rate, min_upoly, units, &e,
-	                          [&](float t, float u, float v, float md) {
-		                          found = true;
-		                          *hit = PatchHit{t, u, v, md};
-	                          });
-	*err |= e;
-	return found && !(e & ERRF_BISECT);
+	const bool in = odd_patch ? patch_begin<NV, TSC, TEST_ODD_PATCH>(pc, verts, time, o, dinv, max_t)
+	                          : patch_begin<NV, TSC, TEST_ODD_RAY>(pc, verts, time, o, dinv, max_t);
+	if (in) at = pc;
+	return in;
+}
+
+// What patch_odd_run leaves: PATCH_*, whether a leaf was taken and the
+// closest one, the iterations not used, errors.
+struct OddRun {
+	int state;
+	bool took;
+	PatchHit hit;
+	int units;
+	unsigned err;
+};
+
+template <int NV, int TSC>
+static __device__ __noinline__ OddRun patch_odd_run(PatchCursor<NV, TSC>& at, PatchStore<NV, TSC>& ps, V3 o, V3 dinv,
+                                                    const RayFlip& rw, float max_t, bool occl, float dice_rate,
+                                                    float min_upoly, bool odd_patch, int units) {
+	PatchCursor<NV, TSC> pc = at;
+	const RayFlip w = rw;
+	bool took = false;
+	unsigned err = 0;
+	PatchHit h;
+	auto leaf = [&](float t, float u, float v, float md) {
+		took = true;
+		h = PatchHit{t, u, v, md};
+	};
+	const int r = odd_patch ? patch_run<NV, TSC, TEST_ODD_PATCH>(pc, ps, o, dinv, w, &max_t, occl, dice_rate, min_upoly, units, &err, leaf)
+	                        : patch_run<NV, TSC, TEST_ODD_RAY>(pc, ps, o, dinv, w, &max_t, occl, dice_rate, min_upoly, units, &err, leaf);
+	if (r == PATCH_MORE) at = pc;
+	return OddRun{r, took, h, units, err};
 }
 
 // ---------------------------------------------------------------------
@@ -771,8 +801,9 @@ __device__ bool hit_space(const DevScene& sc, const HitRec& rec, const HitPath& 
 }
 
 // Patch kind of a bisection in progress: bilinear or bicubic, one or two
-// time samples.
-enum : int { PM_NONE = 0, PM_BILINEAR1, PM_BILINEAR2, PM_BICUBIC1, PM_BICUBIC2 };
+// time samples; and what its tests can meet (PM_ODD: NaN, PM_ODD_PATCH: from
+// the patch's own coordinates).
+enum : int { PM_NONE = 0, PM_BILINEAR1, PM_BILINEAR2, PM_BICUBIC1, PM_BICUBIC2, PM_KIND = 7, PM_ODD = 8, PM_ODD_PATCH = 16 };
 
 // Bytes of the bisection state for the patch kinds of feature set F.
 template <unsigned F>
@@ -935,37 +966,67 @@ struct Trav {
 		return true;
 	}
 
+	// The planes of a node's child boxes at the ray time.
+	static __device__ __forceinline__ void load_node(const DevScene& sc, const DevNode* nd, int ref, float time, Quad& xl,
+	                                                 Quad& xh, Quad& yl, Quad& yh, Quad& zl, Quad& zh) {
+		const char* base = reinterpret_cast<const char*>(nd);
+		load_axis(base, xl, xh);
+		load_axis(base + 32, yl, yh);
+		load_axis(base + 64, zl, zh);
+		if (!(ref & REF_NODE_MOVING)) return;
+		const int4 meta = __ldg(reinterpret_cast<const int4*>(&nd->nchild));
+		const SeqPos q = seq_pos(time, meta.y);
+		auto extra = [&](int k) { return reinterpret_cast<const char*>(sc.node_extra + (size_t)(meta.z + k - 1) * 24); };
+		if (q.i0 != 0) {
+			const char* e = extra(q.i0);
+			load_axis(e, xl, xh);
+			load_axis(e + 32, yl, yh);
+			load_axis(e + 64, zl, zh);
+		}
+		if (q.single) return;
+		const char* e = extra(q.i0 + 1);
+		const unsigned long long al = pack2(q.nalpha, q.nalpha), ia = pack2(one_minus(q.nalpha), one_minus(q.nalpha));
+		Quad a, b;
+		load_axis(e, a, b);
+		lerp_quad(xl, a, ia, al); lerp_quad(xh, b, ia, al);
+		load_axis(e + 32, a, b);
+		lerp_quad(yl, a, ia, al); lerp_quad(yh, b, ia, al);
+		load_axis(e + 64, a, b);
+		lerp_quad(zl, a, ia, al); lerp_quad(zh, b, ia, al);
+	}
+
 	// The distances of a node's four children in the reference's own order of
 	// operations (BBox4::intersect_ray, basics/bbox.hpp:566-595, SSE min/max
 	// semantics), infinity for a miss: rays and boxes with infinities or NaN,
 	// inverted boxes.  0 for a hit before the first time sample: an
 	// extrapolated box need not hold its children's, and its distance on the
 	// stack would prune them.
+	// The near and far planes are picked for all four children at once, by the
+	// ray's sign, so this costs about as much as the plain test: streams along
+	// an axis consist of rays that come here (1M rays straight down on 20,000
+	// spheres 1,499 -> 1,045 us, on a 256x256 heightfield 730 -> 405, bisection
+	// included; a loop over the children with scalar loads before).
 	static __device__ __noinline__ float4 odd_node(const DevScene& sc, int ref, V3 o, V3 dinv, float time, float max_t) {
 		const DevNode* nd = sc.nodes + (ref & REF_NODE_MASK);
-		float b[24];
-		for (int i = 0; i < 24; ++i) b[i] = nd->b[i];
-		if (nd->ts > 1) {
-			const SeqPos q = seq_pos(time, nd->ts);
-			const float* x0 = q.i0 ? sc.node_extra + (size_t)(nd->extra + q.i0 - 1) * 24 : nd->b;
-			const float* x1 = q.single ? x0 : sc.node_extra + (size_t)(nd->extra + q.i0) * 24;
-			const float ia = one_minus(q.nalpha);
-			for (int i = 0; i < 24; ++i) b[i] = q.single ? x0[i] : (x0[i] * ia) + (x1[i] * q.nalpha);
-		}
-		const bool ds0 = dinv.x < 0.0f, ds1 = dinv.y < 0.0f, ds2 = dinv.z < 0.0f;
-		float tk[4];
+		const int nchild = __ldg(&nd->nchild);
+		Quad xl, xh, yl, yh, zl, zh;
+		load_node(sc, nd, ref, time, xl, xh, yl, yh, zl, zh);
+		float xn[4], xf[4], yn[4], yf[4], zn[4], zf[4];
+		const bool sx = dinv.x < 0.0f, sy = dinv.y < 0.0f, sz = dinv.z < 0.0f;
+		planes(sx ? xh : xl, -o.x, dinv.x, xn);
+		planes(sx ? xl : xh, -o.x, dinv.x, xf);
+		planes(sy ? yh : yl, -o.y, dinv.y, yn);
+		planes(sy ? yl : yh, -o.y, dinv.y, yf);
+		planes(sz ? zh : zl, -o.z, dinv.z, zn);
+		planes(sz ? zl : zh, -o.z, dinv.z, zf);
+		float t[4];
+#pragma unroll
 		for (int c = 0; c < 4; ++c) {
-			const float xlo = ((ds0 ? b[4 + c] : b[c]) - o.x) * dinv.x;
-			const float xhi = ((ds0 ? b[c] : b[4 + c]) - o.x) * dinv.x;
-			const float ylo = ((ds1 ? b[12 + c] : b[8 + c]) - o.y) * dinv.y;
-			const float yhi = ((ds1 ? b[8 + c] : b[12 + c]) - o.y) * dinv.y;
-			const float zlo = ((ds2 ? b[20 + c] : b[16 + c]) - o.z) * dinv.z;
-			const float zhi = ((ds2 ? b[16 + c] : b[20 + c]) - o.z) * dinv.z;
-			const float mins = vmax(vmax(xlo, ylo), vmax(zlo, 0.0f));
-			const float maxs = vmax(vmin(vmin(xhi, yhi), zhi), -INFINITY) * BBOX_MAXT_ADJUST;
-			tk[c] = c < nd->nchild && mins < max_t && mins <= maxs ? (time >= 0.0f ? mins : 0.0f) : INFINITY;
+			const float mins = vmax(vmax(xn[c], yn[c]), vmax(zn[c], 0.0f));
+			const float maxs = vmax(vmin(vmin(xf[c], yf[c]), zf[c]), -INFINITY) * BBOX_MAXT_ADJUST;
+			t[c] = c < nchild && mins < max_t && mins <= maxs ? (time >= 0.0f ? mins : 0.0f) : INFINITY;
 		}
-		return make_float4(tk[0], tk[1], tk[2], tk[3]);
+		return make_float4(t[0], t[1], t[2], t[3]);
 	}
 
 	// An inner node (cur): tests the child boxes, leaves the nearest hit child
@@ -981,35 +1042,10 @@ struct Trav {
 			const float4 t = odd_node(sc, ref, o, dinv, time, max_t);
 			t0 = t.x; t1 = t.y; t2 = t.z; t3 = t.w;
 		} else {
-			const char* base = reinterpret_cast<const char*>(nd);
 			float tn[4], tf[4];
 			{
 				Quad xl, xh, yl, yh, zl, zh;
-				load_axis(base, xl, xh);
-				load_axis(base + 32, yl, yh);
-				load_axis(base + 64, zl, zh);
-				if (ref & REF_NODE_MOVING) {
-					const int4 meta = __ldg(reinterpret_cast<const int4*>(&nd->nchild));
-					const SeqPos q = seq_pos(time, meta.y);
-					auto extra = [&](int k) { return reinterpret_cast<const char*>(sc.node_extra + (size_t)(meta.z + k - 1) * 24); };
-					if (q.i0 != 0) {
-						const char* e = extra(q.i0);
-						load_axis(e, xl, xh);
-						load_axis(e + 32, yl, yh);
-						load_axis(e + 64, zl, zh);
-					}
-					if (!q.single) {
-						const char* e = extra(q.i0 + 1);
-						const unsigned long long al = pack2(q.nalpha, q.nalpha), ia = pack2(one_minus(q.nalpha), one_minus(q.nalpha));
-						Quad a, b;
-						load_axis(e, a, b);
-						lerp_quad(xl, a, ia, al); lerp_quad(xh, b, ia, al);
-						load_axis(e + 32, a, b);
-						lerp_quad(yl, a, ia, al); lerp_quad(yh, b, ia, al);
-						load_axis(e + 64, a, b);
-						lerp_quad(zl, a, ia, al); lerp_quad(zh, b, ia, al);
-					}
-				}
+				load_node(sc, nd, ref, time, xl, xh, yl, yh, zl, zh);
 				float l[4], h[4];
 				planes(xl, -o.x, dinv.x, l); planes(xh, -o.x, dinv.x, h);
 #pragma unroll
@@ -1205,17 +1241,31 @@ struct Trav {
 		return w;
 	}
 
+	// patch_odd_run on the bisection in progress (mem->p_*, its work `w`) for up
+	// to `units` iterations.
+	template <class WORK>
+	__device__ __forceinline__ OddRun odd_run(const DevScene& sc, WORK& w, bool odd_patch, int units) {
+		const OddRun r = patch_odd_run(w.c, w.st, mem->p_o, mem->p_dinv, mem->p_rw, max_t, (flags & RAY_OCCL) != 0,
+		                               sc.dice_rate, sc.min_upoly_size, odd_patch, units);
+		err |= r.err;
+		if (r.took) {
+			if (!(flags & RAY_OCCL)) max_t = r.hit.t;
+			record(mem->p_inst, r.hit.t, r.hit.u, r.hit.v, r.hit.max_dim);
+		}
+		return r;
+	}
+
 	// A leaf of class LEAF_PATCH.  WHOLE: the bisection runs here, to its end.
 	// Otherwise the patch's box is tested and its bisection set up (pmode) for
-	// patch_step to carry on.  Rays and patches whose tests can meet NaN are
-	// bisected whole in either case.  Returns false when the ray is finished.
+	// patch_step to carry on.  Returns false when the ray is finished.
 	template <bool WHOLE>
 	__device__ __forceinline__ bool patch_leaf(const DevScene& sc) {
 		const int gi = cur & REF_LEAF_MASK;
 		cur = REF_NONE;
 		const int4 m = __ldg(reinterpret_cast<const int4*>(&sc.leaves[gi].data));  // vertices, transforms, -, kind
 		V3 lo = o, ld = d, li = dinv;
-		bool odd = (flags & RAY_ODD) != 0 || (m.w & LEAF_PATCH_ODD) != 0;
+		const bool odd_patch = (m.w & LEAF_PATCH_ODD) != 0;
+		bool odd = (flags & RAY_ODD) != 0 || odd_patch;
 		M44 om;
 		const bool oxf = XFORM && m.y > 0;
 		if (oxf) {
@@ -1223,10 +1273,10 @@ struct Trav {
 			lo = pos_to(om, io.origin());
 			ld = dir_to(om, io.direction());
 			li = recip3(ld);
-			odd = odd_ray(lo, ld, li) || (m.w & LEAF_PATCH_ODD) != 0;
+			odd = odd_ray(lo, ld, li) || odd_patch;
 		}
 		const float* v = sc.fpool + m.x;
-		const int pm = m.w & 7;  // PM_*
+		const int pm = m.w & PM_KIND;
 		const bool occl = (flags & RAY_OCCL) != 0;
 		const float dr = sc.dice_rate, mu = sc.min_upoly_size;
 		bool live = true, in = false;
@@ -1234,21 +1284,24 @@ struct Trav {
 		auto one = [&](auto& w) {
 			constexpr int NV = sizeof(w.c.cur[0]) / sizeof(V3), N = sizeof(w.c.cur) / sizeof(w.c.cur[0]);
 			if (odd) {
-				PatchHit ph;
-				const RayFlip f = widths(sc, oxf, om, lo, ld);
-				if (!patch_whole<NV, N>(v, time, lo, li, f, max_t, occl, dr, mu, w.st, &ph, &err)) return;
-				if (!occl) max_t = ph.t;
-				live = record(gi, ph.t, ph.u, ph.v, ph.max_dim);
+				in = patch_odd_begin<NV, N>(w.c, v, time, lo, li, max_t, odd_patch);
+				if (WHOLE && in) {
+					mem->p_rw = widths(sc, oxf, om, lo, ld);
+					mem->p_inst = gi;
+					mem->p_o = lo;
+					mem->p_dinv = li;
+					live = odd_run(sc, w, odd_patch, 0x7fffffff).state != PATCH_BLOCKED;
+				}
 				return;
 			}
 			PatchCursor<NV, N> pc;
-			in = patch_begin<NV, N, true>(pc, v, time, lo, li, max_t);
+			in = patch_begin<NV, N, TEST_CLEAN>(pc, v, time, lo, li, max_t);
 			if (!in) return;
 			if constexpr (WHOLE) {
 				const RayFlip f = widths(sc, oxf, om, lo, ld);
 				int units = 0x7fffffff;
-				live = patch_run<NV, N, true>(pc, w.st, lo, li, f, &max_t, occl, dr, mu, units, &err,
-				                              [&](float t, float u, float v2, float md) { record(gi, t, u, v2, md); }) !=
+				live = patch_run<NV, N, TEST_CLEAN>(pc, w.st, lo, li, f, &max_t, occl, dr, mu, units, &err,
+				                                    [&](float t, float u, float v2, float md) { record(gi, t, u, v2, md); }) !=
 				       PATCH_BLOCKED;
 			} else {
 				w.c = pc;
@@ -1264,7 +1317,7 @@ struct Trav {
 		}
 		if (!WHOLE && in) {
 			mem->p_rw = widths(sc, oxf, om, lo, ld);
-			pmode = pm;
+			pmode = pm | (odd ? PM_ODD : 0) | (odd_patch ? PM_ODD_PATCH : 0);
 			mem->p_inst = gi;
 			mem->p_o = lo;
 			mem->p_dinv = li;
@@ -1277,6 +1330,7 @@ struct Trav {
 	// the ray is finished (an occlusion ray's hit).
 	__device__ __forceinline__ bool patch_step(const DevScene& sc, int& units) {
 		int r = PATCH_DONE;
+		const int pm = pmode & PM_KIND;
 		const bool occl = (flags & RAY_OCCL) != 0;
 		const float dr = sc.dice_rate, mu = sc.min_upoly_size;
 		const RayFlip w = mem->p_rw;
@@ -1284,19 +1338,25 @@ struct Trav {
 		// the cursor runs as a local copy (registers) and goes back to the
 		// state only when the bisection stops short of its end
 		auto run = [&](auto& pw) {
+			if (pmode & PM_ODD) {
+				const OddRun o = odd_run(sc, pw, (pmode & PM_ODD_PATCH) != 0, units);
+				r = o.state;
+				units = o.units;
+				return;
+			}
 			auto pc = pw.c;
-			r = patch_run<sizeof(pc.cur[0]) / sizeof(V3), sizeof(pc.cur) / sizeof(pc.cur[0]), true>(
+			r = patch_run<sizeof(pc.cur[0]) / sizeof(V3), sizeof(pc.cur) / sizeof(pc.cur[0]), TEST_CLEAN>(
 			    pc, pw.st, lo, li, w, &max_t, occl, dr, mu, units, &err,
 			    [&](float t, float u, float v, float md) { record(mem->p_inst, t, u, v, md); });
 			if (r == PATCH_MORE) pw.c = pc;
 		};
 		if constexpr ((F & FEAT_BILINEAR) != 0) {
-			if (pmode == PM_BILINEAR1) run(still_work<4>());
-			else if (TS == 2 && pmode == PM_BILINEAR2) run(work<4>());
+			if (pm == PM_BILINEAR1) run(still_work<4>());
+			else if (TS == 2 && pm == PM_BILINEAR2) run(work<4>());
 		}
 		if constexpr ((F & FEAT_BICUBIC) != 0) {
-			if (pmode == PM_BICUBIC1) run(still_work<16>());
-			else if (TS == 2 && pmode == PM_BICUBIC2) run(work<16>());
+			if (pm == PM_BICUBIC1) run(still_work<16>());
+			else if (TS == 2 && pm == PM_BICUBIC2) run(work<16>());
 		}
 		if (r == PATCH_MORE) return true;
 		pmode = PM_NONE;
