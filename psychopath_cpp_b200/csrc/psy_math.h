@@ -31,6 +31,8 @@
 #define PSY_HD inline
 #endif
 
+#define PSY_PI_D 3.14159265358979323846
+
 namespace psy {
 
 static constexpr float BBOX_MAXT_ADJUST = 1.00000024f;  // reference basics/bbox.hpp:20

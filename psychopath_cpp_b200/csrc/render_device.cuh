@@ -18,15 +18,14 @@
 #include "kernels.h"
 #include "shade_geom.cuh"
 #include "psy_libm.cuh"
+#include "shade_math.h"
 
 #define PSY_SPEC_QUAL __device__
 #include "spectral_table.inc"
 
 namespace psy {
 
-#define PSY_HPI_D (PSY_PI_D / 2.0)
 #define PSY_QPI_D (PSY_PI_D / 4.0)
-#define PSY_INV_PI_D (1.0 / PSY_PI_D)
 
 static constexpr float WAVELENGTH_MIN = 380.0f;
 static constexpr float WAVELENGTH_MAX = 700.0f;
@@ -55,23 +54,13 @@ __device__ __forceinline__ float halton_sample(const HaltonDev& hd, uint32_t dim
 	}
 	const uint4 d = __ldg(hd.dims + dim);
 	// The digit groups of the index, most significant factor first: the sum
-	// of perm[digit_g] * pb^(groups - 1 - g), in Horner form.  The division
-	// by pb multiplies by d.x = floor(2^32 / pb): that quotient is right or
-	// one too small (q * (2^32 - d.x * pb) < 2^32 * pb), and the remainder
-	// tells which.  The two hardware-less divisions a group took before were
-	// most of a sample's instructions.
-	const uint32_t pb = d.y;
+	// of perm[digit_g] * pb^(groups - 1 - g), in Horner form.
 	uint32_t q = index;
 	uint32_t sum = 0;
 	for (uint32_t g = 0; g < d.z; ++g) {
-		uint32_t t = __umulhi(q, d.x);
-		uint32_t r = q - t * pb;
-		if (r >= pb) {
-			r -= pb;
-			++t;
-		}
-		sum = sum * pb + (uint32_t)__ldg(hd.perm + d.w + r);
-		q = t;
+		const Division v = divide_by(q, d.y, d.x);
+		sum = sum * d.y + (uint32_t)__ldg(hd.perm + d.w + v.r);
+		q = v.q;
 	}
 	return (float)((double)sum * __ldg(hd.cmul + dim));
 }
@@ -171,52 +160,6 @@ __device__ __forceinline__ V3 uniform_sample_sphere(float u, float v) {
 	float sine, cosine;
 	lm_sincosf(phi, &sine, &cosine);
 	return V3(r * cosine, r * sine, z);
-}
-
-// sphere_lambert (utils/monte_carlo.hpp:207-233).
-// (The reference takes 1 - x of a float x in double and rounds to float.  The
-// double difference is exact but for x below 2^-29 or beyond 2^53, where it
-// rounds like the float one, so the float subtraction gives the same bits.)
-//
-// The cosine tests: |cos a - cos b| <= |a - b|, so where nlcos lies 1e-3 off
-// a limit's cosine (0, +-sin r), the angle lies as far off the limit; rsin is
-// off sin r by at most 2.5e-4 (the rounding of rcos^2) and the arc cosines
-// of the angle tests by less than 1e-6, so both tests agree there.  They
-// spare the arc cosines, and where the cap lies wholly above or below the
-// horizon (most nodes of a light tree walk) all arc functions.  An nlcos past
-// +-1 by rounding (its arc cosine is NaN) takes the angle tests.
-enum : int { CAP_ABOVE, CAP_MOSTLY_ABOVE, CAP_MOSTLY_BELOW, CAP_BELOW, CAP_UNSURE };
-__device__ __forceinline__ int cap_case(float nlcos, float rsin2) {
-	// (on squares: the margin is far above their rounding)
-	const float m = 1e-3f;
-	const float c = fabsf(nlcos), in = c + m, out = c - m;
-	if (out > 0.0f) {
-		if (out * out > rsin2) return c <= 1.0f ? (nlcos > 0.0f ? CAP_ABOVE : CAP_BELOW) : CAP_UNSURE;
-		if (in * in < rsin2) return nlcos > 0.0f ? CAP_MOSTLY_ABOVE : CAP_MOSTLY_BELOW;
-	}
-	return CAP_UNSURE;
-}
-
-// A cap that the horizon cuts, or may (c: cap_case).
-static __device__ __noinline__ float sphere_lambert_cut(float nlcos, float rcos, float rsin2, int c) {
-	if (c == CAP_UNSURE) {
-		const float nl = lm_acosf(nlcos);
-		const float r = lm_acosf(rcos);
-		if ((double)nl < (PSY_HPI_D - (double)r)) return nlcos * rsin2;
-		if ((double)nl < PSY_HPI_D) c = CAP_MOSTLY_ABOVE;
-		else if ((double)nl < (PSY_HPI_D + (double)r)) c = CAP_MOSTLY_BELOW;
-		else return 0.0f;
-	}
-	const float nlsin = (float)sqrt(1.0 - (double)(nlcos * nlcos));
-	const float rsin = sqrtf(rsin2);
-	const float ysin = rcos / nlsin;
-	const float ycos2 = 1.0f - ysin * ysin;  // (float)(1.0 - (double)..)
-	const float ycos = sqrtf(ycos2);
-	const float g = (float)(((((-2.0 * (double)nlsin) * (double)rcos) * (double)ycos) + PSY_HPI_D) -
-	                        (double)lm_asinf(ysin) + (double)(ysin * ycos));
-	const float h = nlcos * ((ycos * sqrtf(rsin2 - ycos2)) + (rsin2 * lm_asinf(ycos / rsin)));
-	if (c == CAP_MOSTLY_ABOVE) return (nlcos * rsin2) + g - h;
-	return (float)((double)(g + h) * PSY_INV_PI_D);
 }
 
 __device__ __forceinline__ float power_heuristic(float a, float b) {
@@ -678,10 +621,10 @@ __device__ __forceinline__ LightProb light_prob(const LightQuery& q, V3 nn, V3 d
 	if (cos_theta_max < 0.0f) return p;
 	p.nlcos = dot(nn, normalized(d));
 	p.rcos = cos_theta_max;
-	p.rsin2 = 1.0f - p.rcos * p.rcos;  // (float)(1.0 - (double)..)
-	const int c = cap_case(p.nlcos, p.rsin2);
-	p.est = c == CAP_ABOVE ? p.nlcos * p.rsin2 : 0.0f;
-	if (c != CAP_ABOVE && c != CAP_BELOW) p.cut = c;
+	const CapEstimate c = sphere_lambert_quick(p.nlcos, p.rcos);
+	p.rsin2 = c.rsin2;
+	p.est = c.est;
+	p.cut = c.cut;
 	return p;
 }
 __device__ __forceinline__ float light_prob_value(const LightProb& p) { return p.e_isa * (0.0f < p.est ? p.est : 0.0f); }

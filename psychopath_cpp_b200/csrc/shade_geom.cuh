@@ -18,8 +18,6 @@
 
 namespace psy {
 
-#define PSY_PI_D 3.14159265358979323846
-
 struct Geo {
 	float u, v;
 	V3 p, dpdu, dpdv, n, dndu, dndv;
