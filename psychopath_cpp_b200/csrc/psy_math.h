@@ -130,7 +130,8 @@ PSY_HD SeqPos seq_pos(float alpha, int count) {
 		p.i0 = count - 1; p.single = 1; p.nalpha = 0.0f;
 	} else {
 		const float temp = alpha * (float)(count - 1);
-		const int index = (int)temp;
+		// (a time far before the first sample must not index before it either)
+		const int index = (int)temp > 0 ? (int)temp : 0;
 		p.i0 = index; p.single = 0; p.nalpha = temp - (float)index;
 	}
 	return p;

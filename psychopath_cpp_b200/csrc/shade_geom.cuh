@@ -114,6 +114,7 @@ __device__ __forceinline__ void patch_at(const float* verts, int tsc, float time
 	int t_index = (int)t_time;
 	const float t_nalpha = t_time - (float)t_index;
 	if (t_index > tsc - 2) t_index = tsc - 2;
+	if (t_index < 0) t_index = 0;
 	Patch<NV> a, b;
 	patch_load<NV>(verts + t_index * NV * 3, &a);
 	patch_load<NV>(verts + (t_index + 1) * NV * 3, &b);

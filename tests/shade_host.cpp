@@ -43,3 +43,13 @@ extern "C" void lambert_plain(unsigned n, const float* nlcos_, const float* rcos
 		         : nl < hpi + r ? (float)((double)(g + h) * (1.0 / PSY_PI_D)) : 0.0f;
 	}
 }
+
+// the place of a time among the samples of a sequence
+extern "C" void positions(unsigned n, const float* time, int count, int* first, int* last, float* alpha) {
+	for (unsigned i = 0; i < n; ++i) {
+		const SeqPos p = seq_pos(time[i], count);
+		first[i] = p.i0;
+		last[i] = p.single ? p.i0 : p.i0 + 1;
+		alpha[i] = p.nalpha;
+	}
+}

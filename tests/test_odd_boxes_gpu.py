@@ -1,6 +1,7 @@
 """Bounding boxes that the traversal's plain node test does not cover:
 inverted ones (a radius below zero).  The reference takes the near plane of an
-axis by the ray's sign (basics/bbox.hpp:566-595), so no ray hits them."""
+axis by the ray's sign (basics/bbox.hpp:566-595), so no ray hits them.  Times
+outside the samples, which can invert a box too."""
 import numpy as np
 import pytest
 
@@ -69,3 +70,15 @@ def test_boxes_extrapolated_before_the_first_sample(ctx, time, hits):
         sc.root.add_object("grow%d" % k, SphereLight([rng.uniform((-5, -5, 0), (5, 5, 2))], [0.5, 1.5], [[1.0] * 3]))
         sc.root.add_instance("grow%d" % k)
     assert bool(trace(ctx, sc, rays, False)["hit"].any()) == hits
+
+
+@pytest.mark.parametrize("scene", ["motion", "instanced"])
+def test_times_far_outside_the_samples(ctx, scene):
+    """Nothing outside the samples is read: the call ends without an error and
+    hits nothing that is not there at any time."""
+    sc = scenes.motion_patch_scene(2) if scene == "motion" else scenes.many_light_scene(4, n_patches=60, n_groups=30, n_lights=50)
+    rays = parity.random_rays(20000, (-4, -4, 0.01), (4, 4, 3), seed=6, occl_frac=0.3)
+    rays["time"][:] = np.random.default_rng(1).choice(np.array([-1.0, -1.5, -3.0, 1.0, 2.5, 7.0], np.float32), 20000)
+    got = trace(ctx, sc, rays, False)
+    assert 1000 < int(got["hit"].sum()) < 20000
+    assert np.all(got["t"][(got["hit"] == 1) & (rays["type"] != 32)] > 0.0)

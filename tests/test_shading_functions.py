@@ -66,3 +66,17 @@ def test_sphere_lambert(lib, near):
     # the same
     assert np.all(same | ((got == 0.0) & (want == 0.0)))
     assert (cut < 0).sum() > n // 20 and (cut >= 0).sum() > n // 20
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 4, 5, 9, 17])
+def test_a_time_s_place_lies_within_the_samples(lib, count):
+    rng = np.random.default_rng(count)
+    t = rng.integers(0, 1 << 32, 200000, dtype=np.uint64).astype(np.uint32).view(F)
+    t = np.concatenate([t, rng.uniform(-3.0, 2.0, 200000).astype(F), np.array([0.0, -0.0, 1.0, np.nextafter(F(1), F(0)),
+                                                                               np.inf, -np.inf, np.nan], F)])
+    first, last, alpha = np.empty(t.size, np.int32), np.empty(t.size, np.int32), np.empty(t.size, F)
+    lib.positions(t.size, p(t), count, p(first), p(last), p(alpha))
+    assert first.min() == 0 and last.max() == count - 1 and np.all(first <= last)
+    inside = (t >= 0) & (t < 1)
+    at = t[inside] * F(count - 1)
+    assert np.array_equal(first[inside], at.astype(np.int32)) and np.array_equal(alpha[inside], at - at.astype(np.int32))
