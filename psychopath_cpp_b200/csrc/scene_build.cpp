@@ -1044,10 +1044,29 @@ static int merge_frames(const std::vector<M44>& a, const float* b, int nb, std::
 	return n;
 }
 
+// The assembly instances of every assembly (their indices in it), assembly
+// after assembly.
+struct SubInstances {
+	std::vector<int> index;
+	std::vector<size_t> first;  // per assembly, and the end
+};
+
+// Entries that assembly `a` unrolls to, at most `limit` + 1.  `known` holds
+// the assemblies done.
+static int unrolled(const BuiltScene& b, const SubInstances& subs, int a, int limit, std::vector<int>* known) {
+	if ((*known)[a]) return (*known)[a];
+	int64_t n = 1;
+	for (size_t s = subs.first[a]; s < subs.first[a + 1] && n <= limit; ++s)
+		n += unrolled(b, subs, b.instances[b.assemblies[a].inst_base + subs.index[s]].data, limit, known);
+	return (*known)[a] = (int)std::min<int64_t>(n, (int64_t)limit + 1);
+}
+
 void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
 	out->leaves.resize(b.instances.size());
-	std::vector<int> rank(b.instances.size(), 0);
+	SubInstances subs;
+	std::vector<int> patch_odd(b.objects.size(), -1);  // per object, when it is first met
 	for (const DevAssembly& as : b.assemblies) {
+		subs.first.push_back(subs.index.size());
 		int r = 0;
 		for (int i = 0; i < as.inst_count; ++i) {
 			const int gi = as.inst_base + i;
@@ -1058,8 +1077,9 @@ void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
 			int cls = LEAF_SIMPLE, pm = 0;
 			if (inst.kind == INST_ASSEMBLY) {
 				cls = LEAF_ENTER;
-				lf.data = rank[gi] = r++;
+				lf.data = r++;
 				lf.asmb = inst.data;
+				subs.index.push_back(i);
 			} else {
 				const DevObject& ob = b.objects[inst.data];
 				const float* p = b.fpool.data() + ob.data;
@@ -1067,9 +1087,14 @@ void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
 					cls = LEAF_PATCH;
 					lf.data = ob.data;
 					pm = (ob.kind == OBJ_BILINEAR ? 1 : 3) + (ob.n0 != 1 ? 1 : 0);
-					const int n = ob.n0 * (ob.kind == OBJ_BILINEAR ? 12 : 48);
-					for (int k = 0; k < n; ++k)
-						if (!(std::fabs(p[k]) < 1e37f)) pm |= LEAF_PATCH_ODD;
+					int& odd = patch_odd[inst.data];
+					if (odd < 0) {
+						const int n = ob.n0 * (ob.kind == OBJ_BILINEAR ? 12 : 48);
+						odd = 0;
+						for (int k = 0; k < n; ++k)
+							if (!(std::fabs(p[k]) < 1e37f)) odd = LEAF_PATCH_ODD;
+					}
+					pm |= odd;
 				} else if (inst.xform_count == 0 && ((ob.kind == OBJ_SPHERE && ob.n0 == 1) ||
 				                                     (ob.kind == OBJ_SPHERE_LIGHT && ob.n0 == 1 && ob.n1 == 1))) {
 					cls = LEAF_SPHERE;
@@ -1079,9 +1104,14 @@ void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
 			lf.kind = pm | (cls << 4);
 		}
 	}
+	subs.first.push_back(subs.index.size());
+	std::vector<int> known(b.assemblies.size(), 0);
+	const int entries = unrolled(b, subs, 0, limit, &known);
+	if (entries > limit) return;
 	// breadth first: an entry's children follow one another
 	std::vector<DevPlace>& pl = out->places;
 	std::vector<float>& fr = out->frames;
+	pl.reserve(entries);
 	const DevAssembly& root = b.assemblies[0];
 	pl.push_back(DevPlace{REF_EMPTY, 0, 0, 0, -1, root.inst_base, -1, root.id_bits, 0, 0, 0});
 	for (size_t k = 0; k < pl.size(); ++k) {
@@ -1090,14 +1120,9 @@ void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
 		const DevAssembly& as = b.assemblies[at.asmb];
 		std::vector<M44> parent(at.frame_count > 0 ? at.frame_count : 0);
 		for (size_t m = 0; m < parent.size(); ++m) std::memcpy(&parent[m], fr.data() + (size_t)(at.frame + m) * 16, sizeof(M44));
-		for (int i = 0; i < as.inst_count; ++i) {
+		for (size_t s = subs.first[at.asmb]; s < subs.first[at.asmb + 1]; ++s) {
+			const int i = subs.index[s];
 			const DevInstance& inst = b.instances[as.inst_base + i];
-			if (inst.kind != INST_ASSEMBLY) continue;
-			if ((int)pl.size() >= limit) {
-				pl.clear();
-				fr.clear();
-				return;
-			}
 			const DevAssembly& sub = b.assemblies[inst.data];
 			DevPlace q = at;
 			q.parent = (int)k;
