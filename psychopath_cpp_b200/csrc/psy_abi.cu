@@ -2,6 +2,7 @@
  * C ABI implementation (include/psy_b200.h): contexts, scene upload, ray
  * tracing entry points, status reporting.
  */
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -158,54 +159,58 @@ struct WaveSet {
 	WaveQueues wq;
 };
 
-static int wave_set(psy_ctx* ctx, const char* prefix, uint64_t P, uint32_t path_length, bool paths_in_hits, WaveSet* ws,
-                    bool adjoint = false) {
-	// one device buffer for all of them (allocating them one by one was most
-	// of a new context's first render)
+// What a wave's buffers depend on.
+struct WaveShape {
+	uint64_t paths;
+	uint32_t path_length;
+	bool paths_in_hits, adjoint;
+};
+
+// Places a wave's buffers from `base` on; returns the bytes they take.
+static size_t wave_layout(char* base, const WaveShape& sh, WaveSet* ws) {
+	const uint64_t P = sh.paths;
 	PathSoA& ps = ws->ps;
 	WaveQueues& wq = ws->wq;
 	WaveBufs& wb = ws->wb;
-	std::memset(ws, 0, sizeof(*ws));
 	wb.cap = (int)P;
-	char* base = nullptr;
 	size_t at = 0;
 	auto place = [&](auto** p, size_t bytes) {
 		*p = base ? reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(base + at) : nullptr;
 		at += (bytes + 255) / 256 * 256;
 	};
-	auto layout = [&]() {
-		at = 0;
-		place(&ps.head, P * 16);
-		place(&ps.col, P * 16);
-		place(&ps.fcol, P * 16);
-		place(&ps.lcol, P * 16);
-		place(&ps.sample, P * 12);
-		if (adjoint) {
-			place(&ps.adj, P * 16);
-			place(&ps.valb, P * 16 * PSY_ADJ_MAX_VERTS);
-			place(&ps.vpid, P * 4 * PSY_ADJ_MAX_VERTS);
-			place(&ps.nee_param, P * 4);
-			place(&ps.vdsc, P * 16 * PSY_ADJ_MAX_VERTS);
-			place(&ps.fexcl, P * 16);
-			place(&ps.nee_base, P * 16);
-		}
-		place(&wq.q0, P * 4);
-		place(&wq.q1, P * 4);
-		place(&wq.counters, sizeof(int) * render_counter_count(path_length));
-		for (float4*& r : wb.ray) place(&r, P * 80);
-		place(&wb.hit_f, P * 16);
-		place(&wb.hit_i, P * (paths_in_hits ? 48 : 16));
-		place(&wb.occl, P);
-	};
-	layout();
+	place(&ps.head, P * 16);
+	place(&ps.col, P * 16);
+	place(&ps.fcol, P * 16);
+	place(&ps.lcol, P * 16);
+	place(&ps.sample, P * 12);
+	if (sh.adjoint) {
+		place(&ps.adj, P * 16);
+		place(&ps.valb, P * 16 * PSY_ADJ_MAX_VERTS);
+		place(&ps.vpid, P * 4 * PSY_ADJ_MAX_VERTS);
+		place(&ps.nee_param, P * 4);
+		place(&ps.vdsc, P * 16 * PSY_ADJ_MAX_VERTS);
+		place(&ps.fexcl, P * 16);
+		place(&ps.nee_base, P * 16);
+	}
+	place(&wq.q0, P * 4);
+	place(&wq.q1, P * 4);
+	place(&wq.counters, sizeof(int) * render_counter_count(sh.path_length));
+	for (float4*& r : wb.ray) place(&r, P * 80);
+	place(&wb.hit_f, P * 16);
+	place(&wb.hit_i, P * (sh.paths_in_hits ? 48 : 16));
+	place(&wb.occl, P);
+	return at;
+}
+
+// A wave's buffers, in one device buffer (allocating them one by one was most
+// of a new context's first render).
+static int wave_set(psy_ctx* ctx, const char* name, const WaveShape& sh, WaveSet* ws) {
+	std::memset(ws, 0, sizeof(*ws));
 	int rc = PSY_OK;
-	base = static_cast<char*>(ctx->scratch_buffer((std::string(prefix) + "wave").c_str(), at, &rc));
+	char* base = static_cast<char*>(ctx->scratch_buffer(name, wave_layout(nullptr, sh, ws), &rc));
 	if (!base) return rc ? rc : PSY_ERR_OOM;
-	layout();
-	// the counters outlive the wave's buffers (psy_profile_counters)
-	wq.rays = static_cast<unsigned long long*>(
-	    ctx->scratch_buffer((std::string(prefix) + "rays").c_str(), 2 * TC_COUNT * sizeof(unsigned long long), &rc));
-	return wq.rays ? PSY_OK : (rc ? rc : PSY_ERR_OOM);
+	wave_layout(base, sh, ws);
+	return PSY_OK;
 }
 
 // Profiling: makes room for `pairs` more traversal-launch timings.  The
@@ -235,10 +240,78 @@ static int timer_reserve(psy_ctx* ctx, int pairs) {
 // Waves in flight.  A wave's launches each end with the longest of its rays
 // or paths, on an ever emptier chip; two waves on two streams fill each
 // other's ends (512x384x16 frame with 50,000 primitives 12.3 -> 11.3 ms,
-// 320x240x16 1.95 -> 1.86, differentiable step 7.4 -> 7.1).  Below PAIR_MIN paths a wave is all latency and two
-// halves of it gain nothing.
+// 320x240x16 1.95 -> 1.86, differentiable step 7.4 -> 7.1).  Below PAIR_MIN
+// paths a wave is all latency and two halves of it gain nothing.
 static constexpr uint64_t AUTO_PATHS = 1ull << 22;  // paths in flight unless the caller says
 static constexpr uint64_t PAIR_MIN = 1ull << 17;
+
+// The waves of `total` paths with `want` of them in flight.
+struct WavePlan {
+	uint64_t paths;  // per wave
+	bool pair;       // two waves in flight, not one after another
+};
+static WavePlan wave_plan(uint64_t total, uint64_t want, bool pair) {
+	want = std::min(std::min<uint64_t>(want, 1ull << 26), total);
+	pair = pair && want >= PAIR_MIN;
+	return {pair ? (want + 1) / 2 : want, pair};
+}
+
+// The context's second stream and its events, made on first use.
+static bool side_stream(psy_ctx* ctx) {
+	if (ctx->side_stream) return true;
+	cudaStream_t s = nullptr;
+	cudaEvent_t a = nullptr, b = nullptr;
+	if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess &&
+	    cudaEventCreateWithFlags(&a, cudaEventDisableTiming) == cudaSuccess &&
+	    cudaEventCreateWithFlags(&b, cudaEventDisableTiming) == cudaSuccess) {
+		ctx->side_stream = s;
+		ctx->fork_event = a;
+		ctx->join_event = b;
+		return true;
+	}
+	cudaGetLastError();
+	if (a) cudaEventDestroy(a);
+	if (s) cudaStreamDestroy(s);
+	return false;
+}
+
+// Whether a pair of waves can run without a new allocation where none may be
+// made: while `st` is captured.
+static bool pair_allowed(psy_ctx* ctx, const char* const name[2], const WaveShape& sh, cudaStream_t st) {
+	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cudaGetLastError();
+	else if (cs != cudaStreamCaptureStatusNone) {
+		WaveSet ws;
+		const size_t bytes = wave_layout(nullptr, sh, &ws);
+		return ctx->side_stream && ctx->scratch[name[0]].bytes >= bytes && ctx->scratch[name[1]].bytes >= bytes;
+	}
+	return side_stream(ctx);
+}
+
+// The buffers of one wave or of a pair.  Without memory for the second one
+// the waves run one after another (*pair is cleared).
+static int wave_sets(psy_ctx* ctx, const char* const name[2], const WaveShape& sh, WaveSet sets[2], bool* pair) {
+	int rc = wave_set(ctx, name[0], sh, &sets[0]);
+	if (rc) return rc;
+	std::memset(&sets[1], 0, sizeof(sets[1]));
+	if (*pair && wave_set(ctx, name[1], sh, &sets[1])) {
+		cudaGetLastError();
+		std::memset(&sets[1], 0, sizeof(sets[1]));
+		*pair = false;
+	}
+	return PSY_OK;
+}
+
+// The traversal counters of a call's waves, which outlive their buffers
+// (psy_profile_counters).
+static int wave_counters(psy_ctx* ctx, const char* name, WaveSet sets[2], cudaStream_t st) {
+	int rc = PSY_OK;
+	const size_t bytes = 2 * TC_COUNT * sizeof(unsigned long long);
+	auto* c = static_cast<unsigned long long*>(ctx->scratch_buffer(name, bytes, &rc));
+	if (!c) return rc ? rc : PSY_ERR_OOM;
+	sets[0].wq.rays = sets[1].wq.rays = c;
+	return ctx_cuda(ctx, cudaMemsetAsync(c, 0, bytes, st), "memset");
+}
 
 struct WavePair {
 	psy_ctx* ctx;
@@ -248,11 +321,6 @@ struct WavePair {
 	int fork(bool pair) {
 		if (!pair) return PSY_OK;
 		int rc;
-		if (!ctx->side_stream &&
-		    ((rc = ctx_cuda(ctx, cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking), "side stream")) ||
-		     (rc = ctx_cuda(ctx, cudaEventCreateWithFlags(&ctx->fork_event, cudaEventDisableTiming), "side stream")) ||
-		     (rc = ctx_cuda(ctx, cudaEventCreateWithFlags(&ctx->join_event, cudaEventDisableTiming), "side stream"))))
-			return rc;
 		if ((rc = ctx_cuda(ctx, cudaEventRecord(ctx->fork_event, st), "side stream")) ||
 		    (rc = ctx_cuda(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->fork_event, 0), "side stream")))
 			return rc;
@@ -276,21 +344,23 @@ static int render_single(psy_ctx* ctx, const psy_render_desc* desc, const Render
 	cudaSetDevice(ctx->device);
 	int rc;
 	const uint64_t total = (uint64_t)desc->width * desc->height * desc->spp;
-	uint64_t want = desc->stream_paths ? desc->stream_paths : AUTO_PATHS;
-	if (want > (1ull << 26)) want = 1ull << 26;
-	if (want > total) want = total;
+	const uint64_t want = desc->stream_paths ? desc->stream_paths : AUTO_PATHS;
+	// whole pixels a wave
+	auto shape = [&](const WavePlan& p) {
+		uint64_t P = (p.paths + (p.pair ? desc->spp - 1 : 0)) / desc->spp * desc->spp;
+		P = std::min(std::max<uint64_t>(P, desc->spp), total);
+		return WaveShape{P, rp.path_length, ctx->dev.places == nullptr, adjoint};
+	};
+	static const char* const name[2] = {"r_wave", "r2_wave"};
 	// (the launches of a profiled render are timed one by one)
-	const bool pair = !desc->stream_paths && want >= PAIR_MIN && !ctx->profiling;
-	uint64_t P = ((pair ? (want + 1) / 2 : want) + (pair ? desc->spp - 1 : 0)) / desc->spp * desc->spp;
-	if (P < desc->spp) P = desc->spp;
-	if (P > total) P = total;
+	WavePlan plan = wave_plan(total, want, !desc->stream_paths && !ctx->profiling);
+	if (plan.pair && !pair_allowed(ctx, name, shape(plan), st)) plan = wave_plan(total, AUTO_PATHS / 2, false);
+	const WaveShape sh = shape(plan);
+	const uint64_t P = sh.paths;
+	bool pair = plan.pair;
 	WaveSet sets[2];
-	for (int k = 0; k < (pair ? 2 : 1); ++k)
-		if ((rc = wave_set(ctx, k ? "r2_" : "r_", P, rp.path_length, ctx->dev.places == nullptr, &sets[k], adjoint))) return rc;
-	sets[1].wq.rays = sets[0].wq.rays;
+	if ((rc = wave_sets(ctx, name, sh, sets, &pair)) || (rc = wave_counters(ctx, "r_rays", sets, st))) return rc;
 	const WaveSet& ws = sets[0];
-	if ((rc = ctx_cuda(ctx, cudaMemsetAsync(ws.wq.rays, 0, 2 * TC_COUNT * sizeof(unsigned long long), st), "memset")))
-		return rc;
 	ctx->last_counts = ws.wq.rays;
 	uint32_t launches = 0, waves = 0;
 	WavePair two{ctx, st};
@@ -413,18 +483,21 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 		features |= sc->dev.features;
 		if (!sc->dev.places) paths_in_hits = true;
 	}
-	uint64_t P = b->stream_paths ? b->stream_paths : (ctx->tuned_stream_paths ? ctx->tuned_stream_paths : AUTO_PATHS);
-	if (P > (1ull << 26)) P = 1ull << 26;
-	if (P > total) P = total;
-	const bool pair = !b->stream_paths && P >= PAIR_MIN;
-	if (pair) P = (P + 1) / 2 + max_spp;
-	if (P < max_spp) P = max_spp;
-	if (P > total) P = total;
+	const uint64_t want = b->stream_paths ? b->stream_paths : (ctx->tuned_stream_paths ? ctx->tuned_stream_paths : AUTO_PATHS);
+	// (waves end on pixel boundaries: two of them hold `want` paths at least)
+	auto shape = [&](const WavePlan& p) {
+		const uint64_t P = std::min(std::max<uint64_t>(p.paths + (p.pair ? max_spp : 0), max_spp), total);
+		return WaveShape{P, max_len, paths_in_hits, false};
+	};
+	static const char* const name[2] = {"b_wave", "b2_wave"};
+	WavePlan plan = wave_plan(total, want, !b->stream_paths);
+	if (plan.pair && !pair_allowed(ctx, name, shape(plan), st)) plan = wave_plan(total, std::min(want, AUTO_PATHS / 2), false);
+	const WaveShape sh = shape(plan);
+	const uint64_t P = sh.paths;
+	bool pair = plan.pair;
 	const int block = (int)(b->block_size ? b->block_size : (ctx->tuned_block ? ctx->tuned_block : 128));
-	WaveSet sets[2] = {};
-	for (int k = 0; k < (pair ? 2 : 1); ++k)
-		if ((rc = wave_set(ctx, k ? "b2_" : "b_", P, max_len, paths_in_hits, &sets[k]))) return rc;
-	sets[1].wq.rays = sets[0].wq.rays;
+	WaveSet sets[2];
+	if ((rc = wave_sets(ctx, name, sh, sets, &pair)) || (rc = wave_counters(ctx, "b_rays", sets, st))) return rc;
 	const WaveSet& ws = sets[0];
 	DevScene* d_scs = static_cast<DevScene*>(ctx->scratch_buffer("b_scenes", sizeof(DevScene) * b->count, &rc));
 	if (!d_scs) return rc;
@@ -436,8 +509,6 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 	if ((rc = ctx_cuda(ctx, cudaMemcpyAsync(d_rps, rps.data(), sizeof(RenderParams) * b->count, cudaMemcpyHostToDevice,
 	                                        st),
 	                   "psy_render_batch: render table")))
-		return rc;
-	if ((rc = ctx_cuda(ctx, cudaMemsetAsync(ws.wq.rays, 0, 2 * TC_COUNT * sizeof(unsigned long long), st), "memset")))
 		return rc;
 	// waves on pixel boundaries
 	std::vector<WaveRange> waves;
