@@ -349,7 +349,8 @@ typedef struct psy_render_desc {
 	uint32_t seed;            /* sampler seed (RenderSettings Seed) */
 	uint32_t path_length;     /* max path segments (PathTraceIntegrator::path_length, default 4) */
 	uint32_t stream_paths;    /* paths per wave, one wave after another; 0 = automatic (up to 2^22 in flight, in two waves) */
-	uint32_t block_size;      /* threads per block for the wavefront kernels, 0 = automatic */
+	uint32_t block_size;      /* 64, 128 or 256 threads per block of the camera kernel and of the traversal of flat
+	                             scenes (the other kernels choose their own); 0 = automatic */
 } psy_render_desc;
 
 typedef struct psy_render_stats {
@@ -499,7 +500,8 @@ typedef struct psy_batch_desc {
 	uint32_t* const* counts;          /* per render: device sample counts, or NULL; the array may be NULL */
 	uint32_t stream_paths;            /* paths per wave, one wave after another; 0 = the context's tuned value, else
 	                                     2^22, in flight in two waves */
-	uint32_t block_size;              /* 64, 128 or 256 threads per block; 0 = tuned value, else 128 */
+	uint32_t block_size;              /* 64, 128 or 256 threads per block of the camera kernel and of the traversal of
+	                                     flat scenes (the other kernels choose their own); 0 = tuned value, else 128 */
 	uint32_t use_graph;               /* 1: launch through a CUDA graph captured once and reused while
 	                                     the batch's launch parameters stay the same */
 } psy_batch_desc;
@@ -512,7 +514,7 @@ typedef struct psy_batch_desc {
 int psy_render_batch(psy_ctx* ctx, const psy_batch_desc* batch, psy_render_stats* stats, void* stream);
 
 typedef struct psy_batch_tuning {
-	uint32_t stream_paths;            /* chosen paths per wave */
+	uint32_t stream_paths;            /* chosen paths in flight */
 	uint32_t block_size;              /* chosen threads per block */
 	float ms;                         /* time of the chosen configuration on the tuning batch */
 	uint32_t trials;                  /* configurations timed */
@@ -520,8 +522,8 @@ typedef struct psy_batch_tuning {
 
 /* Autotuner: times the batch with every sample count divided by
  * spp_divisor (at least 1; scratch films, the batch's films are not
- * touched) for waves of 2^14..2^22 paths and blocks of 64, 128 and 256
- * threads, keeps the fastest in ctx for psy_render_batch calls whose
+ * touched) with 2^14..2^22 paths in flight, as a call with stream_paths 0
+ * runs them, and blocks of 64, 128 and 256 threads, keeps the fastest in ctx for psy_render_batch calls whose
  * configuration fields are 0, and returns it.  Synchronous. */
 int psy_batch_autotune(psy_ctx* ctx, const psy_batch_desc* batch, uint32_t spp_divisor, psy_batch_tuning* out);
 

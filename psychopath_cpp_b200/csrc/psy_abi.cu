@@ -17,6 +17,7 @@
 #include "psy_ctx.h"
 #include "sampler_tables.h"
 #include "scene_build.h"
+#include "wave_plan.h"
 
 using namespace psy;
 
@@ -237,25 +238,6 @@ static int timer_reserve(psy_ctx* ctx, int pairs) {
 	return PSY_OK;
 }
 
-// Waves in flight.  A wave's launches each end with the longest of its rays
-// or paths, on an ever emptier chip; two waves on two streams fill each
-// other's ends (512x384x16 frame with 50,000 primitives 12.3 -> 11.3 ms,
-// 320x240x16 1.95 -> 1.86, differentiable step 7.4 -> 7.1).  Below PAIR_MIN
-// paths a wave is all latency and two halves of it gain nothing.
-static constexpr uint64_t AUTO_PATHS = 1ull << 22;  // paths in flight unless the caller says
-static constexpr uint64_t PAIR_MIN = 1ull << 17;
-
-// The waves of `total` paths with `want` of them in flight.
-struct WavePlan {
-	uint64_t paths;  // per wave
-	bool pair;       // two waves in flight, not one after another
-};
-static WavePlan wave_plan(uint64_t total, uint64_t want, bool pair) {
-	want = std::min(std::min<uint64_t>(want, 1ull << 26), total);
-	pair = pair && want >= PAIR_MIN;
-	return {pair ? (want + 1) / 2 : want, pair};
-}
-
 // The context's second stream and its events, made on first use.
 static bool side_stream(psy_ctx* ctx) {
 	if (ctx->side_stream) return true;
@@ -448,9 +430,18 @@ static int diff_params(psy_ctx* ctx, const psy_diff_desc* d, const char* who, Re
 	return PSY_OK;
 }
 
+// A timed run of the autotuner: the waves of a call without stream_paths on a
+// context tuned to `paths`.  `start` is recorded before the first launch, after
+// what such a call does once (buffers, graph).
+struct BatchTrial {
+	uint32_t paths;
+	cudaEvent_t start;
+};
+
 // The batch: renders laid end to end in one global path space, rendered in
 // waves of at most P paths that end on pixel boundaries.
-static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats* stats, cudaStream_t st) {
+static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats* stats, cudaStream_t st,
+                        const BatchTrial* trial = nullptr) {
 	if (b->count == 0) return PSY_OK;
 	if (!b->scenes || !b->renders || !b->xyz)
 		return ctx_fail(ctx, PSY_ERR_ARG, "psy_render_batch: scenes, renders and xyz are required");
@@ -483,15 +474,12 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 		features |= sc->dev.features;
 		if (!sc->dev.places) paths_in_hits = true;
 	}
-	const uint64_t want = b->stream_paths ? b->stream_paths : (ctx->tuned_stream_paths ? ctx->tuned_stream_paths : AUTO_PATHS);
-	// (waves end on pixel boundaries: two of them hold `want` paths at least)
-	auto shape = [&](const WavePlan& p) {
-		const uint64_t P = std::min(std::max<uint64_t>(p.paths + (p.pair ? max_spp : 0), max_spp), total);
-		return WaveShape{P, max_len, paths_in_hits, false};
-	};
+	auto shape = [&](const WavePlan& p) { return WaveShape{p.paths, max_len, paths_in_hits, false}; };
 	static const char* const name[2] = {"b_wave", "b2_wave"};
-	WavePlan plan = wave_plan(total, want, !b->stream_paths);
-	if (plan.pair && !pair_allowed(ctx, name, shape(plan), st)) plan = wave_plan(total, std::min(want, AUTO_PATHS / 2), false);
+	WavePlan plan = trial ? batch_plan(total, max_spp, 0, trial->paths)
+	                      : batch_plan(total, max_spp, b->stream_paths, ctx->tuned_stream_paths);
+	if (plan.pair && !pair_allowed(ctx, name, shape(plan), st))
+		plan = batch_plan(total, max_spp, (uint32_t)std::min(plan.paths, AUTO_PATHS / 2), 0);
 	const WaveShape sh = shape(plan);
 	const uint64_t P = sh.paths;
 	bool pair = plan.pair;
@@ -604,8 +592,10 @@ static int render_batch(psy_ctx* ctx, const psy_batch_desc* b, psy_render_stats*
 			// the launch count of the captured sequence
 			for (size_t i = 0; i < waves.size(); ++i) launches += 5 + 2 * max_len;
 		}
+		if (trial) cudaEventRecord(trial->start, st);
 		if ((rc = ctx_cuda(ctx, cudaGraphLaunch(ctx->batch_graph, st), "psy_render_batch: graph launch"))) return rc;
 	} else {
+		if (trial) cudaEventRecord(trial->start, st);
 		if ((rc = launch_all(st))) return rc;
 	}
 	if (stats) {
@@ -1194,13 +1184,13 @@ int psy_batch_autotune(psy_ctx* ctx, const psy_batch_desc* b, uint32_t spp_divis
 	psy_batch_tuning best{};
 	best.ms = -1.0f;
 	uint32_t trials = 0;
+	t.stream_paths = 0;
 	for (uint32_t lg = 14; lg <= 22 && rc == PSY_OK; ++lg) {
 		for (uint32_t bi = 0; bi < 3; ++bi) {
-			t.stream_paths = 1u << lg;
+			const BatchTrial timed{1u << lg, e0};
 			t.block_size = blocks[bi];
-			if (trials == 0 && (rc = render_batch(ctx, &t, nullptr, st))) break;  // warm-up
-			cudaEventRecord(e0, st);
-			if ((rc = render_batch(ctx, &t, nullptr, st))) break;
+			if (trials == 0 && (rc = render_batch(ctx, &t, nullptr, st, &timed))) break;  // warm-up
+			if ((rc = render_batch(ctx, &t, nullptr, st, &timed))) break;
 			cudaEventRecord(e1, st);
 			if ((rc = ctx_cuda(ctx, cudaEventSynchronize(e1), "psy_batch_autotune: synchronize"))) break;
 			float ms = 0.0f;
@@ -1208,7 +1198,7 @@ int psy_batch_autotune(psy_ctx* ctx, const psy_batch_desc* b, uint32_t spp_divis
 			++trials;
 			if (best.ms < 0.0f || ms < best.ms) {
 				best.ms = ms;
-				best.stream_paths = t.stream_paths;
+				best.stream_paths = timed.paths;
 				best.block_size = t.block_size;
 			}
 		}
