@@ -100,8 +100,6 @@ int psy_ctx::check_status(cudaStream_t stream) {
 		cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream);
 		cudaStreamSynchronize(stream);
 		if (st & ERRF_STACK) return ctx_fail(this, PSY_ERR_STACK_OVERFLOW, "a traversal stack overflowed (flags %#x)", st);
-		if (st & ERRF_LEVELS)
-			return ctx_fail(this, PSY_ERR_STACK_OVERFLOW, "assembly nesting deeper than supported (flags %#x)", st);
 		if (st & ERRF_MOTION)
 			return ctx_fail(this, PSY_ERR_ARG, "more motion samples than supported (flags %#x)", st);
 		if (st & ERRF_BISECT)

@@ -177,7 +177,7 @@ extern "C" int psy_trace_host_noalloc(psy_ctx* ctx, const psy_ray_soa* rays, uin
 	                   "status read")))
 		return rc;
 	if ((rc = ctx_cuda(ctx, cudaStreamSynchronize(st), "stream synchronize"))) return rc;
-	if (flags & (psy::ERRF_STACK | psy::ERRF_LEVELS))
+	if (flags & psy::ERRF_STACK)
 		return ctx_fail(ctx, PSY_ERR_STACK_OVERFLOW, "psy_trace_host_noalloc: traversal limits exceeded (flags %#x)",
 		                flags);
 	if (flags & psy::ERRF_MOTION)

@@ -31,7 +31,7 @@ enum : int { SHADER_LAMBERT = 0, SHADER_EMIT = 1, SHADER_GTR = 2 };
 enum : int { CLOSURE_NONE = 0, CLOSURE_LAMBERT = 1, CLOSURE_EMIT = 2, CLOSURE_GTR = 3 };
 
 // Device error flags, OR-ed into the context's status word by kernels.
-enum : unsigned { ERRF_STACK = 1u, ERRF_LEVELS = 2u, ERRF_MOTION = 4u, ERRF_TIMEOUT = 8u, ERRF_NOLIGHT = 16u,
+enum : unsigned { ERRF_STACK = 1u, ERRF_MOTION = 4u, ERRF_TIMEOUT = 8u, ERRF_NOLIGHT = 16u,
                   ERRF_BISECT = 32u /* a patch bisection exceeded its step bound */ };
 
 // Scene features that select a compiled variant of the traversal kernels.
@@ -129,12 +129,12 @@ struct alignas(16) DevPlace {
 	int child_base;   // entry of its first assembly instance
 	int frame;        // first matrix of the merged frame
 	int frame_count;  // its motion samples: 0 = no transform, -1 = more than supported
-	int parent;
+	int asmb;
 	int inst_base;    // of its assembly
 	int shader;
 	int id_bits;      // of its assembly
 	uint64_t id;
-	int asmb, pad;
+	int pad[2];
 };
 static_assert(sizeof(DevPlace) == 48, "DevPlace must be 48 bytes");
 // Scenes that unroll to more entries than this are traversed with a level

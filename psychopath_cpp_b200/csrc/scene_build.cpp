@@ -1113,7 +1113,7 @@ void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
 	std::vector<float>& fr = out->frames;
 	pl.reserve(entries);
 	const DevAssembly& root = b.assemblies[0];
-	pl.push_back(DevPlace{REF_EMPTY, 0, 0, 0, -1, root.inst_base, -1, root.id_bits, 0, 0, 0});
+	pl.push_back(DevPlace{REF_EMPTY, 0, 0, 0, 0, root.inst_base, -1, root.id_bits, 0, {0, 0}});
 	for (size_t k = 0; k < pl.size(); ++k) {
 		pl[k].child_base = (int)pl.size();
 		const DevPlace at = pl[k];
@@ -1125,7 +1125,6 @@ void build_tables(const BuiltScene& b, int limit, SceneTables* out) {
 			const DevInstance& inst = b.instances[as.inst_base + i];
 			const DevAssembly& sub = b.assemblies[inst.data];
 			DevPlace q = at;
-			q.parent = (int)k;
 			q.asmb = inst.data;
 			q.inst_base = sub.inst_base;
 			q.id_bits = sub.id_bits;
