@@ -130,8 +130,13 @@ PSY_HD SeqPos seq_pos(float alpha, int count) {
 		p.i0 = count - 1; p.single = 1; p.nalpha = 0.0f;
 	} else {
 		const float temp = alpha * (float)(count - 1);
-		// (a time far before the first sample must not index before it either)
+		// (a time far before the first sample must not index before it either;
+		// the device's conversion to unsigned ends at 0)
+#if defined(__CUDA_ARCH__)
+		const int index = (int)__float2uint_rz(temp);
+#else
 		const int index = (int)temp > 0 ? (int)temp : 0;
+#endif
 		p.i0 = index; p.single = 0; p.nalpha = temp - (float)index;
 	}
 	return p;
