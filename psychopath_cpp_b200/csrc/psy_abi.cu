@@ -778,18 +778,6 @@ int psy_scene_upload_ex(psy_ctx* ctx, const psy_scene_desc* desc, uint32_t flags
 		UP(light_nodes, b->light_nodes);
 		UP(light_extra, b->light_extra);
 	}
-	{
-		// the light tree's children side by side, as the walk reads them
-		const size_t n = b->light_nodes.size() + (ctx->gpu_light_nodes > 0 ? (size_t)ctx->gpu_light_nodes : 0);
-		void* lp = nullptr;
-		if ((rc = ctx_cuda(ctx, cudaMalloc(&lp, (n ? n : 1) * sizeof(DevLightPair)), "cudaMalloc(light_pairs)"))) return rc;
-		ctx->scene_allocs.push_back(lp);
-		ctx->device_bytes += n * sizeof(DevLightPair);
-		d.light_pairs = static_cast<const DevLightPair*>(lp);
-		if ((rc = ctx_cuda(ctx, launch_light_pairs(d.light_nodes, (int)n, static_cast<DevLightPair*>(lp), nullptr),
-		                   "light pairs")))
-			return rc;
-	}
 	UP(assemblies, b->assemblies);
 	UP(instances, b->instances);
 	UP(objects, b->objects);
@@ -805,18 +793,44 @@ int psy_scene_upload_ex(psy_ctx* ctx, const psy_scene_desc* desc, uint32_t flags
 			                REF_MAX_NODES);
 		}
 		build_tables(*b, PSY_MAX_PLACES, &tb);
-		UP(leaves, tb.leaves);
-		UP(places, tb.places);
-		UP(place_frames, tb.frames);
-		std::vector<int> work(node_count + b->assemblies.size());  // node flags, then the assemblies' roots
-		UP(asmb_root, work);
-		int* flags = const_cast<int*>(d.asmb_root);
-		d.asmb_root = flags + node_count;
+		// the tables that the last steps fill or put into form, in one buffer
+		// (a small scene's upload is mostly its allocations)
+		const size_t light_count = b->light_nodes.size() + (ctx->gpu_light_nodes > 0 ? (size_t)ctx->gpu_light_nodes : 0);
+		size_t bytes = 0;
+		auto room = [&](size_t n) {
+			const size_t at = bytes;
+			bytes += (n + 255) / 256 * 256;
+			return at;
+		};
+		const size_t leaf_bytes = tb.leaves.size() * sizeof(DevLeaf), place_bytes = tb.places.size() * sizeof(DevPlace);
+		const size_t frame_bytes = tb.frames.size() * sizeof(float);
+		const size_t leaf_at = room(leaf_bytes), place_at = room(place_bytes), frame_at = room(frame_bytes);
+		const size_t flag_at = room(node_count * sizeof(int)), root_at = room(b->assemblies.size() * sizeof(int));
+		const size_t pair_at = room(light_count * sizeof(DevLightPair));
+		if ((rc = ctx_cuda(ctx, cudaMalloc(&p, bytes), "cudaMalloc(scene tables)"))) return rc;
+		ctx->scene_allocs.push_back(p);
+		ctx->device_bytes += bytes;
+		char* base = static_cast<char*>(p);
+		auto copy = [&](size_t at, const void* from, size_t n) {
+			return n ? ctx_cuda(ctx, cudaMemcpy(base + at, from, n, cudaMemcpyHostToDevice), "cudaMemcpy(scene tables)") : PSY_OK;
+		};
+		if ((rc = copy(leaf_at, tb.leaves.data(), leaf_bytes)) || (rc = copy(place_at, tb.places.data(), place_bytes)) ||
+		    (rc = copy(frame_at, tb.frames.data(), frame_bytes)))
+			return rc;
+		DevPlace* places = tb.places.empty() ? nullptr : reinterpret_cast<DevPlace*>(base + place_at);
+		int* roots = reinterpret_cast<int*>(base + root_at);
+		DevLightPair* pairs = reinterpret_cast<DevLightPair*>(base + pair_at);
+		d.leaves = reinterpret_cast<const DevLeaf*>(base + leaf_at);
+		d.places = places;
+		d.place_frames = reinterpret_cast<const float*>(base + frame_at);
+		d.asmb_root = roots;
+		d.light_pairs = pairs;
 		if ((rc = ctx_cuda(ctx, launch_finish_nodes(const_cast<DevNode*>(d.nodes), const_cast<float*>(d.node_extra),
 		                                            (int)node_count, d.leaves, d.assemblies, (int)b->assemblies.size(),
-		                                            const_cast<DevPlace*>(d.places), (int)tb.places.size(), flags,
-		                                            flags + node_count, nullptr),
-		                   "scene tables")))
+		                                            places, (int)tb.places.size(), reinterpret_cast<int*>(base + flag_at),
+		                                            roots, nullptr),
+		                   "scene tables")) ||
+		    (rc = ctx_cuda(ctx, launch_light_pairs(d.light_nodes, (int)light_count, pairs, nullptr), "light pairs")))
 			return rc;
 	}
 	UP(cam_xforms, b->cam_xforms);
