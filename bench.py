@@ -41,7 +41,7 @@ BYTES_PER_OCCLUSION_RAY = 64
 # DRAM bytes per traced ray of the traversal kernel, from the ncu capture in
 # profiles/trace_wave_kernel_many_light_640x360x4.md (dram read + write of the
 # camera launch / its 460,800 rays)
-TRAFFIC_BYTES_PER_RAY = 1495.0
+TRAFFIC_BYTES_PER_RAY = 1465.0
 BYTES_PER_PATH_EXTRA = 20   # sampler seed 4 + pixel 4 + XYZ 12
 RENDER_RES = (1280, 720)
 RENDER_SPP = 64
@@ -356,7 +356,7 @@ def run_render_ours(args, rank, local, pg, world):
         "config": {"workload": render_workload_name(), "paths_per_step": paths, "path_length": RENDER_PATH_LENGTH,
                    "stream_paths": args.stream_paths or "auto (2^22 in flight)",
                    "parallelism": "replicas" if world > 1 else "single",
-                   "l2": "per-path state (~200 B x 2M paths in flight) larger than L2"},
+                   "l2": "per-path state (~360 B x 4M paths in flight) larger than L2"},
         "mrays_per_s": round(mrays, 2), "rays_per_path": round(rbar, 4),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": hbm, "unit": "GB/s",
                      "frac": round(achieved / hbm, 5), "traffic": round(traffic),

@@ -346,7 +346,9 @@ class Tracer:
 
     def trace(self, rays: dict, fields=("hit", "id", "t", "uv")) -> Dict[str, np.ndarray]:
         """Host-array form (psy_trace_host): returns the requested
-        Intersection fields as numpy arrays."""
+        Intersection fields as numpy arrays.  Below BLOCK_BYTES they are views
+        of one allocation: whoever keeps one field alone and wants the others'
+        memory back copies it."""
         n = len(rays["time"])
         rs, keep = _ray_soa_host(rays)
         # The fields are cut from one block: allocated one by one, arrays of

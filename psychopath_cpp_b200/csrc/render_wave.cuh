@@ -23,8 +23,8 @@
  * which is added to in the same order here), so both leave a vertex together
  * and nothing of the vertex is stored.  (As kernels of their own, hit and
  * shadow shading wrote and read 176 bytes of vertex a path and step, and a
- * small frame waited for twice as many launches: 80x60 preview 525 -> 455 us,
- * 320x240x16 render 2.55 -> 2.26 ms.)
+ * small frame waited for twice as many launches: 80x60 preview 525 -> 443 us,
+ * 320x240x16 render 2.55 -> 2.25 ms.)
  *
  * Rays and hits are stored by queue position (coalesced), path state by path
  * slot.  Finished paths leave their spectrum in the path state; a per-wave
@@ -463,13 +463,12 @@ __global__ void __launch_bounds__(256) camera_gen_kernel(W w, HaltonDev hd, Wave
 //
 // Registers: 128 a thread where a lane's step can be a bicubic split (96
 // floats live); there more warps only push one another's stacks and cursors
-// out of L1 (1280x720x4 many-light frame: 125.7 ms with 2 x 256 threads an
-// SM, 129.4 with 5 x 128, 135.9 with 3 x 192, 140.7 with 3 x 256).  80 in flat
+// out of L1 (1280x720x4 many-light frame: 114.3 ms with 2 x 256 threads an
+// SM, 121.7 with 5 x 128, 127.4 with 3 x 192, 130.6 with 3 x 256).  80 in flat
 // scenes, where more warps hide the walk's latency (512x384x16 with 50,000
-// primitives: 11.10 ms with 3 x 256, 11.15 with 4; 18.2 and 18.9 with 3 and 2
-// before shading was joined).
-// Idle lanes that trigger a refill: 2 of them 135.6 and 11.7 ms, 4 130.1 and
-// 11.5, 8 11.1, 12 10.8 (instanced, flat).
+// primitives: 10.49 ms with 3 x 256, 10.62 with 4, 10.97 with 2).
+// Idle lanes that trigger a refill: 2 of them 118.3 ms, 4 114.3, 8 109.2
+// (instanced); 4 11.04, 8 10.70, 12 10.49 (flat).
 template <unsigned F>
 struct TraceCfg {
 	static constexpr bool NESTED = (F & FEAT_NESTED) != 0;
@@ -1100,7 +1099,7 @@ void launch_wave(const W& w, int mode, uint32_t path_length, const HaltonDev& hd
 		return need < full ? need : full;
 	};
 	// shading blocks: smaller ones for waves that would leave SMs without any
-	// (80x60 preview: 443 us with 512-thread blocks on 10 SMs, 345 with 64 and
+	// (80x60 preview: 443 us with 512-thread blocks on 10 SMs, 338 with 64 and
 	// the rays spread over all warps)
 	int sb = PSY_SHADE_BLOCK;
 	while (sb > 64 && (P + sb - 1) / sb < 2 * g.sms) sb >>= 1;

@@ -50,10 +50,10 @@ struct StreamIO {
 
 // Register cap of the kernel: 64 for flat scenes (spheres, lights, bilinear
 // patches in one level), where more resident warps hide the walk's memory
-// latency (4M rays against the heightfield: 1.06 ms; 1.13 at 80 registers,
-// 1.37 at 128), 128 for the larger variants, whose bicubic bisection spills
-// below that (300,000 mixed rays against instanced patches and spheres:
-// 1.67 ms; 1.71 at 144, 1.72 at 168, 1.87 at 112, 1.94 at 96).
+// latency (4M rays against the heightfield: 0.925 ms; 0.951 at 80 registers,
+// 0.981 at 96, 1.085 at 128), 128 for the larger variants, whose bicubic
+// bisection spills below that (300,000 mixed rays against instanced patches
+// and spheres: 1.58 ms; 1.68 at 144, 1.63 at 168, 1.82 at 112, 1.85 at 96).
 template <unsigned F>
 struct TraceKernelRegs {
 	static constexpr int value = F == FEAT_FLAT ? 64 : 128;
@@ -158,7 +158,7 @@ cudaError_t launch_trace(const DevScene& sc, const RaySoA& rays, const HitSoA& h
 	// A short stream is spread over the SMs, and its warps run on fewer lanes,
 	// whose rays wait less for one another: at least 8 warps an SM as long as
 	// there are rays (1021 rays against a flat scene: 51 us in 8 blocks of 128
-	// threads, 23 so).
+	// threads, 20 so; 148 SMs).
 	const int block = 128;
 	const uint32_t warps = 8 * 148;
 	int lanes = 32;
